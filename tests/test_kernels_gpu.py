@@ -452,3 +452,44 @@ def test_errors_are_reported_not_fatal(ops):
         ops.route(ids.cuda().long(), 4)
     with pytest.raises(Lb.HexaError, match="CUDA tensors only"):
         ops.route(ids, 4)
+
+
+# Both tile sizes of the CUDA-core kernels: every output is one FMA chain in ascending k whichever tile computes it, so a
+# launch wide enough for 128-tiles must reproduce, bit for bit, what narrow launches over column slices (64-tiles) give.
+@pytest.mark.parametrize("dtype,K,N", [(torch.float32, 36, 2052), (torch.float32, 37, 2051), (torch.bfloat16, 130, 2049)])
+@pytest.mark.parametrize("nk", [True, False])
+def test_simt_tile_sizes_agree(ops, dtype, K, N, nk):
+    Lb = L()
+    T, E = 5000, 5
+    ids = make_ids(T, 1, E, 11, skew=True, empty=(2,))
+    r = ops.route(ids.cuda(), E)
+    assert (r.row_capacity // 128) * (-(-N // 128)) >= 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator().manual_seed(K)
+    x = torch.randn(T, K, generator=g).to(dtype)
+    w = torch.randn(E, N, K, generator=g).to(dtype)
+    b = torch.randn(E, N, generator=g)
+    xs = ops.gather_rows(x.cuda(), r)
+    wd = w.cuda() if nk else w.transpose(1, 2).contiguous().cuda()
+    bd = ops._f32(b.cuda())
+    y1 = ops.sorted_buffer(r.row_capacity, N, dtype, "cuda")
+    args = dict(epilogue=Lb.EPI_ACT, act=Lb.ACT_GELU, engine=Lb.ENGINE_SIMT)
+    lay = Lb.B_NK if nk else Lb.B_KN
+    wide = ops.esmm(xs, wd, lay, r, bd, aux=y1, **args)
+    n_pad = int(r.pad_offsets[-1])
+    for c0, c1 in ((0, 64), (1984, N), (N - 3, N)):
+        sl = wd[:, c0:c1] if nk else wd[:, :, c0:c1]
+        a1 = ops.sorted_buffer(r.row_capacity, c1 - c0, dtype, "cuda")
+        got = ops.esmm(xs, sl, lay, r, ops._f32(b[:, c0:c1].cuda()), aux=a1, **args)
+        assert torch.equal(got[:n_pad], wide[:n_pad, c0:c1]) and torch.equal(a1[:n_pad], y1[:n_pad, c0:c1])
+    # the weight gradient, against float64 and slice by slice
+    dw = ops.estmm(wide, xs, r, out_dtype=torch.float32, engine=Lb.ENGINE_SIMT)
+    many = ops.estmm(wide, wide[:, :1024], r, out_dtype=torch.float32, engine=Lb.ENGINE_SIMT)        # 128-tiles
+    few = ops.estmm(wide[:, :64], wide[:, :1024], r, out_dtype=torch.float32, engine=Lb.ENGINE_SIMT)   # 64-tiles
+    assert torch.equal(many[:, :64], few)
+    rows = r.row_token[:n_pad]
+    po = r.pad_offsets.tolist()
+    for e in range(E):
+        want = wide[po[e]:po[e + 1]].double().t() @ xs[po[e]:po[e + 1]].double()
+        # a chain of n fp32 FMAs is within n * 2^-24 of the sum of magnitudes; rows of an expert bound n
+        bound = wide[po[e]:po[e + 1]].double().abs().t() @ xs[po[e]:po[e + 1]].double().abs() * ((po[e + 1] - po[e]) * 2.0 ** -24)
+        assert ((dw[e].double() - want).abs() <= bound + 1e-30).all()
