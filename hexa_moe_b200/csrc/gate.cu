@@ -5,11 +5,17 @@
 // gradient of l with respect to the logits.  The [T,E] score matrix is never written: the backward kernel
 // recomputes the softmax from the logits it has to read anyway.
 //
-// One warp per token, lane l holding columns l, l+32, ...; column sums stay in registers across the tokens of a
-// warp, meet in shared memory once per block (one row per warp, added in warp order) and leave the block as one
-// partial row in the workspace; the block that finishes last adds the partial rows in block order.  Every float
-// sum therefore has a fixed order: mass and loss are bit-identical from run to run.  The only atomics are the
-// integer top-1 histogram and the completion ticket.
+// GShard kernels: a group of G lanes (8 up to 64 experts, 16 up to 128, else 32) per token, lane g holding columns
+// g, g + G, ...: a warp works on 32 / G tokens at once and a reduction over a token is log2(G) shuffles; the next token's
+// row is loaded while this one is worked on.  Sums over a token are added in the order of a 32-lane xor tree over columns
+// modulo 32 whatever G is.  Column sums stay in registers across the tokens of a group, meet in shared memory once per
+// block and leave the block as one partial row (and one row of top-1 counts) in the workspace; gate_finish_kernel adds the
+// rows in a fixed order with all its threads.  A single block finishes by itself.  Nothing has to start at zero and every
+// float sum has a fixed order: mass and loss are bit-identical from run to run.
+// Bound: latency (a token is ~30 dependent shuffles) up to some 10^4 tokens, then the reading of the logits.
+// [131072, 64] top-2: 102 us -> 26 + 10 us (the last block used to add 592 partial rows one after the other, ~50 us of
+// it, after four memsets), the gradient 23 -> 17 us.
+// Load-importance kernels: one warp per token; the block that finishes last adds the partial rows (in block order).
 // Ties: the lowest expert id wins, and the k ids of a token come out in descending score order.  The selection is
 // total: a score that is NaN ranks below every number, so a row of NaN / inf logits (an overflowed fp16 step) still
 // yields k distinct ids in [0, E) - the lowest free columns - and only the loss carries the NaN, as it does through
@@ -24,7 +30,7 @@ namespace {
 constexpr int kGateThreads = 256;
 constexpr int kGateWarps = kGateThreads / 32;
 constexpr int kGateMaxExperts = 512;
-constexpr int kGateMaxBlocks = 1024;   // partial-mass rows the workspace holds
+constexpr int kGateMaxBlocks = 1024;   // partial rows of kGateMaxExperts 32-bit words the workspace holds
 constexpr size_t kGateTicketBytes = 256;
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -60,120 +66,286 @@ __device__ __forceinline__ void warp_softmax(const float* __restrict__ row, int 
   for (int i = 0; i < VPT; ++i) s[i] = s[i] / sum;
 }
 
-template <int VPT>
+// ---- groups of G lanes per token, PER columns per lane ----------------------------------------------------------------
+// Sum over a token's columns in the order of warp_sum over lanes c mod 32 (the columns of one such lane added first).
+template <int G, int PER>
+__device__ __forceinline__ float group_sum(const float (&v)[PER]) {
+  constexpr int R = 32 / G;
+  float cls[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    cls[r] = 0.f;
+#pragma unroll
+    for (int j = r; j < PER; j += R) cls[r] += v[j];
+  }
+#pragma unroll
+  for (int o = R / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int r = 0; r < o; ++r) cls[r] += cls[r + o];
+  float x = cls[0];
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+template <int G, int PER>
+__device__ __forceinline__ void group_load(const float* __restrict__ row, int E, int g, bool valid, float (&v)[PER]) {
+#pragma unroll
+  for (int j = 0; j < PER; ++j) v[j] = (valid && g + G * j < E) ? __ldg(row + g + G * j) : -FLT_MAX;
+}
+
+// logits -> softmax in place; columns >= E come out as 0
+template <int G, int PER>
+__device__ __forceinline__ void group_softmax(int E, int g, float (&s)[PER]) {
+  float m = -FLT_MAX;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) m = fmaxf(m, s[j]);
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+  for (int j = 0; j < PER; ++j) s[j] = g + G * j < E ? expf(s[j] - m) : 0.f;
+  const float sum = group_sum<G, PER>(s);
+#pragma unroll
+  for (int j = 0; j < PER; ++j) s[j] = s[j] / sum;
+}
+
+__device__ __forceinline__ void fold_loss(float part, float* red, int64_t T, int E, float* __restrict__ loss) {
+  // fixed-order block reduction: lanes by xor tree, warps in index order
+  part = warp_sum(part);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float tot = 0.f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += red[w];
+    loss[0] = tot * ((float)E / (float)T) / (float)T;
+  }
+}
+
+// partial: per block E float column sums, then E int top-1 counts
+template <int G, int PER>
 __global__ void __launch_bounds__(kGateThreads)
 gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, int k, int32_t* __restrict__ ids,
                  float* __restrict__ mass, int32_t* __restrict__ first_count, float* __restrict__ loss,
-                 unsigned int* __restrict__ ticket, float* __restrict__ partial) {
-  __shared__ float mass_w[kGateWarps][32 * VPT];
-  __shared__ int cnt_s[32 * VPT];
+                 float* __restrict__ partial) {
+  constexpr int kGroups = 32 / G;
+  __shared__ float mass_w[kGateWarps][G * PER];
+  __shared__ int cnt_s[G * PER];
   __shared__ float red_s[kGateWarps];
-  __shared__ bool last_s;
-  for (int e = threadIdx.x; e < 32 * VPT; e += blockDim.x) cnt_s[e] = 0;
+  for (int e = threadIdx.x; e < G * PER; e += blockDim.x) cnt_s[e] = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t warp0 = (int64_t)blockIdx.x * kGateWarps + warp;
-  const int64_t nwarps = (int64_t)gridDim.x * kGateWarps;
-  float acc[VPT];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane & (G - 1);
+  const int64_t first = ((int64_t)blockIdx.x * kGateWarps + warp) * kGroups;     // this warp's first token of a sweep
+  const int64_t step = (int64_t)gridDim.x * kGateWarps * kGroups;
+  const int grp = lane / G;
+  float acc[PER], next[PER];
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) acc[i] = 0.f;
-  for (int64_t t = warp0; t < T; t += nwarps) {
-    float s[VPT];
-    warp_softmax<VPT>(logits + t * ld, E, lane, s);
+  for (int j = 0; j < PER; ++j) acc[j] = 0.f;
+  group_load<G, PER>(logits + (first + grp) * ld, E, g, first + grp < T, next);
+  for (int64_t t0 = first; t0 < T; t0 += step) {      // uniform across the warp; groups past T carry no token
+    const int64_t t = t0 + grp;
+    const bool live = t < T;
+    float s[PER];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) acc[i] += s[i];
+    for (int j = 0; j < PER; ++j) s[j] = next[j];
+    group_load<G, PER>(logits + (t + step) * ld, E, g, t + step < T, next);
+    group_softmax<G, PER>(E, g, s);
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) acc[j] += s[j];
+    }
     unsigned int taken = 0;
-    for (int j = 0; j < k; ++j) {
+    for (int i = 0; i < k; ++i) {
       // candidates: this lane's free columns; NaN counts as -inf, and the first free column is taken even at -inf,
       // so some lane always has a candidate while fewer than E columns are taken (k <= E is checked by the host)
       float best = -INFINITY;
       int bi = 0x7fffffff;
 #pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        const int c = lane + 32 * i;
-        if (c < E && !((taken >> i) & 1u)) {
-          const float v = s[i] == s[i] ? s[i] : -INFINITY;
+      for (int j = 0; j < PER; ++j) {
+        const int c = g + G * j;
+        if (c < E && !((taken >> j) & 1u)) {
+          const float v = s[j] == s[j] ? s[j] : -INFINITY;
           if (bi == 0x7fffffff || v > best) { best = v; bi = c; }   // ascending c: the first maximum stays
         }
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
+      for (int o = G / 2; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
       }
       const bool valid = (unsigned)bi < (unsigned)E;     // always true; kept so that no index derived from data is trusted
-      if (valid && (bi & 31) == lane) taken |= 1u << (bi >> 5);
-      if (lane == 0) {
-        ids[(int64_t)j * T + t] = valid ? bi : -1;         // -1 is a row the routing kernel skips
-        if (j == 0 && valid) atomicAdd(&cnt_s[bi], 1);
+      if (valid && (bi & (G - 1)) == g) taken |= 1u << (bi / G);
+      if (g == 0 && live) {
+        ids[(int64_t)i * T + t] = valid ? bi : -1;         // -1 is a row the routing kernel skips
+        if (i == 0 && valid) atomicAdd(&cnt_s[bi], 1);
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) mass_w[warp][lane + 32 * i] = acc[i];
+  for (int j = 0; j < PER; ++j) {
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+    if (grp == 0) mass_w[warp][g + G * j] = acc[j];
+  }
   __syncthreads();
+  const bool only = gridDim.x == 1;
+  int32_t* counts = reinterpret_cast<int32_t*>(partial) + (int64_t)blockIdx.x * 2 * E + E;
+  float part = 0.f;
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     float m = 0.f;
 #pragma unroll
     for (int w = 0; w < kGateWarps; ++w) m += mass_w[w][e];
-    partial[(int64_t)blockIdx.x * E + e] = m;
-    if (cnt_s[e]) atomicAdd(&first_count[e], cnt_s[e]);
+    if (only) {
+      mass[e] = m;
+      first_count[e] = cnt_s[e];
+      part += m * (float)cnt_s[e];
+    } else {
+      partial[(int64_t)blockIdx.x * 2 * E + e] = m;
+      counts[e] = cnt_s[e];
+    }
   }
-  // the block that finishes last adds the partial rows (in block order) and folds the two [E] vectors into the loss
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last_s = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last_s) return;
-  __threadfence();
-  float part = 0.f;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  if (only) fold_loss(part, red_s, T, E, loss);
+}
+
+// Adds the blocks' rows: 1024 / E threads per expert take every (1024 / E)-th block, their sums meet in index order.
+constexpr int kFinishThreads = 1024;
+__global__ void __launch_bounds__(kFinishThreads)
+gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int E, float* __restrict__ mass,
+                   int32_t* __restrict__ first_count, float* __restrict__ loss) {
+  __shared__ float m_s[kFinishThreads];
+  __shared__ int c_s[kFinishThreads];
+  __shared__ float red_s[kFinishThreads / 32];
+  const int slices = kFinishThreads / E;
+  const int e = threadIdx.x % E, slice = threadIdx.x / E;
+  if (slice < slices) {
     float m = 0.f;
-    for (unsigned b = 0; b < gridDim.x; ++b) m += __ldcg(partial + (int64_t)b * E + e);
-    mass[e] = m;
-    part += m * (float)__ldcg(first_count + e);
+    int c = 0;
+#pragma unroll 4
+    for (int b = slice; b < blocks; b += slices) {
+      const float* row = partial + (int64_t)b * 2 * E;
+      m += __ldg(row + e);
+      c += __ldg(reinterpret_cast<const int32_t*>(row) + E + e);
+    }
+    m_s[threadIdx.x] = m;
+    c_s[threadIdx.x] = c;
   }
-  // fixed-order block reduction: lanes by xor tree, warps in index order
-  part = warp_sum(part);
-  if (lane == 0) red_s[warp] = part;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float tot = 0.f;
-    for (int w = 0; w < kGateWarps; ++w) tot += red_s[w];
-    loss[0] = tot * ((float)E / (float)T) / (float)T;
+  float part = 0.f;
+  if (threadIdx.x < E) {
+    float m = 0.f;
+    int c = 0;
+    for (int i = 0; i < slices; ++i) { m += m_s[i * E + threadIdx.x]; c += c_s[i * E + threadIdx.x]; }
+    mass[threadIdx.x] = m;
+    first_count[threadIdx.x] = c;
+    part = m * (float)c;
   }
+  fold_loss(part, red_s, T, E, loss);
 }
 
 // dlogits[t,e] = s[t,e] * (g_e - sum_e' s[t,e'] g_e') with g_e = dloss * ce_e / T: the chain rule through
 // mass = column sums of the softmax (ce counts top-1 choices and carries no gradient)
-template <int VPT>
+template <int G, int PER>
 __global__ void __launch_bounds__(kGateThreads)
 gate_loss_grad_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, const int32_t* __restrict__ first_count,
                       const float* __restrict__ dloss, float* __restrict__ dlogits, int64_t ldd) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp0 = (int64_t)blockIdx.x * (kGateThreads / 32) + (threadIdx.x >> 5);
-  const int64_t nwarps = (int64_t)gridDim.x * (kGateThreads / 32);
+  constexpr int kGroups = 32 / G;
+  const int lane = threadIdx.x & 31, g = lane & (G - 1), grp = lane / G;
+  const int64_t first = ((int64_t)blockIdx.x * kGateWarps + (threadIdx.x >> 5)) * kGroups;
+  const int64_t step = (int64_t)gridDim.x * kGateWarps * kGroups;
   const float scale = __ldg(dloss) * ((float)E / (float)T) / (float)T;
-  float g[VPT];
+  float ge[PER], next[PER];
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int c = lane + 32 * i;
-    g[i] = c < E ? scale * (float)__ldg(first_count + c) : 0.f;
+  for (int j = 0; j < PER; ++j) {
+    const int c = g + G * j;
+    ge[j] = c < E ? scale * (float)__ldg(first_count + c) : 0.f;
   }
-  for (int64_t t = warp0; t < T; t += nwarps) {
-    float s[VPT];
-    warp_softmax<VPT>(logits + t * ld, E, lane, s);
-    float dot = 0.f;
+  group_load<G, PER>(logits + (first + grp) * ld, E, g, first + grp < T, next);
+  for (int64_t t0 = first; t0 < T; t0 += step) {
+    const int64_t t = t0 + grp;
+    float s[PER], sg[PER];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) dot += s[i] * g[i];
-    dot = warp_sum(dot);
+    for (int j = 0; j < PER; ++j) s[j] = next[j];
+    group_load<G, PER>(logits + (t + step) * ld, E, g, t + step < T, next);
+    group_softmax<G, PER>(E, g, s);
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int c = lane + 32 * i;
-      if (c < E) dlogits[t * ldd + c] = s[i] * (g[i] - dot);
+    for (int j = 0; j < PER; ++j) sg[j] = s[j] * ge[j];
+    const float dot = group_sum<G, PER>(sg);
+    if (t < T) {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int c = g + G * j;
+        if (c < E) dlogits[t * ldd + c] = s[j] * (ge[j] - dot);
+      }
     }
   }
+}
+
+// ---- the gate projection's operands in 16-bit terms -----------------------------------------------------------------
+// x = hi + mid + lo exactly to fp32's 24 bits, each term the bf16 rounding of what the previous ones left over.
+__device__ __forceinline__ void split_terms(float x, __nv_bfloat16 (&t)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    t[i] = __float2bfloat16_rn(x);
+    x -= __bfloat162float(t[i]);
+  }
+}
+
+template <int V> struct Vec;
+template <> struct Vec<4> { using F = float4; using H = uint2; };
+template <> struct Vec<1> { using F = float; using H = uint16_t; };
+
+// out[r, q * cols + c] = term `order[q]` of src[r, c], four blocks of columns per row: (hi, hi, mid, lo) or, with
+// by_rows, four blocks of rows (lo, mid, hi, hi): src is then one row of rows * cols elements.
+template <int V>
+__global__ void __launch_bounds__(256)
+split_terms_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, int64_t cols, int lo_first, __nv_bfloat16* __restrict__ out) {
+  const int64_t per_row = cols / V;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / per_row, c = (i - r * per_row) * V;
+    const typename Vec<V>::F x = __ldg(reinterpret_cast<const typename Vec<V>::F*>(src + r * ld + c));
+    __align__(8) __nv_bfloat16 t[3][V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      __nv_bfloat16 one[3];
+      split_terms(reinterpret_cast<const float*>(&x)[j], one);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) t[q][j] = one[q];
+    }
+    __nv_bfloat16* o = out + r * 4 * cols + c;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int fwd = q == 0 ? 0 : q - 1, rev = q == 3 ? 0 : 2 - q;      // (hi, hi, mid, lo) / (lo, mid, hi, hi)
+      const typename Vec<V>::H a = *reinterpret_cast<const typename Vec<V>::H*>(t[fwd]);
+      const typename Vec<V>::H b = *reinterpret_cast<const typename Vec<V>::H*>(t[rev]);
+      *reinterpret_cast<typename Vec<V>::H*>(o + q * cols) = lo_first ? b : a;
+    }
+  }
+}
+
+// out[r, c] = (hi + mid) + lo of a row's three blocks of columns, stored in that order or, with lo_first, reversed
+template <int V>
+__global__ void __launch_bounds__(256)
+sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int lo_first, float* __restrict__ out) {
+  using F = typename Vec<V>::F;
+  const int64_t per_row = cols / V;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = i / per_row, c = (i - r * per_row) * V;
+    const float* p = part + r * 3 * cols + c;
+    const F a = __ldg(reinterpret_cast<const F*>(p + (lo_first ? 2 * cols : 0)));
+    const F b = __ldg(reinterpret_cast<const F*>(p + cols));
+    const F d = __ldg(reinterpret_cast<const F*>(p + (lo_first ? 0 : 2 * cols)));
+    F o;
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      reinterpret_cast<float*>(&o)[j] = (reinterpret_cast<const float*>(&a)[j] + reinterpret_cast<const float*>(&b)[j]) +
+                                        reinterpret_cast<const float*>(&d)[j];
+    *reinterpret_cast<F*>(out + r * cols + c) = o;
+  }
+}
+
+unsigned elementwise_grid(int64_t items) {
+  const int64_t want = ceil_div(items, 256), cap = (int64_t)sm_count() * 8;
+  return (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
 
@@ -343,6 +515,28 @@ gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ 
   }
 }
 
+// Blocks of the group kernels: one sweep of a block covers kGateWarps * 32 / G tokens.  Up to four sweeps stay in one block,
+// which then needs no second launch (a sweep costs ~1 us, a launch ~3 us); beyond that, three blocks per SM.
+int gate_group_grid(int64_t T, int G) {
+  const int64_t sweep = kGateWarps * (32 / G);
+  if (T <= 4 * sweep) return 1;
+  int64_t cap = (int64_t)sm_count() * 3;
+  if (cap > kGateMaxBlocks / 2) cap = kGateMaxBlocks / 2;      // a block leaves two rows of words
+  const int64_t want = ceil_div(T, sweep);
+  return (int)(want < cap ? want : cap);
+}
+
+#define HEXA_GATE_DISPATCH(E, LAUNCH)  \
+  do {                                 \
+    if ((E) <= 8) { LAUNCH(8, 1); }    \
+    else if ((E) <= 16) { LAUNCH(8, 2); }  \
+    else if ((E) <= 32) { LAUNCH(8, 4); }  \
+    else if ((E) <= 64) { LAUNCH(8, 8); }  \
+    else if ((E) <= 128) { LAUNCH(16, 8); } \
+    else if ((E) <= 256) { LAUNCH(32, 8); } \
+    else { LAUNCH(32, 16); }           \
+  } while (0);
+
 int gate_grid(int64_t T) {
   const int64_t want = ceil_div(T, kGateThreads / 32);
   int64_t cap = (int64_t)sm_count() * 4;
@@ -372,24 +566,25 @@ extern "C" int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_token
                "hexa_gate_topk: null output or workspace smaller than hexa_gate_workspace_bytes()");
   HEXA_REQUIRE(num_tokens == 0 || (logits && ids && ld >= num_experts), "hexa_gate_topk: null logits/ids or ld < experts");
   HEXA_REQUIRE(aligned16(workspace), "hexa_gate_topk: workspace must be 16-byte aligned");
-  HEXA_CUDA(cudaMemsetAsync(mass, 0, sizeof(float) * num_experts, stream));
-  HEXA_CUDA(cudaMemsetAsync(first_count, 0, sizeof(int32_t) * num_experts, stream));
-  HEXA_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), stream));
-  HEXA_CUDA(cudaMemsetAsync(workspace, 0, 16, stream));
-  if (num_tokens == 0) return HEXA_OK;
-  unsigned int* ticket = static_cast<unsigned int*>(workspace);
+  if (num_tokens == 0) {
+    HEXA_CUDA(cudaMemsetAsync(mass, 0, sizeof(float) * num_experts, stream));
+    HEXA_CUDA(cudaMemsetAsync(first_count, 0, sizeof(int32_t) * num_experts, stream));
+    HEXA_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), stream));
+    return HEXA_OK;
+  }
   float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kGateTicketBytes);
-  const int grid = gate_grid(num_tokens);
-#define HEXA_GATE_FWD(V) \
-  gate_topk_kernel<V><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, top_k, ids, mass, first_count, loss, ticket, partial)
-  const int vpt = (num_experts + 31) / 32;
-  if (vpt <= 1) HEXA_GATE_FWD(1);
-  else if (vpt <= 2) HEXA_GATE_FWD(2);
-  else if (vpt <= 4) HEXA_GATE_FWD(4);
-  else if (vpt <= 8) HEXA_GATE_FWD(8);
-  else HEXA_GATE_FWD(16);
+  int grid = 1;
+#define HEXA_GATE_FWD(G, PER)                                                                                              \
+  grid = gate_group_grid(num_tokens, G);                                                                                   \
+  gate_topk_kernel<G, PER><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, top_k, ids, mass,       \
+                                                              first_count, loss, partial)
+  HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_FWD)
 #undef HEXA_GATE_FWD
   HEXA_LAUNCH_CHECK("gate_topk_kernel");
+  if (grid > 1) {
+    gate_finish_kernel<<<1, kFinishThreads, 0, stream>>>(partial, grid, num_tokens, num_experts, mass, first_count, loss);
+    HEXA_LAUNCH_CHECK("gate_finish_kernel");
+  }
   return HEXA_OK;
 }
 
@@ -401,17 +596,45 @@ extern "C" int hexa_gate_loss_grad(const float* logits, int64_t ld, int64_t num_
   if (num_tokens == 0) return HEXA_OK;
   HEXA_REQUIRE(logits && first_count && dloss && dlogits && ld >= num_experts && ldd >= num_experts,
                "hexa_gate_loss_grad: null pointer or leading dimension < experts");
-  const int grid = gate_grid(num_tokens);
-#define HEXA_GATE_BWD(V) \
-  gate_loss_grad_kernel<V><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, first_count, dloss, dlogits, ldd)
-  const int vpt = (num_experts + 31) / 32;
-  if (vpt <= 1) HEXA_GATE_BWD(1);
-  else if (vpt <= 2) HEXA_GATE_BWD(2);
-  else if (vpt <= 4) HEXA_GATE_BWD(4);
-  else if (vpt <= 8) HEXA_GATE_BWD(8);
-  else HEXA_GATE_BWD(16);
+  int grid = 1;
+#define HEXA_GATE_BWD(G, PER)                                                                                             \
+  grid = gate_group_grid(num_tokens, G);                                                                                  \
+  gate_loss_grad_kernel<G, PER><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, first_count, dloss, \
+                                                                   dlogits, ldd)
+  HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_BWD)
 #undef HEXA_GATE_BWD
   HEXA_LAUNCH_CHECK("gate_loss_grad_kernel");
+  return HEXA_OK;
+}
+
+extern "C" int hexa_gate_split_terms(const float* src, int64_t ld, int64_t rows, int64_t cols, int by_rows, void* out, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  HEXA_REQUIRE(rows >= 0 && cols >= 0 && ld >= cols, "hexa_gate_split_terms: bad sizes");
+  if (rows == 0 || cols == 0) return HEXA_OK;
+  HEXA_REQUIRE(src && out, "hexa_gate_split_terms: null pointer");
+  if (by_rows) {      // blocks of rows: the same as blocks of columns of one long row
+    HEXA_REQUIRE(ld == cols, "hexa_gate_split_terms: blocks of rows need a contiguous source");
+    cols *= rows;
+    ld = cols;
+    rows = 1;
+  }
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  const bool v4 = cols % 4 == 0 && ld % 4 == 0 && aligned16(src) && aligned16(out);
+  if (v4) split_terms_kernel<4><<<elementwise_grid(rows * cols / 4), 256, 0, stream>>>(src, ld, rows, cols, by_rows, o);
+  else split_terms_kernel<1><<<elementwise_grid(rows * cols), 256, 0, stream>>>(src, ld, rows, cols, by_rows, o);
+  HEXA_LAUNCH_CHECK("split_terms_kernel");
+  return HEXA_OK;
+}
+
+extern "C" int hexa_gate_sum_terms(const float* part, int64_t rows, int64_t cols, int lo_first, float* out, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  HEXA_REQUIRE(rows >= 0 && cols >= 0, "hexa_gate_sum_terms: bad sizes");
+  if (rows == 0 || cols == 0) return HEXA_OK;
+  HEXA_REQUIRE(part && out, "hexa_gate_sum_terms: null pointer");
+  const bool v4 = cols % 4 == 0 && aligned16(part) && aligned16(out);
+  if (v4) sum_terms_kernel<4><<<elementwise_grid(rows * cols / 4), 256, 0, stream>>>(part, rows, cols, lo_first, out);
+  else sum_terms_kernel<1><<<elementwise_grid(rows * cols), 256, 0, stream>>>(part, rows, cols, lo_first, out);
+  HEXA_LAUNCH_CHECK("sum_terms_kernel");
   return HEXA_OK;
 }
 

@@ -286,11 +286,34 @@ def gate_max_experts() -> int:
     return int(lib().hexa_gate_max_experts())
 
 
+def gate_split_terms(src: torch.Tensor, by_rows: bool) -> torch.Tensor:
+    """float32 [rows, cols] as bf16 terms hi + mid + lo: [rows, 4 cols] with column blocks (hi, hi, mid, lo) or, by_rows,
+    [4 rows, cols] with row blocks (lo, mid, hi, hi)."""
+    if src.dtype != torch.float32 or not src.is_contiguous():
+        raise L.HexaError("gate_split_terms: src must be contiguous float32")
+    rows, cols = src.shape
+    out = torch.empty((4 * rows, cols) if by_rows else (rows, 4 * cols), dtype=torch.bfloat16, device=src.device)
+    with _Timed("gate"):
+        check(lib().hexa_gate_split_terms(ptr(src), cols, rows, cols, int(by_rows), ptr(out), stream_of(src)), "hexa_gate_split_terms")
+    return out
+
+
+def gate_sum_terms(part: torch.Tensor, rows: int, cols: int, lo_first: bool) -> torch.Tensor:
+    """(hi + mid) + lo of the three column blocks of part [rows, 3 cols], stored as (hi, mid, lo) or, lo_first, reversed."""
+    if part.dtype != torch.float32 or not part.is_contiguous() or part.numel() != 3 * rows * cols:
+        raise L.HexaError("gate_sum_terms: part must be contiguous float32 of 3 * rows * cols elements")
+    out = torch.empty(rows, cols, dtype=torch.float32, device=part.device)
+    with _Timed("gate"):
+        check(lib().hexa_gate_sum_terms(ptr(part), rows, cols, int(lo_first), ptr(out), stream_of(part)), "hexa_gate_sum_terms")
+    return out
+
+
 def gate_topk(logits: torch.Tensor, top_k: int):
     """softmax + top-k + GShard loss of float32 logits [T,E] in one kernel.  Returns (ids int32 [k,T] route-major,
     loss float32 scalar tensor, first_count int32 [E], mass float32 [E])."""
     if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
         raise L.HexaError("gate_topk: logits must be float32 [T,E] with unit inner stride")
+    global LAUNCHES
     T, E = logits.shape
     dev = logits.device
     ids = torch.empty(top_k, T, dtype=torch.int32, device=dev)
@@ -301,6 +324,7 @@ def gate_topk(logits: torch.Tensor, top_k: int):
     with _Timed("gate", 2.0 * T * E * 4):
         check(lib().hexa_gate_topk(ptr(logits), _ld(logits), T, E, top_k, ptr(ids), ptr(mass), ptr(cnt), ptr(loss), ptr(ws),
                                    ws.numel(), stream_of(logits)), "hexa_gate_topk")
+    LAUNCHES += T > (128 if E <= 64 else 64 if E <= 128 else 32)      # beyond one block: a second kernel adds the blocks' rows
     return ids, loss, cnt, mass
 
 

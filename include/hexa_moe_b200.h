@@ -293,6 +293,16 @@ int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_tokens, int num_
 int hexa_gate_loss_grad(const float* logits, int64_t ld, int64_t num_tokens, int num_experts, const int32_t* first_count,
                         const float* dloss, float* dlogits, int64_t ldd, void* stream);
 
+/* Operands of the gate projection of bf16 tokens with an fp32 weight on 16-bit tensor cores (no counterpart in the
+ * reference, which casts the tokens to fp32, gates/top.py:20-25): an fp32 value is hi + mid + lo exactly, each term the
+ * bf16 rounding of what the previous ones left over.
+ * split_terms: out (bf16) = the terms of src [rows, cols] (leading dimension ld).  by_rows = 0: [rows, 4 * cols], the
+ * column blocks (hi, hi, mid, lo); by_rows = 1: [4 * rows, cols], the row blocks (lo, mid, hi, hi), ld = cols.
+ * sum_terms: out [rows, cols] = (hi + mid) + lo of part [rows, 3 * cols], whose column blocks are (hi, mid, lo) or, with
+ * lo_first, (lo, mid, hi). */
+int hexa_gate_split_terms(const float* src, int64_t ld, int64_t rows, int64_t cols, int by_rows, void* out, void* stream);
+int hexa_gate_sum_terms(const float* part, int64_t rows, int64_t cols, int lo_first, float* out, void* stream);
+
 /* The same step for the other auxiliary loss of the reference, the load-importance loss (impls/losses.py:21-43, selected by
  * is_gshard_loss=False; needs gate noise): ids = top-k of the NOISY logits (what torch.topk of softmax(noisy) returns),
  *   importance[e] = sum_t softmax(logits)[t,e],   load[e] = sum_t Phi((softmax(logits)[t,e] - thr_t) / sigma),

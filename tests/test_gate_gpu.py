@@ -187,3 +187,71 @@ def test_module_with_the_load_importance_loss_takes_the_fused_gate():
     assert abs(fused[1] - plain[1]) <= 1e-4 * abs(plain[1])
     for a, b in ((fused[0], plain[0]), (fused[2], plain[2]), (fused[3], plain[3])):
         assert float((a - b).abs().max()) <= 2e-2 * float(b.abs().max())
+
+
+# Edges of the group kernels: the lane-group widths (8 lanes up to 64 experts, 16 up to 128, 32 beyond), column counts
+# around them, token counts around one block's sweeps and around a grid-stride step, and rows with a leading dimension.
+@pytest.mark.parametrize("E", [1, 8, 9, 16, 17, 33, 64, 65, 128, 129, 256, 257, 512])
+@pytest.mark.parametrize("T", [1, 31, 128, 129, 15000])
+def test_group_kernels_at_their_edges(T, E):
+    from hexa_moe_b200 import ops
+    k = min(E, 3)
+    g = torch.Generator(device="cuda").manual_seed(T * 1000 + E)
+    wide = torch.randn(T, E + 3, generator=g, device="cuda") * 2.0
+    logits = wide[:, :E]
+    if E >= 4:
+        logits[T // 2] = float("nan")                     # the lowest free ids, NaN only in the sums
+    ids, loss, first_count, mass = ops.gate_topk(logits, k)
+    live = torch.ones(T, dtype=torch.bool, device="cuda")
+    if E >= 4:
+        assert ids[:, T // 2].tolist() == list(range(k))
+        assert torch.isnan(loss) and torch.isnan(mass).all()
+        live[T // 2] = False
+        ids2, loss, first2, mass = ops.gate_topk(logits[live], k) if T > 1 else (None, None, None, None)
+        if T == 1:
+            return
+        assert torch.equal(ids2, ids[:, live])
+        logits, ids, first_count = logits[live].contiguous(), ids2, first2
+    n = logits.shape[0]
+    scores = F.softmax(logits.double(), dim=1)
+    want = torch.topk(scores, k, dim=1)
+    picked = scores.gather(1, ids.t().long())
+    assert torch.allclose(picked, want.values, rtol=1e-6, atol=0)       # equal up to scores within an ulp of each other
+    assert torch.equal(first_count.long(), torch.bincount(ids[0].long(), minlength=E))
+    assert torch.allclose(mass.double(), scores.sum(0), rtol=1e-5, atol=1e-6)
+    ce = first_count.double() * (E / n)
+    want_loss = (scores.sum(0) * ce).sum() / n
+    assert abs(float(loss) - float(want_loss)) <= 1e-5 * float(want_loss)
+    got = ops.gate_loss_grad(logits, first_count, torch.tensor(2.0, device="cuda"))
+    ge = 2.0 * ce / n
+    want_g = scores * (ge - (scores * ge).sum(1, keepdim=True))
+    # products of fp32 scores (relative error ~1e-6 with expf and the division) with g up to max(g)
+    assert float((got.double() - want_g).abs().max()) <= 4e-6 * float(ge.max())
+
+
+@pytest.mark.parametrize("T,d,E", [(1, 8, 1), (37, 72, 7), (300, 64, 8), (1000, 40, 33)])
+def test_split_precision_gate_terms(T, d, E):
+    """The split projection equals the fp32 products to fp32 accuracy and its gradients agree with the formulation in
+    plain operations that create_graph takes."""
+    from hexa_moe_b200 import ops
+    from hexa_moe_b200.impls.gating import _SplitPrecisionLinear, _split_terms
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(T, d, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    w = torch.randn(E, d, generator=g, device="cuda").requires_grad_(True)
+    t = _split_terms(w.detach(), torch.bfloat16, 3)
+    assert torch.equal(ops.gate_split_terms(w.detach(), True), torch.cat([t[2], t[1], t[0], t[0]], dim=0))
+    dy = torch.randn(T, E, generator=g, device="cuda")
+    t = _split_terms(dy, torch.bfloat16, 3)
+    assert torch.equal(ops.gate_split_terms(dy, False), torch.cat([t[0], t[0], t[1], t[2]], dim=1))
+    y = _SplitPrecisionLinear.apply(x, w)
+    exact = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * ((3 * d + 3) * 2.0 ** -24)      # 3d fp32 additions
+    assert ((y.double() - exact).abs() <= bound + 1e-30).all()
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+    y2 = _SplitPrecisionLinear.apply(x, w)
+    dx2, dw2 = torch.autograd.grad(y2, (x, w), dy, create_graph=True)
+    # dw: 3T fp32 additions either way; dx: one bf16 rounding (2^-8 between neighbours) of sums of 3E terms
+    bw = (dy.double().abs().t() @ x.double().abs()) * ((3 * T + 3) * 2.0 ** -23)
+    assert ((dw - dw2).double().abs() <= bw + 1e-30).all()
+    bx = (dy.double().abs() @ w.double().abs()) * ((3 * E + 3) * 2.0 ** -23)
+    assert ((dx - dx2).double().abs() <= dx.double().abs() * 2.0 ** -7 + bx + 1e-30).all()
