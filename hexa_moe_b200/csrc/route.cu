@@ -1,12 +1,17 @@
 // Routing: segment the T*top_k routed rows into contiguous, padded per-expert segments.
 //
-// Three launches, no host synchronisation, deterministic (equal to a stable sort by expert):
-//   1. route_hist    each warp histograms one chunk of kRowsPerWarp routed rows
-//   2. route_scan    one block: per-expert exclusive scan over chunks, per-expert totals, padded
-//                    segment offsets, tile -> expert table, -1 in the pad slots
-//   3. route_scatter each warp re-reads its chunk and places every row at
-//                    pad_offsets[e] + (rows of e in earlier chunks) + (rows of e earlier in the chunk)
-// HBM traffic: ids are read twice (8 B per routed row), row_token and token_row written once.
+// No host synchronisation, deterministic (equal to a stable sort by expert).  Every row goes to
+//   pad_offsets[e] + (rows of e in earlier blocks) + (rows of e in earlier warps) + (rows of e earlier in the warp's chunk).
+// Bound: latency (the ids of [131072, 2] are 1 MB).  By size:
+//   up to kSmallRows rows, up to 256 experts   one launch: route_place with a single block of 32 warps
+//   block count x experts up to kMaxTotals     two launches: route_count writes every block's histogram, then each block of
+//                                              route_place adds up the histograms itself (a few 10 KB from L2, by all its
+//                                              threads) instead of waiting for one block to scan them serially; the side
+//                                              tables are shared out over the blocks
+//   beyond that (the re-reading would cost more than a scan) three launches: route_hist, route_scan, route_scatter
+// [131072, 2] ids, 64 experts: 10 + 34 + 11 us with the three launches, 5 + 13 us with two; [2048, 2], 8 experts:
+// 7 + 5 + 9 us with three, 8 us with one.
+// HBM traffic: ids are read twice (8 B per routed row; once by the single block), row_token and token_row written once.
 #include <stdarg.h>
 #include <stdlib.h>
 
@@ -178,6 +183,209 @@ __global__ void route_scatter(const int32_t* __restrict__ ids, int64_t T, int to
   }
 }
 
+// ---- one or two launches ------------------------------------------------------------------------------------------------
+constexpr int kIters = 8;                          // rows of a lane: a warp's chunk is at most 256 rows
+constexpr int kCountWarps = 8;
+constexpr int kBlockRows = kCountWarps * 32 * kIters;      // rows of a block when there are several
+constexpr int64_t kSmallRows = 32 * 32 * kIters;           // rows of the single block of 32 warps
+constexpr int kSmallExperts = 256, kCountExperts = 512;    // (WARPS + 4) * E + 2 words of shared memory stay under 48 KB
+constexpr int64_t kMaxTotals = 65536;
+
+struct Ids {
+  const int32_t* p;
+  uint32_t T;
+  int64_t stride_t, stride_k;
+  int E;
+  __device__ __forceinline__ int at(uint32_t f, uint32_t& t, uint32_t& j) const {
+    j = f / T;
+    t = f - j * T;
+    const int e = __ldg(p + (int64_t)t * stride_t + (int64_t)j * stride_k);
+    return e >= 0 && e < E ? e : -1;
+  }
+};
+
+__global__ void __launch_bounds__(kCountWarps * 32)
+route_count(Ids ids, uint32_t n_rows, int32_t* __restrict__ totals) {
+  extern __shared__ int32_t sm[];
+  for (int e = threadIdx.x; e < ids.E; e += blockDim.x) sm[e] = 0;
+  __syncthreads();
+  int e[kIters];
+  const uint32_t f0 = blockIdx.x * (uint32_t)kBlockRows + threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < kIters; ++i) {
+    const uint32_t f = f0 + (uint32_t)i * blockDim.x;
+    uint32_t t, j;
+    e[i] = f < n_rows ? ids.at(f, t, j) : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < kIters; ++i)
+    if (e[i] >= 0) atomicAdd(&sm[e[i]], 1);
+  __syncthreads();
+  for (int x = threadIdx.x; x < ids.E; x += blockDim.x) totals[(int64_t)blockIdx.x * ids.E + x] = sm[x];
+}
+
+struct Tables {
+  int32_t *counts, *seg_offsets, *pad_offsets, *row_token, *token_row, *tile_expert, *pair_block;
+  int64_t row_capacity, pair_cap;
+  int align;
+};
+
+// largest e < E with offs[e] <= x (empty experts share an offset: the last one owns it)
+__device__ __forceinline__ int owner(const int32_t* offs, int E, int32_t x) {
+  int lo = 0, hi = E;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (offs[mid] <= x) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// totals: one histogram per block, or null when this is the only block
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
+route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const int32_t* __restrict__ totals, Tables out) {
+  extern __shared__ int32_t sm[];
+  const int E = ids.E;
+  int32_t* hist = sm;                    // [WARPS][E]: counts, then the next free row of each expert for each warp
+  int32_t* before = hist + WARPS * E;    // [E] rows of earlier blocks
+  int32_t* total = before + E;           // [E]
+  int32_t* pad = total + E;              // [E + 1]
+  int32_t* pair = pad + E + 1;           // [E + 1]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t chunk = (blockIdx.x * (uint32_t)WARPS + (uint32_t)warp) * rows_per_warp;
+  const uint32_t chunk_end = min(chunk + rows_per_warp, n_rows);
+  int e[kIters];
+  uint32_t t[kIters], slot[kIters];      // slot = t * top_k + j
+#pragma unroll
+  for (int i = 0; i < kIters; ++i) {
+    const uint32_t f = chunk + (uint32_t)i * 32 + (uint32_t)lane;
+    e[i] = -1;
+    t[i] = slot[i] = 0;
+    if (f < chunk_end) {
+      uint32_t j;
+      e[i] = ids.at(f, t[i], j);
+      slot[i] = t[i] * (uint32_t)top_k + j;
+    }
+  }
+  for (int x = threadIdx.x; x < (WARPS + 2) * E; x += WARPS * 32) sm[x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kIters; ++i)
+    if (e[i] >= 0) atomicAdd(&hist[warp * E + e[i]], 1);
+  if (totals) {      // integer sums: the order of the additions is immaterial
+    const int slices = max(1, WARPS * 32 / E);
+    for (int x = threadIdx.x; x < slices * E; x += WARPS * 32) {
+      const int ex = x % E;
+      int b_sum = 0, a_sum = 0;
+#pragma unroll 8
+      for (int b = x / E; b < (int)gridDim.x; b += slices) {
+        const int v = __ldg(totals + (int64_t)b * E + ex);
+        a_sum += v;
+        b_sum += b < (int)blockIdx.x ? v : 0;
+      }
+      atomicAdd(&total[ex], a_sum);
+      atomicAdd(&before[ex], b_sum);
+    }
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < E; x += WARPS * 32) {      // exclusive scan over the block's warps
+    int run = before[x];
+#pragma unroll 8
+    for (int w = 0; w < WARPS; ++w) {
+      const int v = hist[w * E + x];
+      hist[w * E + x] = run;
+      run += v;
+    }
+    if (!totals) total[x] = run;
+  }
+  __syncthreads();
+  // exclusive scans over experts (unpadded, padded, pair tiles) by warp 0, 32 experts per step
+  if (warp == 0) {
+    int32_t carry_seg = 0, carry_pad = 0, carry_pair = 0;
+    const bool writes = blockIdx.x == 0;
+    for (int base = 0; base < E; base += 32) {
+      const int x = base + lane;
+      const int32_t c = x < E ? total[x] : 0;
+      const int32_t p = (c + out.align - 1) / out.align * out.align;
+      const int32_t q = (p / kRowTile + 1) / 2;      // two 128-row blocks each, the last one may be half empty
+      int32_t ic = c, ip = p, iq = q;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t tc = __shfl_up_sync(0xffffffffu, ic, o), tp = __shfl_up_sync(0xffffffffu, ip, o);
+        const int32_t tq = __shfl_up_sync(0xffffffffu, iq, o);
+        if (lane >= o) { ic += tc; ip += tp; iq += tq; }
+      }
+      if (x < E) {
+        pad[x] = carry_pad + ip - p;
+        pair[x] = carry_pair + iq - q;
+        if (writes) {
+          out.counts[x] = c;
+          out.seg_offsets[x] = carry_seg + ic - c;
+          out.pad_offsets[x] = carry_pad + ip - p;
+        }
+      }
+      carry_seg += __shfl_sync(0xffffffffu, ic, 31);
+      carry_pad += __shfl_sync(0xffffffffu, ip, 31);
+      carry_pair += __shfl_sync(0xffffffffu, iq, 31);
+    }
+    if (lane == 0) {
+      pad[E] = carry_pad;
+      pair[E] = carry_pair;
+      if (writes) { out.seg_offsets[E] = carry_seg; out.pad_offsets[E] = carry_pad; }
+    }
+  }
+  __syncthreads();
+  // this warp's rows, 32 at a time in order
+  for (int x = lane; x < E; x += 32) hist[warp * E + x] += pad[x];
+  __syncwarp();
+  int32_t* cur = hist + warp * E;
+#pragma unroll
+  for (int i = 0; i < kIters; ++i) {
+    const uint32_t f = chunk + (uint32_t)i * 32;
+    if (f >= chunk_end) break;      // uniform across the warp
+    const unsigned peers = __match_any_sync(0xffffffffu, e[i]);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    int32_t pos = -1;
+    if (e[i] >= 0) pos = cur[e[i]] + rank;
+    __syncwarp();
+    if (e[i] >= 0 && rank == 0) cur[e[i]] += __popc(peers);
+    __syncwarp();
+    if (f + (uint32_t)lane < chunk_end) {
+      out.token_row[slot[i]] = pos;
+      if (pos >= 0) out.row_token[pos] = (int32_t)t[i];
+    }
+  }
+  // side tables, shared out over the grid
+  const int64_t tid = (int64_t)blockIdx.x * (WARPS * 32) + threadIdx.x, threads = (int64_t)gridDim.x * (WARPS * 32);
+  if (out.pair_block) {      // entry = (first 128-row block) * 2 + (the next block belongs to the same expert)
+    for (int64_t i = tid; i < out.pair_cap; i += threads) {
+      int32_t v = -1;
+      if (i < pair[E]) {
+        const int x = owner(pair, E, (int32_t)i);
+        const int32_t o = ((int32_t)i - pair[x]) * 2, nb = (pad[x + 1] - pad[x]) / kRowTile;
+        v = (pad[x] / kRowTile + o) * 2 + (o + 1 < nb ? 1 : 0);
+      }
+      out.pair_block[i] = v;
+    }
+  }
+  for (int64_t i = tid; i < out.row_capacity / out.align; i += threads) {
+    const int32_t row = (int32_t)(i * out.align);
+    out.tile_expert[i] = row < pad[E] ? owner(pad, E, row) : -1;
+  }
+  for (int64_t i = tid; i < (int64_t)E * out.align; i += threads) {      // pad slots
+    const int x = (int)(i / out.align), o = (int)(i % out.align);
+    const int32_t row = pad[x] + total[x] + o;
+    if (row < pad[x + 1]) out.row_token[row] = -1;
+  }
+}
+
+// 1, 2 or 3 launches, see the head of this file
+int route_plan(int64_t n_rows, int E) {
+  if (n_rows <= kSmallRows && E <= kSmallExperts) return 1;
+  if (n_rows > 0 && E <= kCountExperts && ceil_div(n_rows, kBlockRows) * E <= kMaxTotals) return 2;
+  return 3;
+}
+
 }  // namespace
 
 // ---- error plumbing shared by every translation unit ------------------------------------------
@@ -310,9 +518,29 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
     set_error("hexa_route: workspace %zu bytes < required %zu", workspace_bytes, need);
     return HEXA_ERR_WORKSPACE;
   }
+  HEXA_REQUIRE(pair_block == nullptr || align == kRowTile, "hexa_route: the pair-tile list needs align = %d", kRowTile);
   const int64_t n_rows = T * top_k;
-  const int64_t n_chunks = ceil_div(n_rows, kRowsPerWarp);
   const int64_t row_cap = hexa_route_row_capacity(T, top_k, E, align);
+  const int64_t pair_cap = pair_block ? hexa_route_pair_capacity(T, top_k, E) : 0;
+  const int plan = route_plan(n_rows, E);
+  if (plan <= 2) {
+    const Ids in{ids, (uint32_t)(T > 0 ? T : 1), stride_t, stride_k, E};
+    const Tables out{counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block, row_cap, pair_cap, align};
+    if (plan == 1) {
+      const uint32_t rows_per_warp = (uint32_t)ceil_div(ceil_div(n_rows, 32), 32) * 32;
+      route_place<32><<<1, 1024, (36 * (size_t)E + 2) * sizeof(int32_t), stream>>>(in, top_k, (uint32_t)n_rows, rows_per_warp, nullptr, out);
+    } else {
+      const unsigned blocks = (unsigned)ceil_div(n_rows, kBlockRows);
+      int32_t* totals = (int32_t*)workspace;      // blocks * E words, fewer than the chunk histograms of the third plan
+      route_count<<<blocks, kCountWarps * 32, (size_t)E * sizeof(int32_t), stream>>>(in, (uint32_t)n_rows, totals);
+      HEXA_LAUNCH_CHECK("route_count");
+      route_place<kCountWarps><<<blocks, kCountWarps * 32, ((kCountWarps + 4) * (size_t)E + 2) * sizeof(int32_t), stream>>>(
+          in, top_k, (uint32_t)n_rows, 32 * kIters, totals, out);
+    }
+    HEXA_LAUNCH_CHECK("route_place");
+    return HEXA_OK;
+  }
+  const int64_t n_chunks = ceil_div(n_rows, kRowsPerWarp);
   int32_t* chunk_hist = (int32_t*)workspace;
   int warps = (int)(48 * 1024 / (4 * (int64_t)E));
   warps = warps < 1 ? 1 : (warps > 8 ? 8 : warps);
@@ -322,11 +550,10 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
                                                                                 chunk_hist);
     HEXA_LAUNCH_CHECK("route_hist");
   }
-  HEXA_REQUIRE(pair_block == nullptr || align == kRowTile, "hexa_route: the pair-tile list needs align = %d", kRowTile);
   int32_t* pair_off = chunk_hist + (size_t)(n_chunks > 0 ? n_chunks : 1) * E;
   route_scan<<<1, 1024, (2 * (size_t)E + 1) * sizeof(int32_t), stream>>>(
       chunk_hist, n_chunks, E, align, row_cap, counts, seg_offsets, pad_offsets, row_token, tile_expert, pair_off, pair_block,
-      pair_block ? hexa_route_pair_capacity(T, top_k, E) : 0);
+      pair_cap);
   HEXA_LAUNCH_CHECK("route_scan");
   if (n_chunks > 0) {
     route_scatter<<<(unsigned)ceil_div(n_chunks, warps), warps * 32, smem, stream>>>(
@@ -334,4 +561,8 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
     HEXA_LAUNCH_CHECK("route_scatter");
   }
   return HEXA_OK;
+}
+
+extern "C" int hexa_route_launches(int64_t T, int top_k, int E) {
+  return T < 0 || top_k <= 0 || E <= 0 ? 0 : route_plan(T * top_k, E);
 }

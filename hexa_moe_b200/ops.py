@@ -22,7 +22,7 @@ from ._lib import check, dt, lib, ptr, stream_of
 # (name, start_event, end_event, algorithmic_work, algorithmic_bytes) with CUDA events recorded on the launching stream.
 LAUNCHES = 0
 PROFILE = None
-_KERNELS_PER_CALL = dict(route=3, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1)
+_KERNELS_PER_CALL = dict(route=1, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1)
 
 
 class _Timed:
@@ -66,6 +66,7 @@ class Routing:
 
 def route(ids: torch.Tensor, num_experts: int, align: int = L.ROW_TILE, route_major: bool = False) -> Routing:
     """Segment routed rows by expert.  ids: int32 [T, k] (or [k, T] when route_major)."""
+    global LAUNCHES
     if ids.dtype != torch.int32:
         raise L.HexaError("route: ids must be int32")
     if ids.dim() != 2:
@@ -92,6 +93,8 @@ def route(ids: torch.Tensor, num_experts: int, align: int = L.ROW_TILE, route_ma
         check(lib().hexa_route(ptr(ids), T, k, st, sk, num_experts, align, ptr(r.counts), ptr(r.seg_offsets), ptr(r.pad_offsets),
                                ptr(r.row_token), ptr(r.token_row), ptr(r.tile_expert), ptr(r.pair_block), ptr(ws), ws.numel(), s),
               "hexa_route")
+    if T * k > 8192 or num_experts > 256:
+        LAUNCHES += lib().hexa_route_launches(T, k, num_experts) - 1
     return r
 
 

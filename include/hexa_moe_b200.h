@@ -112,6 +112,9 @@ size_t hexa_route_workspace_bytes(int64_t num_tokens, int top_k, int num_experts
 /* Entries of the optional pair-tile list (align = 128 only): row_capacity/256 + E + 1. */
 int64_t hexa_route_pair_capacity(int64_t num_tokens, int top_k, int num_experts);
 
+/* How many kernels hexa_route launches for a size (1 to 3; 0 for bad sizes). */
+int hexa_route_launches(int64_t num_tokens, int top_k, int num_experts);
+
 /* ids: expert id of routed row (t,j) at ids[t*stride_t + j*stride_k]; ids outside [0,E) are
  * skipped (their token_row entry is -1).
  * Outputs (device, int32): counts[E], seg_offsets[E+1] (exclusive scan of counts),

@@ -493,3 +493,35 @@ def test_simt_tile_sizes_agree(ops, dtype, K, N, nk):
         # a chain of n fp32 FMAs is within n * 2^-24 of the sum of magnitudes; rows of an expert bound n
         bound = wide[po[e]:po[e + 1]].double().abs().t() @ xs[po[e]:po[e + 1]].double().abs() * ((po[e + 1] - po[e]) * 2.0 ** -24)
         assert ((dw[e].double() - want).abs() <= bound + 1e-30).all()
+
+
+# One launch, two launches and three: sizes around a warp's chunk, the single block's capacity, a block's rows of the
+# two-launch form, the expert limits of both, strided id tensors, ids out of range, no rows for most experts.
+@pytest.mark.parametrize("T,k,E,launches", [(0, 2, 4, 1), (1, 1, 256, 1), (33, 3, 7, 1), (4096, 2, 64, 1), (8192, 1, 256, 1), (8193, 1, 64, 2),
+                                            (9001, 1, 257, 2), (2048, 4, 512, 2), (70000, 3, 64, 2), (16385, 2, 8, 2),
+                                            (600, 2, 513, 3), (200000, 4, 400, 3)])
+@pytest.mark.parametrize("align", [128, 16])
+def test_route_launch_forms(ops, T, k, E, launches, align):
+    Lb = L()
+    assert Lb.lib().hexa_route_launches(T, k, E) == launches
+    g = torch.Generator().manual_seed(T + E)
+    ids = torch.randint(-1, E + 1, (T, k), generator=g, dtype=torch.int32)
+    if E > 8:
+        ids[T // 2:] = ids[T // 2:] % 3
+    dev = ids.cuda()
+    wide = torch.full((T, 2 * k + 1), -7, dtype=torch.int32, device="cuda")
+    wide[:, 1::2] = dev
+    forms = [(dev, False), (dev.t().contiguous(), True), (wide[:, 1::2], False), (wide.t()[1::2], True)]
+    want = O.route(ids, E, align)
+    n_pad = want["n_pad"]
+    for src, major in forms:
+        r = ops.route(src, E, align, route_major=major)
+        for name in ("counts", "seg_offsets", "pad_offsets"):
+            assert torch.equal(getattr(r, name).cpu(), want[name]), name
+        assert torch.equal(r.row_token.cpu()[:n_pad], want["row_token"])
+        assert torch.equal(r.token_row.cpu()[: T * k], want["token_row"])
+        te = r.tile_expert.cpu()
+        assert torch.equal(te[: n_pad // align], want["tile_expert"]) and (te[n_pad // align: r.row_capacity // align] == -1).all()
+        if align == 128:
+            pb, n = r.pair_block.cpu(), want["pair_block"].numel()
+            assert torch.equal(pb[:n], want["pair_block"]) and (pb[n:] == -1).all()
