@@ -122,20 +122,20 @@ __device__ __forceinline__ void fold_loss(float part, float* red, int64_t T, int
 }
 
 // partial: per block E float column sums, then E int top-1 counts
-template <int G, int PER>
-__global__ void __launch_bounds__(kGateThreads)
+template <int G, int PER, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, int k, int32_t* __restrict__ ids,
                  float* __restrict__ mass, int32_t* __restrict__ first_count, float* __restrict__ loss,
                  float* __restrict__ partial) {
   constexpr int kGroups = 32 / G;
-  __shared__ float mass_w[kGateWarps][G * PER];
+  __shared__ float mass_w[WARPS][G * PER];
   __shared__ int cnt_s[G * PER];
-  __shared__ float red_s[kGateWarps];
+  __shared__ float red_s[WARPS];
   for (int e = threadIdx.x; e < G * PER; e += blockDim.x) cnt_s[e] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane & (G - 1);
-  const int64_t first = ((int64_t)blockIdx.x * kGateWarps + warp) * kGroups;     // this warp's first token of a sweep
-  const int64_t step = (int64_t)gridDim.x * kGateWarps * kGroups;
+  const int64_t first = ((int64_t)blockIdx.x * WARPS + warp) * kGroups;     // this warp's first token of a sweep
+  const int64_t step = (int64_t)gridDim.x * WARPS * kGroups;
   const int grp = lane / G;
   float acc[PER], next[PER];
 #pragma unroll
@@ -194,7 +194,7 @@ gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E,
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     float m = 0.f;
 #pragma unroll
-    for (int w = 0; w < kGateWarps; ++w) m += mass_w[w][e];
+    for (int w = 0; w < WARPS; ++w) m += mass_w[w][e];
     if (only) {
       mass[e] = m;
       first_count[e] = cnt_s[e];
@@ -515,16 +515,17 @@ gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ 
   }
 }
 
-// Blocks of the group kernels: one sweep of a block covers kGateWarps * 32 / G tokens.  Up to four sweeps stay in one block,
-// which then needs no second launch (a sweep costs ~1 us, a launch ~3 us); beyond that, three blocks per SM.
+// Blocks of the group kernels: one sweep of a block covers kGateWarps * 32 / G tokens, three blocks per SM at most.
 int gate_group_grid(int64_t T, int G) {
-  const int64_t sweep = kGateWarps * (32 / G);
-  if (T <= 4 * sweep) return 1;
   int64_t cap = (int64_t)sm_count() * 3;
   if (cap > kGateMaxBlocks / 2) cap = kGateMaxBlocks / 2;      // a block leaves two rows of words
-  const int64_t want = ceil_div(T, sweep);
+  const int64_t want = ceil_div(T, kGateWarps * (32 / G));
   return (int)(want < cap ? want : cap);
 }
+// Tokens that one block takes by itself, saving the second launch (~3 us): four sweeps at ~1 us each, of 32 warps where
+// their column sums fit in shared memory.
+constexpr int lone_warps(int G) { return G < 32 ? 32 : kGateWarps; }
+constexpr int64_t lone_tokens(int G) { return 4 * lone_warps(G) * (32 / G); }
 
 #define HEXA_GATE_DISPATCH(E, LAUNCH)  \
   do {                                 \
@@ -575,9 +576,15 @@ extern "C" int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_token
   float* partial = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kGateTicketBytes);
   int grid = 1;
 #define HEXA_GATE_FWD(G, PER)                                                                                              \
-  grid = gate_group_grid(num_tokens, G);                                                                                   \
-  gate_topk_kernel<G, PER><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, top_k, ids, mass,       \
-                                                              first_count, loss, partial)
+  if (num_tokens <= lone_tokens(G)) {                                                                                      \
+    gate_topk_kernel<G, PER, lone_warps(G)><<<1, lone_warps(G) * 32, 0, stream>>>(logits, ld, num_tokens, num_experts,     \
+                                                                                  top_k, ids, mass, first_count, loss,     \
+                                                                                  partial);                                \
+  } else {                                                                                                                 \
+    grid = gate_group_grid(num_tokens, G);                                                                                 \
+    gate_topk_kernel<G, PER, kGateWarps><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, top_k,    \
+                                                                            ids, mass, first_count, loss, partial);        \
+  }
   HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_FWD)
 #undef HEXA_GATE_FWD
   HEXA_LAUNCH_CHECK("gate_topk_kernel");

@@ -327,7 +327,7 @@ def gate_topk(logits: torch.Tensor, top_k: int):
     with _Timed("gate", 2.0 * T * E * 4):
         check(lib().hexa_gate_topk(ptr(logits), _ld(logits), T, E, top_k, ptr(ids), ptr(mass), ptr(cnt), ptr(loss), ptr(ws),
                                    ws.numel(), stream_of(logits)), "hexa_gate_topk")
-    LAUNCHES += T > (128 if E <= 64 else 64 if E <= 128 else 32)      # beyond one block: a second kernel adds the blocks' rows
+    LAUNCHES += T > (512 if E <= 64 else 256 if E <= 128 else 32)      # beyond one block: a second kernel adds the blocks' rows
     return ids, loss, cnt, mass
 
 

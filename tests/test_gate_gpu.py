@@ -192,7 +192,7 @@ def test_module_with_the_load_importance_loss_takes_the_fused_gate():
 # Edges of the group kernels: the lane-group widths (8 lanes up to 64 experts, 16 up to 128, 32 beyond), column counts
 # around them, token counts around one block's sweeps and around a grid-stride step, and rows with a leading dimension.
 @pytest.mark.parametrize("E", [1, 8, 9, 16, 17, 33, 64, 65, 128, 129, 256, 257, 512])
-@pytest.mark.parametrize("T", [1, 31, 128, 129, 15000])
+@pytest.mark.parametrize("T", [1, 33, 256, 257, 512, 513, 15000])
 def test_group_kernels_at_their_edges(T, E):
     from hexa_moe_b200 import ops
     k = min(E, 3)
