@@ -95,7 +95,7 @@ def lib():
 
 ERR_DEVICE = -5
 _STATUS_CODES = {1: "the TMA producer waited for a free ring slot", 2: "the MMA issuer waited for a drained accumulator",
-                 3: "the MMA issuer waited for operands", 4: "an epilogue warp waited for an accumulator"}
+                 3: "the MMA issuer waited for operands", 4: "an epilogue warp waited for an accumulator", 5: "an epilogue warp waited for the saved pre-activation"}
 
 
 def check(status: int, what: str):

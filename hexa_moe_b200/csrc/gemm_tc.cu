@@ -16,11 +16,22 @@
 //   warp 1      MMA issuer (only in the pair's leader CTA when CTAS = 2): one thread issues tcgen05.mma
 //               (K = 16 per instruction) into one of two TMEM accumulators; tcgen05.commit frees ring slots
 //               and publishes finished accumulators (multicast to both CTAs of a pair)
-//   warps 2..   epilogue (EW = 16 or 8 warps, template parameter): tcgen05.ld of the accumulator (lane quadrant =
-//               warp % 4, each group of four warps owns a column range), fused epilogue math; ESMM results go through
-//               a 64B-swizzled staging tile and one TMA store per 128x32 block, ESTMM stores from registers.  The
-//               MMA and producer threads share their issue slots with the epilogue warps of their sub-partition:
-//               16 warps finish a tile's epilogue sooner (short k-loops), 8 leave the role threads more slots
+//   warps 2..17 epilogue: tcgen05.ld of the accumulator (lane quadrant = warp % 4, each group of four warps owns a column
+//               range), fused epilogue math; results go through 64B-swizzled staging tiles and one TMA store per 128x32
+//               block (ESTMM with fp32, accumulating, split or scattered output stores from registers).  A kernel per
+//               epilogue (Out below), because they want different things of shared memory:
+//                 ACT     two staging tiles per group, pre-activation and output side by side: one wait and one pair of
+//                         barriers per block instead of two
+//                 DACT    two staging tiles per group that first receive the saved pre-activation by TMA, a block ahead,
+//                         and are overwritten in place by the result.  Reading it with per-thread loads (32 rows x 16 B
+//                         per instruction, each behind the previous block's math) cost 214 us where this costs 171
+//                         ([32768 rows, 3072 x 768], bf16, GELU'; 1336 where 1240 at [131072, 4096 x 1024] skewed)
+//                 STAGED  ESTMM's 16-bit [E, m, n] outputs: 145 us with register stores (a row per lane, half-used
+//                         sectors), 75 through the staging tile (32 experts x 4096 x 1024 from 144 rows each; long
+//                         segments measure the same either way)
+//               The tile's bias is put into shared memory by the group a tile ahead (fc1 + GELU of the first shape: 209 ->
+//               196 us on one box, the 16 per-thread global loads of a block sat in front of the math).  Loading all 32
+//               columns of a block from TMEM at once instead of 16 + 16 spilled and was 20 % slower.
 // so the epilogue of tile i overlaps the MMAs of tile i+1.  Every mbarrier wait is bounded: after ~2 s a CTA
 // raises an abort flag, records a code in the status word and drains; both CTAs of a pair always reach the
 // closing cluster barrier.
@@ -304,23 +315,30 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                : "memory");
 }
 
-template <int BN, int CTAS, int EW, int MODE> struct Cfg {
-  static constexpr int kThreads = 32 * (2 + EW);
-  // ESTMM stores from registers and needs no staging tile: its ring gets the space (one more 32 KB slot), which is what
-  // a loop bounded by the latency of a ring slot's round trip (MMA done -> slot refilled) converts into throughput
-#ifndef HEXA_TC_RING_SLOTS      // build-time override for experiments with the ring depth (0 = the defaults below)
-#define HEXA_TC_RING_SLOTS 0
-#endif
+// What the epilogue does with an accumulator.  ESMM: HEXA_EPI_LINEAR / HEXA_EPI_ACT / HEXA_EPI_DACT; ESTMM: stores from
+// registers (any output form) or through staging tiles (16-bit [E, m, n] outputs).
+enum Out { OUT_LINEAR = HEXA_EPI_LINEAR, OUT_ACT = HEXA_EPI_ACT, OUT_DACT = HEXA_EPI_DACT, OUT_REGISTERS = 3, OUT_STAGED = 4 };
+
+template <int BN, int CTAS, int MODE, int OUT> struct Cfg {
+  static constexpr int kEpiWarps = 16;
+  static constexpr int kThreads = 32 * (2 + kEpiWarps);
+  static constexpr int kParts = kEpiWarps / 4;          // groups of four warps; each owns BN / kParts columns of every tile
+  static constexpr int kBlocks = BN / kParts / 32;      // as this many 128 x 32 blocks
 #ifndef HEXA_TC_SMEM_SLACK      // bytes kept for aligning the dynamic shared memory base to 1 KB by hand
 #define HEXA_TC_SMEM_SLACK 1024
 #endif
-  static constexpr int kStages = (BN == 256 && CTAS == 1) ? 4 : (HEXA_TC_RING_SLOTS ? HEXA_TC_RING_SLOTS : (MODE == ESTMM ? 7 : 6));
+  // 128 x 32 staging tiles per group: one where the epilogue has nothing to wait for but its own stores; two where it
+  // writes two outputs (ACT) or reads the saved pre-activation through the same tile (DACT); none for register stores.
+  // The ring has the rest of the shared memory (32 KB per slot; 48 KB for single-CTA 256-column tiles).
+  static constexpr int kBufs = OUT == OUT_REGISTERS ? 0 : (OUT == OUT_ACT || OUT == OUT_DACT) ? 2 : 1;
   static constexpr uint32_t kBBytes = (BN / CTAS) * BLOCK_K * 2;   // this CTA's share of the B tile
   static constexpr uint32_t kStageBytes = kABytes + kBBytes;
   static constexpr uint32_t kTmemCols = 2 * BN;  // two accumulators; 256 or 512, a power of two
   static constexpr uint32_t kStoreBufBytes = 128 * 64;   // [128 rows x 32 16-bit columns]
-  static constexpr uint32_t kStoreBytes = MODE == ESTMM ? 0 : (EW / 4) * kStoreBufBytes;  // one buffer per group of four epilogue warps
-  static constexpr size_t kSmemBytes = HEXA_TC_SMEM_SLACK + (size_t)kStages * kStageBytes + kStoreBytes + 256 /*barriers*/;
+  static constexpr uint32_t kStoreBytes = kBufs * kParts * kStoreBufBytes;
+  static constexpr uint32_t kBiasBytes = MODE == ESTMM ? 0 : BN * 4;      // the tile's bias, a part per group
+  static constexpr int kStages = (232448 - HEXA_TC_SMEM_SLACK - 512 - kBiasBytes - kStoreBytes) / kStageBytes;
+  static constexpr size_t kSmemBytes = HEXA_TC_SMEM_SLACK + (size_t)kStages * kStageBytes + kStoreBytes + kBiasBytes + 512 /*barriers*/;
   static_assert(kSmemBytes <= 232448, "more shared memory than one CTA can have (227 KB)");
 };
 
@@ -395,6 +413,11 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, const void* 
                "r"(c0), "r"(c1)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* tm, const void* src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tm), "r"(smem_u32(src)),
+               "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void bulk_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
@@ -413,43 +436,80 @@ __device__ __forceinline__ void stage_row(uint8_t* buf, int r, const uint32_t (&
     *reinterpret_cast<uint4*>(row + ((c ^ x) << 4)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
 }
 
+// Half of that row: 16 columns = chunks 2 hf and 2 hf + 1.
+__device__ __forceinline__ void stage_half(uint8_t* buf, int r, int hf, const uint32_t (&w)[8]) {
+  uint8_t* row = buf + r * 64;
+  const int x = (r >> 1) & 3;
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    *reinterpret_cast<uint4*>(row + (((2 * hf + c) ^ x) << 4)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+}
+__device__ __forceinline__ void load_half(const uint8_t* buf, int r, int hf, uint32_t (&w)[8]) {
+  const uint8_t* row = buf + r * 64;
+  const int x = (r >> 1) & 3;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const uint4 a = *reinterpret_cast<const uint4*>(row + (((2 * hf + c) ^ x) << 4));
+    w[4 * c] = a.x; w[4 * c + 1] = a.y; w[4 * c + 2] = a.z; w[4 * c + 3] = a.w;
+  }
+}
+
 // Values of 16 columns of one row for the two possible outputs of the ESMM epilogue: y = acc + bias packed as it
 // is (the saved pre-activation), o = the layer output of this GEMM.  Rows that are padding come out as zeros without a
 // select per element: their accumulator is exactly zero (the A operand's pad rows are zeros), the caller has masked
 // their bias, and every activation here maps 0 to 0 (the derivative epilogue multiplies the zero accumulator).  Working
 // on 16 columns at a time keeps few enough values live for the compiler to interleave the independent activations.
-template <int EPI, int ACT, int is_bf16>
-__device__ __forceinline__ void epi_values16(const float (&f)[16], const uint16_t* xp, int ncols, uint32_t* y, uint32_t* o) {
-  if (EPI == HEXA_EPI_DACT) {
+template <int OUT, int ACT, int is_bf16>
+__device__ __forceinline__ void epi_values16(const float (&f)[16], const uint32_t (&x)[8], uint32_t* y, uint32_t* o) {
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      // columns at or beyond ncols do not exist (the TMA store clips them): do not read aux there
-      const uint4 a = g * 8 < ncols ? *reinterpret_cast<const uint4*>(xp + g * 8) : make_uint4(0, 0, 0, 0);
-      const uint32_t* ap = reinterpret_cast<const uint32_t*>(&a);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        o[4 * g + i] = pack2(f[8 * g + 2 * i] * act_grad_fast<ACT>(unpack_lo(ap[i], is_bf16)),
-                             f[8 * g + 2 * i + 1] * act_grad_fast<ACT>(unpack_hi(ap[i], is_bf16)), is_bf16);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (EPI == HEXA_EPI_ACT) {
-        y[i] = pack2(f[2 * i], f[2 * i + 1], is_bf16);
-        o[i] = pack2(act_fast<ACT>(f[2 * i]), act_fast<ACT>(f[2 * i + 1]), is_bf16);
-      } else {
-        o[i] = pack2(f[2 * i], f[2 * i + 1], is_bf16);
-      }
+  for (int i = 0; i < 8; ++i) {
+    if (OUT == OUT_DACT) {
+      o[i] = pack2(f[2 * i] * act_grad_fast<ACT>(unpack_lo(x[i], is_bf16)),
+                   f[2 * i + 1] * act_grad_fast<ACT>(unpack_hi(x[i], is_bf16)), is_bf16);
+    } else if (OUT == OUT_ACT) {
+      y[i] = pack2(f[2 * i], f[2 * i + 1], is_bf16);
+      o[i] = pack2(act_fast<ACT>(f[2 * i]), act_fast<ACT>(f[2 * i + 1]), is_bf16);
+    } else {
+      o[i] = pack2(f[2 * i], f[2 * i + 1], is_bf16);
     }
   }
 }
+template <int OUT>
+__device__ __forceinline__ void epi_dispatch16(int act, int is_bf16, const float (&f)[16], const uint32_t (&x)[8], uint32_t* y, uint32_t* o) {
+  // one specialisation per (activation, 16-bit flavour): no per-element branches
+#define HEXA_EPI_CASE(A_)                                                  \
+  case A_:                                                                 \
+    if (is_bf16) epi_values16<OUT, A_, 1>(f, x, y, o);                     \
+    else epi_values16<OUT, A_, 0>(f, x, y, o);                             \
+    break;
+  if (OUT == OUT_LINEAR) act = HEXA_ACT_NONE;
+  switch (act) {
+    HEXA_EPI_CASE(HEXA_ACT_RELU)
+    HEXA_EPI_CASE(HEXA_ACT_GELU)
+    HEXA_EPI_CASE(HEXA_ACT_GELU_TANH)
+    HEXA_EPI_CASE(HEXA_ACT_SILU)
+    default:
+      if (is_bf16) epi_values16<OUT, HEXA_ACT_NONE, 1>(f, x, y, o);
+      else epi_values16<OUT, HEXA_ACT_NONE, 0>(f, x, y, o);
+  }
+#undef HEXA_EPI_CASE
+}
 
-template <int BN, int MODE, int CTAS, int EW>
-__global__ void __launch_bounds__(32 * (2 + EW), 1)
+// The tile list as the epilogue walks it (ESMM): the entry of the next tile is requested while this one is worked on.
+// entry = (first 128-row block of the tile) * 2 + (the second block is this expert's as well), -1 past the end.
+template <int CTAS>
+__device__ __forceinline__ int tile_entry(const Params& p, uint32_t t, uint32_t row_tiles) {
+  const uint32_t row_tile = t / p.nt;
+  if (row_tile >= row_tiles) return -1;
+  return CTAS == 2 ? __ldg(p.pair_block + row_tile) : (int)(row_tile * 2);
+}
+
+template <int BN, int MODE, int CTAS, int OUT>
+__global__ void __launch_bounds__(Cfg<BN, CTAS, MODE, OUT>::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX, const Params p) {
-  using C = Cfg<BN, CTAS, EW, MODE>;
-  constexpr int kEpiWarps = EW;
+  using C = Cfg<BN, CTAS, MODE, OUT>;
+  constexpr int kEpiWarps = C::kEpiWarps;
   constexpr int kStages = C::kStages;
   constexpr int BNH = BN / CTAS;          // B columns this CTA loads
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -459,7 +519,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     return;                                                  // uniform: every thread of every CTA sees the same base offset
   }
   uint8_t* store_bufs = smem + (size_t)kStages * C::kStageBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(store_bufs + C::kStoreBytes);
+  float* bias_s = reinterpret_cast<float*>(store_bufs + C::kStoreBytes);      // [BN] ESMM
+  uint64_t* bars = reinterpret_cast<uint64_t*>(store_bufs + C::kStoreBytes + C::kBiasBytes);
   uint64_t* full = bars;                  // [kStages]  producers -> MMA     (used in the leader CTA)
   uint64_t* empty = bars + kStages;       // [kStages]  MMA -> producer      (one per CTA, multicast commit)
   uint64_t* acc_full = bars + 2 * kStages;        // [2] MMA -> epilogue     (one per CTA, multicast commit)
@@ -467,6 +528,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* group_abort = abort_flag + 1;   // [4]: one per group of four epilogue warps
+  uint64_t* aux_full = bars + 2 * kStages + 8;   // [kParts][2] DACT: the saved pre-activation is in the group's staging tile
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CTAS == 2 ? (int)cluster_ctarank() : 0;    // 0 = leader of the pair
@@ -478,6 +540,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], kEpiWarps * CTAS); }
     *abort_flag = 0;
     for (int g = 0; g < kEpiWarps / 4; ++g) group_abort[g] = 0;
+    if (OUT == OUT_DACT)
+      for (int g = 0; g < 2 * C::kParts; ++g) mbar_init(&aux_full[g], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {  // the allocating warp also frees; with CTAS = 2 the same warp of both CTAs takes part
@@ -618,40 +682,64 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue (every CTA, its own 128 rows)
-    constexpr int kParts = kEpiWarps / 4;   // groups of four warps; each group owns BN / kParts columns of every tile
     const int q = warp & 3;                 // TMEM lane quadrant this warp may read
     const int part = (warp - 2) >> 2;
     const int is_bf16 = p.is_bf16;
-    const bool leader = (q == 2) && lane == 0;   // the first warp of every group of four issues the group's TMA stores
-    uint8_t* buf = store_bufs + (size_t)part * C::kStoreBufBytes;
+    const bool leader = (q == 2) && lane == 0;   // the first warp of every group of four issues the group's TMA copies
+    uint8_t* bufs = store_bufs + (size_t)part * C::kBufs * C::kStoreBufBytes;
+    const int rloc = q * 32 + lane;
+    const int part_col = part * (BN / C::kParts);
     bool ok = true;
-    Tile tile;
     int it = -1;
-    for (uint32_t t = tile_first; ok && get_tile<BN, MODE, CTAS>(p, t, rank, tile); t += tile_step) {
-      if (MODE != ESTMM && tile.skip) continue;
-      ++it;
-      const int acc = it & 1;
-      const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-      // The four warps of a group meet at named barriers inside the tile, so they must leave together: each warp
-      // publishes a failed wait, the group synchronises, and all four read the same verdict.
+    // The four warps of a group meet at named barriers inside the tile, so they must leave together: each warp
+    // publishes a failed wait, the group synchronises, and all four read the same verdict.
+    auto accumulator_ready = [&](int acc, uint32_t acc_phase) {
       if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, 4, p.wait_limit_ns) && lane == 0) group_abort[part] = 1;
       group_sync(1 + part);
-      if (group_abort[part]) { ok = false; break; }
-      tc_fence_after();
-      const int rloc = q * 32 + lane;
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
+      return group_abort[part] == 0;
+    };
+    auto accumulator_drained = [&](int acc) {      // hand it back to the (leader's) MMA warp
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CTAS == 2 && rank != 0) mbar_arrive_cluster(map_to_cta(&acc_empty[acc], 0));
+        else mbar_arrive(&acc_empty[acc]);
+      }
+    };
+    if constexpr (MODE == ESTMM) {
+      Tile tile;
+      for (uint32_t t = tile_first; get_tile<BN, MODE, CTAS>(p, t, rank, tile); t += tile_step) {
+        ++it;
+        const int acc = it & 1;
+        if (!accumulator_ready(acc, (uint32_t)(it >> 1) & 1u)) break;
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
 #pragma unroll 1
-      for (int cc = 0; cc < BN / kParts / 32; ++cc) {
-        const int cloc = part * (BN / kParts) + cc * 32;
-        const int64_t gcol = (int64_t)tile.col0 + cloc;
-        if (gcol >= p.n || !tile.valid) break;  // uniform across the four warps of a group
-        if (MODE == ESTMM) {
+        for (int cc = 0; cc < C::kBlocks; ++cc) {
+          const int cloc = part_col + cc * 32;
+          const int64_t gcol = (int64_t)tile.col0 + cloc;
+          if (gcol >= p.n || !tile.valid) break;  // uniform across the four warps of a group
           uint32_t v[32];
           if (tile.num_kb > 0) {
             tmem_ld32(t_row + (uint32_t)cloc, v);
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+          if constexpr (OUT == OUT_STAGED) {      // rows and columns beyond the output are clipped by the store
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]), is_bf16);
+            if (leader) bulk_wait_read<0>();   // the previous store has finished reading the buffer
+            group_sync(1 + part);
+            stage_row(bufs, rloc, w);
+            fence_async_smem();
+            group_sync(1 + part);
+            if (leader) {
+              tma_store_3d(&tmC, bufs, (int)gcol, tile.m0, tile.e);
+              bulk_commit();
+            }
+            continue;
           }
           const int64_t mrow = (int64_t)tile.m0 + rloc;
           if (mrow < p.m && p.splits > 1) {
@@ -706,105 +794,149 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               }
             }
           }
-        } else {
-          const int64_t r = (int64_t)tile.row0 + rloc;
+        }
+        accumulator_drained(acc);
+      }
+    } else {
+      const uint32_t row_tiles = CTAS == 2 ? (uint32_t)p.max_pairs : (uint32_t)(p.pad_offsets[p.E] / BLOCK_M);
+      uint32_t t = tile_first;
+      int entry = tile_entry<CTAS>(p, t, row_tiles);
+      int e = entry >= 0 ? __ldg(p.tile_expert + (entry >> 1)) : -1;
+      uint32_t seq = 0;             // DACT: blocks done so far; block i uses staging tile i & 1
+      bool requested = false;       // DACT, leader: the block about to start has its aux load under way
+      auto request_aux = [&](uint32_t block, int64_t col, int row0) {
+        uint64_t* bar = &aux_full[part * 2 + (block & 1)];
+        mbar_expect_tx(bar, C::kStoreBufBytes);
+        tma_load_2d(bufs + (block & 1) * C::kStoreBufBytes, &tmX, bar, (int)col, row0);
+      };
+      // Thread i of a group holds the bias of the group's i-th column of the tile ahead; it goes to shared memory before the
+      // first barrier of its tile, which every thread reaches after the last barrier (hence after all reads) of the one before.
+      constexpr int kPartCols = BN / C::kParts;
+      const int gi = q * 32 + lane;
+      auto bias_of = [&](int expert, uint32_t tile_index) {
+        const int64_t col = (int64_t)(tile_index % p.nt) * BN + part_col + gi;
+        return p.bias && gi < kPartCols && col < p.n ? __ldg(p.bias + (int64_t)expert * p.ldbias + col) : 0.f;
+      };
+      float bias_next = entry >= 0 && e >= 0 ? bias_of(e, t) : 0.f;
+      while (ok && entry >= 0 && e >= 0) {
+        const uint32_t t_next = t + tile_step;
+        if (gi < kPartCols) bias_s[part_col + gi] = bias_next;
+        const int next = tile_entry<CTAS>(p, t_next, row_tiles);
+        const int e_next = next >= 0 ? __ldg(p.tile_expert + (next >> 1)) : -1;
+        if (e >= p.e_begin && e < p.e_end) {
+          ++it;
+          const int acc = it & 1;
+          const bool valid = rank == 0 || (entry & 1);
+          const int row0 = ((entry >> 1) + rank) * BLOCK_M;
+          const int64_t col0 = (int64_t)(t % p.nt) * BN;
+          const int64_t r = (int64_t)row0 + rloc;
           // a pad row skips the bias, which is the only thing that could make it non-zero
-          const bool live = p.row_token == nullptr || p.row_token[r] >= 0;
-          uint32_t yv[16], ov[16];
+          const bool live = p.bias != nullptr && valid && (p.row_token == nullptr || p.row_token[r] >= 0);
+          if (!accumulator_ready(acc, (uint32_t)(it >> 1) & 1u)) break;
+          tc_fence_after();
+          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
+#pragma unroll 1
+          for (int cc = 0; cc < C::kBlocks; ++cc) {
+            const int cloc = part_col + cc * 32;
+            const int64_t gcol = col0 + cloc;
+            if (gcol >= p.n || !valid) break;  // uniform across the four warps of a group
+            uint8_t* buf = bufs + (OUT == OUT_DACT ? (seq & 1) * C::kStoreBufBytes : 0);
+            if (OUT == OUT_DACT) {
+              // The other staging tile is free once its store has read it and the whole group is past its column sums
+              // (the barrier): the next block's saved pre-activation is requested now and lands during this one.
+              if (cc > 0) group_sync(1 + part);      // the first block's barrier was accumulator_ready's
+              if (leader) {
+                bulk_wait_read<0>();
+                if (!requested) request_aux(seq, gcol, row0);
+                requested = false;
+                if (cc + 1 < C::kBlocks && gcol + 32 < p.n) {
+                  request_aux(seq + 1, gcol + 32, row0);
+                  requested = true;
+                } else if (next >= 0 && (rank == 0 || (next & 1)) && e_next >= p.e_begin && e_next < p.e_end) {
+                  const int64_t col_next = (int64_t)(t_next % p.nt) * BN + part_col;
+                  if (col_next < p.n) {
+                    request_aux(seq + 1, col_next, ((next >> 1) + rank) * BLOCK_M);
+                    requested = true;
+                  }
+                }
+              }
+              __syncwarp();
+              if (!mbar_wait_fast(&aux_full[part * 2 + (seq & 1)], (seq >> 1) & 1u, abort_flag, p.status, 5, p.wait_limit_ns) && lane == 0)
+                group_abort[part] = 1;
+            }
+            const bool two = OUT == OUT_ACT && p.aux != nullptr && !(p.debug & 16);
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            const int64_t hcol = gcol + hf * 16;
-            const int ncols = (int)min((int64_t)16, p.n - hcol);   // <= 0: nothing of this half exists
-            uint32_t v[16];
-            tmem_ld16(t_row + (uint32_t)(cloc + hf * 16), v);      // ESMM tiles always have k-blocks
-            float f[16];
+            for (int hf = 0; hf < 2; ++hf) {
+              uint32_t v[16];
+              tmem_ld16(t_row + (uint32_t)(cloc + hf * 16), v);      // ESMM tiles always have k-blocks
+              float f[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
-            if (p.bias && ncols > 0 && live) {
-              const float* bp = p.bias + (int64_t)tile.e * p.ldbias + hcol;
+              for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(v[i]);
+              if (live) {
+                const float4* bp = reinterpret_cast<const float4*>(bias_s + cloc + hf * 16);
 #pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                if (g * 4 < ncols) {
-                  const float4 bv = __ldg(reinterpret_cast<const float4*>(bp + g * 4));
+                for (int g = 0; g < 4; ++g) {
+                  const float4 bv = bp[g];
                   f[4 * g] += bv.x; f[4 * g + 1] += bv.y; f[4 * g + 2] += bv.z; f[4 * g + 3] += bv.w;
                 }
               }
+              uint32_t x[8], y[8], o[8];
+              if (OUT == OUT_DACT) load_half(buf, rloc, hf, x);      // columns past the end came in as zeros
+              if (p.debug & 8) epi_dispatch16<OUT_LINEAR>(0, is_bf16, f, x, y, o);
+              else epi_dispatch16<OUT>(p.act, is_bf16, f, x, y, o);
+              // registers -> swizzled staging tile(s) -> one TMA store per 128x32 block (full 128-byte lines to L2)
+              if (OUT != OUT_DACT && hf == 0) {      // (DACT writes over its own row of the saved pre-activation)
+                if (leader) bulk_wait_read<0>();     // the previous stores have finished reading the buffers
+                group_sync(1 + part);
+              }
+              stage_half(buf, rloc, hf, o);
+              if (two) stage_half(buf + C::kStoreBufBytes, rloc, hf, y);
             }
-            const uint16_t* xp = p.aux ? reinterpret_cast<const uint16_t*>(p.aux) + r * p.ldaux + hcol : nullptr;
-            uint32_t* yh = yv + hf * 8;
-            uint32_t* oh = ov + hf * 8;
-            // one specialisation per (epilogue, activation, 16-bit flavour): no per-element branches
-#define HEXA_EPI_CASE(E_, A_)                                                                          \
-  case E_ * 8 + A_:                                                                                    \
-    if (is_bf16) epi_values16<E_, A_, 1>(f, xp, ncols, yh, oh);                                        \
-    else epi_values16<E_, A_, 0>(f, xp, ncols, yh, oh);                                                \
-    break;
-            switch ((p.debug & 8) ? 99 : p.epilogue * 8 + p.act) {
-              HEXA_EPI_CASE(HEXA_EPI_ACT, HEXA_ACT_RELU)
-              HEXA_EPI_CASE(HEXA_EPI_ACT, HEXA_ACT_GELU)
-              HEXA_EPI_CASE(HEXA_EPI_ACT, HEXA_ACT_GELU_TANH)
-              HEXA_EPI_CASE(HEXA_EPI_ACT, HEXA_ACT_SILU)
-              HEXA_EPI_CASE(HEXA_EPI_ACT, HEXA_ACT_NONE)
-              HEXA_EPI_CASE(HEXA_EPI_DACT, HEXA_ACT_RELU)
-              HEXA_EPI_CASE(HEXA_EPI_DACT, HEXA_ACT_GELU)
-              HEXA_EPI_CASE(HEXA_EPI_DACT, HEXA_ACT_GELU_TANH)
-              HEXA_EPI_CASE(HEXA_EPI_DACT, HEXA_ACT_SILU)
-              default:
-                if (is_bf16) epi_values16<HEXA_EPI_LINEAR, HEXA_ACT_NONE, 1>(f, xp, ncols, yh, oh);
-                else epi_values16<HEXA_EPI_LINEAR, HEXA_ACT_NONE, 0>(f, xp, ncols, yh, oh);
-                break;
-            }
-#undef HEXA_EPI_CASE
-          }
-          // registers -> swizzled staging tile -> one TMA store per 128x32 block (full 128-byte lines to L2)
-          const bool two = (p.epilogue == HEXA_EPI_ACT) && p.aux != nullptr && !(p.debug & 16);
-          for (int o = (p.debug & 32) ? 2 : (two ? 0 : 1); o < 2; ++o) {
-            if (leader) bulk_wait_read<0>();   // the previous store has finished reading the buffer
-            group_sync(1 + part);
-            stage_row(buf, rloc, o == 0 ? yv : ov);
             fence_async_smem();
             group_sync(1 + part);
-            if (leader) {
-              tma_store_2d(o == 0 ? &tmX : &tmC, buf, (int)gcol, tile.row0);
+            if (OUT == OUT_DACT && group_abort[part]) { ok = false; break; }
+            if (leader && !(p.debug & 32)) {
+              if (two) tma_store_2d(&tmX, buf + C::kStoreBufBytes, (int)gcol, row0);
+              tma_store_2d(&tmC, buf, (int)gcol, row0);
               bulk_commit();
             }
+            ++seq;
+            if (p.colsum != nullptr && !(p.debug & 32)) {
+              // Column sums of the block that now sits in the staging tile (the output as stored).  The warp whose TMEM
+              // quadrant is q takes the 16-byte chunk q of every row: lane = (row mod 8) * 4 + 32-bit word within the
+              // chunk (two columns), 16 rows per lane, then the eight row classes meet through three shuffles.  The eight
+              // rows of one load fall into eight different groups of four banks (rows r, r+1 differ by 64 bytes, rows
+              // r, r+2 by the swizzle): one conflict-free 128-byte wavefront per load.  Nothing else is synchronised:
+              // every thread has finished reading before it arrives at the barrier that precedes the next write of the buffer.
+              const int w4 = lane & 3, ro = lane >> 2;
+              const uint8_t* src = buf + ro * 64 + ((q ^ ((ro >> 1) & 3)) << 4) + w4 * 4;   // (r >> 1) & 3 == (ro >> 1) & 3 for r = 8 i + ro
+              float s0 = 0.f, s1 = 0.f;
+  #pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint32_t v = *reinterpret_cast<const uint32_t*>(src + i * 512);
+                s0 += unpack_lo(v, is_bf16);
+                s1 += unpack_hi(v, is_bf16);
+              }
+  #pragma unroll
+              for (int d = 4; d < 32; d <<= 1) {
+                s0 += __shfl_xor_sync(0xffffffffu, s0, d);
+                s1 += __shfl_xor_sync(0xffffffffu, s1, d);
+              }
+              const int64_t col = gcol + q * 8 + w4 * 2;
+              if (ro == 0 && col < p.n) {
+                float* dst = p.colsum + (int64_t)(row0 / BLOCK_M) * p.n + col;
+                dst[0] = s0;
+                if (col + 1 < p.n) dst[1] = s1;
+              }
+            }
           }
-          if (p.colsum != nullptr && !(p.debug & 32)) {
-            // Column sums of the block that now sits in the staging tile (the output as stored).  The warp whose TMEM
-            // quadrant is q takes the 16-byte chunk q of every row: lane = (row mod 8) * 4 + 32-bit word within the
-            // chunk (two columns), 16 rows per lane, then the eight row classes meet through three shuffles.  The eight
-            // rows of one load fall into eight different groups of four banks (rows r, r+1 differ by 64 bytes, rows
-            // r, r+2 by the swizzle): one conflict-free 128-byte wavefront per load.  Nothing else is synchronised:
-            // every thread has finished reading before it arrives at the barrier that precedes the next write of the buffer.
-            const int w4 = lane & 3, ro = lane >> 2;
-            const uint8_t* src = buf + ro * 64 + ((q ^ ((ro >> 1) & 3)) << 4) + w4 * 4;   // (r >> 1) & 3 == (ro >> 1) & 3 for r = 8 i + ro
-            float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const uint32_t v = *reinterpret_cast<const uint32_t*>(src + i * 512);
-              s0 += unpack_lo(v, is_bf16);
-              s1 += unpack_hi(v, is_bf16);
-            }
-#pragma unroll
-            for (int d = 4; d < 32; d <<= 1) {
-              s0 += __shfl_xor_sync(0xffffffffu, s0, d);
-              s1 += __shfl_xor_sync(0xffffffffu, s1, d);
-            }
-            const int64_t col = gcol + q * 8 + w4 * 2;
-            if (ro == 0 && col < p.n) {
-              float* dst = p.colsum + (int64_t)(tile.row0 / BLOCK_M) * p.n + col;
-              dst[0] = s0;
-              if (col + 1 < p.n) dst[1] = s1;
-            }
-          }
+          if (!ok) break;
+          accumulator_drained(acc);
         }
-      }
-      // accumulator drained: hand it back to the (leader's) MMA warp
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if (CTAS == 2 && rank != 0) mbar_arrive_cluster(map_to_cta(&acc_empty[acc], 0));
-        else mbar_arrive(&acc_empty[acc]);
+        bias_next = next >= 0 && e_next >= 0 ? bias_of(e_next, t_next) : 0.f;
+        t = t_next;
+        entry = next;
+        e = e_next;
       }
     }
     if (leader) bulk_wait_all();   // staging buffers must outlive the stores that read them
@@ -892,13 +1024,13 @@ int make_map(CUtensorMap* tm, const void* base, int is_bf16, int rank, const uin
   return HEXA_OK;
 }
 
-template <int BN, int MODE, int CTAS, int EW>
-int launch_ew(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX, const Params& p,
+template <int BN, int MODE, int CTAS, int OUT>
+int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX, const Params& p,
               int64_t max_tiles, cudaStream_t stream) {
-  using C = Cfg<BN, CTAS, EW, MODE>;
+  using C = Cfg<BN, CTAS, MODE, OUT>;
   static bool attr_set[64] = {false};
   static int max_clusters[64] = {0};
-  auto kernel = gemm_tc_kernel<BN, MODE, CTAS, EW>;
+  auto kernel = gemm_tc_kernel<BN, MODE, CTAS, OUT>;
   int dev = 0;
   HEXA_CUDA(cudaGetDevice(&dev));
   HEXA_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
@@ -932,7 +1064,7 @@ int launch_ew(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap&
   }
   cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tmA, tmB, tmC, tmX, p);
   if (e != cudaSuccess) {
-    set_error("launch of gemm_tc_kernel<%d,%d,%d,%d> failed: %s", BN, MODE, CTAS, EW, cudaGetErrorString(e));
+    set_error("launch of gemm_tc_kernel<%d,%d,%d,%d> failed: %s", BN, MODE, CTAS, OUT, cudaGetErrorString(e));
     return HEXA_ERR_CUDA;
   }
   return HEXA_OK;
@@ -943,22 +1075,12 @@ int env_int(const char* name, int dflt) {
   return s ? atoi(s) : dflt;
 }
 
-// Epilogue warps of a launch: HEXA_TC_EPI_WARPS (8 or 16, read at every launch so that one process can compare the two)
-// or, by default, 8 for long k-loops and 16 for short ones, where the epilogue of a tile has to keep pace with few MMAs.
-int epi_warps_for(int64_t num_kb_typical) {
-  const int forced = env_int("HEXA_TC_EPI_WARPS", 0);
-  if (forced == 4 || forced == 8 || forced == 16) return forced;
-  const int64_t threshold = env_int("HEXA_TC_EPI_WARPS_KB", 0);     // 0: always 16 (the faster setting at K = 768 and, for the
-                                                                     // launches with an activation, at K = 2048 as well)
-  return (threshold > 0 && num_kb_typical >= threshold) ? 8 : 16;
-}
-
 template <int BN, int MODE, int CTAS>
-int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX, const Params& p,
-           int64_t max_tiles, cudaStream_t stream, int epi_warps) {
-  if (epi_warps == 4) return launch_ew<BN, MODE, CTAS, 4>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
-  if (epi_warps == 8) return launch_ew<BN, MODE, CTAS, 8>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
-  return launch_ew<BN, MODE, CTAS, 16>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
+int launch_esmm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmX, const Params& p,
+                int64_t max_tiles, cudaStream_t stream) {
+  if (p.epilogue == HEXA_EPI_ACT) return launch<BN, MODE, CTAS, OUT_ACT>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
+  if (p.epilogue == HEXA_EPI_DACT) return launch<BN, MODE, CTAS, OUT_DACT>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
+  return launch<BN, MODE, CTAS, OUT_LINEAR>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
 }
 // HEXA_TC_CTAS=1 keeps every GEMM on single-CTA tiles (for A/B measurements); default: CTA pairs where they apply.
 bool pairs_enabled() { static int v = -1; if (v < 0) v = env_int("HEXA_TC_CTAS", 2) == 1 ? 0 : 1; return v == 1; }
@@ -1018,7 +1140,7 @@ int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int6
     int rc = make_map(&tmC, c, is_bf16, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
     if (rc) return rc;
     tmX = tmC;
-    if (aux && epilogue == HEXA_EPI_ACT) {
+    if (aux && epilogue != HEXA_EPI_LINEAR) {
       uint64_t strx[1] = {(uint64_t)ldaux * 2};
       rc = make_map(&tmX, aux, is_bf16, 2, dims, strx, box, CU_TENSOR_MAP_SWIZZLE_64B);
       if (rc) return rc;
@@ -1034,18 +1156,17 @@ int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int6
   const int64_t NT = ceil_div(n_out, BN);
   HEXA_REQUIRE((row_cap / BLOCK_M + E + 1) * NT < (int64_t)0x7fffffff, "hexa_esmm: too many output tiles for a 32-bit tile index");
   p.nt = (uint32_t)NT;
-  const int ew = epi_warps_for(ceil_div(k, BLOCK_K));
   if (ctas == 2) {
     const int64_t max_tiles = p.max_pairs * NT;
-    return b_layout == HEXA_B_NK ? launch<256, ESMM_NK, 2>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew)
-                                 : launch<256, ESMM_KN, 2>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew);
+    return b_layout == HEXA_B_NK ? launch_esmm<256, ESMM_NK, 2>(tmA, tmB, tmC, tmX, p, max_tiles, stream)
+                                 : launch_esmm<256, ESMM_KN, 2>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
   }
   const int64_t max_tiles = (row_cap / BLOCK_M) * NT;
   if (b_layout == HEXA_B_NK)
-    return BN == 256 ? launch<256, ESMM_NK, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew)
-                     : launch<128, ESMM_NK, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew);
-  return BN == 256 ? launch<256, ESMM_KN, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew)
-                   : launch<128, ESMM_KN, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream, ew);
+    return BN == 256 ? launch_esmm<256, ESMM_NK, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream)
+                     : launch_esmm<128, ESMM_NK, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
+  return BN == 256 ? launch_esmm<256, ESMM_KN, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream)
+                   : launch_esmm<128, ESMM_KN, 1>(tmA, tmB, tmC, tmX, p, max_tiles, stream);
 }
 
 bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, const void* out, int64_t ldo,
@@ -1124,12 +1245,22 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   p.nt = (uint32_t)ceil_div(n, BN);
   p.per_expert = (uint32_t)(ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN) * splits);
   p.total_tiles = (uint32_t)max_tiles;
-  // ESTMM stores straight from registers; the two output maps are unused placeholders
   int rc;
-  const int ew = epi_warps_for(row_cap / BLOCK_K / (E * (int64_t)splits));
-  if (ctas == 2) rc = launch<256, ESTMM, 2>(tmA, tmB, tmA, tmA, p, max_tiles, stream, ew);
-  else rc = BN == 256 ? launch<256, ESTMM, 1>(tmA, tmB, tmA, tmA, p, max_tiles, stream, ew)
-                      : launch<128, ESTMM, 1>(tmA, tmB, tmA, tmA, p, max_tiles, stream, ew);
+  const bool staged = n_split == 0 && m_split >= m && !beta && !p.out_f32 && splits == 1;
+  CUtensorMap tmC = tmA;      // a placeholder for register stores
+  if (staged) {
+    uint64_t dims[3] = {(uint64_t)n, (uint64_t)m, (uint64_t)E};
+    uint64_t str[2] = {(uint64_t)ldo * 2, (uint64_t)o_estride * 2};
+    uint32_t box[3] = {32, BLOCK_M, 1};
+    rc = make_map(&tmC, out, is_bf16, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc) return rc;
+    if (ctas == 2) return launch<256, ESTMM, 2, OUT_STAGED>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+    return BN == 256 ? launch<256, ESTMM, 1, OUT_STAGED>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
+                     : launch<128, ESTMM, 1, OUT_STAGED>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+  }
+  if (ctas == 2) rc = launch<256, ESTMM, 2, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+  else rc = BN == 256 ? launch<256, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
+                      : launch<128, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
   if (rc != HEXA_OK || splits == 1) return rc;
   const int64_t total = (int64_t)E * m * (n / 4);
   int64_t blocks = ceil_div(total, 256);
