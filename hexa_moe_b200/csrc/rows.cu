@@ -3,7 +3,9 @@
 // Bytes per unit (what the roofline of these kernels is computed from):
 //   gather   reads cols*size per real row, writes cols*size per padded row, 4 B of row_token per row
 //   combine  reads top_k*cols*size and writes cols*size per token, 4*top_k B of token_row
-//   ESS      reads cols*size per padded row once; partials add 4*cols B per 128 rows (write + read)
+//   ESS      reads cols*size per padded row once; partials add 4*cols B per 128 rows (write + read).  The gather that
+//            makes the rows can sum them on the way (hexa_gather_rows_ess): then only the partials are read.  [262144, 2048]
+//            bf16 by token: gather 318 + first pass 193 us apart, 392 us together.
 #include "hexa_common.cuh"
 
 namespace hexa {
@@ -136,31 +138,49 @@ __global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes
 }
 
 // ---- ESS pass 1: column sums of one 128-row tile (one expert) ------------------------------------
-// block = 64 column groups x 4 row groups; a thread sums 32 rows of V adjacent columns.
-template <typename T>
-__global__ void __launch_bounds__(256)
-ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ pad_offsets, int E,
-                   int64_t cols, float* __restrict__ partial) {
+// block = 32 column groups x 8 row groups; a thread sums 16 rows of V adjacent columns, eight loads in flight.
+// GATHER: the rows come from src[row_token[row]] (zeros for pad rows) and are written to dst as well.
+constexpr int kEssCx = 32, kEssRy = 8;
+template <typename T, bool GATHER>
+__global__ void __launch_bounds__(kEssCx * kEssRy)
+ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ row_token,
+                   const int32_t* __restrict__ pad_offsets, int E, int64_t cols, T* __restrict__ dst, int64_t dst_ld,
+                   float* __restrict__ partial) {
   constexpr int V = 16 / sizeof(T);
-  __shared__ float red[4][64 * V];
+  __shared__ float red[kEssRy][kEssCx * V];
+  __shared__ int32_t tok_s[kRowTile];
   const int64_t n_pad = pad_offsets[E];
   const int64_t row0 = (int64_t)blockIdx.y * kRowTile;
   if (row0 >= n_pad) return;
-  const int cx = threadIdx.x & 63, ry = threadIdx.x >> 6;
-  const int64_t col = ((int64_t)blockIdx.x * 64 + cx) * V;
+  if (GATHER) {
+    if (threadIdx.x < kRowTile) tok_s[threadIdx.x] = __ldg(row_token + row0 + threadIdx.x);
+    __syncthreads();
+  }
+  const int cx = threadIdx.x & (kEssCx - 1), ry = threadIdx.x / kEssCx;
+  const int64_t col = ((int64_t)blockIdx.x * kEssCx + cx) * V;
   float acc[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) acc[i] = 0.f;
   if (col < cols) {
-    const bool vec_ok = (col + V <= cols) && (src_ld % V == 0);
-    for (int r = ry; r < kRowTile; r += 4) {
-      const T* p = src + (row0 + r) * src_ld + col;
-      if (vec_ok) {
-        uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
+    const bool vec_ok = GATHER || ((col + V <= cols) && (src_ld % V == 0));      // GATHER: checked by the host
+    if (vec_ok) {
+#pragma unroll 8
+      for (int r = ry; r < kRowTile; r += kEssRy) {
+        uint4 raw = make_uint4(0, 0, 0, 0);
+        if (GATHER) {
+          const int32_t tok = tok_s[r];
+          if (tok >= 0) raw = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)tok * src_ld + col));
+          *reinterpret_cast<uint4*>(dst + (row0 + r) * dst_ld + col) = raw;
+        } else {
+          raw = __ldg(reinterpret_cast<const uint4*>(src + (row0 + r) * src_ld + col));
+        }
         const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] += to_f32<T>(v[i]);
-      } else {
+      }
+    } else {
+      for (int r = ry; r < kRowTile; r += kEssRy) {
+        const T* p = src + (row0 + r) * src_ld + col;
 #pragma unroll
         for (int i = 0; i < V; ++i)
           if (col + i < cols) acc[i] += to_f32<T>(p[i]);
@@ -170,27 +190,40 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
 #pragma unroll
   for (int i = 0; i < V; ++i) red[ry][cx * V + i] = acc[i];
   __syncthreads();
-  if (ry == 0 && col < cols) {
+  for (int c = threadIdx.x; c < kEssCx * V; c += kEssCx * kEssRy) {
+    const int64_t gc = (int64_t)blockIdx.x * kEssCx * V + c;
+    if (gc >= cols) continue;
+    float s = red[0][c];
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      if (col + i < cols) {
-        float s = red[0][cx * V + i] + red[1][cx * V + i] + red[2][cx * V + i] + red[3][cx * V + i];
-        partial[(int64_t)blockIdx.y * cols + col + i] = s;
-      }
-    }
+    for (int y = 1; y < kEssRy; ++y) s += red[y][c];
+    partial[(int64_t)blockIdx.y * cols + gc] = s;
   }
 }
 
-// ---- ESS pass 2: per expert, add its tiles' partial rows in ascending order ---------------------
-__global__ void ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
-                                 int64_t cols, float* __restrict__ out, int64_t ldo) {
+// ---- ESS pass 2: per expert, add its tiles' partial rows -----------------------------------------
+// 32 columns x 8 slices of the tiles per block, each slice in ascending order, then the slices in order: an expert with
+// 144 tiles is 18 dependent additions deep (one thread per column walked all of them: 13 us for [18432, 512] and its
+// hidden gradient, 5 us now).
+__global__ void __launch_bounds__(256)
+ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
+                 int64_t cols, float* __restrict__ out, int64_t ldo) {
+  __shared__ float red[8][32];
   const int e = blockIdx.y;
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+  const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int64_t c = (int64_t)blockIdx.x * 32 + cx;
   const int64_t t0 = pad_offsets[e] / kRowTile, t1 = pad_offsets[e + 1] / kRowTile;
   float s = 0.f;
-  for (int64_t t = t0; t < t1; ++t) s += partial[t * cols + c];
-  out[(int64_t)e * ldo + c] = s;
+  if (c < cols) {
+#pragma unroll 8
+    for (int64_t t = t0 + slice; t < t1; t += 8) s += __ldg(partial + t * cols + c);
+  }
+  red[slice][cx] = s;
+  __syncthreads();
+  if (slice == 0 && c < cols) {
+#pragma unroll
+    for (int y = 1; y < 8; ++y) s += red[y][cx];
+    out[(int64_t)e * ldo + c] = s;
+  }
 }
 
 }  // namespace
@@ -267,26 +300,64 @@ int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int 
   const int64_t tiles = ceil_div(row_cap, kRowTile);
   if (tiles > 0) {
     const int V = 16 / (int)dtype_size(dtype);
-    dim3 grid((unsigned)ceil_div(cols, 64 * V), (unsigned)tiles);
+    dim3 grid((unsigned)ceil_div(cols, kEssCx * V), (unsigned)tiles);
     HEXA_REQUIRE(tiles <= 65535, "hexa_ess: more than 65535 row tiles (row_capacity %lld)", (long long)row_cap);
+#define HEXA_ESS(T)                                                                                                          \
+  ess_partial_kernel<T, false><<<grid, kEssCx * kEssRy, 0, stream>>>((const T*)src, src_ld, nullptr, pad_offsets, E, cols, nullptr, 0, partial)
     switch (dtype) {
-      case HEXA_F32: ess_partial_kernel<float><<<grid, 256, 0, stream>>>((const float*)src, src_ld, pad_offsets, E, cols, partial); break;
-      case HEXA_F16: ess_partial_kernel<__half><<<grid, 256, 0, stream>>>((const __half*)src, src_ld, pad_offsets, E, cols, partial); break;
-      case HEXA_BF16: ess_partial_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)src, src_ld, pad_offsets, E, cols, partial); break;
+      case HEXA_F32: HEXA_ESS(float); break;
+      case HEXA_F16: HEXA_ESS(__half); break;
+      case HEXA_BF16: HEXA_ESS(__nv_bfloat16); break;
       default: HEXA_REQUIRE(false, "hexa_ess: bad dtype %d", dtype);
     }
+#undef HEXA_ESS
     HEXA_LAUNCH_CHECK("ess_partial");
   }
   return ess_finish(partial, pad_offsets, E, cols, out, ldo, stream);
 }
 
 int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, float* out, int64_t ldo, cudaStream_t stream) {
-  dim3 grid2((unsigned)ceil_div(cols, 256), (unsigned)E);
+  dim3 grid2((unsigned)ceil_div(cols, 32), (unsigned)E);
   ess_final_kernel<<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, out, ldo);
   HEXA_LAUNCH_CHECK("ess_final");
   return HEXA_OK;
 }
 }  // namespace hexa
+
+extern "C" int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32_t* row_token, const int32_t* pad_offsets,
+                                    int E, int64_t row_cap, int64_t cols, void* dst, int64_t dst_ld, float* sums,
+                                    int64_t ld_sums, int dtype, void* workspace, size_t workspace_bytes, void* stream_) {
+  cudaStream_t stream = (cudaStream_t)stream_;
+  HEXA_REQUIRE(row_token && pad_offsets && dst && sums && workspace, "hexa_gather_rows_ess: null pointer");
+  HEXA_REQUIRE(E > 0 && E <= 65535 && row_cap >= 0 && cols > 0 && src_ld >= cols && dst_ld >= cols && ld_sums >= cols,
+               "hexa_gather_rows_ess: bad sizes");
+  HEXA_REQUIRE(dtype == HEXA_F32 || dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gather_rows_ess: bad dtype %d", dtype);
+  HEXA_REQUIRE(aligned16(dst), "hexa_gather_rows_ess: dst must be 16-byte aligned");
+  const size_t need = hexa_ess_workspace_bytes(row_cap, cols);
+  if (workspace_bytes < need) {
+    set_error("hexa_gather_rows_ess: workspace %zu bytes < required %zu", workspace_bytes, need);
+    return HEXA_ERR_WORKSPACE;
+  }
+  const int64_t tiles = ceil_div(row_cap, kRowTile), V = 16 / (int64_t)dtype_size(dtype);
+  // one pass where every row is whole 16-byte groups on both sides; otherwise the two operators one after the other
+  const bool one = tiles > 0 && row_cap % kRowTile == 0 && tiles <= 65535 && cols % V == 0 && src_ld % V == 0 && dst_ld % V == 0 &&
+                   aligned16(src);
+  if (!one) {
+    const int rc = hexa_gather_rows(src, src_ld, row_token, pad_offsets, E, row_cap, cols, dst, dst_ld, dtype, stream_);
+    if (rc != HEXA_OK) return rc;
+    return ess_launch(dst, dst_ld, pad_offsets, E, row_cap, cols, sums, ld_sums, dtype, (float*)workspace, stream);
+  }
+  dim3 grid((unsigned)ceil_div(cols, kEssCx * V), (unsigned)tiles);
+#define HEXA_GATHER_ESS(T)                                                                                                   \
+  ess_partial_kernel<T, true><<<grid, kEssCx * kEssRy, 0, stream>>>((const T*)src, src_ld, row_token, pad_offsets, E, cols, (T*)dst, \
+                                                                    dst_ld, (float*)workspace)
+  if (dtype == HEXA_F32) HEXA_GATHER_ESS(float);
+  else if (dtype == HEXA_F16) HEXA_GATHER_ESS(__half);
+  else HEXA_GATHER_ESS(__nv_bfloat16);
+#undef HEXA_GATHER_ESS
+  HEXA_LAUNCH_CHECK("gather_rows_ess");
+  return ess_finish((const float*)workspace, pad_offsets, E, cols, sums, ld_sums, stream);
+}
 
 extern "C" int hexa_ess(const void* src, int64_t src_ld, const int32_t* pad_offsets, int E, int64_t row_cap,
                         int64_t cols, float* out, int64_t ldo, int dtype, void* workspace, size_t workspace_bytes,

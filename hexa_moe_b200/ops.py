@@ -124,6 +124,23 @@ def gather_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = Non
     return out
 
 
+def gather_rows_ess(src: torch.Tensor, r: Routing):
+    """(gather_rows(src), ess of the result) from one pass over the rows."""
+    global LAUNCHES
+    if r.align % L.ROW_TILE:
+        raise L.HexaError("gather_rows_ess: routing must be aligned to 128 rows")
+    cols = src.shape[1]
+    out = sorted_buffer(r.row_capacity, cols, src.dtype, src.device)
+    sums = torch.empty(r.num_experts, cols, dtype=torch.float32, device=src.device)
+    ws = torch.empty(max(lib().hexa_ess_workspace_bytes(r.row_capacity, cols), 4), dtype=torch.uint8, device=src.device)
+    with _Timed("gather", 2.0 * r.num_tokens * r.top_k * cols * src.element_size()):
+        check(lib().hexa_gather_rows_ess(ptr(src), _ld(src), ptr(r.row_token), ptr(r.pad_offsets), r.num_experts, r.row_capacity,
+                                         cols, ptr(out), _ld(out), ptr(sums), _ld(sums), dt(src), ptr(ws), ws.numel(),
+                                         stream_of(src)), "hexa_gather_rows_ess")
+    LAUNCHES += 1          # the second pass of ESS over the tile sums
+    return out, sums
+
+
 def combine_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Sorted rows -> token order with the unweighted sum over the k routes."""
     cols = src.shape[1]
@@ -463,8 +480,7 @@ def moe_backward_fc2(st: LayerState, dy, w2, act_id: int, has_b2=True, grad_dtyp
     Split from the fc1 half so a caller can start reducing dw2/db2 across ranks while fc1 runs.  want_db1: the fc1
     half will need the bias gradient ESS(dh); with a fused activation the GEMM that writes dh sums it on the way."""
     r = st.routing
-    dys = gather_rows(dy.contiguous(), r)
-    db2 = ess(dys, r) if has_b2 else None
+    dys, db2 = gather_rows_ess(dy.contiguous(), r) if has_b2 else (gather_rows(dy.contiguous(), r), None)
     dw2 = estmm(st.h, dys, r, out_dtype=grad_dtype, engine=engine, ranks=ranks, out=dw_out, tag="dw2")
     if act_id >= 0:
         dh = _hidden_gradient(st, dys, w2, act_id, engine, want_db1)
@@ -583,8 +599,12 @@ def dense_backward(st: LayerState, dy, w1, w2, act_id: int, has_b1=True, has_b2=
     bias gradients are float32."""
     r = st.routing
     T = r.num_tokens
-    dys = _dense_rows(dy, r)
-    db2 = ess(dys, r).view(-1) if has_b2 else None
+    if has_b2 and dy.shape[0] != r.row_capacity:
+        dys, db2 = gather_rows_ess(dy.contiguous(), r)
+    else:
+        dys = _dense_rows(dy, r)
+        db2 = ess(dys, r) if has_b2 else None
+    db2 = None if db2 is None else db2.view(-1)
     dw2 = estmm(st.h, dys, r, out_dtype=grad_dtype, engine=engine)[0]
     dh = _hidden_gradient(st, dys, w2.unsqueeze(0), act_id, engine, has_b1)
     db1 = (st.db1 if st.db1 is not None else ess(dh, r)).view(-1) if has_b1 else None

@@ -137,6 +137,13 @@ int hexa_gather_rows(const void* src, int64_t src_ld, const int32_t* row_token, 
                      int num_experts, int64_t row_capacity, int64_t cols, void* dst, int64_t dst_ld,
                      int dtype, void* stream);
 
+/* hexa_gather_rows and hexa_ess of its result in one pass over the rows: sums[e,:] (fp32 [E, cols], ld_sums) = sum of
+ * expert e's rows of dst, the same additions in the same order as hexa_ess(dst).  Needs segments aligned to 128 rows;
+ * workspace: hexa_ess_workspace_bytes(row_capacity, cols) bytes, contents irrelevant. */
+int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32_t* row_token, const int32_t* pad_offsets,
+                         int num_experts, int64_t row_capacity, int64_t cols, void* dst, int64_t dst_ld, float* sums,
+                         int64_t ld_sums, int dtype, void* workspace, size_t workspace_bytes, void* stream);
+
 /* dst[t,:] = sum_j src[token_row[t*top_k + j],:] (fp32 accumulation, fixed order j = 0..k-1). */
 int hexa_combine_rows(const void* src, int64_t src_ld, const int32_t* token_row, int64_t num_tokens,
                       int top_k, int64_t cols, void* dst, int64_t dst_ld, int dtype, void* stream);

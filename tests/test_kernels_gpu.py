@@ -525,3 +525,23 @@ def test_route_launch_forms(ops, T, k, E, launches, align):
         if align == 128:
             pb, n = r.pair_block.cpu(), want["pair_block"].numel()
             assert torch.equal(pb[:n], want["pair_block"]) and (pb[n:] == -1).all()
+
+
+# Gather with column sums: whole and ragged 16-byte groups, more columns than one block's, empty experts, a row pitch.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,cols", [(1, 8), (777, 264), (700, 203), (5000, 1032)])
+def test_gather_with_sums_is_gather_then_ess(ops, dtype, T, cols):
+    E, k = 6, 2
+    ids = make_ids(T, k, E, 3, skew=True, empty=(2,))
+    r = ops.route(ids.cuda(), E)
+    x = torch.randn(T, cols + 8, generator=torch.Generator().manual_seed(T)).to(dtype).cuda()[:, :cols]
+    n_pad = int(r.pad_offsets[-1])
+    rows, sums = ops.gather_rows_ess(x, r)
+    want = ops.gather_rows(x, r)
+    assert torch.equal(rows[:n_pad], want[:n_pad])
+    assert torch.equal(sums, ops.ess(want, r))
+    # n additions of fp32 stay within n * 2^-24 of the sum of magnitudes
+    for e in range(E):
+        tok = r.row_token[r.pad_offsets[e]: r.pad_offsets[e + 1]].long()
+        seg = x[tok[tok >= 0]].double()
+        assert ((sums[e].double() - seg.sum(0)).abs() <= seg.abs().sum(0) * (len(seg) * 2.0 ** -24) + 1e-30).all()
