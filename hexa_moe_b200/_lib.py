@@ -70,6 +70,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_host = None
 
 
 class HexaError(RuntimeError):
@@ -92,6 +93,23 @@ def lib():
                     fn.restype, fn.argtypes = res, args
                 _lib = handle
     return _lib
+
+
+def host():
+    """The native wrapper module (csrc/host.cpp), bound to the library once.  Fails loudly if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        with _lock:
+            if _host is None:
+                try:
+                    from . import _host as module
+                except ImportError as e:
+                    raise HexaError(f"hexa_moe_b200/_host.so cannot be loaded ({e}): build it with "
+                                    "`python -m hexa_moe_b200.build` (there is no fallback path)")
+                module.bind(LIB_PATH, HexaError, ensure_status_word, _STATUS_CODES)
+                _host = module
+    return _host
 
 
 ERR_DEVICE = -5
@@ -163,4 +181,4 @@ def stream_of(t: torch.Tensor) -> int:
     idx = t.device.index
     if idx not in _status_words:
         ensure_status_word(torch.cuda.current_device() if idx is None else idx)
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if idx is None else idx)

@@ -1,0 +1,318 @@
+// Native side of the operator wrappers in ops.py: output and scratch allocation, pointer / stride / dtype plumbing, the
+// current stream, error translation - everything between a Python call and the C ABI of include/hexa_moe_b200.h.
+//
+// Why: a layer step is ~20 launches of a few microseconds each at small sizes, and a wrapper that collects two dozen
+// pointers, strides and sizes in Python and hands them to ctypes cost ~20 us per operator.  Here it is one call:
+// 16 tokens forward 370 -> 204 us, the README layer's step 941 -> 593 us, 4608 tokens x 32 experts 1037 -> 709 us.
+// The C ABI is bound at run time from the library that _lib.py has loaded (bind()), so this module links against torch only.
+// The interpreter lock is released around every library call: a launch can block on a full queue, and the thread that
+// would resolve the stall may need the lock.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/hexa_moe_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+struct Api {
+#define HEXA_API(X)                                                                                                            \
+  X(hexa_last_error_string) X(hexa_pending_device_status) X(hexa_route_row_capacity) X(hexa_route_workspace_bytes)             \
+  X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
+  X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
+  X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
+  X(hexa_gate_split_terms) X(hexa_gate_sum_terms)
+#define HEXA_FIELD(name) decltype(&::name) name = nullptr;
+  HEXA_API(HEXA_FIELD)
+} api;
+
+struct Bound {      // what _lib.py hands over; lives as long as the process (nothing to release after the interpreter)
+  py::object error, ensure_status_word;
+  py::dict status_text;
+};
+Bound* bound = nullptr;
+bool status_installed[64] = {false};
+
+[[noreturn]] void fail(const std::string& message) {
+  PyErr_SetString(bound->error.ptr(), message.c_str());
+  throw py::error_already_set();
+}
+
+// Raise on a non-zero return code, and on a code that a kernel launched earlier left in the device's status word.
+void check(int rc, const char* what) {
+  if (rc != 0) fail(std::string(what) + " failed (" + std::to_string(rc) + "): " + api.hexa_last_error_string());
+  const int code = api.hexa_pending_device_status();
+  if (code != 0) {
+    const py::int_ key(code);
+    const std::string text = bound->status_text.contains(key) ? bound->status_text[key].cast<std::string>() : "unknown";
+    fail(std::string(what) + ": a kernel on this device gave up a bounded wait (status code " + std::to_string(code) + ": " + text +
+         "); results since then are incomplete (" + std::to_string(HEXA_ERR_DEVICE) + ")");
+  }
+}
+
+template <typename F> void call(const char* what, F&& f) {
+  int rc;
+  {
+    py::gil_scoped_release nogil;
+    rc = f();
+  }
+  check(rc, what);
+}
+
+void* stream_of(const Tensor& t) {
+  if (!t.is_cuda()) fail("hexa_moe_b200 operators run on CUDA tensors only (no CPU path)");
+  const int dev = t.get_device();
+  if (dev < 0 || dev >= 64 || !status_installed[dev]) {
+    bound->ensure_status_word(dev);
+    if (dev >= 0 && dev < 64) status_installed[dev] = true;
+  }
+  return c10::cuda::getCurrentCUDAStream(dev).stream();
+}
+
+int dt(const Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kFloat: return HEXA_F32;
+    case at::kHalf: return HEXA_F16;
+    case at::kBFloat16: return HEXA_BF16;
+    default: fail(std::string("unsupported dtype ") + c10::toString(t.scalar_type()));
+  }
+}
+
+int64_t ld(const Tensor& t) {
+  if (t.dim() != 2 || t.stride(1) != 1) fail("expected a 2-D tensor with unit inner stride");
+  return t.stride(0);
+}
+
+void* ptr(const Tensor& t) { return t.data_ptr(); }
+void* ptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
+const int32_t* i32(const Tensor& t) { return static_cast<const int32_t*>(t.data_ptr()); }
+const int32_t* i32(const OptTensor& t) { return t.has_value() ? i32(*t) : nullptr; }
+
+Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
+  return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+}
+Tensor scratch(size_t bytes, const Tensor& like) { return empty({(int64_t)(bytes < 4 ? 4 : bytes)}, at::kByte, like); }
+
+// [rows, cols] whose row pitch is a multiple of 8 elements (16 bytes of 16-bit data), as the TMA-fed GEMMs need
+Tensor sorted_buffer(int64_t rows, int64_t cols, at::ScalarType type, const Tensor& like) {
+  const int64_t pitch = (cols + 7) / 8 * 8;
+  Tensor t = empty({rows, pitch}, type, like);
+  return pitch == cols ? t : t.narrow(1, 0, cols);
+}
+
+// (counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block | None, T, k, row_capacity, launches)
+py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
+  if (ids.scalar_type() != at::kInt) fail("route: ids must be int32");
+  if (ids.dim() != 2) fail("route: ids must be 2-D");
+  const int dt_ = route_major ? 1 : 0;
+  const int64_t T = ids.size(dt_), k = ids.size(1 - dt_), st = ids.stride(dt_), sk = ids.stride(1 - dt_);
+  void* s = stream_of(ids);
+  const int64_t cap = api.hexa_route_row_capacity(T, (int)k, E, align);
+  if (cap < 0) fail("route: bad sizes");
+  auto ints = [&](int64_t n) { return empty({n < 1 ? 1 : n}, at::kInt, ids); };
+  OptTensor pairs;
+  if (align == 128) pairs = ints(api.hexa_route_pair_capacity(T, (int)k, E));
+  Tensor counts = ints(E), seg = ints(E + 1), pad = ints(E + 1), row_token = ints(cap), token_row = ints(T * k), tiles = ints(cap / align);
+  Tensor ws = scratch(api.hexa_route_workspace_bytes(T, (int)k, E), ids);
+  auto out = [](const Tensor& t) { return static_cast<int32_t*>(t.data_ptr()); };
+  call("hexa_route", [&] {
+    return api.hexa_route(i32(ids), T, (int)k, st, sk, E, align, out(counts), out(seg), out(pad), out(row_token), out(token_row),
+                          out(tiles), pairs ? out(*pairs) : nullptr, ptr(ws), (size_t)ws.numel(), s);
+  });
+  return py::make_tuple(counts, seg, pad, row_token, token_row, tiles, pairs, T, k, cap, api.hexa_route_launches(T, (int)k, E));
+}
+
+Tensor gather_rows(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
+  const int64_t cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = out_ ? *out_ : sorted_buffer(cap, cols, src.scalar_type(), src);
+  const int type = dt(src);
+  const int64_t lds = ld(src), ldo = ld(out);
+  call("hexa_gather_rows", [&] { return api.hexa_gather_rows(ptr(src), lds, i32(row_token), i32(pad_offsets), E, cap, cols, ptr(out), ldo, type, s); });
+  return out;
+}
+
+std::tuple<Tensor, Tensor> gather_rows_ess(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap) {
+  const int64_t cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = sorted_buffer(cap, cols, src.scalar_type(), src), sums = empty({E, cols}, at::kFloat, src);
+  Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
+  const int type = dt(src);
+  const int64_t lds = ld(src), ldo = ld(out);
+  call("hexa_gather_rows_ess", [&] {
+    return api.hexa_gather_rows_ess(ptr(src), lds, i32(row_token), i32(pad_offsets), E, cap, cols, ptr(out), ldo,
+                                    static_cast<float*>(ptr(sums)), cols, type, ptr(ws), (size_t)ws.numel(), s);
+  });
+  return {out, sums};
+}
+
+Tensor combine_rows(const Tensor& src, const Tensor& token_row, int64_t T, int top_k, const OptTensor& out_) {
+  const int64_t cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = out_ ? *out_ : empty({T, cols}, src.scalar_type(), src);
+  const int type = dt(src);
+  const int64_t lds = ld(src), ldo = ld(out);
+  call("hexa_combine_rows", [&] { return api.hexa_combine_rows(ptr(src), lds, i32(token_row), T, top_k, cols, ptr(out), ldo, type, s); });
+  return out;
+}
+
+Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_expert, const Tensor& pad_offsets, const Tensor& row_token,
+            const OptTensor& pair_block, int E, int64_t cap, const OptTensor& bias, int epilogue, int act, const OptTensor& aux,
+            const OptTensor& out_, int engine, int64_t n_out, int64_t k, int e0, int e1, const OptTensor& sums) {
+  if (a.scalar_type() != b.scalar_type())
+    fail(std::string("esmm: a is ") + c10::toString(a.scalar_type()) + " but b is " + c10::toString(b.scalar_type()));
+  if (bias && bias->scalar_type() != at::kFloat) fail("esmm: bias must be float32");
+  if (sums && (e0 != 0 || e1 != E || sums->scalar_type() != at::kFloat || sums->dim() != 2 || sums->size(0) != E || sums->size(1) != n_out ||
+               sums->stride(1) != 1))
+    fail("esmm: sums must be float32 [E, n_out] and needs the full expert range");
+  void* s = stream_of(a);
+  const int type = dt(a);
+  Tensor out = out_ ? *out_ : sorted_buffer(cap, n_out, a.scalar_type(), a);
+  const int64_t lda = ld(a), ldo = ld(out), ldbias = bias ? ld(*bias) : 0, ldaux = aux ? ld(*aux) : 0;
+  const float* bp = static_cast<const float*>(ptr(bias));
+  if (sums) {
+    Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, n_out), a);
+    call("hexa_esmm_ess", [&] {
+      return api.hexa_esmm_ess(ptr(a), lda, ptr(b), b_layout, b.stride(1), b.stride(0), bp, ldbias, ptr(aux), ldaux, ptr(out), ldo,
+                               i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, type, epilogue, act,
+                               engine, static_cast<float*>(ptr(sums)), sums->stride(0), ptr(ws), (size_t)ws.numel(), s);
+    });
+    return out;
+  }
+  call("hexa_esmm", [&] {
+    return api.hexa_esmm_experts(ptr(a), lda, ptr(b), b_layout, b.stride(1), b.stride(0), bp, ldbias, ptr(aux), ldaux, ptr(out), ldo,
+                                 i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, type, epilogue,
+                                 act, engine, e0, e1, s);
+  });
+  return out;
+}
+
+// out given: its strides say where results go ([E, m, n], or [ranks, E, m / ranks, n] with ranks > 1)
+Tensor estmm(const Tensor& p, const Tensor& q, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_,
+             std::optional<at::ScalarType> out_dtype, int beta, int engine, int64_t ranks) {
+  const int64_t m = p.size(1), n = q.size(1);
+  if (p.scalar_type() != q.scalar_type()) fail("estmm: p and q dtypes differ");
+  const at::ScalarType type = out_dtype.value_or(p.scalar_type());
+  Tensor out;
+  int64_t ldo, estride, m_split = 0, split_stride = 0;
+  if (ranks > 1) {
+    if (m % ranks) fail("estmm: the row count must be divisible by ranks");
+    out = out_ ? *out_ : empty({ranks, E, m / ranks, n}, type, p);
+    ldo = out.stride(2); estride = out.stride(1); m_split = m / ranks; split_stride = out.stride(0);
+  } else {
+    if (!out_ && beta) fail("estmm: beta=1 needs an existing out");
+    out = out_ ? *out_ : empty({E, m, n}, type, p);
+    ldo = out.stride(1); estride = out.stride(0);
+  }
+  if (out.stride(-1) != 1) fail("estmm: out must have unit inner stride");
+  void* s = stream_of(p);
+  const int in_type = dt(p), o_type = dt(out);
+  const int64_t ldp = ld(p), ldq = ld(q);
+  const size_t bytes = engine != HEXA_ENGINE_SIMT ? api.hexa_estmm_workspace_bytes(E, cap, m, n, in_type) : 0;
+  OptTensor ws;
+  if (bytes) ws = scratch(bytes, p);
+  call("hexa_estmm", [&] {
+    return api.hexa_estmm(ptr(p), ldp, ptr(q), ldq, i32(pad_offsets), E, cap, m, n, ptr(out), ldo, estride, m_split, split_stride, in_type,
+                          o_type, beta, engine, ptr(ws), bytes, s);
+  });
+  return out;
+}
+
+Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
+  const int64_t cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = out_ ? *out_ : empty({E, cols}, at::kFloat, src);
+  Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
+  const int type = dt(src);
+  const int64_t lds = ld(src), ldo = ld(out);
+  call("hexa_ess", [&] {
+    return api.hexa_ess(ptr(src), lds, i32(pad_offsets), E, cap, cols, static_cast<float*>(ptr(out)), ldo, type, ptr(ws), (size_t)ws.numel(), s);
+  });
+  return out;
+}
+
+// ---- the step before routing ---------------------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor, Tensor, Tensor> gate_topk(const Tensor& logits, int top_k) {
+  if (logits.scalar_type() != at::kFloat || logits.dim() != 2 || logits.stride(1) != 1)
+    fail("gate_topk: logits must be float32 [T,E] with unit inner stride");
+  const int64_t T = logits.size(0), E = logits.size(1);
+  void* s = stream_of(logits);
+  Tensor ids = empty({top_k, T}, at::kInt, logits), mass = empty({E}, at::kFloat, logits), cnt = empty({E}, at::kInt, logits);
+  Tensor loss = empty({}, at::kFloat, logits), ws = scratch(api.hexa_gate_workspace_bytes(), logits);
+  call("hexa_gate_topk", [&] {
+    return api.hexa_gate_topk(static_cast<const float*>(ptr(logits)), logits.stride(0), T, (int)E, top_k, static_cast<int32_t*>(ptr(ids)),
+                              static_cast<float*>(ptr(mass)), static_cast<int32_t*>(ptr(cnt)), static_cast<float*>(ptr(loss)), ptr(ws),
+                              (size_t)ws.numel(), s);
+  });
+  return {ids, loss, cnt, mass};
+}
+
+Tensor gate_loss_grad(const Tensor& logits, const Tensor& first_count, const Tensor& dloss_) {
+  const int64_t T = logits.size(0), E = logits.size(1);
+  void* s = stream_of(logits);
+  Tensor out = empty({T, E}, at::kFloat, logits);
+  const Tensor dloss = dloss_.detach().to(at::kFloat).reshape({1}).contiguous();
+  const int64_t ldl = ld(logits);
+  call("hexa_gate_loss_grad", [&] {
+    return api.hexa_gate_loss_grad(static_cast<const float*>(ptr(logits)), ldl, T, (int)E, i32(first_count),
+                                   static_cast<const float*>(ptr(dloss)), static_cast<float*>(ptr(out)), E, s);
+  });
+  return out;
+}
+
+Tensor gate_split_terms(const Tensor& src, bool by_rows) {
+  if (src.scalar_type() != at::kFloat || src.dim() != 2 || !src.is_contiguous()) fail("gate_split_terms: src must be contiguous float32");
+  const int64_t rows = src.size(0), cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = by_rows ? empty({4 * rows, cols}, at::kBFloat16, src) : empty({rows, 4 * cols}, at::kBFloat16, src);
+  call("hexa_gate_split_terms", [&] { return api.hexa_gate_split_terms(static_cast<const float*>(ptr(src)), cols, rows, cols, by_rows, ptr(out), s); });
+  return out;
+}
+
+Tensor gate_sum_terms(const Tensor& part, int64_t rows, int64_t cols, bool lo_first) {
+  if (part.scalar_type() != at::kFloat || !part.is_contiguous() || part.numel() != 3 * rows * cols)
+    fail("gate_sum_terms: part must be contiguous float32 of 3 * rows * cols elements");
+  void* s = stream_of(part);
+  Tensor out = empty({rows, cols}, at::kFloat, part);
+  call("hexa_gate_sum_terms", [&] {
+    return api.hexa_gate_sum_terms(static_cast<const float*>(ptr(part)), rows, cols, lo_first, static_cast<float*>(ptr(out)), s);
+  });
+  return out;
+}
+
+void bind(const std::string& path, py::object error, py::object ensure, py::dict text) {
+  void* handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (!handle) throw std::runtime_error(dlerror());
+#define HEXA_BIND(name)                                                  \
+  api.name = reinterpret_cast<decltype(api.name)>(dlsym(handle, #name)); \
+  if (!api.name) throw std::runtime_error(path + " does not export " #name);
+  HEXA_API(HEXA_BIND)
+  bound = new Bound{std::move(error), std::move(ensure), std::move(text)};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  m.def("bind", &bind);
+  m.def("route", &route);
+  m.def("gather_rows", &gather_rows);
+  m.def("gather_rows_ess", &gather_rows_ess);
+  m.def("combine_rows", &combine_rows);
+  m.def("esmm", &esmm);
+  m.def("estmm", &estmm);
+  m.def("ess", &ess);
+  m.def("gate_topk", &gate_topk);
+  m.def("gate_loss_grad", &gate_loss_grad);
+  m.def("gate_split_terms", &gate_split_terms);
+  m.def("gate_sum_terms", &gate_sum_terms);
+}

@@ -365,10 +365,8 @@ class MoE_Cascaded(torch.nn.Module):
         x = input.reshape(-1, original_shape[-reserve_dims:].numel())
         if torch.is_autocast_enabled():
             x = x.to(torch.get_autocast_gpu_dtype() if x.is_cuda else torch.get_autocast_cpu_dtype())
-        else:
-            for p in self.parameters():
-                x = x.to(p.dtype)
-                break
+        elif self.total_depth_moe + self.total_depth_mlp:      # the dtype of the module's first parameter
+            x = x.to((self.batched_fc1_w if self.total_depth_moe else self.mlp_fc1_w)[0].dtype)
 
         if not is_moe:
             y = MLP_Implement.apply(cfg, x, self.mlp_fc1_w[i_mlp], self.mlp_fc2_w[i_mlp], self.mlp_fc1_b[i_mlp],
@@ -385,9 +383,9 @@ class MoE_Cascaded(torch.nn.Module):
         cfg.stage = i_moe
 
         loc = self.local_dim_list[i_moe]
-        w1 = self.batched_fc1_w[i_moe][:, :loc]
-        w2 = self.batched_fc2_w[i_moe][:, :loc]
-        b1 = self.batched_fc1_bias[i_moe][:, :loc] if self.has_fc1_bias else None
+        own = lambda t: t if t.shape[1] == loc else t[:, :loc]      # this rank's slice, when the storage is wider
+        w1, w2 = own(self.batched_fc1_w[i_moe]), own(self.batched_fc2_w[i_moe])
+        b1 = own(self.batched_fc1_bias[i_moe]) if self.has_fc1_bias else None
         b2 = self.batched_fc2_bias[i_moe] if self.has_fc2_bias else None
         y = FusedMoE_Shared_CudaCore.apply(cfg, x, w1, w2, b1, b2).to(x.dtype)
         y = y.view(list(original_shape[:-reserve_dims]) + list(y.shape[-reserve_dims:])).to(original_dtype)

@@ -204,7 +204,14 @@ def simplified_extract_critical(scores, top_k, loss_fn=losses.gshard_loss):
 
 
 def _stack_ids(indices_: List[Tensor], device) -> Tensor:
-    """k int vectors [T] -> one int32 [k, T] tensor (route-major, what the routing kernel reads)."""
+    """k int vectors [T] -> one int32 [k, T] tensor (route-major, what the routing kernel reads).  Vectors that already
+    are the consecutive rows of such a tensor (what the gate step hands out) are taken as they lie, without a copy."""
+    first = indices_[0]
+    T = first.numel()
+    start, store = first.data_ptr(), first.untyped_storage().data_ptr()
+    if T and all(i.dtype == torch.int32 and i.device == device and i.numel() == T and i.is_contiguous()
+                 and i.data_ptr() == start + 4 * T * j and i.untyped_storage().data_ptr() == store for j, i in enumerate(indices_)):
+        return first.as_strided((len(indices_), T), (T, 1))
     return torch.stack([i.reshape(-1).to(device=device, dtype=torch.int32) for i in indices_], dim=0).contiguous()
 
 

@@ -2,7 +2,7 @@
 single-device MoE layer forward/backward assembled from them.
 
 Everything here runs CUDA kernels from libhexa_moe_b200.so on the current stream of the input's
-device; no function has a CPU or PyTorch fallback.  Buffers in "sorted-row" layout have
+device, most of it through the native wrappers of csrc/host.cpp; no function has a CPU or PyTorch fallback.  Buffers in "sorted-row" layout have
 `row_capacity` rows of which the first pad_offsets[E] are meaningful (pad rows hold zeros).
 """
 from __future__ import annotations
@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import _lib as L
-from ._lib import check, dt, lib, ptr, stream_of
+from ._lib import check, dt, host, lib, ptr, stream_of
 
 
 # ---- optional per-call instrumentation (used by bench.py; off by default) --------------------------
@@ -23,6 +23,16 @@ from ._lib import check, dt, lib, ptr, stream_of
 LAUNCHES = 0
 PROFILE = None
 _KERNELS_PER_CALL = dict(route=1, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1)
+
+
+def _run(name, work, nbytes, fn, args):
+    """fn(*args), counted and, when PROFILE is on, timed."""
+    global LAUNCHES
+    if PROFILE is None:
+        LAUNCHES += _KERNELS_PER_CALL[name.split(":")[0]]
+        return fn(*args)
+    with _Timed(name, work, nbytes):
+        return fn(*args)
 
 
 class _Timed:
@@ -67,35 +77,10 @@ class Routing:
 def route(ids: torch.Tensor, num_experts: int, align: int = L.ROW_TILE, route_major: bool = False) -> Routing:
     """Segment routed rows by expert.  ids: int32 [T, k] (or [k, T] when route_major)."""
     global LAUNCHES
-    if ids.dtype != torch.int32:
-        raise L.HexaError("route: ids must be int32")
-    if ids.dim() != 2:
-        raise L.HexaError("route: ids must be 2-D")
-    if route_major:
-        k, T = ids.shape
-        st, sk = ids.stride(1), ids.stride(0)
-    else:
-        T, k = ids.shape
-        st, sk = ids.stride(0), ids.stride(1)
-    s = stream_of(ids)
-    dev = ids.device
-    cap = lib().hexa_route_row_capacity(T, k, num_experts, align)
-    if cap < 0:
-        raise L.HexaError("route: bad sizes")
-    i32 = dict(dtype=torch.int32, device=dev)
-    pairs = torch.empty(lib().hexa_route_pair_capacity(T, k, num_experts), **i32) if align == L.ROW_TILE else None
-    r = Routing(torch.empty(num_experts, **i32), torch.empty(num_experts + 1, **i32), torch.empty(num_experts + 1, **i32),
-                torch.empty(max(cap, 1), **i32), torch.empty(max(T * k, 1), **i32), torch.empty(max(cap // align, 1), **i32),
-                pairs, T, k, num_experts, align, cap)
-    ws_bytes = lib().hexa_route_workspace_bytes(T, k, num_experts)
-    ws = torch.empty(max(ws_bytes, 4), dtype=torch.uint8, device=dev)
-    with _Timed("route", 12.0 * T * k):
-        check(lib().hexa_route(ptr(ids), T, k, st, sk, num_experts, align, ptr(r.counts), ptr(r.seg_offsets), ptr(r.pad_offsets),
-                               ptr(r.row_token), ptr(r.token_row), ptr(r.tile_expert), ptr(r.pair_block), ptr(ws), ws.numel(), s),
-              "hexa_route")
-    if T * k > 8192 or num_experts > 256:
-        LAUNCHES += lib().hexa_route_launches(T, k, num_experts) - 1
-    return r
+    out = _run("route", 12.0 * ids.numel(), 0.0, host().route, (ids, num_experts, align, route_major))
+    LAUNCHES += out[-1] - 1
+    counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, cap, _ = out
+    return Routing(counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, num_experts, align, cap)
 
 
 def sorted_buffer(rows: int, cols: int, dtype, device) -> torch.Tensor:
@@ -115,13 +100,8 @@ def _ld(t: torch.Tensor) -> int:
 
 def gather_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Token order -> sorted rows: out[row] = src[row_token[row]] (zeros for pad rows)."""
-    cols = src.shape[1]
-    if out is None:
-        out = sorted_buffer(r.row_capacity, cols, src.dtype, src.device)
-    with _Timed("gather", 2.0 * r.num_tokens * r.top_k * cols * src.element_size()):
-        check(lib().hexa_gather_rows(ptr(src), _ld(src), ptr(r.row_token), ptr(r.pad_offsets), r.num_experts, r.row_capacity,
-                                     cols, ptr(out), _ld(out), dt(src), stream_of(src)), "hexa_gather_rows")
-    return out
+    return _run("gather", 2.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().gather_rows,
+                (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity, out))
 
 
 def gather_rows_ess(src: torch.Tensor, r: Routing):
@@ -129,27 +109,15 @@ def gather_rows_ess(src: torch.Tensor, r: Routing):
     global LAUNCHES
     if r.align % L.ROW_TILE:
         raise L.HexaError("gather_rows_ess: routing must be aligned to 128 rows")
-    cols = src.shape[1]
-    out = sorted_buffer(r.row_capacity, cols, src.dtype, src.device)
-    sums = torch.empty(r.num_experts, cols, dtype=torch.float32, device=src.device)
-    ws = torch.empty(max(lib().hexa_ess_workspace_bytes(r.row_capacity, cols), 4), dtype=torch.uint8, device=src.device)
-    with _Timed("gather", 2.0 * r.num_tokens * r.top_k * cols * src.element_size()):
-        check(lib().hexa_gather_rows_ess(ptr(src), _ld(src), ptr(r.row_token), ptr(r.pad_offsets), r.num_experts, r.row_capacity,
-                                         cols, ptr(out), _ld(out), ptr(sums), _ld(sums), dt(src), ptr(ws), ws.numel(),
-                                         stream_of(src)), "hexa_gather_rows_ess")
     LAUNCHES += 1          # the second pass of ESS over the tile sums
-    return out, sums
+    return _run("gather", 2.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().gather_rows_ess,
+                (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity))
 
 
 def combine_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Sorted rows -> token order with the unweighted sum over the k routes."""
-    cols = src.shape[1]
-    if out is None:
-        out = torch.empty(r.num_tokens, cols, dtype=src.dtype, device=src.device)
-    with _Timed("combine", (r.top_k + 1.0) * r.num_tokens * cols * src.element_size()):
-        check(lib().hexa_combine_rows(ptr(src), _ld(src), ptr(r.token_row), r.num_tokens, r.top_k, cols, ptr(out), _ld(out),
-                                      dt(src), stream_of(src)), "hexa_combine_rows")
-    return out
+    return _run("combine", (r.top_k + 1.0) * r.num_tokens * src.shape[1] * src.element_size(), 0.0, host().combine_rows,
+                (src, r.token_row, r.num_tokens, r.top_k, out))
 
 
 def esmm(a: torch.Tensor, b: torch.Tensor, b_layout: int, r: Routing, bias: Optional[torch.Tensor] = None,
@@ -172,36 +140,18 @@ def esmm(a: torch.Tensor, b: torch.Tensor, b_layout: int, r: Routing, bias: Opti
         kk, nn = b.shape[1], b.shape[2]
     n_out = nn if n_out is None else n_out
     k = kk if k is None else k
-    if a.dtype != b.dtype:
-        raise L.HexaError(f"esmm: a is {a.dtype} but b is {b.dtype}")
-    if bias is not None and bias.dtype != torch.float32:
-        raise L.HexaError("esmm: bias must be float32")
-    if out is None:
-        out = sorted_buffer(r.row_capacity, n_out, a.dtype, a.device)
-    rows_ = r.num_tokens * r.top_k
-    es_ = a.element_size()
-    nbytes = es_ * (rows_ * k + r.num_experts * n_out * k + rows_ * n_out * (1 if epilogue == L.EPI_LINEAR else 2))
     e0, e1 = (0, r.num_experts) if experts is None else experts
-    share = (e1 - e0) / max(r.num_experts, 1)        # work of a group, taken as its share of the experts
+    work = nbytes = 0.0
+    if PROFILE is not None:
+        es, rows = a.element_size(), r.num_tokens * r.top_k
+        share = (e1 - e0) / max(r.num_experts, 1)        # work of a group, taken as its share of the experts
+        work = 2.0 * rows * n_out * k * share
+        nbytes = float(es * (rows * k + r.num_experts * n_out * k + rows * n_out * (1 if epilogue == L.EPI_LINEAR else 2))) * share
     if sums is not None:
-        if experts is not None or sums.dtype != torch.float32 or tuple(sums.shape) != (r.num_experts, n_out) or sums.stride(1) != 1:
-            raise L.HexaError("esmm: sums must be float32 [E, n_out] and needs the full expert range")
-        ws = torch.empty(max(lib().hexa_ess_workspace_bytes(r.row_capacity, n_out), 4), dtype=torch.uint8, device=a.device)
-        with _Timed("esmm:" + (tag or "epilogue%d" % epilogue), 2.0 * rows_ * n_out * k, float(nbytes)):
-            check(lib().hexa_esmm_ess(ptr(a), _ld(a), ptr(b), b_layout, b.stride(1), b.stride(0), ptr(bias),
-                                      0 if bias is None else _ld(bias), ptr(aux), 0 if aux is None else _ld(aux), ptr(out),
-                                      _ld(out), ptr(r.tile_expert), ptr(r.pad_offsets), ptr(r.row_token), ptr(r.pair_block),
-                                      r.num_experts, r.row_capacity, n_out, k, dt(a), epilogue, act, engine, ptr(sums),
-                                      sums.stride(0), ptr(ws), ws.numel(), stream_of(a)), "hexa_esmm_ess")
         LAUNCHES += 1          # the second pass of ESS over the block sums
-        return out
-    with _Timed("esmm:" + (tag or "epilogue%d" % epilogue), 2.0 * rows_ * n_out * k * share, float(nbytes) * share):
-        check(lib().hexa_esmm_experts(ptr(a), _ld(a), ptr(b), b_layout, b.stride(1), b.stride(0), ptr(bias),
-                                      0 if bias is None else _ld(bias), ptr(aux), 0 if aux is None else _ld(aux), ptr(out),
-                                      _ld(out), ptr(r.tile_expert), ptr(r.pad_offsets), ptr(r.row_token), ptr(r.pair_block),
-                                      r.num_experts, r.row_capacity, n_out, k, dt(a), epilogue, act, engine, e0, e1,
-                                      stream_of(a)), "hexa_esmm")
-    return out
+    return _run("esmm:" + (tag or "epilogue%d" % epilogue), work, nbytes, host().esmm,
+                (a, b, b_layout, r.tile_expert, r.pad_offsets, r.row_token, r.pair_block, r.num_experts, r.row_capacity, bias,
+                 epilogue, act, aux, out, engine, n_out, k, e0, e1, sums))
 
 
 def estmm(p: torch.Tensor, q: torch.Tensor, r: Routing, out_dtype: Optional[torch.dtype] = None,
@@ -234,28 +184,13 @@ def estmm(p: torch.Tensor, q: torch.Tensor, r: Routing, out_dtype: Optional[torc
                                            ptrs, ranks, o0.stride(1), o0.stride(0), m // ranks, dt(p), dt(o0), stream_of(p)),
                   "hexa_estmm_scatter")
         return out
-    if ranks > 1:
-        if m % ranks:
-            raise L.HexaError("estmm: the row count must be divisible by ranks")
-        if out is None:
-            out = torch.empty(ranks, r.num_experts, m // ranks, n, dtype=out_dtype or p.dtype, device=p.device)
-        ldo, estride, m_split, split_stride = out.stride(2), out.stride(1), m // ranks, out.stride(0)
-    else:
-        if out is None:
-            if beta:
-                raise L.HexaError("estmm: beta=1 needs an existing out")
-            out = torch.empty(r.num_experts, m, n, dtype=out_dtype or p.dtype, device=p.device)
-        ldo, estride, m_split, split_stride = out.stride(1), out.stride(0), 0, 0
-    if out.stride(-1) != 1:
-        raise L.HexaError("estmm: out must have unit inner stride")
-    ws_bytes = lib().hexa_estmm_workspace_bytes(r.num_experts, r.row_capacity, m, n, dt(p)) if engine != L.ENGINE_SIMT else 0
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=p.device) if ws_bytes else None
-    with _Timed("estmm:" + (tag or "dw"), 2.0 * rows_ * m * n,
-                float(p.element_size() * rows_ * (m + n) + out.element_size() * r.num_experts * m * n)):
-        check(lib().hexa_estmm(ptr(p), _ld(p), ptr(q), _ld(q), ptr(r.pad_offsets), r.num_experts, r.row_capacity, m, n, ptr(out),
-                               ldo, estride, m_split, split_stride, dt(p), dt(out), beta, engine, ptr(ws), ws_bytes,
-                               stream_of(p)), "hexa_estmm")
-    return out
+    work = nbytes = 0.0
+    if PROFILE is not None:
+        work = 2.0 * rows_ * m * n
+        o_size = (out.element_size() if out is not None else torch.finfo(out_dtype or p.dtype).bits // 8)
+        nbytes = float(p.element_size() * rows_ * (m + n) + o_size * r.num_experts * m * n)
+    return _run("estmm:" + (tag or "dw"), work, nbytes, host().estmm,
+                (p, q, r.pad_offsets, r.num_experts, r.row_capacity, out, out_dtype, beta, engine, ranks))
 
 
 def copy_2d(dst: torch.Tensor, dst_pitch: int, src: torch.Tensor, src_pitch: int, width: int, height: int, stream: int = None):
@@ -281,15 +216,8 @@ def ess(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> to
     """out[e] = sum of expert e's rows of src, float32 [E, cols]."""
     if r.align % L.ROW_TILE:
         raise L.HexaError("ess: routing must be aligned to 128 rows")
-    cols = src.shape[1]
-    if out is None:
-        out = torch.empty(r.num_experts, cols, dtype=torch.float32, device=src.device)
-    nbytes = lib().hexa_ess_workspace_bytes(r.row_capacity, cols)
-    ws = torch.empty(max(nbytes, 4), dtype=torch.uint8, device=src.device)
-    with _Timed("ess", 1.0 * r.num_tokens * r.top_k * cols * src.element_size()):
-        check(lib().hexa_ess(ptr(src), _ld(src), ptr(r.pad_offsets), r.num_experts, r.row_capacity, cols, ptr(out), _ld(out),
-                             dt(src), ptr(ws), ws.numel(), stream_of(src)), "hexa_ess")
-    return out
+    return _run("ess", 1.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().ess,
+                (src, r.pad_offsets, r.num_experts, r.row_capacity, out))
 
 
 def mask_pad_rows(buf: torch.Tensor, r: Routing) -> torch.Tensor:
@@ -309,54 +237,27 @@ def gate_max_experts() -> int:
 def gate_split_terms(src: torch.Tensor, by_rows: bool) -> torch.Tensor:
     """float32 [rows, cols] as bf16 terms hi + mid + lo: [rows, 4 cols] with column blocks (hi, hi, mid, lo) or, by_rows,
     [4 rows, cols] with row blocks (lo, mid, hi, hi)."""
-    if src.dtype != torch.float32 or not src.is_contiguous():
-        raise L.HexaError("gate_split_terms: src must be contiguous float32")
-    rows, cols = src.shape
-    out = torch.empty((4 * rows, cols) if by_rows else (rows, 4 * cols), dtype=torch.bfloat16, device=src.device)
-    with _Timed("gate"):
-        check(lib().hexa_gate_split_terms(ptr(src), cols, rows, cols, int(by_rows), ptr(out), stream_of(src)), "hexa_gate_split_terms")
-    return out
+    return _run("gate", 0.0, 0.0, host().gate_split_terms, (src, by_rows))
 
 
 def gate_sum_terms(part: torch.Tensor, rows: int, cols: int, lo_first: bool) -> torch.Tensor:
     """(hi + mid) + lo of the three column blocks of part [rows, 3 cols], stored as (hi, mid, lo) or, lo_first, reversed."""
-    if part.dtype != torch.float32 or not part.is_contiguous() or part.numel() != 3 * rows * cols:
-        raise L.HexaError("gate_sum_terms: part must be contiguous float32 of 3 * rows * cols elements")
-    out = torch.empty(rows, cols, dtype=torch.float32, device=part.device)
-    with _Timed("gate"):
-        check(lib().hexa_gate_sum_terms(ptr(part), rows, cols, int(lo_first), ptr(out), stream_of(part)), "hexa_gate_sum_terms")
-    return out
+    return _run("gate", 0.0, 0.0, host().gate_sum_terms, (part, rows, cols, lo_first))
 
 
 def gate_topk(logits: torch.Tensor, top_k: int):
     """softmax + top-k + GShard loss of float32 logits [T,E] in one kernel.  Returns (ids int32 [k,T] route-major,
     loss float32 scalar tensor, first_count int32 [E], mass float32 [E])."""
-    if logits.dtype != torch.float32 or logits.dim() != 2 or logits.stride(1) != 1:
-        raise L.HexaError("gate_topk: logits must be float32 [T,E] with unit inner stride")
     global LAUNCHES
+    out = _run("gate", 8.0 * logits.numel(), 0.0, host().gate_topk, (logits, top_k))
     T, E = logits.shape
-    dev = logits.device
-    ids = torch.empty(top_k, T, dtype=torch.int32, device=dev)
-    mass = torch.empty(E, dtype=torch.float32, device=dev)
-    cnt = torch.empty(E, dtype=torch.int32, device=dev)
-    loss = torch.empty((), dtype=torch.float32, device=dev)
-    ws = torch.empty(int(lib().hexa_gate_workspace_bytes()), dtype=torch.uint8, device=dev)
-    with _Timed("gate", 2.0 * T * E * 4):
-        check(lib().hexa_gate_topk(ptr(logits), _ld(logits), T, E, top_k, ptr(ids), ptr(mass), ptr(cnt), ptr(loss), ptr(ws),
-                                   ws.numel(), stream_of(logits)), "hexa_gate_topk")
     LAUNCHES += T > (512 if E <= 64 else 256 if E <= 128 else 32)      # beyond one block: a second kernel adds the blocks' rows
-    return ids, loss, cnt, mass
+    return out
 
 
 def gate_loss_grad(logits: torch.Tensor, first_count: torch.Tensor, dloss: torch.Tensor) -> torch.Tensor:
     """Gradient of gate_topk's loss with respect to the logits, scaled by the device scalar dloss."""
-    T, E = logits.shape
-    out = torch.empty(T, E, dtype=torch.float32, device=logits.device)
-    dloss = dloss.detach().to(torch.float32).reshape(1).contiguous()
-    with _Timed("gate", 2.0 * T * E * 4):
-        check(lib().hexa_gate_loss_grad(ptr(logits), _ld(logits), T, E, ptr(first_count), ptr(dloss), ptr(out), _ld(out),
-                                        stream_of(logits)), "hexa_gate_loss_grad")
-    return out
+    return _run("gate", 8.0 * logits.numel(), 0.0, host().gate_loss_grad, (logits, first_count, dloss))
 
 
 def gate_topk_load_importance(logits: torch.Tensor, logits_w_noise: torch.Tensor, top_k: int, sigma: float):
