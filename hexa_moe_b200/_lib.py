@@ -39,6 +39,7 @@ SIGNATURES = {
     "hexa_route_pair_capacity": (i64, [i64, ci, ci]),
     "hexa_route_launches": (ci, [i64, ci, ci]),
     "hexa_route": (ci, [vp, i64, ci, i64, i64, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
+    "hexa_ids_from_lists": (ci, [vp, vp, i64, ci, i64, vp, vp]),
     "hexa_gather_rows": (ci, [vp, i64, vp, vp, ci, i64, i64, vp, i64, ci, vp]),
     "hexa_gather_rows_ess": (ci, [vp, i64, vp, vp, ci, i64, i64, vp, i64, vp, i64, ci, vp, sz, vp]),
     "hexa_combine_rows": (ci, [vp, i64, vp, i64, ci, i64, vp, i64, ci, vp]),

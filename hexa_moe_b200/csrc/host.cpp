@@ -31,7 +31,7 @@ struct Api {
   X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
   X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
   X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
-  X(hexa_gate_split_terms) X(hexa_gate_sum_terms)
+  X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists)
 #define HEXA_FIELD(name) decltype(&::name) name = nullptr;
   HEXA_API(HEXA_FIELD)
 } api;
@@ -130,6 +130,16 @@ py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
                           out(tiles), pairs ? out(*pairs) : nullptr, ptr(ws), (size_t)ws.numel(), s);
   });
   return py::make_tuple(counts, seg, pad, row_token, token_row, tiles, pairs, T, k, cap, api.hexa_route_launches(T, (int)k, E));
+}
+
+Tensor ids_from_lists(int64_t num_toks, const Tensor& tok_ids_, const Tensor& exp_ids_, int chunk) {
+  const Tensor tok_ids = tok_ids_.to(at::kInt).contiguous(), exp_ids = exp_ids_.to(at::kInt).contiguous();
+  void* s = stream_of(tok_ids);
+  Tensor ids = empty({num_toks}, at::kInt, tok_ids);
+  call("hexa_ids_from_lists", [&] {
+    return api.hexa_ids_from_lists(i32(tok_ids), i32(exp_ids), tok_ids.numel(), chunk, num_toks, static_cast<int32_t*>(ptr(ids)), s);
+  });
+  return ids;
 }
 
 Tensor gather_rows(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
@@ -305,6 +315,7 @@ void bind(const std::string& path, py::object error, py::object ensure, py::dict
 PYBIND11_MODULE(_host, m) {
   m.def("bind", &bind);
   m.def("route", &route);
+  m.def("ids_from_lists", &ids_from_lists);
   m.def("gather_rows", &gather_rows);
   m.def("gather_rows_ess", &gather_rows_ess);
   m.def("combine_rows", &combine_rows);

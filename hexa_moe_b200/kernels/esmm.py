@@ -12,9 +12,7 @@ from .basics import MAX_TOKEN_CHUNK
 def ids_from_lists(num_toks, tok_ids_list, exp_ids_list):
     """Expert id per token (-1: token not in any segment) from the reference's (tok_ids + 1, exp_ids) lists."""
     assert tok_ids_list.shape[0] == MAX_TOKEN_CHUNK * exp_ids_list.shape[0]
-    ids = torch.full((num_toks + 1,), -1, dtype=torch.int32, device=tok_ids_list.device)
-    ids[tok_ids_list.long()] = exp_ids_list.repeat_interleave(MAX_TOKEN_CHUNK).to(torch.int32)
-    return ids[1:].contiguous()          # slot 0 collected the pad entries
+    return ops.ids_from_lists(num_toks, tok_ids_list, exp_ids_list, MAX_TOKEN_CHUNK)
 
 
 def ESMM(toks, w, b, tok_ids_list, exp_ids_list):

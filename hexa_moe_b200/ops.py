@@ -22,7 +22,7 @@ from ._lib import check, dt, host, lib, ptr, stream_of
 # (name, start_event, end_event, algorithmic_work, algorithmic_bytes) with CUDA events recorded on the launching stream.
 LAUNCHES = 0
 PROFILE = None
-_KERNELS_PER_CALL = dict(route=1, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1)
+_KERNELS_PER_CALL = dict(route=1, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1, lists=1)
 
 
 def _run(name, work, nbytes, fn, args):
@@ -81,6 +81,12 @@ def route(ids: torch.Tensor, num_experts: int, align: int = L.ROW_TILE, route_ma
     LAUNCHES += out[-1] - 1
     counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, cap, _ = out
     return Routing(counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, num_experts, align, cap)
+
+
+def ids_from_lists(num_toks: int, tok_ids: torch.Tensor, exp_ids: torch.Tensor, chunk: int) -> torch.Tensor:
+    """int32 [num_toks] expert id per token (-1: in no segment) from lists of token ids + 1 (0: pad), `chunk` entries per
+    element of exp_ids."""
+    return _run("lists", 0.0, 0.0, host().ids_from_lists, (num_toks, tok_ids, exp_ids, chunk))
 
 
 def sorted_buffer(rows: int, cols: int, dtype, device) -> torch.Tensor:

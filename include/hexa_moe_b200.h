@@ -128,6 +128,11 @@ int hexa_route(const int32_t* ids, int64_t num_tokens, int top_k, int64_t stride
                int32_t* row_token, int32_t* token_row, int32_t* tile_expert, int32_t* pair_block,
                void* workspace, size_t workspace_bytes, void* stream);
 
+/* One expert id per token from the reference's operator-level lists (kernels/esmm.py:249-263): tok_ids[n] holds token
+ * ids + 1 (0 = pad) and entry i belongs to expert exp_ids[i / chunk].  ids[num_tokens]: -1 for tokens in no segment. */
+int hexa_ids_from_lists(const int32_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_tokens, int32_t* ids,
+                        void* stream);
+
 /* ---- row movement between token order and sorted-row order (the reference gathers rows by
  *      tok_ids inside its kernels, kernels/esmm.py:95-101, and sums the k routes in Python,
  *      impls/layers.py:254-258) ---- */

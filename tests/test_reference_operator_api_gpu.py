@@ -73,3 +73,18 @@ def test_fused_ess_estmm_equal_reference_where_it_is_correct(golden_dir):
         assert np.abs(got_dw[written] - dw_ref[written]).max() / np.abs(dw_ref[written]).max() < 2e-3
         counts = np.bincount(routing.cpu().numpy(), minlength=E)
         assert (got_ess[counts == 0] == 0).all() and (got_dw[counts == 0] == 0).all()
+
+
+@pytest.mark.parametrize("T,n,dtype", [(1, 16, torch.int32), (300, 4096, torch.int32), (257, 320, torch.int64), (40, 0, torch.int32)])
+def test_expert_ids_from_lists(T, n, dtype):
+    """Pads (0), tokens in no segment, a list longer than a block and an empty one, against the indexing formulation."""
+    from hexa_moe_b200.kernels.esmm import ids_from_lists
+    g = torch.Generator().manual_seed(T + n)
+    tok = torch.zeros(n, dtype=torch.int64)
+    slots = torch.randperm(n, generator=g)[: min(T * 2 // 3 + 1, n)]
+    tok[slots] = torch.randperm(T, generator=g)[: len(slots)] + 1
+    exp = torch.randint(0, 9, (n // 16,), generator=g, dtype=torch.int32)
+    want = torch.full((T + 1,), -1, dtype=torch.int32)
+    want[tok] = exp.repeat_interleave(16)
+    got = ids_from_lists(T, tok.to(dtype).cuda(), exp.cuda())
+    assert got.dtype == torch.int32 and torch.equal(got.cpu(), want[1:])
