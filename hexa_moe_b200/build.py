@@ -17,7 +17,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhexa_moe_b200.so")
 HOST = os.path.join(HERE, "_host.so")
-SOURCES = ["route.cu", "rows.cu", "gemm_simt.cu", "gemm_tc.cu", "ops_api.cu", "peer.cu", "gate.cu"]
+SOURCES = ["route.cu", "rows.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_f32.cu", "ops_api.cu", "peer.cu", "gate.cu"]
 
 
 def _nvcc():

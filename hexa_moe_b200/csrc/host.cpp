@@ -29,7 +29,7 @@ struct Api {
 #define HEXA_API(X)                                                                                                            \
   X(hexa_last_error_string) X(hexa_pending_device_status) X(hexa_route_row_capacity) X(hexa_route_workspace_bytes)             \
   X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
-  X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
+  X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_f32_workspace_bytes) X(hexa_esmm_f32) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
   X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
   X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists)
 #define HEXA_FIELD(name) decltype(&::name) name = nullptr;
@@ -176,6 +176,19 @@ Tensor combine_rows(const Tensor& src, const Tensor& token_row, int64_t T, int t
   return out;
 }
 
+Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
+  const int64_t cols = src.size(1);
+  void* s = stream_of(src);
+  Tensor out = out_ ? *out_ : empty({E, cols}, at::kFloat, src);
+  Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
+  const int type = dt(src);
+  const int64_t lds = ld(src), ldo = ld(out);
+  call("hexa_ess", [&] {
+    return api.hexa_ess(ptr(src), lds, i32(pad_offsets), E, cap, cols, static_cast<float*>(ptr(out)), ldo, type, ptr(ws), (size_t)ws.numel(), s);
+  });
+  return out;
+}
+
 Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_expert, const Tensor& pad_offsets, const Tensor& row_token,
             const OptTensor& pair_block, int E, int64_t cap, const OptTensor& bias, int epilogue, int act, const OptTensor& aux,
             const OptTensor& out_, int engine, int64_t n_out, int64_t k, int e0, int e1, const OptTensor& sums) {
@@ -190,6 +203,21 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
   Tensor out = out_ ? *out_ : sorted_buffer(cap, n_out, a.scalar_type(), a);
   const int64_t lda = ld(a), ldo = ld(out), ldbias = bias ? ld(*bias) : 0, ldaux = aux ? ld(*aux) : 0;
   const float* bp = static_cast<const float*>(ptr(bias));
+  const size_t planes = type == HEXA_F32 && engine == HEXA_ENGINE_AUTO && pair_block && e0 == 0 && e1 == E
+                            ? api.hexa_esmm_f32_workspace_bytes(E, cap, n_out, k) : 0;
+  if (planes) {
+    {
+      Tensor ws = scratch(planes, a);
+      auto f = [](void* v) { return static_cast<float*>(v); };
+      call("hexa_esmm_f32", [&] {
+        return api.hexa_esmm_f32(f(ptr(a)), lda, f(ptr(b)), b_layout, b.stride(1), b.stride(0), bp, ldbias, f(ptr(aux)), ldaux, f(ptr(out)),
+                                 ldo, i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, epilogue,
+                                 act, ptr(ws), (size_t)ws.numel(), s);
+      });
+    }
+    if (sums) ess(out, pad_offsets, E, cap, sums);
+    return out;
+  }
   if (sums) {
     Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, n_out), a);
     call("hexa_esmm_ess", [&] {
@@ -234,19 +262,6 @@ Tensor estmm(const Tensor& p, const Tensor& q, const Tensor& pad_offsets, int E,
   call("hexa_estmm", [&] {
     return api.hexa_estmm(ptr(p), ldp, ptr(q), ldq, i32(pad_offsets), E, cap, m, n, ptr(out), ldo, estride, m_split, split_stride, in_type,
                           o_type, beta, engine, ptr(ws), bytes, s);
-  });
-  return out;
-}
-
-Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
-  const int64_t cols = src.size(1);
-  void* s = stream_of(src);
-  Tensor out = out_ ? *out_ : empty({E, cols}, at::kFloat, src);
-  Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
-  const int type = dt(src);
-  const int64_t lds = ld(src), ldo = ld(out);
-  call("hexa_ess", [&] {
-    return api.hexa_ess(ptr(src), lds, i32(pad_offsets), E, cap, cols, static_cast<float*>(ptr(out)), ldo, type, ptr(ws), (size_t)ws.numel(), s);
   });
   return out;
 }

@@ -72,6 +72,31 @@ extern "C" int hexa_esmm(const void* a, int64_t lda, const void* b, int b_layout
                            row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, engine, 0, E, stream_);
 }
 
+extern "C" size_t hexa_esmm_f32_workspace_bytes(int E, int64_t row_cap, int64_t n_out, int64_t k) {
+  return esmm_f32_workspace_bytes(E, row_cap, n_out, k);
+}
+
+extern "C" int hexa_esmm_f32(const float* a, int64_t lda, const float* b, int b_layout, int64_t ldb, int64_t b_estride,
+                             const float* bias, int64_t ldbias, float* aux, int64_t ldaux, float* c, int64_t ldc,
+                             const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token,
+                             const int32_t* pair_block, int E, int64_t row_cap, int64_t n_out, int64_t k, int epilogue, int act,
+                             void* workspace, size_t workspace_bytes, void* stream_) {
+  // one result, two engines: the tensor cores need scratch, 16-byte rows to store to and the pair-tile list
+  const size_t need = esmm_f32_workspace_bytes(E, row_cap, n_out, k);
+  const bool planes = need > 0 && workspace && workspace_bytes >= need && aligned16(workspace) && a && b && c && tile_expert && pad_offsets &&
+                      pair_block && row_cap % kRowTile == 0 && lda >= k && ldc >= n_out && (!aux || ldaux >= n_out) &&
+                      (!bias || ldbias >= n_out) && (b_layout == HEXA_B_NK || b_layout == HEXA_B_KN) &&
+                      ldb >= (b_layout == HEXA_B_NK ? k : n_out) && epilogue >= HEXA_EPI_LINEAR && epilogue <= HEXA_EPI_DACT &&
+                      act >= HEXA_ACT_NONE && act <= HEXA_ACT_SILU && (epilogue != HEXA_EPI_DACT || aux) && aligned16(c) && ldc % 4 == 0 &&
+                      (epilogue != HEXA_EPI_ACT || !aux || (aligned16(aux) && ldaux % 4 == 0));
+  if (!planes)      // also the place where bad arguments are refused
+    return hexa_esmm_experts(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token,
+                             pair_block, E, row_cap, n_out, k, HEXA_F32, epilogue, act, HEXA_ENGINE_AUTO, 0, E, stream_);
+  HEXA_CHECK_DEVICE_STATUS("hexa_esmm_f32");
+  return esmm_f32_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token,
+                         pair_block, E, row_cap, n_out, k, epilogue, act, (cudaStream_t)stream_, workspace);
+}
+
 extern "C" int hexa_esmm_ess(const void* a, int64_t lda, const void* b, int b_layout, int64_t ldb, int64_t b_estride,
                              const float* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
                              const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token,
@@ -111,7 +136,9 @@ extern "C" int hexa_esmm_ess(const void* a, int64_t lda, const void* b, int b_la
 }
 
 extern "C" size_t hexa_estmm_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n, int dtype) {
-  if (E <= 0 || row_cap <= 0 || m <= 0 || n <= 0 || (dtype != HEXA_F16 && dtype != HEXA_BF16)) return 0;
+  if (E <= 0 || row_cap <= 0 || m <= 0 || n <= 0) return 0;
+  if (dtype == HEXA_F32) return estmm_f32_workspace_bytes(E, row_cap, m, n);
+  if (dtype != HEXA_F16 && dtype != HEXA_BF16) return 0;
   return estmm_tc_workspace_bytes(E, row_cap, m, n);
 }
 
@@ -139,6 +166,12 @@ extern "C" int hexa_estmm(const void* p, int64_t ldp, const void* q, int64_t ldq
   if (engine != HEXA_ENGINE_SIMT && tc_ok)
     return estmm_tc_launch(p, ldp, q, ldq, pad_offsets, E, row_cap, m, n, out, ldo, o_estride, m_split, split_stride, dtype, out_dtype,
                            beta, stream, nullptr, 0, workspace, workspace_bytes);
+  if (dtype == HEXA_F32 && engine == HEXA_ENGINE_AUTO && workspace && aligned16(workspace) && !beta && m_split >= m && aligned16(out) &&
+      ldo % 4 == 0 && o_estride % 4 == 0) {
+    const size_t need = estmm_f32_workspace_bytes(E, row_cap, m, n);
+    if (need > 0 && workspace_bytes >= need)
+      return estmm_f32_launch(p, ldp, q, ldq, pad_offsets, E, row_cap, m, n, out, ldo, o_estride, stream, workspace);
+  }
   return estmm_simt_launch(p, ldp, q, ldq, pad_offsets, E, m, n, out, ldo, o_estride, m_split, split_stride, dtype, out_dtype, beta,
                            stream);
 }

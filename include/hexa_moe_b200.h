@@ -239,6 +239,18 @@ int hexa_ess(const void* src, int64_t src_ld, const int32_t* pad_offsets, int nu
              int64_t row_capacity, int64_t cols, float* out, int64_t ldo, int dtype, void* workspace,
              size_t workspace_bytes, void* stream);
 
+/* hexa_esmm on fp32 data with scratch: where it pays (by sizes) and the arguments allow, the products run on the tensor
+ * cores as six bf16 term products per k-block with fp32 additions between k-blocks, closer to the exact result than the
+ * FMA chain of the CUDA-core kernel, which computes the call otherwise and whenever an operand holds a value that is not
+ * finite or beyond bf16's range.  workspace: hexa_esmm_f32_workspace_bytes() bytes (0: none is used), contents irrelevant.
+ * hexa_estmm does the same for fp32 inputs given hexa_estmm_workspace_bytes(..., HEXA_F32). */
+size_t hexa_esmm_f32_workspace_bytes(int num_experts, int64_t row_capacity, int64_t n_out, int64_t k);
+int hexa_esmm_f32(const float* a, int64_t lda, const float* b, int b_layout, int64_t ldb, int64_t b_estride,
+                  const float* bias, int64_t ldbias, float* aux, int64_t ldaux, float* c, int64_t ldc,
+                  const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token,
+                  const int32_t* pair_block, int num_experts, int64_t row_capacity, int64_t n_out, int64_t k, int epilogue,
+                  int act, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ESMM and ESS of its output in one pass.  No counterpart as a single call: the reference computes the hidden
  * gradient and then sums it per expert in its fused backward kernel (task 2 of launch_fused_grad_bias_*,
  * kernels/fused.py:111-141, reading the gradient back).  Arguments up to `engine` are hexa_esmm's.  Additionally

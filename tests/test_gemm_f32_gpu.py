@@ -1,0 +1,128 @@
+"""fp32 ESMM / ESTMM on the tensor cores (three bf16 planes per operand, fp32 additions between k-blocks) against float64 and
+against the CUDA-core kernel: never further from the exact result than the FMA chain, zero pad rows, and the FMA chain's own
+answer wherever an operand holds a value that has no planes.  Sizes are just beyond the point where the path is taken."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _need_cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def _mods():
+    from hexa_moe_b200 import _lib as L, ops
+    return L, ops
+
+
+def _routing(ops, T, E, k, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    logits = torch.randn(T, E, generator=g, device="cuda") - 0.3 * torch.arange(E, device="cuda")
+    logits[:, min(1, E - 1)] = -100.0 if E > k else 0.0                     # an empty expert
+    return ops.route(torch.topk(logits, k, dim=1).indices.to(torch.int32), E), g
+
+
+def _data(shape, g, kind):
+    x = torch.randn(shape, generator=g, device="cuda")
+    return {"normal": x, "positive": x.abs(), "wide": x * torch.exp2(torch.randint(-20, 20, shape, generator=g, device="cuda").float())}[kind]
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("kind", ["normal", "positive", "wide"])
+@pytest.mark.parametrize("T,K,N,nk", [(12000, 256, 512, True), (12000, 250, 1028, False), (9000, 321, 1000, True), (9000, 324, 1012, False),
+                                      (7000, 1088, 272, False), (6000, 200, 2048, True)])
+def test_esmm_is_closer_than_the_fma_chain(T, K, N, nk, kind):
+    L, ops = _mods()
+    r, g = _routing(ops, T, 5, 2, K)
+    assert L.lib().hexa_esmm_f32_workspace_bytes(5, r.row_capacity, N, K) > 0
+    x = _data((T, K), g, kind)
+    w = torch.randn(5, N, K, generator=g, device="cuda")
+    if kind == "positive":
+        w = w.abs()
+    b = torch.randn(5, N, generator=g, device="cuda")
+    xs = ops.gather_rows(x, r)
+    wd, lay = (w, L.B_NK) if nk else (w.transpose(1, 2).contiguous(), L.B_KN)
+    n_pad = int(r.pad_offsets[-1])
+    po = r.pad_offsets.tolist()
+    exact = torch.zeros(n_pad, N, dtype=torch.float64, device="cuda")
+    for e in range(5):
+        exact[po[e]:po[e + 1]] = xs[po[e]:po[e + 1]].double() @ w[e].double().t()
+    got = ops.esmm(xs, wd, lay, r)[:n_pad]
+    chain = ops.esmm(xs, wd, lay, r, engine=L.ENGINE_SIMT)[:n_pad]
+    assert not torch.equal(got, chain)                      # the other path did run
+    assert _rel(got, exact) <= _rel(chain, exact) and _rel(got, exact) < 4e-7
+    live = r.row_token[:n_pad] >= 0
+    assert (got[~live] == 0).all()
+    exact[live] += b.double()[r.tile_expert[: n_pad // 128].repeat_interleave(128).long()][live]
+    # epilogues: both ways round the same formulas in fp32 from sums that close (1e-5 is the fp32 tolerance of the operators)
+    for epi, act in ((L.EPI_ACT, L.ACT_GELU), (L.EPI_ACT, L.ACT_SILU), (L.EPI_DACT, L.ACT_GELU), (L.EPI_DACT, L.ACT_RELU)):
+        outs = []
+        for eng in (L.ENGINE_AUTO, L.ENGINE_SIMT):
+            aux = ops.sorted_buffer(r.row_capacity, N, torch.float32, "cuda")
+            if epi == L.EPI_DACT:
+                aux.copy_(torch.randn(aux.shape, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda"))
+            y = ops.esmm(xs, wd, lay, r, b, epi, act, aux=aux, engine=eng)
+            outs.append((y[:n_pad], aux[:n_pad]))
+        (y0, a0), (y1, a1) = outs
+        assert (y0[~live] == 0).all()
+        assert float((y0 - y1).norm() / y1.norm()) < 3e-6 and float((a0 - a1).norm() / a1.norm()) < 3e-6
+        if epi == L.EPI_ACT:
+            assert _rel(a0, exact) <= _rel(a1, exact)
+
+
+@pytest.mark.parametrize("kind", ["normal", "positive", "wide"])
+@pytest.mark.parametrize("T,m,n,E", [(9000, 516, 1000, 4), (9000, 1001, 260, 7), (20000, 1001, 500, 7), (30000, 1000, 700, 3)])
+def test_estmm_is_closer_than_the_fma_chain(T, m, n, E, kind):
+    L, ops = _mods()
+    r, g = _routing(ops, T, E, 2, m)
+    assert L.lib().hexa_estmm_workspace_bytes(E, r.row_capacity, m, n, L.F32) > 0
+    p, q = ops.gather_rows(_data((T, m), g, kind), r), ops.gather_rows(_data((T, n), g, kind), r)
+    got = ops.estmm(p, q, r)
+    chain = ops.estmm(p, q, r, engine=L.ENGINE_SIMT)
+    po = r.pad_offsets.tolist()
+    exact = torch.stack([p[po[e]:po[e + 1]].double().t() @ q[po[e]:po[e + 1]].double() for e in range(E)])
+    if n % 4 == 0:
+        assert not torch.equal(got, chain)
+    assert _rel(got, exact) <= _rel(chain, exact) and _rel(got, exact) < 6e-7
+    assert (got[1] == 0).all() or E <= 2
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("where", ["a", "b"])
+def test_values_without_planes_take_the_fma_chain(bad, where):
+    L, ops = _mods()
+    T, K, N, E = 12000, 256, 512, 4
+    r, g = _routing(ops, T, E, 2, 3)
+    x = torch.randn(T, K, generator=g, device="cuda")
+    w = torch.randn(E, N, K, generator=g, device="cuda")
+    (x if where == "a" else w[2])[17, 5] = bad
+    xs = ops.gather_rows(x, r)
+    n_pad = int(r.pad_offsets[-1])
+    y1, y2 = torch.empty(r.row_capacity, N, device="cuda"), torch.empty(r.row_capacity, N, device="cuda")
+    got = ops.esmm(xs, w, L.B_NK, r, None, L.EPI_ACT, L.ACT_GELU, aux=y1)[:n_pad]
+    want = ops.esmm(xs, w, L.B_NK, r, None, L.EPI_ACT, L.ACT_GELU, aux=y2, engine=L.ENGINE_SIMT)[:n_pad]
+    assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), want.nan_to_num(7.0, 8.0, 9.0))
+    assert torch.equal(y1[:n_pad].nan_to_num(7.0, 8.0, 9.0), y2[:n_pad].nan_to_num(7.0, 8.0, 9.0))
+    dw, dw2 = ops.estmm(y1, xs, r), ops.estmm(y1, xs, r, engine=L.ENGINE_SIMT)
+    if where == "a":
+        assert torch.equal(dw.nan_to_num(7.0, 8.0, 9.0), dw2.nan_to_num(7.0, 8.0, 9.0))
+
+
+def test_tiny_values_keep_their_products():
+    """Terms that fall below bf16's normal range: the result stays as close as the FMA chain's."""
+    L, ops = _mods()
+    r, g = _routing(ops, 12000, 4, 2, 5)
+    x = torch.randn(12000, 256, generator=g, device="cuda") * 1e-30
+    w = torch.randn(4, 512, 256, generator=g, device="cuda")
+    xs = ops.gather_rows(x, r)
+    n_pad = int(r.pad_offsets[-1])
+    po = r.pad_offsets.tolist()
+    exact = torch.cat([xs[po[e]:po[e + 1]].double() @ w[e].double().t() for e in range(4)])
+    got = _rel(ops.esmm(xs, w, L.B_NK, r)[:n_pad], exact)
+    assert got <= _rel(ops.esmm(xs, w, L.B_NK, r, engine=L.ENGINE_SIMT)[:n_pad], exact)
