@@ -521,7 +521,7 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
     HEXA_LAUNCH_CHECK("epilogue_rows_kernel");
   }
   return esmm_simt_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token, E,
-                          row_cap, n_out, k, HEXA_F32, epilogue, act, stream, 0, E, flags, n_flags);
+                          row_cap, n_out, k, HEXA_F32, epilogue, act, stream, 0, E, 0, flags, n_flags);
 }
 
 int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets, int E, int64_t row_cap,

@@ -20,23 +20,25 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
 int estmm_f32_launch(const void* p, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets, int E, int64_t row_cap,
                      int64_t m, int64_t n, void* out, int64_t ldo, int64_t o_estride, cudaStream_t stream, void* workspace);
 // The CUDA-core launchers below can be told to do nothing unless one of `n_flags` device words is set (null: always run).
-int esmm_simt_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const float*, int64_t, void*, int64_t, void*,
+// (their bias, and that of esmm_tc_launch, is fp32 or, with bias16, of the data's 16-bit type)
+int esmm_simt_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const void*, int64_t, void*, int64_t, void*,
                      int64_t, const int32_t*, const int32_t*, const int32_t*, int, int64_t, int64_t, int64_t, int, int, int,
-                     cudaStream_t, int e_begin, int e_end, const int32_t* flags = nullptr, int n_flags = 0);
+                     cudaStream_t, int e_begin, int e_end, int bias16 = 0, const int32_t* flags = nullptr, int n_flags = 0);
 int estmm_simt_launch(const void*, int64_t, const void*, int64_t, const int32_t*, int, int64_t, int64_t, void*, int64_t,
                       int64_t, int64_t, int64_t, int, int, int, cudaStream_t, const int32_t* flags = nullptr, int n_flags = 0);
 bool esmm_tc_supported(const void*, int64_t, const void*, int64_t, int64_t, const void*, int64_t, const void*, int64_t,
                        const float*, int64_t, int64_t, int);
-int esmm_tc_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const float*, int64_t, void*, int64_t, void*,
+int esmm_tc_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const void*, int64_t, void*, int64_t, void*,
                    int64_t, const int32_t*, const int32_t*, const int32_t*, const int32_t*, int, int64_t, int64_t, int64_t, int,
-                   int, int, cudaStream_t, int e_begin, int e_end, float* colsum = nullptr);
+                   int, int, cudaStream_t, int e_begin, int e_end, int bias16, float* colsum = nullptr);
 bool estmm_tc_supported(const void*, int64_t, const void*, int64_t, const void*, int64_t, int64_t, int64_t, int64_t, int, int);
 int estmm_tc_launch(const void*, int64_t, const void*, int64_t, const int32_t*, int, int64_t, int64_t, int64_t, void*, int64_t,
                     int64_t, int64_t, int64_t, int, int, int, cudaStream_t, void* const* split_out = nullptr, int n_split = 0,
                     void* workspace = nullptr, size_t workspace_bytes = 0);
 size_t estmm_tc_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n);
 // rows.cu: both passes of ESS, and its second pass alone (per expert, the partial rows of its 128-row blocks added in order)
-int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int E, int64_t row_cap, int64_t cols, float* out,
-               int64_t ldo, int dtype, float* partial, cudaStream_t stream);
-int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, float* out, int64_t ldo, cudaStream_t stream);
+int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int E, int64_t row_cap, int64_t cols, void* out,
+               int64_t ldo, int out_dtype, int dtype, float* partial, cudaStream_t stream);
+int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, void* out, int64_t ldo, int out_dtype,
+               cudaStream_t stream);
 }  // namespace hexa

@@ -169,10 +169,11 @@ __device__ __forceinline__ bool wanted(const int32_t* __restrict__ flags, int n_
 template <typename T, int TILE, bool B_NK, bool VEC>
 __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
 esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, int64_t ldb,
-                 int64_t b_estride, const float* __restrict__ bias, int64_t ldbias, T* __restrict__ aux, int64_t ldaux,
+                 int64_t b_estride, const void* __restrict__ bias, int64_t ldbias, T* __restrict__ aux, int64_t ldaux,
                  T* __restrict__ c, int64_t ldc, const int32_t* __restrict__ tile_expert,
                  const int32_t* __restrict__ pad_offsets, const int32_t* __restrict__ row_token, int E, int64_t n_out,
-                 int64_t k, int epilogue, int act, int e_begin, int e_end, const int32_t* __restrict__ flags, int n_flags) {
+                 int64_t k, int epilogue, int act, int e_begin, int e_end, int bias16,
+                 const int32_t* __restrict__ flags, int n_flags) {
   if (!wanted(flags, n_flags)) return;
   const int64_t row0 = (int64_t)blockIdx.y * TILE;
   if (row0 >= pad_offsets[E]) return;
@@ -204,7 +205,10 @@ esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           float v = f[j];
-          if (bias && n + j < n_out) v += bias[(int64_t)e * ldbias + n + j];
+          if (bias && n + j < n_out) {
+            const int64_t at = (int64_t)e * ldbias + n + j;
+            v += bias16 ? to_f32<T>(static_cast<const T*>(bias)[at]) : static_cast<const float*>(bias)[at];
+          }
           y[j] = live ? v : 0.f;
           if (epilogue == HEXA_EPI_ACT) v = act_apply(act, v);
           else if (epilogue == HEXA_EPI_DACT) v = v * act_grad(act, x[j]);
@@ -274,10 +278,10 @@ bool use_large_tile(int64_t tiles128) { return tiles128 >= 2 * (int64_t)sm_count
 }  // namespace
 
 int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, int64_t ldb, int64_t b_estride,
-                     const float* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
+                     const void* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
                      const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token, int E,
                      int64_t row_cap, int64_t n_out, int64_t k, int dtype, int epilogue, int act, cudaStream_t stream,
-                     int e_begin, int e_end, const int32_t* flags, int n_flags) {
+                     int e_begin, int e_end, int bias16, const int32_t* flags, int n_flags) {
   if (row_cap == 0 || e_begin >= e_end) return HEXA_OK;
   if (e_begin < 0) e_begin = 0;
   HEXA_REQUIRE(row_cap / 64 <= 65535, "hexa_esmm (simt): row_capacity %lld too large", (long long)row_cap);
@@ -291,7 +295,7 @@ int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, in
   esmm_simt_kernel<T, TILE, NK, VEC><<<grid, kThreads, 0, stream>>>((const T*)a, lda, (const T*)b, ldb, b_estride, bias, \
                                                                     ldbias, (T*)aux, ldaux, (T*)c, ldc, tile_expert,   \
                                                                     pad_offsets, row_token, E, n_out, k, epilogue, act, \
-                                                                    e_begin, e_end, flags, n_flags)
+                                                                    e_begin, e_end, bias16, flags, n_flags)
 #define HEXA_ESMM_SIMT_T(T, VEC)                              \
   do {                                                        \
     if (large && nk) HEXA_ESMM_SIMT(T, 128, true, VEC);       \

@@ -64,8 +64,9 @@ struct Params {
   const int32_t* row_token;
   const int32_t* pair_block;   // CTAS = 2, ESMM: per pair tile (first 128-row block) * 2 + (second block belongs to the same expert), -1 ends the list
   int64_t max_pairs;
-  const float* bias;
+  const void* bias;
   int64_t ldbias;
+  int bias16;       // the bias is of the data's type instead of fp32
   void* aux;
   int64_t ldaux;
   void* c;          // ESMM: c ; ESTMM: out
@@ -568,7 +569,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int gi = q * 32 + lane;
       auto bias_of = [&](int expert, uint32_t tile_index) {
         const int64_t col = (int64_t)(tile_index % p.nt) * BN + part_col + gi;
-        return p.bias && gi < kPartCols && col < p.n ? __ldg(p.bias + (int64_t)expert * p.ldbias + col) : 0.f;
+        if (p.bias == nullptr || gi >= kPartCols || col >= p.n) return 0.f;
+        const int64_t at = (int64_t)expert * p.ldbias + col;
+        if (!p.bias16) return __ldg(static_cast<const float*>(p.bias) + at);
+        return unpack_lo(__ldg(static_cast<const uint16_t*>(p.bias) + at), is_bf16);
       };
       float bias_next = entry >= 0 && e >= 0 ? bias_of(e, t) : 0.f;
       while (ok && entry >= 0 && e >= 0) {
@@ -862,10 +866,10 @@ bool esmm_tc_supported(const void* a, int64_t lda, const void* b, int64_t ldb, i
 }
 
 int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int64_t ldb, int64_t b_estride,
-                   const float* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
+                   const void* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
                    const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token,
                    const int32_t* pair_block, int E, int64_t row_cap, int64_t n_out, int64_t k, int dtype, int epilogue,
-                   int act, cudaStream_t stream, int e_begin, int e_end, float* colsum) {
+                   int act, cudaStream_t stream, int e_begin, int e_end, int bias16, float* colsum) {
   if (row_cap == 0 || e_begin >= e_end) return HEXA_OK;
   const int is_bf16 = dtype == HEXA_BF16;
   const int BN = n_out > 128 ? 256 : 128;
@@ -909,7 +913,7 @@ int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int6
   Params p{};
   p.tile_expert = tile_expert; p.pad_offsets = pad_offsets; p.row_token = row_token;
   p.pair_block = pair_block; p.max_pairs = row_cap / (2 * BLOCK_M) + E;
-  p.bias = bias; p.ldbias = ldbias; p.aux = aux; p.ldaux = ldaux; p.c = c; p.ldc = ldc;
+  p.bias = bias; p.ldbias = ldbias; p.bias16 = bias16; p.aux = aux; p.ldaux = ldaux; p.c = c; p.ldc = ldc;
   p.n = n_out; p.k = k; p.m = 0; p.E = E; p.e_begin = e_begin; p.e_end = e_end;
   p.epilogue = epilogue; p.act = act; p.is_bf16 = is_bf16; p.colsum = colsum;
   p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();

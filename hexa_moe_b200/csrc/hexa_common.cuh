@@ -56,6 +56,13 @@ int tc_debug_flags();     // HEXA_TC_DEBUG / hexa_set_tc_debug
     }                                                                                \
   } while (0)
 
+// Splits a dtype argument into the data type and its flags; false when a flag comes with a type that is not 16 bits wide
+// or is none of `allowed`.
+inline bool take_flags(int& dtype, int allowed, int& flags) {
+  flags = dtype & ~0xff;
+  dtype &= 0xff;
+  return (flags & ~allowed) == 0 && (flags == 0 || dtype == HEXA_F16 || dtype == HEXA_BF16);
+}
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t dtype_size(int dt) { return dt == HEXA_F32 ? 4 : 2; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -88,6 +88,9 @@ int dt(const Tensor& t) {
   }
 }
 
+// A bias or sum operand is fp32 or of the data's own 16-bit type, which a flag on the dtype says.
+bool same16(const Tensor& t, const Tensor& data) { return t.scalar_type() == data.scalar_type() && data.scalar_type() != at::kFloat; }
+
 int64_t ld(const Tensor& t) {
   if (t.dim() != 2 || t.stride(1) != 1) fail("expected a 2-D tensor with unit inner stride");
   return t.stride(0);
@@ -152,12 +155,13 @@ Tensor gather_rows(const Tensor& src, const Tensor& row_token, const Tensor& pad
   return out;
 }
 
-std::tuple<Tensor, Tensor> gather_rows_ess(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap) {
+std::tuple<Tensor, Tensor> gather_rows_ess(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap, at::ScalarType sums_type) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
-  Tensor out = sorted_buffer(cap, cols, src.scalar_type(), src), sums = empty({E, cols}, at::kFloat, src);
+  Tensor out = sorted_buffer(cap, cols, src.scalar_type(), src), sums = empty({E, cols}, sums_type, src);
+  if (sums_type != at::kFloat && !same16(sums, src)) fail("gather_rows_ess: sums are float32 or of the data's 16-bit type");
   Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
-  const int type = dt(src);
+  const int type = dt(src) | (sums_type != at::kFloat ? HEXA_SUMS_16 : 0);
   const int64_t lds = ld(src), ldo = ld(out);
   call("hexa_gather_rows_ess", [&] {
     return api.hexa_gather_rows_ess(ptr(src), lds, i32(row_token), i32(pad_offsets), E, cap, cols, ptr(out), ldo,
@@ -176,12 +180,13 @@ Tensor combine_rows(const Tensor& src, const Tensor& token_row, int64_t T, int t
   return out;
 }
 
-Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
+Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_, at::ScalarType out_type) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
-  Tensor out = out_ ? *out_ : empty({E, cols}, at::kFloat, src);
+  Tensor out = out_ ? *out_ : empty({E, cols}, out_type, src);
+  if (out.scalar_type() != at::kFloat && !same16(out, src)) fail("ess: the result is float32 or of the data's 16-bit type");
   Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
-  const int type = dt(src);
+  const int type = dt(src) | (out.scalar_type() != at::kFloat ? HEXA_SUMS_16 : 0);
   const int64_t lds = ld(src), ldo = ld(out);
   call("hexa_ess", [&] {
     return api.hexa_ess(ptr(src), lds, i32(pad_offsets), E, cap, cols, static_cast<float*>(ptr(out)), ldo, type, ptr(ws), (size_t)ws.numel(), s);
@@ -194,12 +199,12 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
             const OptTensor& out_, int engine, int64_t n_out, int64_t k, int e0, int e1, const OptTensor& sums) {
   if (a.scalar_type() != b.scalar_type())
     fail(std::string("esmm: a is ") + c10::toString(a.scalar_type()) + " but b is " + c10::toString(b.scalar_type()));
-  if (bias && bias->scalar_type() != at::kFloat) fail("esmm: bias must be float32");
-  if (sums && (e0 != 0 || e1 != E || sums->scalar_type() != at::kFloat || sums->dim() != 2 || sums->size(0) != E || sums->size(1) != n_out ||
+  if (bias && bias->scalar_type() != at::kFloat && !same16(*bias, a)) fail("esmm: bias must be float32 or of the data's 16-bit type");
+  if (sums && (e0 != 0 || e1 != E || (sums->scalar_type() != at::kFloat && !same16(*sums, a)) || sums->dim() != 2 || sums->size(0) != E || sums->size(1) != n_out ||
                sums->stride(1) != 1))
-    fail("esmm: sums must be float32 [E, n_out] and needs the full expert range");
+    fail("esmm: sums must be [E, n_out], float32 or of the data's 16-bit type, and needs the full expert range");
   void* s = stream_of(a);
-  const int type = dt(a);
+  const int type = dt(a) | (bias && bias->scalar_type() != at::kFloat ? HEXA_BIAS_16 : 0);
   Tensor out = out_ ? *out_ : sorted_buffer(cap, n_out, a.scalar_type(), a);
   const int64_t lda = ld(a), ldo = ld(out), ldbias = bias ? ld(*bias) : 0, ldaux = aux ? ld(*aux) : 0;
   const float* bp = static_cast<const float*>(ptr(bias));
@@ -215,14 +220,15 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
                                  act, ptr(ws), (size_t)ws.numel(), s);
       });
     }
-    if (sums) ess(out, pad_offsets, E, cap, sums);
+    if (sums) ess(out, pad_offsets, E, cap, sums, at::kFloat);
     return out;
   }
   if (sums) {
+    const int sums_flag = sums->scalar_type() != at::kFloat ? HEXA_SUMS_16 : 0;
     Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, n_out), a);
     call("hexa_esmm_ess", [&] {
       return api.hexa_esmm_ess(ptr(a), lda, ptr(b), b_layout, b.stride(1), b.stride(0), bp, ldbias, ptr(aux), ldaux, ptr(out), ldo,
-                               i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, type, epilogue, act,
+                               i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, type | sums_flag, epilogue, act,
                                engine, static_cast<float*>(ptr(sums)), sums->stride(0), ptr(ws), (size_t)ws.numel(), s);
     });
     return out;

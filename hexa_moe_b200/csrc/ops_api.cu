@@ -38,6 +38,9 @@ extern "C" int hexa_esmm_experts(const void* a, int64_t lda, const void* b, int 
                                  int epilogue, int act, int engine, int expert_begin, int expert_end, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   HEXA_REQUIRE(a && b && c && tile_expert && pad_offsets, "hexa_esmm: null pointer");
+  int flags;
+  HEXA_REQUIRE(take_flags(dtype, HEXA_BIAS_16, flags), "hexa_esmm: bad dtype %d", dtype);
+  const int bias16 = flags != 0;
   HEXA_REQUIRE(expert_begin >= 0 && expert_begin <= expert_end && expert_end <= E,
                "hexa_esmm: expert range [%d, %d) is not inside [0, %d)", expert_begin, expert_end, E);
   HEXA_REQUIRE(E > 0 && row_cap >= 0 && row_cap % kRowTile == 0 && n_out > 0 && k > 0,
@@ -51,16 +54,16 @@ extern "C" int hexa_esmm_experts(const void* a, int64_t lda, const void* b, int 
   HEXA_REQUIRE(epilogue != HEXA_EPI_DACT || aux, "hexa_esmm: HEXA_EPI_DACT needs the saved pre-activation in aux");
   HEXA_REQUIRE(engine >= HEXA_ENGINE_AUTO && engine <= HEXA_ENGINE_SIMT, "hexa_esmm: bad engine %d", engine);
   HEXA_CHECK_DEVICE_STATUS("hexa_esmm");
-  const bool tc_ok = esmm_tc_supported(a, lda, b, ldb, b_estride, aux, ldaux, c, ldc, bias, ldbias, n_out, dtype);
+  const bool tc_ok = esmm_tc_supported(a, lda, b, ldb, b_estride, aux, ldaux, c, ldc, bias16 ? nullptr : bias, ldbias, n_out, dtype);
   if (engine == HEXA_ENGINE_TCGEN05 && !tc_ok) {
     set_error("hexa_esmm: tcgen05 engine needs 16-bit data, 16-byte aligned pointers and leading dimensions / n_out that are multiples of 8");
     return HEXA_ERR_UNSUPPORTED;
   }
   if (engine != HEXA_ENGINE_SIMT && tc_ok)
     return esmm_tc_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets,
-                          row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, stream, expert_begin, expert_end);
+                          row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, stream, expert_begin, expert_end, bias16);
   return esmm_simt_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets,
-                          row_token, E, row_cap, n_out, k, dtype, epilogue, act, stream, expert_begin, expert_end);
+                          row_token, E, row_cap, n_out, k, dtype, epilogue, act, stream, expert_begin, expert_end, bias16);
 }
 
 extern "C" int hexa_esmm(const void* a, int64_t lda, const void* b, int b_layout, int64_t ldb, int64_t b_estride,
@@ -106,18 +109,22 @@ extern "C" int hexa_esmm_ess(const void* a, int64_t lda, const void* b, int b_la
   cudaStream_t stream = (cudaStream_t)stream_;
   HEXA_REQUIRE(sums && workspace && ld_sums >= n_out, "hexa_esmm_ess: sums / workspace missing or ld_sums too small");
   HEXA_REQUIRE(E > 0 && E <= 65535 && row_cap >= 0 && n_out > 0, "hexa_esmm_ess: bad sizes");
+  const int with_bias_flag = dtype & ~HEXA_SUMS_16;
+  int flags;
+  HEXA_REQUIRE(take_flags(dtype, HEXA_BIAS_16 | HEXA_SUMS_16, flags), "hexa_esmm_ess: bad dtype %d", dtype);
+  const int bias16 = (flags & HEXA_BIAS_16) != 0, out_dtype = flags & HEXA_SUMS_16 ? dtype : HEXA_F32;
   const size_t need = hexa_ess_workspace_bytes(row_cap, n_out);
   if (workspace_bytes < need) {
     set_error("hexa_esmm_ess: workspace %zu bytes < required %zu", workspace_bytes, need);
     return HEXA_ERR_WORKSPACE;
   }
   const bool fused = a && b && c && engine != HEXA_ENGINE_SIMT &&
-                     esmm_tc_supported(a, lda, b, ldb, b_estride, aux, ldaux, c, ldc, bias, ldbias, n_out, dtype);
+                     esmm_tc_supported(a, lda, b, ldb, b_estride, aux, ldaux, c, ldc, bias16 ? nullptr : bias, ldbias, n_out, dtype);
   if (!fused) {   // same result in two passes: the GEMM, then ESS over its output
     int rc = hexa_esmm_experts(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets,
-                               row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, engine, 0, E, stream_);
+                               row_token, pair_block, E, row_cap, n_out, k, with_bias_flag, epilogue, act, engine, 0, E, stream_);
     if (rc != HEXA_OK) return rc;
-    return ess_launch(c, ldc, pad_offsets, E, row_cap, n_out, sums, ld_sums, dtype, (float*)workspace, stream);
+    return ess_launch(c, ldc, pad_offsets, E, row_cap, n_out, sums, ld_sums, out_dtype, dtype, (float*)workspace, stream);
   }
   // the checks of hexa_esmm_experts, then the tcgen05 launch with the block sums switched on
   HEXA_REQUIRE(tile_expert && pad_offsets, "hexa_esmm_ess: null pointer");
@@ -130,9 +137,9 @@ extern "C" int hexa_esmm_ess(const void* a, int64_t lda, const void* b, int b_la
   HEXA_REQUIRE(epilogue != HEXA_EPI_DACT || aux, "hexa_esmm_ess: HEXA_EPI_DACT needs the saved pre-activation in aux");
   HEXA_CHECK_DEVICE_STATUS("hexa_esmm_ess");
   int rc = esmm_tc_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets,
-                          row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, stream, 0, E, (float*)workspace);
+                          row_token, pair_block, E, row_cap, n_out, k, dtype, epilogue, act, stream, 0, E, bias16, (float*)workspace);
   if (rc != HEXA_OK) return rc;
-  return ess_finish((const float*)workspace, pad_offsets, E, n_out, sums, ld_sums, stream);
+  return ess_finish((const float*)workspace, pad_offsets, E, n_out, sums, ld_sums, out_dtype, stream);
 }
 
 extern "C" size_t hexa_estmm_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n, int dtype) {

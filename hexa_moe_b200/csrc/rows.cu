@@ -204,9 +204,10 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
 // 32 columns x 8 slices of the tiles per block, each slice in ascending order, then the slices in order: an expert with
 // 144 tiles is 18 dependent additions deep (one thread per column walked all of them: 13 us for [18432, 512] and its
 // hidden gradient, 5 us now).
+template <typename TO>
 __global__ void __launch_bounds__(256)
 ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
-                 int64_t cols, float* __restrict__ out, int64_t ldo) {
+                 int64_t cols, TO* __restrict__ out, int64_t ldo) {
   __shared__ float red[8][32];
   const int e = blockIdx.y;
   const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
@@ -222,7 +223,7 @@ ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ 
   if (slice == 0 && c < cols) {
 #pragma unroll
     for (int y = 1; y < 8; ++y) s += red[y][cx];
-    out[(int64_t)e * ldo + c] = s;
+    out[(int64_t)e * ldo + c] = from_f32<TO>(s);
   }
 }
 
@@ -293,10 +294,10 @@ extern "C" size_t hexa_ess_workspace_bytes(int64_t row_cap, int64_t cols) {
 }
 
 namespace hexa {
-int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, float* out, int64_t ldo, cudaStream_t stream);
+int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, void* out, int64_t ldo, int out_dtype, cudaStream_t stream);
 // Shared by hexa_ess and the entry points built on it: both passes on caller-provided scratch.
 int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int E, int64_t row_cap, int64_t cols,
-               float* out, int64_t ldo, int dtype, float* partial, cudaStream_t stream) {
+               void* out, int64_t ldo, int out_dtype, int dtype, float* partial, cudaStream_t stream) {
   const int64_t tiles = ceil_div(row_cap, kRowTile);
   if (tiles > 0) {
     const int V = 16 / (int)dtype_size(dtype);
@@ -313,12 +314,15 @@ int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int 
 #undef HEXA_ESS
     HEXA_LAUNCH_CHECK("ess_partial");
   }
-  return ess_finish(partial, pad_offsets, E, cols, out, ldo, stream);
+  return ess_finish(partial, pad_offsets, E, cols, out, ldo, out_dtype, stream);
 }
 
-int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, float* out, int64_t ldo, cudaStream_t stream) {
+int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, void* out, int64_t ldo, int out_dtype,
+               cudaStream_t stream) {
   dim3 grid2((unsigned)ceil_div(cols, 32), (unsigned)E);
-  ess_final_kernel<<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, out, ldo);
+  if (out_dtype == HEXA_F16) ess_final_kernel<__half><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (__half*)out, ldo);
+  else if (out_dtype == HEXA_BF16) ess_final_kernel<__nv_bfloat16><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (__nv_bfloat16*)out, ldo);
+  else ess_final_kernel<float><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (float*)out, ldo);
   HEXA_LAUNCH_CHECK("ess_final");
   return HEXA_OK;
 }
@@ -331,7 +335,10 @@ extern "C" int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32
   HEXA_REQUIRE(row_token && pad_offsets && dst && sums && workspace, "hexa_gather_rows_ess: null pointer");
   HEXA_REQUIRE(E > 0 && E <= 65535 && row_cap >= 0 && cols > 0 && src_ld >= cols && dst_ld >= cols && ld_sums >= cols,
                "hexa_gather_rows_ess: bad sizes");
-  HEXA_REQUIRE(dtype == HEXA_F32 || dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gather_rows_ess: bad dtype %d", dtype);
+  int flags;
+  const bool dtype_ok = take_flags(dtype, HEXA_SUMS_16, flags);
+  HEXA_REQUIRE(dtype_ok && (dtype == HEXA_F32 || dtype == HEXA_F16 || dtype == HEXA_BF16), "hexa_gather_rows_ess: bad dtype %d", dtype);
+  const int out_dtype = flags ? dtype : HEXA_F32;
   HEXA_REQUIRE(aligned16(dst), "hexa_gather_rows_ess: dst must be 16-byte aligned");
   const size_t need = hexa_ess_workspace_bytes(row_cap, cols);
   if (workspace_bytes < need) {
@@ -345,7 +352,7 @@ extern "C" int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32
   if (!one) {
     const int rc = hexa_gather_rows(src, src_ld, row_token, pad_offsets, E, row_cap, cols, dst, dst_ld, dtype, stream_);
     if (rc != HEXA_OK) return rc;
-    return ess_launch(dst, dst_ld, pad_offsets, E, row_cap, cols, sums, ld_sums, dtype, (float*)workspace, stream);
+    return ess_launch(dst, dst_ld, pad_offsets, E, row_cap, cols, sums, ld_sums, out_dtype, dtype, (float*)workspace, stream);
   }
   dim3 grid((unsigned)ceil_div(cols, kEssCx * V), (unsigned)tiles);
 #define HEXA_GATHER_ESS(T)                                                                                                   \
@@ -356,13 +363,15 @@ extern "C" int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32
   else HEXA_GATHER_ESS(__nv_bfloat16);
 #undef HEXA_GATHER_ESS
   HEXA_LAUNCH_CHECK("gather_rows_ess");
-  return ess_finish((const float*)workspace, pad_offsets, E, cols, sums, ld_sums, stream);
+  return ess_finish((const float*)workspace, pad_offsets, E, cols, sums, ld_sums, out_dtype, stream);
 }
 
 extern "C" int hexa_ess(const void* src, int64_t src_ld, const int32_t* pad_offsets, int E, int64_t row_cap,
                         int64_t cols, float* out, int64_t ldo, int dtype, void* workspace, size_t workspace_bytes,
                         void* stream_) {
   HEXA_REQUIRE(src && pad_offsets && out && workspace, "hexa_ess: null pointer");
+  int flags;
+  HEXA_REQUIRE(take_flags(dtype, HEXA_SUMS_16, flags), "hexa_ess: bad dtype %d", dtype);
   HEXA_REQUIRE(E > 0 && E <= 65535 && row_cap >= 0 && cols > 0 && src_ld >= cols && ldo >= cols, "hexa_ess: bad sizes");
   HEXA_REQUIRE(aligned16(src), "hexa_ess: src must be 16-byte aligned");
   const size_t need = hexa_ess_workspace_bytes(row_cap, cols);
@@ -370,7 +379,7 @@ extern "C" int hexa_ess(const void* src, int64_t src_ld, const int32_t* pad_offs
     set_error("hexa_ess: workspace %zu bytes < required %zu", workspace_bytes, need);
     return HEXA_ERR_WORKSPACE;
   }
-  return ess_launch(src, src_ld, pad_offsets, E, row_cap, cols, out, ldo, dtype, (float*)workspace, (cudaStream_t)stream_);
+  return ess_launch(src, src_ld, pad_offsets, E, row_cap, cols, out, ldo, flags ? dtype : HEXA_F32, dtype, (float*)workspace, (cudaStream_t)stream_);
 }
 
 // ---- ESS on library-owned scratch -------------------------------------------------------------------
@@ -408,5 +417,5 @@ extern "C" int hexa_ess_static(const void* src, int64_t src_ld, const int32_t* p
     __atomic_store_n(&dev_addr[dev], scratch, __ATOMIC_RELEASE);
   }
   // Nothing in the scratch has to start at zero: pass 1 overwrites every partial row that pass 2 reads.
-  return ess_launch(src, src_ld, pad_offsets, E, row_cap, cols, out, ldo, dtype, scratch, (cudaStream_t)stream_);
+  return ess_launch(src, src_ld, pad_offsets, E, row_cap, cols, out, ldo, HEXA_F32, dtype, scratch, (cudaStream_t)stream_);
 }

@@ -225,6 +225,11 @@ def _cast(w: Optional[Tensor], dtype) -> Optional[Tensor]:
     return w if w.dtype == dtype else w.to(dtype)
 
 
+def _common_dtype(b1, b2):
+    """The dtype of the biases there are, None when they differ."""
+    return b1 or b2 if b1 is None or b2 is None or b1 == b2 else None
+
+
 # ------------------------------------------------------------------------------------------------
 # dense FFN (the layers either side of every MoE layer)
 # ------------------------------------------------------------------------------------------------
@@ -279,7 +284,8 @@ class MLP_Implement(torch.autograd.Function):
             (w1, w2), st = ctx.w, ctx.state
             ctx.state = ctx.w = None
             dx, dw1, dw2, db1, db2 = cfg.backend.dense_backward(st, dy.contiguous(), w1, w2, cfg.act_id,
-                                                                has_b1=ctx.has_b1, has_b2=ctx.has_b2)
+                                                                has_b1=ctx.has_b1, has_b2=ctx.has_b2,
+                                                                bias_grad_dtype=_common_dtype(*ctx.param_dtypes[2:]))
             pd = ctx.param_dtypes
             dw1, dw2 = dw1.to(pd[0]), dw2.to(pd[1])
             db1 = None if db1 is None else db1.to(pd[2])
@@ -417,7 +423,9 @@ class FusedMoE_Shared_CudaCore(torch.autograd.Function):
             # reduce-scatter reads (no packing pass)
             packed = W > 1 and x_is_cuda(dy) and _is_nccl(cfg.group) and all(s_ == split[0] for s_ in split)
             kw = dict(ranks=W) if packed else {}
-            kw2 = dict(kw, dw_out=cfg.cache.grad_buffer("fc2", stage)) if packed else {}
+            if W == 1 and x_is_cuda(dy):
+                kw["bias_grad_dtype"] = _common_dtype(b1_dt, b2_dt)
+            kw2 = dict(kw, dw_out=cfg.cache.grad_buffer("fc2", stage)) if packed else dict(kw)
             dh, dw2, db2 = be.moe_backward_fc2(st, dy, w2, cfg.act_id, has_b2=ctx.has_b2, grad_dtype=w2_dt, want_db1=ctx.has_b1, **kw2)
             # By default the reduced gradients are added to the parameters' .grad by a callback at the end of the
             # backward pass (nothing waits for the transfer); HEXA_DEFER_GRADS=0 returns them through autograd instead

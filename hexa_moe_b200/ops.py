@@ -110,14 +110,14 @@ def gather_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = Non
                 (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity, out))
 
 
-def gather_rows_ess(src: torch.Tensor, r: Routing):
+def gather_rows_ess(src: torch.Tensor, r: Routing, sums_dtype: torch.dtype = torch.float32):
     """(gather_rows(src), ess of the result) from one pass over the rows."""
     global LAUNCHES
     if r.align % L.ROW_TILE:
         raise L.HexaError("gather_rows_ess: routing must be aligned to 128 rows")
     LAUNCHES += 1          # the second pass of ESS over the tile sums
     return _run("gather", 2.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().gather_rows_ess,
-                (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity))
+                (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity, sums_dtype))
 
 
 def combine_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -133,8 +133,8 @@ def esmm(a: torch.Tensor, b: torch.Tensor, b_layout: int, r: Routing, bias: Opti
          sums: Optional[torch.Tensor] = None) -> torch.Tensor:
     """c[row] = a[row] x b[expert(row)] with the fused epilogue.  b: [E, n_out, k] (B_NK) or [E, k, n_out] (B_KN);
     b may be a view with arbitrary expert / row strides (unit inner stride).  experts = (first, end): only the rows of
-    those experts are computed (the other rows of `out` are left as they are).  sums: a float32 [E, n_out] tensor that
-    receives the per-expert column sums of the output (ESS of `out`) from the same launch."""
+    those experts are computed (the other rows of `out` are left as they are).  bias: [E, n_out], float32 or of a's 16-bit
+    type.  sums: an [E, n_out] tensor, float32 or of a's 16-bit type, that receives the per-expert column sums of the output (ESS of `out`) from the same launch."""
     global LAUNCHES
     if r.align % L.ROW_TILE:
         raise L.HexaError("esmm: routing must be aligned to 128 rows")
@@ -218,12 +218,12 @@ def mean_slices(local: torch.Tensor, recv: torch.Tensor, n_recv: int, world: int
           "hexa_mean_slices")
 
 
-def ess(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out[e] = sum of expert e's rows of src, float32 [E, cols]."""
+def ess(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    """out[e] = sum of expert e's rows of src, [E, cols], float32 or (rounded once at the end) of src's 16-bit type."""
     if r.align % L.ROW_TILE:
         raise L.HexaError("ess: routing must be aligned to 128 rows")
     return _run("ess", 1.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().ess,
-                (src, r.pad_offsets, r.num_experts, r.row_capacity, out))
+                (src, r.pad_offsets, r.num_experts, r.row_capacity, out, out_dtype))
 
 
 def mask_pad_rows(buf: torch.Tensor, r: Routing) -> torch.Tensor:
@@ -328,6 +328,18 @@ def _f32(t):
     return out[..., :n]
 
 
+def _bias(t, x):
+    """Bias as the epilogue reads it: as it is when it has the 16-bit type of the data, else in fp32."""
+    if t is not None and t.dtype == x.dtype and x.dtype != torch.float32 and t.stride(-1) == 1:
+        return t.detach()
+    return _f32(t)
+
+
+def _sums_dtype(wanted, data):
+    """Bias gradients are summed in float32; they leave in `wanted` when the kernels can round to it themselves."""
+    return wanted if wanted is not None and wanted == data.dtype else torch.float32
+
+
 def moe_forward(x, ids, w1, w2, b1, b2, act_id: int, act_fn=None, route_major=False, engine=L.ENGINE_AUTO,
                 need_state=True, before_fc2=None, fc1_groups=None):
     """y[t] = sum_j fc2(act(fc1(x[t]; e_j)); e_j).  x [T,d]; ids int32 [T,k] ([k,T] if route_major);
@@ -340,7 +352,7 @@ def moe_forward(x, ids, w1, w2, b1, b2, act_id: int, act_fn=None, route_major=Fa
     E = w1.shape[0]
     r = route(ids, E, L.ROW_TILE, route_major=route_major)
     xs = gather_rows(x, r)
-    b1f, b2f = _f32(b1), _f32(b2)
+    b1f, b2f = _bias(b1, x), _bias(b2, x)
     H = w1.shape[1]
     y1 = sorted_buffer(r.row_capacity, H, x.dtype, x.device)
     g = None
@@ -372,25 +384,27 @@ def moe_forward(x, ids, w1, w2, b1, b2, act_id: int, act_fn=None, route_major=Fa
     return y, (LayerState(r, xs, y1, h, g) if need_state else None)
 
 
-def _hidden_gradient(st: LayerState, dys, w2, act_id: int, engine, want_db1: bool):
+def _hidden_gradient(st: LayerState, dys, w2, act_id: int, engine, want_db1: bool, sums_dtype=torch.float32):
     """dh = dys W2^T * act'(y1) for a fused activation; with want_db1 the same launch leaves ESS(dh) in st.db1."""
     r = st.routing
     st.db1 = None
     if want_db1 and os.environ.get("HEXA_FUSED_ESS", "1") != "0":
-        st.db1 = torch.empty(r.num_experts, w2.shape[1], dtype=torch.float32, device=dys.device)
+        st.db1 = torch.empty(r.num_experts, w2.shape[1], dtype=sums_dtype, device=dys.device)
     return esmm(dys, w2, L.B_NK, r, None, L.EPI_DACT, act_id, aux=st.y1, engine=engine, tag="fc2_dgrad_dact", sums=st.db1)
 
 
 def moe_backward_fc2(st: LayerState, dy, w2, act_id: int, has_b2=True, grad_dtype=None, engine=L.ENGINE_AUTO, ranks=1,
-                     dw_out=None, want_db1=False):
+                     dw_out=None, want_db1=False, bias_grad_dtype=None):
     """First half of the layer backward: (dh [cap,H] = dy W2^T * act'(y1), dw2 [E,H,d_out], db2 [E,d_out] | None).
     Split from the fc1 half so a caller can start reducing dw2/db2 across ranks while fc1 runs.  want_db1: the fc1
-    half will need the bias gradient ESS(dh); with a fused activation the GEMM that writes dh sums it on the way."""
+    half will need the bias gradient ESS(dh); with a fused activation the GEMM that writes dh sums it on the way.
+    bias_grad_dtype: bias gradients leave in this type where that is the data's own 16-bit type, else in float32."""
     r = st.routing
-    dys, db2 = gather_rows_ess(dy.contiguous(), r) if has_b2 else (gather_rows(dy.contiguous(), r), None)
+    sums = _sums_dtype(bias_grad_dtype, dy)
+    dys, db2 = gather_rows_ess(dy.contiguous(), r, sums) if has_b2 else (gather_rows(dy.contiguous(), r), None)
     dw2 = estmm(st.h, dys, r, out_dtype=grad_dtype, engine=engine, ranks=ranks, out=dw_out, tag="dw2")
     if act_id >= 0:
-        dh = _hidden_gradient(st, dys, w2, act_id, engine, want_db1)
+        dh = _hidden_gradient(st, dys, w2, act_id, engine, want_db1, sums)
     else:
         dh = esmm(dys, w2, L.B_NK, r, None, L.EPI_LINEAR, engine=engine, tag="fc2_dgrad")
         dh.mul_(st.act_grad)
@@ -399,12 +413,12 @@ def moe_backward_fc2(st: LayerState, dy, w2, act_id: int, has_b2=True, grad_dtyp
 
 
 def moe_backward_fc1(st: LayerState, dh, w1, has_b1=True, grad_dtype=None, engine=L.ENGINE_AUTO, ranks=1,
-                     after_dw=None, dw_out=None):
+                     after_dw=None, dw_out=None, bias_grad_dtype=None):
     """Second half: (dx [T,d], dw1 [E,H,d], db1 [E,H] | None) from dh.  after_dw(dw1, db1), if given, is called on the
     host as soon as both parameter gradients are enqueued, before the input-gradient GEMM: a caller can start
     reducing them across ranks while that GEMM runs."""
     r = st.routing
-    db1 = (st.db1 if st.db1 is not None else ess(dh, r)) if has_b1 else None
+    db1 = (st.db1 if st.db1 is not None else ess(dh, r, out_dtype=_sums_dtype(bias_grad_dtype, dh))) if has_b1 else None
     st.db1 = None
     dw1 = estmm(dh, st.xs, r, out_dtype=grad_dtype, engine=engine, ranks=ranks, out=dw_out, tag="dw1")
     if after_dw is not None:
@@ -495,26 +509,28 @@ def dense_forward(x, w1, w2, b1, b2, act_id: int, need_state=True, engine=L.ENGI
     r = dense_routing(T, x.device)
     xs = _dense_rows(x, r)
     y1 = sorted_buffer(r.row_capacity, w1.shape[0], x.dtype, x.device)
-    h = esmm(xs, w1.unsqueeze(0), L.B_NK, r, None if b1 is None else _f32(b1).unsqueeze(0), L.EPI_ACT, act_id, aux=y1,
+    h = esmm(xs, w1.unsqueeze(0), L.B_NK, r, None if b1 is None else _bias(b1, x).unsqueeze(0), L.EPI_ACT, act_id, aux=y1,
              engine=engine)
-    ys = esmm(h, w2.unsqueeze(0), L.B_KN, r, None if b2 is None else _f32(b2).unsqueeze(0), L.EPI_LINEAR, engine=engine)
+    ys = esmm(h, w2.unsqueeze(0), L.B_KN, r, None if b2 is None else _bias(b2, x).unsqueeze(0), L.EPI_LINEAR, engine=engine)
     return ys[:T], (LayerState(r, xs, y1, h, None) if need_state else None)
 
 
-def dense_backward(st: LayerState, dy, w1, w2, act_id: int, has_b1=True, has_b2=True, grad_dtype=None, engine=L.ENGINE_AUTO):
+def dense_backward(st: LayerState, dy, w1, w2, act_id: int, has_b1=True, has_b2=True, grad_dtype=None, engine=L.ENGINE_AUTO,
+                   bias_grad_dtype=None):
     """Gradients of dense_forward: (dx [T,d], dw1 [H,d], dw2 [H,d_out], db1 [H] | None, db2 [d_out] | None);
-    bias gradients are float32."""
+    bias gradients are float32, or bias_grad_dtype where that is the data's own 16-bit type."""
+    sums = _sums_dtype(bias_grad_dtype, dy)
     r = st.routing
     T = r.num_tokens
     if has_b2 and dy.shape[0] != r.row_capacity:
-        dys, db2 = gather_rows_ess(dy.contiguous(), r)
+        dys, db2 = gather_rows_ess(dy.contiguous(), r, sums)
     else:
         dys = _dense_rows(dy, r)
-        db2 = ess(dys, r) if has_b2 else None
+        db2 = ess(dys, r, out_dtype=sums) if has_b2 else None
     db2 = None if db2 is None else db2.view(-1)
     dw2 = estmm(st.h, dys, r, out_dtype=grad_dtype, engine=engine)[0]
-    dh = _hidden_gradient(st, dys, w2.unsqueeze(0), act_id, engine, has_b1)
-    db1 = (st.db1 if st.db1 is not None else ess(dh, r)).view(-1) if has_b1 else None
+    dh = _hidden_gradient(st, dys, w2.unsqueeze(0), act_id, engine, has_b1, sums)
+    db1 = (st.db1 if st.db1 is not None else ess(dh, r, out_dtype=sums)).view(-1) if has_b1 else None
     st.db1 = None
     dw1 = estmm(dh, st.xs, r, out_dtype=grad_dtype, engine=engine)[0]
     dxs = esmm(dh, w1.unsqueeze(0), L.B_KN, r, None, L.EPI_LINEAR, engine=engine)

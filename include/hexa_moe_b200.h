@@ -40,6 +40,11 @@ typedef enum {
 } hexa_status;
 
 typedef enum { HEXA_F32 = 0, HEXA_F16 = 1, HEXA_BF16 = 2 } hexa_dtype;
+/* Added to a 16-bit dtype argument: the fp32 operand in question holds values of that dtype instead (the pointer is cast,
+ * leading dimensions count its elements).  Accumulation is fp32 either way.
+ *   HEXA_BIAS_16  bias of hexa_esmm / hexa_esmm_experts / hexa_esmm_ess (no padding or alignment of its rows is needed)
+ *   HEXA_SUMS_16  sums / out of hexa_ess, hexa_gather_rows_ess and hexa_esmm_ess, rounded once from the fp32 sums */
+enum { HEXA_BIAS_16 = 0x100, HEXA_SUMS_16 = 0x200 };
 
 /* Activation fused into the ESMM epilogue (HEXA_ACT_NONE: plain linear). */
 typedef enum {

@@ -545,3 +545,35 @@ def test_gather_with_sums_is_gather_then_ess(ops, dtype, T, cols):
         tok = r.row_token[r.pad_offsets[e]: r.pad_offsets[e + 1]].long()
         seg = x[tok[tok >= 0]].double()
         assert ((sums[e].double() - seg.sum(0)).abs() <= seg.abs().sum(0) * (len(seg) * 2.0 ** -24) + 1e-30).all()
+
+
+# Biases and column sums of the data's own 16-bit type: the same values as the fp32 operands holding them / rounded once.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("K,N,engine", [(64, 264, "auto"), (72, 203, "auto"), (37, 41, "auto"), (64, 100, "simt"), (64, 96, "auto")])
+def test_16_bit_bias_and_sums(ops, dtype, K, N, engine):
+    Lb = L()
+    eng = Lb.ENGINE_SIMT if engine == "simt" else Lb.ENGINE_AUTO
+    T, k, E = 900, 2, 5
+    r = ops.route(make_ids(T, k, E, 21, skew=True, empty=(1,)).cuda(), E)
+    g = torch.Generator().manual_seed(N)
+    xs = ops.gather_rows(torch.randn(T, K, generator=g).to(dtype).cuda(), r)
+    w = torch.randn(E, N, K, generator=g).to(dtype).cuda()
+    wide = torch.randn(E, N + 3, generator=g).to(dtype).cuda()
+    n_pad = int(r.pad_offsets[-1])
+    for b in (wide[:, :N], wide[:, 1:N + 1]):                       # rows that start and end anywhere
+        outs = []
+        for bias in (b, ops._f32(b)):
+            s16, s32 = (torch.empty(E, N, dtype=t, device="cuda") for t in (dtype, torch.float32))
+            y = ops.esmm(xs, w, Lb.B_NK, r, bias, Lb.EPI_ACT, Lb.ACT_GELU, engine=eng, sums=s32)
+            y2 = ops.esmm(xs, w, Lb.B_NK, r, bias, Lb.EPI_ACT, Lb.ACT_GELU, engine=eng, sums=s16)
+            assert torch.equal(y[:n_pad], y2[:n_pad]) and torch.equal(s16, s32.to(dtype))
+            outs.append((y[:n_pad], s32))
+        assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert torch.equal(ops.ess(xs, r, out_dtype=dtype), ops.ess(xs, r).to(dtype))
+    x = torch.randn(T, K, generator=g).to(dtype).cuda()
+    assert torch.equal(ops.gather_rows_ess(x, r, dtype)[1], ops.gather_rows_ess(x, r)[1].to(dtype))
+    with pytest.raises(Lb.HexaError):
+        ops.ess(xs, r, out_dtype=torch.float64)
+    f = torch.zeros(r.row_capacity, 8, device="cuda")
+    with pytest.raises(Lb.HexaError):
+        ops.ess(f, r, out_dtype=torch.bfloat16)                     # only the data's own type
