@@ -208,7 +208,8 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
   Tensor out = out_ ? *out_ : sorted_buffer(cap, n_out, a.scalar_type(), a);
   const int64_t lda = ld(a), ldo = ld(out), ldbias = bias ? ld(*bias) : 0, ldaux = aux ? ld(*aux) : 0;
   const float* bp = static_cast<const float*>(ptr(bias));
-  const size_t planes = type == HEXA_F32 && engine == HEXA_ENGINE_AUTO && pair_block && e0 == 0 && e1 == E
+  const bool relu = epilogue == HEXA_EPI_ACT && act == HEXA_ACT_RELU;      // stays with the FMA chain, see hexa_esmm_f32
+  const size_t planes = type == HEXA_F32 && engine == HEXA_ENGINE_AUTO && pair_block && e0 == 0 && e1 == E && !relu
                             ? api.hexa_esmm_f32_workspace_bytes(E, cap, n_out, k) : 0;
   if (planes) {
     {

@@ -84,13 +84,16 @@ extern "C" int hexa_esmm_f32(const float* a, int64_t lda, const float* b, int b_
                              const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token,
                              const int32_t* pair_block, int E, int64_t row_cap, int64_t n_out, int64_t k, int epilogue, int act,
                              void* workspace, size_t workspace_bytes, void* stream_) {
-  // one result, two engines: the tensor cores need scratch, 16-byte rows to store to and the pair-tile list
+  // one result, two engines: the tensor cores need scratch, 16-byte rows to store to and the pair-tile list.  A ReLU's
+  // pre-activations stay with the FMA chain: its derivative jumps at zero, so two roundings of a sum that ends within 1e-7
+  // of zero give different gradient masks, and which kernel computes a call depends on its size.
   const size_t need = esmm_f32_workspace_bytes(E, row_cap, n_out, k);
   const bool planes = need > 0 && workspace && workspace_bytes >= need && aligned16(workspace) && a && b && c && tile_expert && pad_offsets &&
                       pair_block && row_cap % kRowTile == 0 && lda >= k && ldc >= n_out && (!aux || ldaux >= n_out) &&
                       (!bias || ldbias >= n_out) && (b_layout == HEXA_B_NK || b_layout == HEXA_B_KN) &&
                       ldb >= (b_layout == HEXA_B_NK ? k : n_out) && epilogue >= HEXA_EPI_LINEAR && epilogue <= HEXA_EPI_DACT &&
-                      act >= HEXA_ACT_NONE && act <= HEXA_ACT_SILU && (epilogue != HEXA_EPI_DACT || aux) && aligned16(c) && ldc % 4 == 0 &&
+                      act >= HEXA_ACT_NONE && act <= HEXA_ACT_SILU && (epilogue != HEXA_EPI_DACT || aux) &&
+                      !(epilogue == HEXA_EPI_ACT && act == HEXA_ACT_RELU) && aligned16(c) && ldc % 4 == 0 &&
                       (epilogue != HEXA_EPI_ACT || !aux || (aligned16(aux) && ldaux % 4 == 0));
   if (!planes)      // also the place where bad arguments are refused
     return hexa_esmm_experts(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token,

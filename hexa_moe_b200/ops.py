@@ -367,7 +367,9 @@ def moe_forward(x, ids, w1, w2, b1, b2, act_id: int, act_fn=None, route_major=Fa
         for e0, e1, ready in groups:
             if ready is not None:
                 ready()
-            esmm(xs, w1, L.B_NK, r, b1f, L.EPI_LINEAR, out=y1, engine=engine, tag="fc1_forward", experts=(e0, e1))
+            # an unknown activation may have kinks: its fp32 pre-activations are FMA chains at every size, as a ReLU's are
+            esmm(xs, w1, L.B_NK, r, b1f, L.EPI_LINEAR, out=y1, tag="fc1_forward", experts=(e0, e1),
+                 engine=L.ENGINE_SIMT if engine == L.ENGINE_AUTO and x.dtype == torch.float32 else engine)
         if need_state:
             with torch.enable_grad():
                 yy = y1.detach().requires_grad_(True)

@@ -126,3 +126,15 @@ def test_tiny_values_keep_their_products():
     exact = torch.cat([xs[po[e]:po[e + 1]].double() @ w[e].double().t() for e in range(4)])
     got = _rel(ops.esmm(xs, w, L.B_NK, r)[:n_pad], exact)
     assert got <= _rel(ops.esmm(xs, w, L.B_NK, r, engine=L.ENGINE_SIMT)[:n_pad], exact)
+
+
+def test_relu_masks_do_not_depend_on_the_path():
+    L, ops = _mods()
+    r, g = _routing(ops, 12000, 5, 2, 9)
+    x = torch.randn(12000, 256, generator=g, device="cuda")
+    w = torch.randn(5, 512, 256, generator=g, device="cuda")
+    xs = ops.gather_rows(x, r)
+    n_pad = int(r.pad_offsets[-1])
+    a = [torch.empty(r.row_capacity, 512, device="cuda") for _ in range(2)]
+    y = [ops.esmm(xs, w, L.B_NK, r, None, L.EPI_ACT, L.ACT_RELU, aux=a[i], engine=e)[:n_pad] for i, e in enumerate((L.ENGINE_AUTO, L.ENGINE_SIMT))]
+    assert torch.equal(y[0], y[1]) and torch.equal(a[0][:n_pad], a[1][:n_pad])
