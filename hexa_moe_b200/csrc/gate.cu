@@ -343,6 +343,145 @@ sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int
   }
 }
 
+// ---- the gate projection of few tokens, straight on the CUDA cores -----------------------------------------------------
+// logits = x W^T with x 16-bit [T, d], W fp32 [E, d] and fp32 FMAs: for small T the split operands' three launches (or, for
+// fp16 tokens, a cast and an fp32 GEMM with too few blocks) cost more than the products.  A warp takes 4 tokens x 4 experts,
+// its lanes 8 consecutive elements of every 256 of d, so an operand value loaded once meets four of the other side, and the 16
+// sums meet in 16 shuffles.  Bound: the latency of d / 256 rounds of loads.  [2048, 768], 8 experts: 4 us (fp16 with a
+// cast and a GEMM 22, bf16 in split terms 7 in three launches); [16, 1024], 32 experts: 4 us (split terms 7).
+template <typename T>
+__device__ __forceinline__ void load8(const T* __restrict__ p, bool live, float (&v)[8]) {
+  uint4 raw = make_uint4(0, 0, 0, 0);
+  if (live) raw = __ldg(reinterpret_cast<const uint4*>(p));
+  const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(e[i]);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128)
+gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restrict__ w, int64_t tokens, int E, int64_t d, float* __restrict__ logits) {
+  const int lane = threadIdx.x & 31;
+  const int64_t groups = (E + 3) / 4;
+  const int64_t tile = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int64_t t0 = tile / groups * 4;
+  const int e0 = (int)(tile % groups) * 4;
+  if (t0 >= tokens) return;      // uniform across the warp
+  float acc[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+  for (int64_t c = lane * 8; c < d; c += 256) {
+    float xv[4][8];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) load8<T>(x + (t0 + a) * ldx + c, t0 + a < tokens, xv[a]);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+      if (e0 + b < E) {
+        lo = __ldg(reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c));
+        hi = __ldg(reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c + 4));
+      }
+      const float wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[a * 4 + b] = fmaf(xv[a][i], wv[i], acc[a * 4 + b]);
+    }
+  }
+  // sums over the lanes, halving the values a lane is responsible for: lane l ends with value l / 2
+#pragma unroll
+  for (int o = 16; o >= 2; o >>= 1) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int i = 0; i < o / 2; ++i) {
+      const float mine = upper ? acc[i + o / 2] : acc[i], theirs = upper ? acc[i] : acc[i + o / 2];
+      acc[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+    }
+  }
+  const float sum = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+  const int v = lane >> 1;
+  const int64_t t = t0 + (v >> 2);
+  const int e = e0 + (v & 3);
+  if ((lane & 1) == 0 && t < tokens && e < E) logits[t * E + e] = sum;
+}
+
+// dx = g W, 16-bit [T, d]: a thread owns 8 columns of 4 tokens
+template <typename T>
+__global__ void __launch_bounds__(128)
+gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w, int64_t tokens, int E, int64_t d, T* __restrict__ dx) {
+  const int64_t chunks = d / 8;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t0 = i / chunks * 4, c = (i % chunks) * 8;
+  if (t0 >= tokens) return;
+  float acc[4][8];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
+#pragma unroll 2
+  for (int e = 0; e < E; ++e) {
+    const float4 lo = __ldg(reinterpret_cast<const float4*>(w + (int64_t)e * d + c)), hi = __ldg(reinterpret_cast<const float4*>(w + (int64_t)e * d + c + 4));
+    const float wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const float gv = t0 + a < tokens ? __ldg(g + (t0 + a) * E + e) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[a][j] = fmaf(gv, wv[j], acc[a][j]);
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    if (t0 + a >= tokens) break;
+    uint4 raw;
+    T* o = reinterpret_cast<T*>(&raw);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = from_f32<T>(acc[a][j]);
+    *reinterpret_cast<uint4*>(dx + (t0 + a) * d + c) = raw;
+  }
+}
+
+// dW = g^T x, fp32 [E, d]: a block owns 32 columns of 4 experts; 64 token slices of 4 column lanes, added in slice order
+template <typename T>
+__global__ void __launch_bounds__(256)
+gate_project_dw_kernel(const float* __restrict__ g, const T* __restrict__ x, int64_t ldx, int64_t tokens, int E, int64_t d, float* __restrict__ dw) {
+  __shared__ float red[64][33];
+  const int cl = threadIdx.x & 3, slice = threadIdx.x >> 2;
+  const int64_t c = (int64_t)blockIdx.x * 32 + cl * 8;
+  const int e0 = blockIdx.y * 4;
+  float acc[4][8];
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[b][j] = 0.f;
+#pragma unroll 4
+  for (int64_t t = slice; t < tokens; t += 64) {
+    float xv[8];
+    load8<T>(x + t * ldx + c, c < d, xv);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float gv = e0 + b < E ? __ldg(g + t * E + e0 + b) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[b][j] = fmaf(gv, xv[j], acc[b][j]);
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[slice][cl * 8 + j] = acc[b][j];
+    __syncthreads();
+    // eight threads per column add eight slices each, then meet by shuffles
+    const int col = threadIdx.x >> 3, part = threadIdx.x & 7;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += red[part * 8 + i][col];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const int64_t oc = (int64_t)blockIdx.x * 32 + col;
+    if (part == 0 && e0 + b < E && oc < d) dw[(int64_t)(e0 + b) * d + oc] = s;
+  }
+}
+
 unsigned elementwise_grid(int64_t items) {
   const int64_t want = ceil_div(items, 256), cap = (int64_t)sm_count() * 8;
   return (unsigned)(want < cap ? (want > 0 ? want : 1) : cap);
@@ -704,5 +843,43 @@ extern "C" int hexa_gate_load_importance_grad(const float* logits, const float* 
   else HEXA_GATE_LIG(16);
 #undef HEXA_GATE_LIG
   HEXA_LAUNCH_CHECK("gate_li_grad_kernel");
+  return HEXA_OK;
+}
+
+extern "C" int hexa_gate_project(const void* x, int64_t ldx, const float* w, int64_t tokens, int num_experts, int64_t d, int dtype,
+                                 float* logits, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  HEXA_REQUIRE(tokens >= 0 && num_experts >= 1 && d >= 8 && d % 8 == 0 && ldx >= d && ldx % 8 == 0, "hexa_gate_project: bad sizes (d and ldx must be multiples of 8)");
+  HEXA_REQUIRE(dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project: 16-bit tokens only");
+  if (tokens == 0) return HEXA_OK;
+  HEXA_REQUIRE(x && w && logits && aligned16(x) && aligned16(w), "hexa_gate_project: null or unaligned pointer");
+  const int64_t tiles = ceil_div(tokens, 4) * ceil_div(num_experts, 4);
+  HEXA_REQUIRE(ceil_div(tiles, 4) < INT32_MAX, "hexa_gate_project: too many tokens");
+  const unsigned grid = (unsigned)ceil_div(tiles, 4);
+  if (dtype == HEXA_F16) gate_project_kernel<__half><<<grid, 128, 0, stream>>>((const __half*)x, ldx, w, tokens, num_experts, d, logits);
+  else gate_project_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)x, ldx, w, tokens, num_experts, d, logits);
+  HEXA_LAUNCH_CHECK("gate_project_kernel");
+  return HEXA_OK;
+}
+
+extern "C" int hexa_gate_project_grad(const float* g, const void* x, int64_t ldx, const float* w, int64_t tokens, int num_experts,
+                                      int64_t d, int dtype, void* dx, float* dw, void* stream_) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  HEXA_REQUIRE(tokens >= 1 && num_experts >= 1 && d >= 8 && d % 8 == 0 && ldx >= d && ldx % 8 == 0, "hexa_gate_project_grad: bad sizes (d and ldx must be multiples of 8)");
+  HEXA_REQUIRE(dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project_grad: 16-bit tokens only");
+  HEXA_REQUIRE(g && (!dx || (w && aligned16(w) && aligned16(dx))) && (!dw || (x && aligned16(x))), "hexa_gate_project_grad: null or unaligned pointer");
+  const int64_t blocks = ceil_div(ceil_div(tokens, 4) * (d / 8), 128);
+  HEXA_REQUIRE(blocks < INT32_MAX && ceil_div(num_experts, 4) <= 65535, "hexa_gate_project_grad: too many tokens or experts");
+  if (dx) {
+    if (dtype == HEXA_F16) gate_project_dx_kernel<__half><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__half*)dx);
+    else gate_project_dx_kernel<__nv_bfloat16><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__nv_bfloat16*)dx);
+    HEXA_LAUNCH_CHECK("gate_project_dx_kernel");
+  }
+  if (dw) {
+    const dim3 grid((unsigned)ceil_div(d, 32), (unsigned)ceil_div(num_experts, 4));
+    if (dtype == HEXA_F16) gate_project_dw_kernel<__half><<<grid, 256, 0, stream>>>(g, (const __half*)x, ldx, tokens, num_experts, d, dw);
+    else gate_project_dw_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(g, (const __nv_bfloat16*)x, ldx, tokens, num_experts, d, dw);
+    HEXA_LAUNCH_CHECK("gate_project_dw_kernel");
+  }
   return HEXA_OK;
 }

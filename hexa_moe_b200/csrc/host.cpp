@@ -31,7 +31,8 @@ struct Api {
   X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
   X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_f32_workspace_bytes) X(hexa_esmm_f32) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
   X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
-  X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists)
+  X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists)       \
+  X(hexa_gate_project) X(hexa_gate_project_grad)
 #define HEXA_FIELD(name) decltype(&::name) name = nullptr;
   HEXA_API(HEXA_FIELD)
 } api;
@@ -322,6 +323,35 @@ Tensor gate_sum_terms(const Tensor& part, int64_t rows, int64_t cols, bool lo_fi
   return out;
 }
 
+Tensor gate_project(const Tensor& x, const Tensor& w) {
+  if (w.scalar_type() != at::kFloat || w.dim() != 2 || !w.is_contiguous() || x.dim() != 2 || x.size(1) != w.size(1))
+    fail("gate_project: w must be contiguous float32 [E, d] and x [T, d]");
+  void* s = stream_of(x);
+  const int type = dt(x);
+  const int64_t ldx = ld(x), T = x.size(0), E = w.size(0);
+  Tensor out = empty({T, E}, at::kFloat, x);
+  call("hexa_gate_project", [&] {
+    return api.hexa_gate_project(ptr(x), ldx, static_cast<const float*>(ptr(w)), T, (int)E, x.size(1), type, static_cast<float*>(ptr(out)), s);
+  });
+  return out;
+}
+
+std::tuple<OptTensor, OptTensor> gate_project_grad(const Tensor& g, const Tensor& x, const Tensor& w, bool want_dx, bool want_dw) {
+  if (g.scalar_type() != at::kFloat || g.dim() != 2 || !g.is_contiguous() || g.size(0) != x.size(0) || g.size(1) != w.size(0) || !w.is_contiguous())
+    fail("gate_project_grad: g must be contiguous float32 [T, E]");
+  void* s = stream_of(g);
+  const int type = dt(x);
+  const int64_t ldx = ld(x);
+  OptTensor dx, dw;
+  if (want_dx) dx = empty({x.size(0), x.size(1)}, x.scalar_type(), x);
+  if (want_dw) dw = empty({w.size(0), w.size(1)}, at::kFloat, x);
+  call("hexa_gate_project_grad", [&] {
+    return api.hexa_gate_project_grad(static_cast<const float*>(ptr(g)), ptr(x), ldx, static_cast<const float*>(ptr(w)), x.size(0), (int)w.size(0),
+                                      x.size(1), type, ptr(dx), static_cast<float*>(ptr(dw)), s);
+  });
+  return {dx, dw};
+}
+
 void bind(const std::string& path, py::object error, py::object ensure, py::dict text) {
   void* handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
   if (!handle) throw std::runtime_error(dlerror());
@@ -346,6 +376,8 @@ PYBIND11_MODULE(_host, m) {
   m.def("ess", &ess);
   m.def("gate_topk", &gate_topk);
   m.def("gate_loss_grad", &gate_loss_grad);
+  m.def("gate_project", &gate_project);
+  m.def("gate_project_grad", &gate_project_grad);
   m.def("gate_split_terms", &gate_split_terms);
   m.def("gate_sum_terms", &gate_sum_terms);
 }

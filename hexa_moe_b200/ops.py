@@ -240,6 +240,19 @@ def gate_max_experts() -> int:
     return int(lib().hexa_gate_max_experts())
 
 
+def gate_project(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """float32 logits x w^T of 16-bit tokens [T,d] and a float32 weight [E,d], fp32 products and sums (few tokens)."""
+    return _run("gate", 2.0 * x.shape[0] * w.numel(), 0.0, host().gate_project, (x, w))
+
+
+def gate_project_grad(g: torch.Tensor, x: torch.Tensor, w: torch.Tensor, want_dx: bool, want_dw: bool):
+    """(dx = g w in x's type, dw = g^T x in float32) of gate_project, None where not wanted."""
+    global LAUNCHES
+    LAUNCHES += int(want_dx) + int(want_dw) - 1
+    return _run("gate", 2.0 * x.shape[0] * w.numel() * (int(want_dx) + int(want_dw)), 0.0, host().gate_project_grad,
+                (g, x, w, want_dx, want_dw))
+
+
 def gate_split_terms(src: torch.Tensor, by_rows: bool) -> torch.Tensor:
     """float32 [rows, cols] as bf16 terms hi + mid + lo: [rows, 4 cols] with column blocks (hi, hi, mid, lo) or, by_rows,
     [4 rows, cols] with row blocks (lo, mid, hi, hi)."""

@@ -336,6 +336,14 @@ int hexa_gate_loss_grad(const float* logits, int64_t ld, int64_t num_tokens, int
 int hexa_gate_split_terms(const float* src, int64_t ld, int64_t rows, int64_t cols, int by_rows, void* out, void* stream);
 int hexa_gate_sum_terms(const float* part, int64_t rows, int64_t cols, int lo_first, float* out, void* stream);
 
+/* The projection itself for few tokens, fp32 products and sums on the CUDA cores: logits [tokens, experts] = x W^T with x
+ * 16-bit [tokens, d] (leading dimension ldx) and W fp32 [experts, d]; and its gradients from g [tokens, experts]:
+ * dx (dtype, [tokens, d]) = g W, dw (fp32, [experts, d]) = g^T x, either may be null.  d, ldx multiples of 8. */
+int hexa_gate_project(const void* x, int64_t ldx, const float* w, int64_t tokens, int num_experts, int64_t d, int dtype,
+                      float* logits, void* stream);
+int hexa_gate_project_grad(const float* g, const void* x, int64_t ldx, const float* w, int64_t tokens, int num_experts,
+                           int64_t d, int dtype, void* dx, float* dw, void* stream);
+
 /* The same step for the other auxiliary loss of the reference, the load-importance loss (impls/losses.py:21-43, selected by
  * is_gshard_loss=False; needs gate noise): ids = top-k of the NOISY logits (what torch.topk of softmax(noisy) returns),
  *   importance[e] = sum_t softmax(logits)[t,e],   load[e] = sum_t Phi((softmax(logits)[t,e] - thr_t) / sigma),

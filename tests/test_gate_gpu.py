@@ -255,3 +255,30 @@ def test_split_precision_gate_terms(T, d, E):
     assert ((dw - dw2).double().abs() <= bw + 1e-30).all()
     bx = (dy.double().abs() @ w.double().abs()) * ((3 * E + 3) * 2.0 ** -23)
     assert ((dx - dx2).double().abs() <= dx.double().abs() * 2.0 ** -7 + bx + 1e-30).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,d,E", [(1, 8, 1), (5, 264, 3), (63, 72, 7), (300, 64, 33), (4096, 200, 8), (130, 1024, 64)])
+def test_direct_gate_projection(T, d, E, dtype):
+    """Few-token projection and its gradients: within the bound of an fp32 sum of that many terms of the exact values, and
+    in agreement with the formulation that create_graph takes."""
+    from hexa_moe_b200.impls.gating import _DirectLinear, _direct_linear_applies
+    g = torch.Generator(device="cuda").manual_seed(d + T)
+    lin = torch.nn.Linear(d, E, bias=False, device="cuda")
+    x = torch.randn(T, d + 8, generator=g, device="cuda").to(dtype)[:, :d].requires_grad_(True)      # a row pitch
+    assert _direct_linear_applies(lin, x)
+    w, dy = lin.weight, torch.randn(T, E, generator=g, device="cuda")
+    y = _DirectLinear.apply(x, w)
+    X, W, DY = x.detach().double(), w.detach().double(), dy.double()
+    assert ((y.double() - X @ W.t()).abs() <= X.abs() @ W.abs().t() * (d * 2.0 ** -24) + 1e-30).all()
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+    assert dx.dtype == dtype and dw.dtype == torch.float32
+    assert ((dw.double() - DY.t() @ X).abs() <= DY.abs().t() @ X.abs() * (max(T, 8) * 2.0 ** -24) + 1e-30).all()
+    half = torch.finfo(dtype).eps / 2                      # one rounding of an fp32 sum of E terms (tiny: fp16's subnormals)
+    want = DY @ W
+    assert ((dx.double() - want).abs() <= want.abs() * half * 1.01 + DY.abs() @ W.abs() * (E * 2.0 ** -24) + 3e-8).all()
+    dx2, dw2 = torch.autograd.grad(_DirectLinear.apply(x, w), (x, w), dy, create_graph=True)
+    assert ((dx2 - dx).double().abs() <= want.abs() * half * 2.1 + DY.abs() @ W.abs() * (E * 2.0 ** -23) + 6e-8).all()
+    assert ((dw2 - dw).double().abs() <= DY.abs().t() @ X.abs() * (max(T, 8) * 2.0 ** -23) + 1e-30).all()
+    only = torch.autograd.grad(_DirectLinear.apply(x.detach(), w), w, dy)[0]
+    assert torch.equal(only, dw)
