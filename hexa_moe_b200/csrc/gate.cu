@@ -344,8 +344,8 @@ sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int
 }
 
 // ---- the gate projection of few tokens, straight on the CUDA cores -----------------------------------------------------
-// logits = x W^T with x 16-bit [T, d], W fp32 [E, d] and fp32 FMAs: for small T the split operands' three launches (or, for
-// fp16 tokens, a cast and an fp32 GEMM with too few blocks) cost more than the products.  A warp takes 4 tokens x 4 experts,
+// logits = x W^T with x [T, d], W fp32 [E, d] and fp32 FMAs: for small T the split operands' three launches (or, for fp16
+// and fp32 tokens, an fp32 GEMM with too few blocks) cost more than the products.  A warp takes 4 tokens x 4 experts,
 // its lanes 8 consecutive elements of every 256 of d, so an operand value loaded once meets four of the other side, and the 16
 // sums meet in 16 shuffles.  Bound: the latency of d / 256 rounds of loads.  [2048, 768], 8 experts: 4 us (fp16 with a
 // cast and a GEMM 22, bf16 in split terms 7 in three launches); [16, 1024], 32 experts: 4 us (split terms 7).
@@ -356,6 +356,13 @@ __device__ __forceinline__ void load8(const T* __restrict__ p, bool live, float 
   const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(e[i]);
+}
+
+template <>
+__device__ __forceinline__ void load8<float>(const float* __restrict__ p, bool live, float (&v)[8]) {
+  float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+  if (live) { lo = __ldg(reinterpret_cast<const float4*>(p)); hi = __ldg(reinterpret_cast<const float4*>(p) + 1); }
+  v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
 }
 
 template <typename T>
@@ -405,7 +412,7 @@ gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restric
   if ((lane & 1) == 0 && t < tokens && e < E) logits[t * E + e] = sum;
 }
 
-// dx = g W, 16-bit [T, d]: a thread owns 8 columns of 4 tokens
+// dx = g W, [T, d]: a thread owns 8 columns of 4 tokens
 template <typename T>
 __global__ void __launch_bounds__(128)
 gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w, int64_t tokens, int E, int64_t d, T* __restrict__ dx) {
@@ -432,11 +439,12 @@ gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w,
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     if (t0 + a >= tokens) break;
-    uint4 raw;
-    T* o = reinterpret_cast<T*>(&raw);
+    __align__(16) T o[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = from_f32<T>(acc[a][j]);
-    *reinterpret_cast<uint4*>(dx + (t0 + a) * d + c) = raw;
+#pragma unroll
+    for (int j = 0; j < (int)(8 * sizeof(T) / 16); ++j)
+      reinterpret_cast<uint4*>(dx + (t0 + a) * d + c)[j] = reinterpret_cast<const uint4*>(o)[j];
   }
 }
 
@@ -850,13 +858,14 @@ extern "C" int hexa_gate_project(const void* x, int64_t ldx, const float* w, int
                                  float* logits, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   HEXA_REQUIRE(tokens >= 0 && num_experts >= 1 && d >= 8 && d % 8 == 0 && ldx >= d && ldx % 8 == 0, "hexa_gate_project: bad sizes (d and ldx must be multiples of 8)");
-  HEXA_REQUIRE(dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project: 16-bit tokens only");
+  HEXA_REQUIRE(dtype == HEXA_F32 || dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project: bad dtype %d", dtype);
   if (tokens == 0) return HEXA_OK;
   HEXA_REQUIRE(x && w && logits && aligned16(x) && aligned16(w), "hexa_gate_project: null or unaligned pointer");
   const int64_t tiles = ceil_div(tokens, 4) * ceil_div(num_experts, 4);
   HEXA_REQUIRE(ceil_div(tiles, 4) < INT32_MAX, "hexa_gate_project: too many tokens");
   const unsigned grid = (unsigned)ceil_div(tiles, 4);
-  if (dtype == HEXA_F16) gate_project_kernel<__half><<<grid, 128, 0, stream>>>((const __half*)x, ldx, w, tokens, num_experts, d, logits);
+  if (dtype == HEXA_F32) gate_project_kernel<float><<<grid, 128, 0, stream>>>((const float*)x, ldx, w, tokens, num_experts, d, logits);
+  else if (dtype == HEXA_F16) gate_project_kernel<__half><<<grid, 128, 0, stream>>>((const __half*)x, ldx, w, tokens, num_experts, d, logits);
   else gate_project_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)x, ldx, w, tokens, num_experts, d, logits);
   HEXA_LAUNCH_CHECK("gate_project_kernel");
   return HEXA_OK;
@@ -866,18 +875,20 @@ extern "C" int hexa_gate_project_grad(const float* g, const void* x, int64_t ldx
                                       int64_t d, int dtype, void* dx, float* dw, void* stream_) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   HEXA_REQUIRE(tokens >= 1 && num_experts >= 1 && d >= 8 && d % 8 == 0 && ldx >= d && ldx % 8 == 0, "hexa_gate_project_grad: bad sizes (d and ldx must be multiples of 8)");
-  HEXA_REQUIRE(dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project_grad: 16-bit tokens only");
+  HEXA_REQUIRE(dtype == HEXA_F32 || dtype == HEXA_F16 || dtype == HEXA_BF16, "hexa_gate_project_grad: bad dtype %d", dtype);
   HEXA_REQUIRE(g && (!dx || (w && aligned16(w) && aligned16(dx))) && (!dw || (x && aligned16(x))), "hexa_gate_project_grad: null or unaligned pointer");
   const int64_t blocks = ceil_div(ceil_div(tokens, 4) * (d / 8), 128);
   HEXA_REQUIRE(blocks < INT32_MAX && ceil_div(num_experts, 4) <= 65535, "hexa_gate_project_grad: too many tokens or experts");
   if (dx) {
-    if (dtype == HEXA_F16) gate_project_dx_kernel<__half><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__half*)dx);
+    if (dtype == HEXA_F32) gate_project_dx_kernel<float><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (float*)dx);
+    else if (dtype == HEXA_F16) gate_project_dx_kernel<__half><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__half*)dx);
     else gate_project_dx_kernel<__nv_bfloat16><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__nv_bfloat16*)dx);
     HEXA_LAUNCH_CHECK("gate_project_dx_kernel");
   }
   if (dw) {
     const dim3 grid((unsigned)ceil_div(d, 32), (unsigned)ceil_div(num_experts, 4));
-    if (dtype == HEXA_F16) gate_project_dw_kernel<__half><<<grid, 256, 0, stream>>>(g, (const __half*)x, ldx, tokens, num_experts, d, dw);
+    if (dtype == HEXA_F32) gate_project_dw_kernel<float><<<grid, 256, 0, stream>>>(g, (const float*)x, ldx, tokens, num_experts, d, dw);
+    else if (dtype == HEXA_F16) gate_project_dw_kernel<__half><<<grid, 256, 0, stream>>>(g, (const __half*)x, ldx, tokens, num_experts, d, dw);
     else gate_project_dw_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(g, (const __nv_bfloat16*)x, ldx, tokens, num_experts, d, dw);
     HEXA_LAUNCH_CHECK("gate_project_dw_kernel");
   }

@@ -241,7 +241,7 @@ def gate_max_experts() -> int:
 
 
 def gate_project(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """float32 logits x w^T of 16-bit tokens [T,d] and a float32 weight [E,d], fp32 products and sums (few tokens)."""
+    """float32 logits x w^T of tokens [T,d] and a float32 weight [E,d], fp32 products and sums (few tokens)."""
     return _run("gate", 2.0 * x.shape[0] * w.numel(), 0.0, host().gate_project, (x, w))
 
 

@@ -337,7 +337,7 @@ int hexa_gate_split_terms(const float* src, int64_t ld, int64_t rows, int64_t co
 int hexa_gate_sum_terms(const float* part, int64_t rows, int64_t cols, int lo_first, float* out, void* stream);
 
 /* The projection itself for few tokens, fp32 products and sums on the CUDA cores: logits [tokens, experts] = x W^T with x
- * 16-bit [tokens, d] (leading dimension ldx) and W fp32 [experts, d]; and its gradients from g [tokens, experts]:
+ * [tokens, d] of `dtype` (leading dimension ldx) and W fp32 [experts, d]; and its gradients from g [tokens, experts]:
  * dx (dtype, [tokens, d]) = g W, dw (fp32, [experts, d]) = g^T x, either may be null.  d, ldx multiples of 8. */
 int hexa_gate_project(const void* x, int64_t ldx, const float* w, int64_t tokens, int num_experts, int64_t d, int dtype,
                       float* logits, void* stream);

@@ -257,7 +257,7 @@ def test_split_precision_gate_terms(T, d, E):
     assert ((dx - dx2).double().abs() <= dx.double().abs() * 2.0 ** -7 + bx + 1e-30).all()
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("T,d,E", [(1, 8, 1), (5, 264, 3), (63, 72, 7), (300, 64, 33), (4096, 200, 8), (130, 1024, 64)])
 def test_direct_gate_projection(T, d, E, dtype):
     """Few-token projection and its gradients: within the bound of an fp32 sum of that many terms of the exact values, and
