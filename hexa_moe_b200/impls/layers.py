@@ -235,13 +235,19 @@ def _common_dtype(b1, b2):
 # ------------------------------------------------------------------------------------------------
 def _dense_on_kernels(cfg, x: Tensor) -> bool:
     """16-bit CUDA tokens with an activation the GEMM epilogue knows run as a one-expert layer on the grouped-GEMM
-    kernels (fused bias + activation, fused activation derivative); anything else is plain PyTorch."""
+    kernels (fused bias + activation, fused activation derivative); anything else is plain PyTorch.
+
+    Tokens at least 64 wide: forward + backward at widths 64 to 248 and 16 to 65000 tokens 295-440 us against 430-1106 with
+    PyTorch operations.  A ReLU takes the kernels from 256 on: the two ways round a pre-activation differently (once from
+    the fp32 sum here, before and after the bias there), which moves a derivative that jumps at zero by more than the
+    rounding itself.  HEXA_DENSE_MIN_DIM sets the width for all."""
     if os.environ.get("HEXA_DENSE_KERNELS", "1") == "0":        # A/B switch: keep the dense FFN on PyTorch ops
         return False
+    from .. import _lib
+    least = os.environ.get("HEXA_DENSE_MIN_DIM") or (256 if getattr(cfg, "act_id", -1) == _lib.ACT_RELU else 64)
     return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and getattr(cfg, "act_id", -1) >= 0
             and getattr(cfg, "backend", None) is not None and hasattr(cfg.backend, "dense_forward")
-            and x.shape[0] > 0 and x.shape[1] % 8 == 0
-            and x.shape[1] >= int(os.environ.get("HEXA_DENSE_MIN_DIM", "256")))
+            and x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.shape[1] >= int(least))
 
 
 class MLP_Implement(torch.autograd.Function):

@@ -255,3 +255,40 @@ def test_dense_ffn_on_the_grouped_gemm_kernels(dtype, tokens):
         assert g.shape == w.shape
         assert rel_err(g, w) <= 2e-2
         assert rel_err(g, p_) <= 3e-2
+
+
+@pytest.mark.parametrize("dim,act,on_kernels", [(64, "gelu", True), (72, "silu", True), (56, "gelu", False), (64, "relu", False), (256, "relu", True)])
+def test_dense_depth_widths_on_the_kernels(dim, act, on_kernels):
+    """Which widths run as a one-expert layer, and that both ways agree to the 16-bit tolerance."""
+    import os
+    import torch.nn.functional as F
+    from hexa_moe import moe as hmoe
+    from hexa_moe_b200 import ops
+    torch.manual_seed(dim)
+    fn = {"gelu": lambda t: F.gelu(t), "silu": F.silu, "relu": F.relu}[act]
+    m = hmoe.MoE_Cascaded(gate_type={'type': 'top', 'k': 1}, model_dim_list=[dim], moe_idx_list=[], mlp_ratio=4,
+                          num_global_experts=1, total_depth=1, data_centric=True, activation_fn=fn)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.normal_(0, 0.1)
+    m = m.to(torch.bfloat16).cuda()
+    x, dy = torch.randn(333, dim, device="cuda").bfloat16(), torch.randn(333, dim, device="cuda").bfloat16()
+
+    def run():
+        m.zero_grad()
+        xi = x.clone().requires_grad_(True)
+        before = ops.LAUNCHES
+        y, _ = m(0, xi)
+        y.backward(dy)
+        return ops.LAUNCHES > before, [y.detach(), xi.grad] + [p.grad for p in m.parameters()]
+
+    used, got = run()
+    assert used == on_kernels
+    os.environ["HEXA_DENSE_KERNELS"] = "0"
+    try:
+        _, want = run()
+    finally:
+        del os.environ["HEXA_DENSE_KERNELS"]
+    if act != "relu":
+        for a, b in zip(got, want):
+            assert float((a.float() - b.float()).norm()) <= 1.2e-2 * float(b.float().norm())
