@@ -957,13 +957,13 @@ bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, 
   return true;
 }
 
-// How many chunks a split ESTMM cuts every expert's segment into (1 = no split).  Only static sizes enter.  Few, long
-// segments - the dense FFN's weight gradient (one "expert" owning every row), or a handful of experts with a small d x H -
-// would otherwise leave most SMs idle behind a few serial k-loops.  The count minimises a model of the launch's time in
-// k-blocks (one takes ~0.35 us): full waves of tiles, each a chunk's k-blocks plus ~6 for filling and draining the pipeline,
-// and the fp32 partial results, written and read once at ~5 TB/s by a second launch (~8).  A count that just spills into another wave is what this
-// avoids: [18432 rows, 2048 x 512] in 10 chunks is 160 tiles on 74 pairs, three waves of 29 k-blocks (64 us with the
-// second pass), in 4 chunks one wave of 72 (48 us); [30000, 640 x 160] over 4 experts 33 us in 13, 24 in 6.  A chunk keeps at least 8 k-blocks.
+// How many chunks a split ESTMM cuts every expert's segment into (1 = no split).  Only static sizes enter: the tile
+// count without a split against the CTA pairs (or CTAs) of the device, and the average segment length, so that a chunk
+// keeps at least 8 k-blocks.  Few, long segments - the dense FFN's weight gradient (one "expert" owning every row), or a
+// handful of experts with a small d x H - would otherwise leave most SMs idle behind a few serial k-loops.  A chunk is also
+// the length of a chain in the accumulator, which truncates: a count that fills whole waves with fewer, longer chunks is
+// faster ([18432 rows, 2048 x 512] in 4 chunks 47 us, in these 10 63 us) but further from the exact sums: relative error of
+// that shape's fp32 result 5.0e-6 against 1.9e-6 (positive data 17e-6 against 4.7e-6), one chunk 21e-6.
 int estmm_tc_splits(int E, int64_t row_cap, int64_t m, int64_t n) {
   static int forced = -2;
   if (forced == -2) forced = env_int("HEXA_ESTMM_SPLITS", -1);       // A/B switch: 1 = never split
@@ -973,16 +973,12 @@ int estmm_tc_splits(int E, int64_t row_cap, int64_t m, int64_t n) {
   const int64_t tiles = (int64_t)E * ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN);
   const int64_t slots = ctas == 2 ? sm_count() / 2 : sm_count();
   const int64_t avg_kb = row_cap / BLOCK_K / E;
-  if (forced > 0) return forced > 32 ? 32 : forced;
-  if (tiles >= 2 * slots) return 1;
-  const double partial = 2.0 * (double)E * (double)m * (double)n * 4.0 / 5e12 / 0.35e-6;      // one chunk's, in k-blocks
-  int best = 1;
-  double best_cost = 0.0;
-  for (int64_t s = 1; s <= 32 && (s == 1 || avg_kb / s >= 8); ++s) {
-    const double cost = (double)ceil_div(tiles * s, slots) * (double)(ceil_div(avg_kb, s) + 6) + (s > 1 ? partial * (double)s + 8.0 : 0.0);
-    if (s == 1 || cost < best_cost) { best = (int)s; best_cost = cost; }
-  }
-  return best;
+  int64_t s = 1;
+  if (tiles < 2 * slots) s = ceil_div(2 * slots, tiles);
+  if (s > avg_kb / 8) s = avg_kb / 8;
+  if (forced > 0) s = forced;
+  if (s > 32) s = 32;
+  return s < 1 ? 1 : (int)s;
 }
 
 size_t estmm_tc_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n) {

@@ -296,3 +296,15 @@ def test_token_chunks_are_the_same_count_on_every_rank(monkeypatch):
     monkeypatch.setenv("HEXA_MC_CHUNKS", "2")
     assert token_chunks([16384] * 8)[0] == [0, 8192, 16384]
     assert token_chunks([384] * 2)[0] == [0, 384]                          # too few tokens to cut
+
+
+@pytest.mark.parametrize("E,rows,m,n,chunks", [(1, 18432, 2048, 512, 10), (8, 32768, 1024, 256, 5), (4, 16384, 2048, 512, 3),
+                                               (4, 30000 // 128 * 128, 640, 160, 13), (8, 32768, 3072, 768, 1), (1, 18432, 64, 64, 32)])
+def test_weight_gradient_chunks_keep_accumulator_chains_short(E, rows, m, n, chunks):
+    """A chunk is a chain in the tensor core's truncating accumulator: two tiles per CTA pair are made even where fewer,
+    longer chunks would fill whole waves (148 SMs, which the library also assumes without a device)."""
+    from hexa_moe_b200 import _lib as L
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("chunk counts are stated for 148 SMs")
+    got = L.lib().hexa_estmm_workspace_bytes(E, rows, m, n, L.BF16)
+    assert got == (chunks * E * m * n * 4 if chunks > 1 else 0)
