@@ -40,6 +40,7 @@ SIGNATURES = {
     "hexa_route_launches": (ci, [i64, ci, ci]),
     "hexa_route": (ci, [vp, i64, ci, i64, i64, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "hexa_ids_from_lists": (ci, [vp, vp, i64, ci, i64, vp, vp]),
+    "hexa_ids_from_lists_i64": (ci, [vp, vp, i64, ci, i64, vp, vp]),
     "hexa_gather_rows": (ci, [vp, i64, vp, vp, ci, i64, i64, vp, i64, ci, vp]),
     "hexa_gather_rows_ess": (ci, [vp, i64, vp, vp, ci, i64, i64, vp, i64, vp, i64, ci, vp, sz, vp]),
     "hexa_combine_rows": (ci, [vp, i64, vp, i64, ci, i64, vp, i64, ci, vp]),
@@ -112,14 +113,23 @@ def host():
                 except ImportError as e:
                     raise HexaError(f"hexa_moe_b200/_host.so cannot be loaded ({e}): build it with "
                                     "`python -m hexa_moe_b200.build` (there is no fallback path)")
-                module.bind(LIB_PATH, HexaError, ensure_status_word, _STATUS_CODES)
+                module.bind(LIB_PATH, HexaError, ensure_status_word, status_text)
                 _host = module
     return _host
 
 
 ERR_DEVICE = -5
+STATUS_BAD_TOKEN = 6
 _STATUS_CODES = {1: "the TMA producer waited for a free ring slot", 2: "the MMA issuer waited for a drained accumulator",
-                 3: "the MMA issuer waited for operands", 4: "an epilogue warp waited for an accumulator", 5: "an epilogue warp waited for the saved pre-activation"}
+                 3: "the MMA issuer waited for operands", 4: "an epilogue warp waited for an accumulator",
+                 5: "an epilogue warp waited for the saved pre-activation",
+                 STATUS_BAD_TOKEN: "a list names a token beyond the number of tokens"}
+
+
+def status_text(code: int) -> str:
+    what = "was given an index out of range" if code == STATUS_BAD_TOKEN else "gave up a bounded wait"
+    return (f"a kernel on this device {what} (status code {code}: {_STATUS_CODES.get(code, 'unknown')}); "
+            f"results since then are incomplete ({ERR_DEVICE})")
 
 
 def check(status: int, what: str):
@@ -130,8 +140,7 @@ def check(status: int, what: str):
     if _status_words:
         code = lib().hexa_pending_device_status()
         if code:
-            raise HexaError(f"{what}: a kernel on this device gave up a bounded wait (status code {code}: "
-                            f"{_STATUS_CODES.get(code, 'unknown')}); results since then are incomplete ({ERR_DEVICE})")
+            raise HexaError(f"{what}: {status_text(code)}")
 
 
 # One status word per device in pinned host memory: kernels store a code there when a wait inside them runs out,

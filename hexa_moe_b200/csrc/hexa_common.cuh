@@ -18,14 +18,27 @@ int status_pending();     // code an earlier kernel left in the current device's
 uint64_t wait_limit_ns(); // limit of the bounded waits inside kernels, see hexa_set_wait_limit_ns
 int tc_debug_flags();     // HEXA_TC_DEBUG / hexa_set_tc_debug
 
+constexpr int kStatusBadToken = 6;   // status code of hexa_ids_from_lists; the others come from bounded waits
+// The status word may live in device memory or in pinned host memory (where the host can poll it without a copy), so
+// it is written with plain stores: the first code to arrive stays, and which of two simultaneous codes wins is immaterial.
+__device__ __forceinline__ void report_status(int32_t* status, int code) {
+  if (status) {
+    volatile int32_t* s = status;
+    if (*s == 0) *s = code;
+    __threadfence_system();
+  }
+}
+
 // Entry points that launch kernels with bounded waits refuse to run once such a wait has been given up on this
 // device: what those kernels wrote is incomplete, and so is everything computed from it.
 #define HEXA_CHECK_DEVICE_STATUS(name)                                                                     \
   do {                                                                                                     \
     const int code_ = ::hexa::status_pending();                                                            \
     if (code_ != 0) {                                                                                      \
-      ::hexa::set_error("%s: an earlier kernel on this device gave up a bounded wait (status code %d); "   \
-                        "its outputs are incomplete.  Clear the status word to continue", name, code_);    \
+      ::hexa::set_error("%s: an earlier kernel on this device %s (status code %d); "                       \
+                        "its outputs are incomplete.  Clear the status word to continue", name,            \
+                        code_ == ::hexa::kStatusBadToken ? "met a token id out of range"                   \
+                                                         : "gave up a bounded wait", code_);               \
       return HEXA_ERR_DEVICE;                                                                              \
     }                                                                                                      \
   } while (0)

@@ -31,15 +31,14 @@ struct Api {
   X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
   X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_f32_workspace_bytes) X(hexa_esmm_f32) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
   X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
-  X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists)       \
+  X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists) X(hexa_ids_from_lists_i64)                          \
   X(hexa_gate_project) X(hexa_gate_project_grad)
 #define HEXA_FIELD(name) decltype(&::name) name = nullptr;
   HEXA_API(HEXA_FIELD)
 } api;
 
 struct Bound {      // what _lib.py hands over; lives as long as the process (nothing to release after the interpreter)
-  py::object error, ensure_status_word;
-  py::dict status_text;
+  py::object error, ensure_status_word, status_text;
 };
 Bound* bound = nullptr;
 bool status_installed[64] = {false};
@@ -53,12 +52,7 @@ bool status_installed[64] = {false};
 void check(int rc, const char* what) {
   if (rc != 0) fail(std::string(what) + " failed (" + std::to_string(rc) + "): " + api.hexa_last_error_string());
   const int code = api.hexa_pending_device_status();
-  if (code != 0) {
-    const py::int_ key(code);
-    const std::string text = bound->status_text.contains(key) ? bound->status_text[key].cast<std::string>() : "unknown";
-    fail(std::string(what) + ": a kernel on this device gave up a bounded wait (status code " + std::to_string(code) + ": " + text +
-         "); results since then are incomplete (" + std::to_string(HEXA_ERR_DEVICE) + ")");
-  }
+  if (code != 0) fail(std::string(what) + ": " + bound->status_text(code).cast<std::string>());
 }
 
 template <typename F> void call(const char* what, F&& f) {
@@ -78,6 +72,12 @@ void* stream_of(const Tensor& t) {
     if (dev >= 0 && dev < 64) status_installed[dev] = true;
   }
   return c10::cuda::getCurrentCUDAStream(dev).stream();
+}
+
+// Kernels take raw pointers: an operand on another device, or on the host, has to be refused here.
+void on_device_of(const Tensor& anchor, std::initializer_list<const Tensor*> others) {
+  for (const Tensor* t : others)
+    if (t->device() != anchor.device()) fail("operands are on different devices: " + anchor.device().str() + " and " + t->device().str());
 }
 
 int dt(const Tensor& t) {
@@ -137,11 +137,16 @@ py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
 }
 
 Tensor ids_from_lists(int64_t num_toks, const Tensor& tok_ids_, const Tensor& exp_ids_, int chunk) {
-  const Tensor tok_ids = tok_ids_.to(at::kInt).contiguous(), exp_ids = exp_ids_.to(at::kInt).contiguous();
-  void* s = stream_of(tok_ids);
+  void* s = stream_of(tok_ids_);
+  on_device_of(tok_ids_, {&exp_ids_});
+  const bool narrow = tok_ids_.scalar_type() == at::kInt;      // anything else is read as 64 bits: an id must not wrap
+  const Tensor tok_ids = tok_ids_.to(narrow ? at::kInt : at::kLong).contiguous(), exp_ids = exp_ids_.to(at::kInt).contiguous();
+  if (chunk < 1 || tok_ids.numel() > (int64_t)chunk * exp_ids.numel()) fail("ids_from_lists: more token ids than the expert ids cover");
   Tensor ids = empty({num_toks}, at::kInt, tok_ids);
   call("hexa_ids_from_lists", [&] {
-    return api.hexa_ids_from_lists(i32(tok_ids), i32(exp_ids), tok_ids.numel(), chunk, num_toks, static_cast<int32_t*>(ptr(ids)), s);
+    return narrow ? api.hexa_ids_from_lists(i32(tok_ids), i32(exp_ids), tok_ids.numel(), chunk, num_toks, static_cast<int32_t*>(ptr(ids)), s)
+                  : api.hexa_ids_from_lists_i64(static_cast<const int64_t*>(ptr(tok_ids)), i32(exp_ids), tok_ids.numel(), chunk, num_toks,
+                                                static_cast<int32_t*>(ptr(ids)), s);
   });
   return ids;
 }
@@ -352,7 +357,7 @@ std::tuple<OptTensor, OptTensor> gate_project_grad(const Tensor& g, const Tensor
   return {dx, dw};
 }
 
-void bind(const std::string& path, py::object error, py::object ensure, py::dict text) {
+void bind(const std::string& path, py::object error, py::object ensure, py::object text) {
   void* handle = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
   if (!handle) throw std::runtime_error(dlerror());
 #define HEXA_BIND(name)                                                  \

@@ -380,15 +380,21 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
 }
 
 // One expert id per token from the reference's lists: entry i of tok_ids is a token id + 1 (0: pad) and belongs to expert
-// exp_ids[i / chunk].  Slot 0 is the pads' and is not part of the result; a negative entry counts from the end, as an index does.
+// exp_ids[i / chunk].  Slot 0 is the pads' and is not part of the result; a negative entry counts from the end, as an index
+// does, and an entry outside [-(num_toks + 1), num_toks] is an error: it writes nothing and leaves a code in the status word.
+template <typename I>
 __global__ void __launch_bounds__(256)
-ids_from_lists_kernel(const int32_t* __restrict__ tok_ids, const int32_t* __restrict__ exp_ids, int64_t n, int chunk, int64_t num_toks,
-                      int32_t* __restrict__ ids) {
+ids_from_lists_kernel(const I* __restrict__ tok_ids, const int32_t* __restrict__ exp_ids, int64_t n, int chunk, int64_t num_toks,
+                      int32_t* __restrict__ ids, int32_t* status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int64_t slot = __ldg(tok_ids + i);
+  int64_t slot = (int64_t)__ldg(tok_ids + i);
+  if (slot > num_toks || slot < -(num_toks + 1)) {
+    report_status(status, kStatusBadToken);
+    return;
+  }
   if (slot < 0) slot += num_toks + 1;
-  if (slot > 0 && slot <= num_toks) ids[slot - 1] = __ldg(exp_ids + i / chunk);
+  if (slot > 0) ids[slot - 1] = __ldg(exp_ids + i / chunk);
 }
 
 // 1, 2 or 3 launches, see the head of this file
@@ -579,15 +585,24 @@ extern "C" int hexa_route_launches(int64_t T, int top_k, int E) {
   return T < 0 || top_k <= 0 || E <= 0 ? 0 : route_plan(T * top_k, E);
 }
 
-extern "C" int hexa_ids_from_lists(const int32_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_toks, int32_t* ids,
-                                   void* stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
+namespace {
+template <typename I>
+int ids_from_lists(const I* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_toks, int32_t* ids, cudaStream_t stream) {
   HEXA_REQUIRE(n >= 0 && chunk > 0 && num_toks >= 0 && ceil_div(n, 256) < INT32_MAX, "hexa_ids_from_lists: bad sizes");
-  if (num_toks == 0) return HEXA_OK;
-  HEXA_REQUIRE(ids && (n == 0 || (tok_ids && exp_ids)), "hexa_ids_from_lists: null pointer");
-  HEXA_CUDA(cudaMemsetAsync(ids, 0xFF, (size_t)num_toks * sizeof(int32_t), stream));      // -1: token in no segment
+  HEXA_REQUIRE((num_toks == 0 || ids) && (n == 0 || (tok_ids && exp_ids)), "hexa_ids_from_lists: null pointer");
+  if (num_toks > 0) HEXA_CUDA(cudaMemsetAsync(ids, 0xFF, (size_t)num_toks * sizeof(int32_t), stream));      // -1: token in no segment
   if (n == 0) return HEXA_OK;
-  ids_from_lists_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, stream>>>(tok_ids, exp_ids, n, chunk, num_toks, ids);
+  ids_from_lists_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, stream>>>(tok_ids, exp_ids, n, chunk, num_toks, ids, status_word());
   HEXA_LAUNCH_CHECK("ids_from_lists_kernel");
   return HEXA_OK;
+}
+}  // namespace
+
+extern "C" int hexa_ids_from_lists(const int32_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_toks, int32_t* ids,
+                                   void* stream_) {
+  return ids_from_lists(tok_ids, exp_ids, n, chunk, num_toks, ids, (cudaStream_t)stream_);
+}
+extern "C" int hexa_ids_from_lists_i64(const int64_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_toks,
+                                       int32_t* ids, void* stream_) {
+  return ids_from_lists(reinterpret_cast<const long long*>(tok_ids), exp_ids, n, chunk, num_toks, ids, (cudaStream_t)stream_);
 }

@@ -51,16 +51,6 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
   return t;
 }
 
-// The status word may live in device memory or in pinned host memory (where the host can poll it without a copy), so
-// it is written with plain stores: the first code to arrive stays, and which of two simultaneous codes wins is immaterial.
-__device__ __forceinline__ void report_status(int32_t* status, int code) {
-  if (status) {
-    volatile int32_t* s = status;
-    if (*s == 0) *s = code;
-    __threadfence_system();
-  }
-}
-
 // Bounded wait.  Returns false when this CTA is aborting (its own limit ran out or another role's did).
 __device__ __noinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int32_t* status, int code,
                                        uint64_t limit_ns) {

@@ -85,7 +85,7 @@ const char* hexa_last_error_string(void);
  * memory (cudaHostAlloc / cudaHostRegister), which the host can read at any time without a copy or a synchronisation.
  * A kernel that gives up a wait stores a non-zero code there (1 = producer waiting for a free ring slot, 2 = MMA
  * issuer waiting for a drained accumulator, 3 = MMA issuer waiting for operands, 4 = epilogue waiting for an
- * accumulator), lets copies in flight land, frees its tensor memory and returns; its outputs are incomplete.
+ * accumulator, 5 = epilogue waiting for the saved pre-activation), lets copies in flight land, frees its tensor memory and returns; its outputs are incomplete.
  * One word per device, shared by all host threads (forward and backward of a training step are launched from
  * different threads).  With a word in pinned host memory, hexa_esmm / hexa_estmm / hexa_estmm_scatter return
  * HEXA_ERR_DEVICE without launching while the word is non-zero; the caller zeroes the word to continue.
@@ -134,9 +134,12 @@ int hexa_route(const int32_t* ids, int64_t num_tokens, int top_k, int64_t stride
                void* workspace, size_t workspace_bytes, void* stream);
 
 /* One expert id per token from the reference's operator-level lists (kernels/esmm.py:249-263): tok_ids[n] holds token
- * ids + 1 (0 = pad) and entry i belongs to expert exp_ids[i / chunk].  ids[num_tokens]: -1 for tokens in no segment. */
+ * ids + 1 (0 = pad) and entry i belongs to expert exp_ids[i / chunk].  ids[num_tokens]: -1 for tokens in no segment.
+ * A negative entry counts from the end.  An entry that names no token writes nothing and leaves code 6 in the status word. */
 int hexa_ids_from_lists(const int32_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_tokens, int32_t* ids,
                         void* stream);
+int hexa_ids_from_lists_i64(const int64_t* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_tokens, int32_t* ids,
+                            void* stream);
 
 /* ---- row movement between token order and sorted-row order (the reference gathers rows by
  *      tok_ids inside its kernels, kernels/esmm.py:95-101, and sums the k routes in Python,

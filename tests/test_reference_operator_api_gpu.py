@@ -88,3 +88,33 @@ def test_expert_ids_from_lists(T, n, dtype):
     want[tok] = exp.repeat_interleave(16)
     got = ids_from_lists(T, tok.to(dtype).cuda(), exp.cuda())
     assert got.dtype == torch.int32 and torch.equal(got.cpu(), want[1:])
+
+
+def test_expert_ids_refuse_lists_on_another_device():
+    from hexa_moe_b200 import _lib as L, ops
+    tok, exp = torch.ones(16, dtype=torch.int32), torch.zeros(1, dtype=torch.int32)
+    for a, b in ((tok.cuda(), exp), (tok, exp.cuda())):
+        with pytest.raises(L.HexaError):
+            ops.ids_from_lists(4, a, b, 16)
+    with pytest.raises(L.HexaError, match="cover"):                   # 16 entries per expert id
+        ops.ids_from_lists(4, tok.cuda().repeat(2), exp.cuda(), 16)
+
+
+@pytest.mark.parametrize("bad,dtype", [(6, torch.int32), (-7, torch.int32), (6, torch.int64), ((1 << 32) + 2, torch.int64)])
+def test_expert_ids_report_a_token_that_is_not_there(bad, dtype):
+    """The kernel's bounds check skips the entry and leaves a code that the next call raises; entries that index, from
+    either end, are taken."""
+    from hexa_moe_b200 import _lib as L, ops
+    tok = torch.tensor([1, 5, -1, -6] + [0] * 12, dtype=dtype)
+    exp = torch.tensor([3], dtype=torch.int32).cuda()
+    assert ops.ids_from_lists(5, tok.cuda(), exp, 16).tolist() == [3, -1, -1, -1, 3]
+    tok[7] = bad
+    ids = ops.ids_from_lists(5, tok.cuda(), exp, 16)
+    torch.cuda.synchronize()
+    assert ids.tolist() == [3, -1, -1, -1, 3] and L.device_status() == L.STATUS_BAD_TOKEN
+    try:
+        with pytest.raises(L.HexaError, match="index out of range"):
+            ops.route(ids.view(-1, 1), 4)
+    finally:
+        L.clear_device_status()
+    ops.route(ids.view(-1, 1), 4)
