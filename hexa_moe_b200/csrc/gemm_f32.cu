@@ -51,6 +51,7 @@ struct Params {
   int64_t n, k, m;
   int E;
   uint32_t nt, per_expert, total_tiles;
+  int debug;      // test aid (hexa_set_tc_debug): bit 2 = the producer neither loads nor arrives, every wait runs into its limit
   int32_t* status;
   uint64_t wait_limit_ns;
 };
@@ -137,6 +138,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           uint8_t* sA = smem + (size_t)stage * kStageBytes;
           uint8_t* sB = sA + kOperandBytes;
           const uint32_t lead_full = lead_full0 + 8u * (uint32_t)stage;
+          if (p.debug & 4) {
+            if (++stage == kStages) { stage = 0; phase ^= 1; }
+            continue;
+          }
           if (rank == 0) mbar_expect_tx(&full[stage], 2 * kStageBytes);      // both CTAs' bytes
           if (MODE == TN) {      // 64 columns of all three planes per load
             const int r = tile.row0 + kb * BLOCK_K;
@@ -215,7 +220,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       bool good = true;
       for (int kb = 0; kb < tile.num_kb; ++kb, ++chunk) {
         const uint32_t acc = chunk & 1;
-        if (!(good = mbar_wait(&acc_full[acc], (chunk >> 1) & 1u, abort_flag, p.status, 4, p.wait_limit_ns))) break;
+        // one verdict per warp: what follows is for all 32 lanes or none
+        good = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (chunk >> 1) & 1u, abort_flag, p.status, 4, p.wait_limit_ns));
+        if (!good) break;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BLOCK_N + (uint32_t)(part * kPartCols);
 #pragma unroll
@@ -506,7 +513,7 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
   p.max_pairs = row_cap / (2 * BLOCK_M) + E;
   p.bias = bias; p.ldbias = ldbias; p.n = n_out; p.k = k; p.E = E;
   p.nt = (uint32_t)ceil_div(n_out, BLOCK_N);
-  p.status = status_word(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
   HEXA_REQUIRE((row_cap / BLOCK_M + E + 1) * (int64_t)p.nt < (int64_t)0x7fffffff, "hexa_esmm: too many output tiles for a 32-bit tile index");
   const int64_t max_tiles = p.max_pairs * (int64_t)p.nt;
   rc = nk ? launch<NK>(tmA, tmB, tmC, p, max_tiles, stream) : launch<KN>(tmA, tmB, tmC, p, max_tiles, stream);
@@ -549,7 +556,7 @@ int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, co
   HEXA_REQUIRE(per_expert * E < (int64_t)0x7fffffff, "hexa_estmm: too many output tiles for a 32-bit tile index");
   p.per_expert = (uint32_t)per_expert;
   p.total_tiles = (uint32_t)(per_expert * E);
-  p.status = status_word(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
   rc = launch<TN>(tmA, tmB, tmC, p, per_expert * E, stream);
   if (rc) return rc;
   return estmm_simt_launch(pp, ldp, q, ldq, pad_offsets, E, m, n, out, ldo, o_estride, m, 0, HEXA_F32, HEXA_F32, 0, stream, flags, n_flags);

@@ -73,6 +73,59 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_keeps_working(ops, n_ou
     assert torch.equal(again[:n_pad], good[:n_pad]) and L.device_status() == 0
 
 
+@pytest.mark.parametrize("form", ["nk", "kn", "tn"])
+def test_a_wait_that_runs_out_in_the_fp32_kernel(ops, form):
+    """The same for fp32 data on the tensor cores (ESMM with either weight layout, ESTMM)."""
+    from hexa_moe_b200 import _lib as L
+    lib = L.lib()
+    T, E, K, N = 12000, 4, 256, 512
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = ops.route(torch.randint(0, E, (T, 1), generator=g, device="cuda").to(torch.int32), E)
+    xs = ops.gather_rows(torch.randn(T, K, generator=g, device="cuda"), r)
+    n_pad = int(r.pad_offsets[-1])
+    stream = torch.cuda.current_stream().cuda_stream
+    if form == "tn":
+        q = ops.gather_rows(torch.randn(T, 2048, generator=g, device="cuda"), r)
+        run = lambda: ops.estmm(xs, q, r)
+        out = torch.empty(E, K, 2048, device="cuda")
+        ws = torch.empty(lib.hexa_estmm_workspace_bytes(E, r.row_capacity, K, 2048, L.F32), dtype=torch.uint8, device="cuda")
+        raw = lambda: lib.hexa_estmm(xs.data_ptr(), K, q.data_ptr(), 2048, r.pad_offsets.data_ptr(), E, r.row_capacity, K, 2048,
+                                     out.data_ptr(), 2048, K * 2048, 0, 0, L.F32, L.F32, 0, L.ENGINE_AUTO, ws.data_ptr(), ws.numel(), stream)
+    else:
+        w = torch.randn(E, N, K, generator=g, device="cuda")
+        w, lay = (w, L.B_NK) if form == "nk" else (w.transpose(1, 2).contiguous(), L.B_KN)
+        run = lambda: ops.esmm(xs, w, lay, r)[:n_pad]
+        out = torch.empty(r.row_capacity, N, device="cuda")
+        ws = torch.empty(lib.hexa_esmm_f32_workspace_bytes(E, r.row_capacity, N, K), dtype=torch.uint8, device="cuda")
+        raw = lambda: lib.hexa_esmm_f32(xs.data_ptr(), K, w.data_ptr(), lay, w.stride(1), w.stride(0), None, 0, None, 0, out.data_ptr(), N,
+                                        r.tile_expert.data_ptr(), r.pad_offsets.data_ptr(), r.row_token.data_ptr(),
+                                        r.pair_block.data_ptr(), E, r.row_capacity, N, K, L.EPI_LINEAR, L.ACT_NONE, ws.data_ptr(),
+                                        ws.numel(), stream)
+    assert ws.numel() > 0
+    good = run().clone()
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+    try:
+        assert lib.hexa_set_wait_limit_ns(5_000_000) == 0 and lib.hexa_set_tc_debug(4) == 0
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        assert raw() == 0                             # the failure happens on the device
+        t1.record()
+        torch.cuda.synchronize()
+        assert t0.elapsed_time(t1) < 1000.0
+    finally:
+        lib.hexa_set_tc_debug(0)
+        lib.hexa_set_wait_limit_ns(2_000_000_000)
+    code = L.device_status()
+    assert code in (1, 2, 3, 4), code
+    with pytest.raises(L.HexaError, match="bounded wait"):
+        run()
+    L.clear_device_status()
+    assert torch.equal(run(), good)
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+
+
 def test_status_word_is_shared_by_host_threads(ops):
     """Backward runs on the autograd engine's thread: the word installed from the main thread must be the one a
     kernel launched from another thread reports to."""
