@@ -9,8 +9,12 @@
 //   k = 128: 2.0e-7 / 0.8e-7    512: 4.1e-7 / 1.0e-7    2048: 8.1e-7 / 1.3e-7    8192: 1.6e-6 / 2.2e-7
 // (positive data, the worst for truncation: 1.7 / 0.9, 3.5 / 1.0, 7.0 / 1.2, 14 / 2.0 e-7; with 128-deep blocks the bias
 // doubles and reaches the FMA chain's error at k = 128, over the whole k it exceeds it).
-// A value that is not finite, or that a bf16 cannot hold, has no such planes: the split raises a flag and the CUDA-core
-// kernel, launched behind, redoes the whole operator (it returns at once when no flag is set).
+// Not every operand has such planes.  A value that is not finite, or that a bf16 cannot hold, has none; one below 2^-109 has a
+// third term under bf16's smallest step, 2^-133 (operands of 2^-116: 2.2e-6 where the FMA chain has 2.9e-7, of 2^-124: 5.6e-4);
+// products that leave fp32's range come out of six terms of either sign as NaN where a chain gives infinity; and when every
+// product lies near the lower end (2^-64 x 2^-64) the chain is closer.  So the split takes the largest magnitude of either
+// operand and looks for values without planes, an idle warp of the GEMM makes one verdict of it (planes_hold), and the
+// CUDA-core kernel, launched behind, redoes the whole operator where the verdict says so (else it returns at once).
 //
 // Bound: the tensor pipe, six MMAs where bf16 data needs one.  A CTA pair computes a 256 x 256 tile (each CTA its own 128
 // rows of A and half of B, as the 16-bit kernel does); a stage is one k-block of both operands' three planes, 96 KB per
@@ -20,8 +24,6 @@
 // (epilogue_rows_kernel): in the epilogue they would hold up the next tile's k-blocks.
 // fp32 layer of 8192 tokens, d=512, hidden 2048, 8 experts, top-2 (a launch, CUDA cores / this): fc1 + GELU 811 / 274 us,
 // fc2 790 / 233, GELU' 848 / 300, weight gradient 822 / 235.
-#include <float.h>
-
 #include "gemm_launch.h"
 #include "hexa_common.cuh"
 #include "tc_ptx.cuh"
@@ -51,6 +53,10 @@ struct Params {
   int64_t n, k, m;
   int E;
   uint32_t nt, per_expert, total_tiles;
+  const uint32_t* maxima;   // [2][n_maxima] per block of the split: largest magnitude of a, of b (bits; kNoPlanes: a value without planes)
+  int n_maxima;
+  int terms;                // the most products one result can have
+  int32_t* redo;            // the verdict, for the kernel behind this one
   int debug;      // test aid (hexa_set_tc_debug): bit 2 = the producer neither loads nor arrives, every wait runs into its limit
   int32_t* status;
   uint64_t wait_limit_ns;
@@ -60,6 +66,18 @@ struct Tile {
   int e, row0, col0, m0, num_kb;
   bool valid;      // this CTA has rows to store
 };
+
+constexpr uint32_t kNoPlanes = 0xffffffffu;
+
+// May the products be made from planes?  amax, bmax: bits of the operands' largest magnitudes.
+__device__ __forceinline__ bool planes_hold(uint32_t amax, uint32_t bmax, int terms) {
+  if (amax == kNoPlanes || bmax == kNoPlanes) return false;
+  if (amax == 0 || bmax == 0) return true;      // all zero
+  const int ea = (int)(amax >> 23) - 126, eb = (int)(bmax >> 23) - 126;      // |a| < 2^ea, |b| < 2^eb
+  const int log_terms = 32 - __clz(terms);                                   // terms < 2^log_terms
+  return ea + eb + log_terms <= 127      // no partial sum reaches 2^128
+         && ea + eb >= -100;             // the largest products carry all their terms
+}
 
 template <int MODE>
 __device__ __forceinline__ bool get_tile(const Params& p, uint32_t t, int rank, Tile& tile) {
@@ -204,6 +222,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
     }
+    if (blockIdx.x == 1) {      // the second CTA of the first pair issues nothing
+      uint32_t amax = 0, bmax = 0;
+      for (int i = lane; i < p.n_maxima; i += 32) {
+        amax = max(amax, __ldg(p.maxima + i));
+        bmax = max(bmax, __ldg(p.maxima + p.n_maxima + i));
+      }
+      amax = __reduce_max_sync(0xffffffffu, amax);
+      bmax = __reduce_max_sync(0xffffffffu, bmax);
+      if (lane == 0) *p.redo = planes_hold(amax, bmax, p.terms) ? 0 : 1;
+    }
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ epilogue (every CTA, its own 128 rows)
@@ -296,14 +324,24 @@ struct Side {
   int vec;                              // rows are whole 16-byte groups
 };
 
-// A warp per row, both operands in one launch; flags[block] = some value of this block's rows has no planes.
+// Magnitude of a value as ordered bits, kNoPlanes where three bf16 terms cannot hold it: not finite, rounded to infinity by
+// the first term, or so small that the third falls below bf16's smallest step.
+__device__ __forceinline__ uint32_t magnitude(float x) {
+  const uint32_t m = __float_as_uint(x) & 0x7fffffffu;
+  constexpr uint32_t least = (uint32_t)(127 - 109) << 23, most = 0x7f7f7fffu;      // the largest value that rounds to a finite bf16
+  return m - least <= most - least || m == 0 ? m : kNoPlanes;
+}
+
+// A warp per row, both operands in one launch; maxima[block], maxima[blocks + block] = the largest magnitude of this block's
+// rows of a and of b.
 __global__ void __launch_bounds__(256)
-split_planes_kernel(const Side a, const Side b, int32_t* __restrict__ flags) {
+split_planes_kernel(const Side a, const Side b, uint32_t* __restrict__ maxima) {
+  __shared__ uint32_t seen[2][8];
   const int lane = threadIdx.x & 31;
   const int64_t rows_a = a.limit ? min((int64_t)*a.limit, a.rows) : a.rows * a.E;
   const int64_t rows_b = b.limit ? min((int64_t)*b.limit, b.rows) : b.rows * b.E;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  int bad = 0;
+  uint32_t most[2] = {0, 0};
   for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < rows_a + rows_b; w += warps) {
     const bool first = w < rows_a;
     const Side& s = first ? a : b;
@@ -311,37 +349,47 @@ split_planes_kernel(const Side a, const Side b, int32_t* __restrict__ flags) {
     const float* src = s.src + e * s.estride + r * s.ld;
     __nv_bfloat16* dst = s.dst + flat * s.pitch;
     const int64_t plane = s.plane;
+    uint32_t m = 0;
     if (s.vec) {
       for (int64_t c = lane * 4; c < s.cols; c += 128) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(src + c));
         float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m = max(m, magnitude(x[i]));
 #pragma unroll
         for (int q = 0; q < kPlanes; ++q) {
           __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[0], x[1]), __floats2bfloat162_rn(x[2], x[3])};
           *reinterpret_cast<uint2*>(dst + q * plane + c) = *reinterpret_cast<const uint2*>(h);
           x[0] -= __low2float(h[0]); x[1] -= __high2float(h[0]);
           x[2] -= __low2float(h[1]); x[3] -= __high2float(h[1]);
-          if (q == 0) {      // inf - inf and NaN - NaN leave NaN, a finite value beyond bf16 leaves -inf
-#pragma unroll
-            for (int i = 0; i < 4; ++i) bad |= !(fabsf(x[i]) <= FLT_MAX);
-          }
         }
       }
     } else {
       for (int64_t c = lane; c < s.cols; c += 32) {
         float x = src[c];
+        m = max(m, magnitude(x));
 #pragma unroll
         for (int q = 0; q < kPlanes; ++q) {
           const __nv_bfloat16 h = __float2bfloat16_rn(x);
           dst[q * plane + c] = h;
           x -= __bfloat162float(h);
-          if (q == 0) bad |= !(fabsf(x) <= FLT_MAX);
         }
       }
     }
+    if (first) most[0] = max(most[0], m);
+    else most[1] = max(most[1], m);
   }
-  bad = __syncthreads_or(bad);
-  if (threadIdx.x == 0) flags[blockIdx.x] = bad;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const uint32_t m = __reduce_max_sync(0xffffffffu, most[i]);
+    if (lane == 0) seen[i][threadIdx.x >> 5] = m;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    uint32_t m = 0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) m = max(m, seen[threadIdx.x][i]);
+    maxima[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = m;
+  }
 }
 
 // c = act(x) (x may be c itself) or c = c * act'(x), x [rows, cols], over the rows in use
@@ -373,7 +421,7 @@ epilogue_rows_kernel(const float* x, int64_t ldx, float* c, int64_t ldc, const i
 
 // ---- host side --------------------------------------------------------------------------------------------------------------
 constexpr int kMaxSplitBlocks = 2048;
-constexpr size_t kFlagBytes = kMaxSplitBlocks * sizeof(int32_t);
+constexpr size_t kFlagBytes = (2 * kMaxSplitBlocks + 64) * sizeof(int32_t);      // the blocks' maxima, the verdict
 constexpr size_t kMaxWorkspace = (size_t)2 << 30;      // scratch a call may take; beyond it the CUDA cores do the work
 
 int64_t pitch_of(int64_t cols) { return (cols + 7) / 8 * 8; }
@@ -393,14 +441,19 @@ bool pays(int64_t tiles, int64_t kb, double split_values, double pass_values, in
   return tc * 1.15 < flops / (large ? 44e6 : 30e6);
 }
 
-int split_launch(const Side& a, const Side& b, int32_t* flags, int* n_flags, cudaStream_t stream) {
+// Writes both operands' planes and tells `p` where their maxima are and the verdict goes.
+int split_launch(const Side& a, const Side& b, uint8_t* ws, int64_t terms, Params& p, cudaStream_t stream) {
   const int64_t want = ceil_div(a.rows * a.E + b.rows * b.E, 8);
   int64_t blocks = (int64_t)sm_count() * 8;
   if (blocks > kMaxSplitBlocks) blocks = kMaxSplitBlocks;
   if (want < blocks) blocks = want > 0 ? want : 1;
-  split_planes_kernel<<<(unsigned)blocks, 256, 0, stream>>>(a, b, flags);
+  uint32_t* maxima = reinterpret_cast<uint32_t*>(ws);
+  split_planes_kernel<<<(unsigned)blocks, 256, 0, stream>>>(a, b, maxima);
   HEXA_LAUNCH_CHECK("split_planes_kernel");
-  *n_flags = (int)blocks;
+  p.maxima = maxima;
+  p.n_maxima = (int)blocks;
+  p.terms = (int)(terms < INT32_MAX ? terms : INT32_MAX);
+  p.redo = reinterpret_cast<int32_t*>(ws) + 2 * kMaxSplitBlocks;
   return HEXA_OK;
 }
 
@@ -490,12 +543,11 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
                     const int32_t* pad_offsets, const int32_t* row_token, const int32_t* pair_block, int E, int64_t row_cap,
                     int64_t n_out, int64_t k, int epilogue, int act, cudaStream_t stream, void* workspace) {
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  int32_t* flags = reinterpret_cast<int32_t*>(ws);
   const bool nk = b_layout == HEXA_B_NK;
   const Side sa = make_side(a, lda, 0, 1, row_cap, k, pad_offsets + E, ws + kFlagBytes);
   const Side sb = make_side(b, ldb, b_estride, E, nk ? n_out : k, nk ? k : n_out, nullptr, ws + kFlagBytes + plane_bytes(row_cap, k));
-  int n_flags = 0;
-  int rc = split_launch(sa, sb, flags, &n_flags, stream);
+  Params p{};
+  int rc = split_launch(sa, sb, ws, k, p, stream);
   if (rc) return rc;
   CUtensorMap tmA, tmB, tmC;
   if ((rc = plane_map(&tmA, sa, false, BLOCK_K, BLOCK_M))) return rc;
@@ -508,7 +560,6 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
     const uint32_t box[2] = {kSlab, BLOCK_M};
     if ((rc = encode_tensor_map(&tmC, pre ? aux : c, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
   }
-  Params p{};
   p.tile_expert = tile_expert; p.pad_offsets = pad_offsets; p.row_token = row_token; p.pair_block = pair_block;
   p.max_pairs = row_cap / (2 * BLOCK_M) + E;
   p.bias = bias; p.ldbias = ldbias; p.n = n_out; p.k = k; p.E = E;
@@ -528,17 +579,16 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
     HEXA_LAUNCH_CHECK("epilogue_rows_kernel");
   }
   return esmm_simt_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token, E,
-                          row_cap, n_out, k, HEXA_F32, epilogue, act, stream, 0, E, 0, flags, n_flags);
+                          row_cap, n_out, k, HEXA_F32, epilogue, act, stream, 0, E, 0, p.redo);
 }
 
 int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets, int E, int64_t row_cap,
                      int64_t m, int64_t n, void* out, int64_t ldo, int64_t o_estride, cudaStream_t stream, void* workspace) {
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  int32_t* flags = reinterpret_cast<int32_t*>(ws);
   const Side sp = make_side(pp, ldp, 0, 1, row_cap, m, pad_offsets + E, ws + kFlagBytes);
   const Side sq = make_side(q, ldq, 0, 1, row_cap, n, pad_offsets + E, ws + kFlagBytes + plane_bytes(row_cap, m));
-  int n_flags = 0;
-  int rc = split_launch(sp, sq, flags, &n_flags, stream);
+  Params p{};
+  int rc = split_launch(sp, sq, ws, row_cap, p, stream);
   if (rc) return rc;
   CUtensorMap tmA, tmB, tmC;
   if ((rc = plane_map(&tmA, sp, false, 64, BLOCK_K))) return rc;
@@ -549,7 +599,6 @@ int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, co
     const uint32_t box[3] = {kSlab, BLOCK_M, 1};
     if ((rc = encode_tensor_map(&tmC, out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
   }
-  Params p{};
   p.pad_offsets = pad_offsets; p.n = n; p.m = m; p.E = E;
   p.nt = (uint32_t)ceil_div(n, BLOCK_N);
   const int64_t per_expert = ceil_div(m, 2 * BLOCK_M) * (int64_t)p.nt;
@@ -559,7 +608,7 @@ int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, co
   p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
   rc = launch<TN>(tmA, tmB, tmC, p, per_expert * E, stream);
   if (rc) return rc;
-  return estmm_simt_launch(pp, ldp, q, ldq, pad_offsets, E, m, n, out, ldo, o_estride, m, 0, HEXA_F32, HEXA_F32, 0, stream, flags, n_flags);
+  return estmm_simt_launch(pp, ldp, q, ldq, pad_offsets, E, m, n, out, ldo, o_estride, m, 0, HEXA_F32, HEXA_F32, 0, stream, p.redo);
 }
 
 }  // namespace hexa

@@ -19,13 +19,13 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
                     int64_t n_out, int64_t k, int epilogue, int act, cudaStream_t stream, void* workspace);
 int estmm_f32_launch(const void* p, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets, int E, int64_t row_cap,
                      int64_t m, int64_t n, void* out, int64_t ldo, int64_t o_estride, cudaStream_t stream, void* workspace);
-// The CUDA-core launchers below can be told to do nothing unless one of `n_flags` device words is set (null: always run).
+// The CUDA-core launchers below can be told to do nothing unless a device word is set (`only_if`; null: always run).
 // (their bias, and that of esmm_tc_launch, is fp32 or, with bias16, of the data's 16-bit type)
 int esmm_simt_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const void*, int64_t, void*, int64_t, void*,
                      int64_t, const int32_t*, const int32_t*, const int32_t*, int, int64_t, int64_t, int64_t, int, int, int,
-                     cudaStream_t, int e_begin, int e_end, int bias16 = 0, const int32_t* flags = nullptr, int n_flags = 0);
+                     cudaStream_t, int e_begin, int e_end, int bias16 = 0, const int32_t* only_if = nullptr);
 int estmm_simt_launch(const void*, int64_t, const void*, int64_t, const int32_t*, int, int64_t, int64_t, void*, int64_t,
-                      int64_t, int64_t, int64_t, int, int, int, cudaStream_t, const int32_t* flags = nullptr, int n_flags = 0);
+                      int64_t, int64_t, int64_t, int, int, int, cudaStream_t, const int32_t* only_if = nullptr);
 bool esmm_tc_supported(const void*, int64_t, const void*, int64_t, int64_t, const void*, int64_t, const void*, int64_t,
                        const float*, int64_t, int64_t, int);
 int esmm_tc_launch(const void*, int64_t, const void*, int, int64_t, int64_t, const void*, int64_t, void*, int64_t, void*,

@@ -158,13 +158,8 @@ __device__ __forceinline__ void contract(Acc<TILE>& acc, const T* __restrict__ a
   }
 }
 
-// True when one of the words is set, or when there are none to look at (every thread gets the same answer).
-__device__ __forceinline__ bool wanted(const int32_t* __restrict__ flags, int n_flags) {
-  if (flags == nullptr) return true;
-  int any = 0;
-  for (int i = threadIdx.x; i < n_flags; i += kThreads) any |= __ldg(flags + i);
-  return __syncthreads_or(any) != 0;
-}
+// A launch with a condition does nothing unless that word is set.
+__device__ __forceinline__ bool wanted(const int32_t* __restrict__ only_if) { return only_if == nullptr || __ldg(only_if) != 0; }
 
 template <typename T, int TILE, bool B_NK, bool VEC>
 __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
@@ -173,8 +168,8 @@ esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, 
                  T* __restrict__ c, int64_t ldc, const int32_t* __restrict__ tile_expert,
                  const int32_t* __restrict__ pad_offsets, const int32_t* __restrict__ row_token, int E, int64_t n_out,
                  int64_t k, int epilogue, int act, int e_begin, int e_end, int bias16,
-                 const int32_t* __restrict__ flags, int n_flags) {
-  if (!wanted(flags, n_flags)) return;
+                 const int32_t* __restrict__ only_if) {
+  if (!wanted(only_if)) return;
   const int64_t row0 = (int64_t)blockIdx.y * TILE;
   if (row0 >= pad_offsets[E]) return;
   const int e = tile_expert[row0 / kRowTile];
@@ -233,8 +228,8 @@ template <typename T, typename TO, int TILE, bool VEC>
 __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
 estmm_simt_kernel(const T* __restrict__ p, int64_t ldp, const T* __restrict__ q, int64_t ldq,
                   const int32_t* __restrict__ pad_offsets, int64_t m, int64_t n, TO* __restrict__ out, int64_t ldo,
-                  int64_t o_estride, int64_t m_split, int64_t split_stride, int beta, const int32_t* __restrict__ flags, int n_flags) {
-  if (!wanted(flags, n_flags)) return;
+                  int64_t o_estride, int64_t m_split, int64_t split_stride, int beta, const int32_t* __restrict__ only_if) {
+  if (!wanted(only_if)) return;
   const int e = blockIdx.z;
   const int64_t m0 = (int64_t)blockIdx.y * TILE, n0 = (int64_t)blockIdx.x * TILE;
   Acc<TILE> acc;
@@ -281,7 +276,7 @@ int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, in
                      const void* bias, int64_t ldbias, void* aux, int64_t ldaux, void* c, int64_t ldc,
                      const int32_t* tile_expert, const int32_t* pad_offsets, const int32_t* row_token, int E,
                      int64_t row_cap, int64_t n_out, int64_t k, int dtype, int epilogue, int act, cudaStream_t stream,
-                     int e_begin, int e_end, int bias16, const int32_t* flags, int n_flags) {
+                     int e_begin, int e_end, int bias16, const int32_t* only_if) {
   if (row_cap == 0 || e_begin >= e_end) return HEXA_OK;
   if (e_begin < 0) e_begin = 0;
   HEXA_REQUIRE(row_cap / 64 <= 65535, "hexa_esmm (simt): row_capacity %lld too large", (long long)row_cap);
@@ -295,7 +290,7 @@ int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, in
   esmm_simt_kernel<T, TILE, NK, VEC><<<grid, kThreads, 0, stream>>>((const T*)a, lda, (const T*)b, ldb, b_estride, bias, \
                                                                     ldbias, (T*)aux, ldaux, (T*)c, ldc, tile_expert,   \
                                                                     pad_offsets, row_token, E, n_out, k, epilogue, act, \
-                                                                    e_begin, e_end, bias16, flags, n_flags)
+                                                                    e_begin, e_end, bias16, only_if)
 #define HEXA_ESMM_SIMT_T(T, VEC)                              \
   do {                                                        \
     if (large && nk) HEXA_ESMM_SIMT(T, 128, true, VEC);       \
@@ -320,7 +315,7 @@ int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, in
 
 int estmm_simt_launch(const void* p, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets, int E,
                       int64_t m, int64_t n, void* out, int64_t ldo, int64_t o_estride, int64_t m_split, int64_t split_stride,
-                      int dtype, int out_dtype, int beta, cudaStream_t stream, const int32_t* flags, int n_flags) {
+                      int dtype, int out_dtype, int beta, cudaStream_t stream, const int32_t* only_if) {
   HEXA_REQUIRE(ceil_div(m, 64) <= 65535 && E <= 65535, "hexa_estmm (simt): grid too large");
   const bool vec = dtype == HEXA_F32 && aligned16(p) && aligned16(q) && aligned16(out) && ldp % 4 == 0 && ldq % 4 == 0 && ldo % 4 == 0 &&
                    o_estride % 4 == 0 && split_stride % 4 == 0 && m % 4 == 0 && n % 4 == 0;
@@ -329,8 +324,7 @@ int estmm_simt_launch(const void* p, int64_t ldp, const void* q, int64_t ldq, co
   dim3 grid((unsigned)ceil_div(n, tile), (unsigned)ceil_div(m, tile), (unsigned)E);
 #define HEXA_ESTMM_SIMT_V(T, TO, TILE, VEC)                                                                             \
   estmm_simt_kernel<T, TO, TILE, VEC><<<grid, kThreads, 0, stream>>>((const T*)p, ldp, (const T*)q, ldq, pad_offsets, m, n, \
-                                                                     (TO*)out, ldo, o_estride, m_split, split_stride, beta, flags, \
-                                                                     n_flags)
+                                                                     (TO*)out, ldo, o_estride, m_split, split_stride, beta, only_if)
 #define HEXA_ESTMM_SIMT(T, TO, VEC)                    \
   do {                                                 \
     if (large) HEXA_ESTMM_SIMT_V(T, TO, 128, VEC);     \

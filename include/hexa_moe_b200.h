@@ -250,7 +250,8 @@ int hexa_ess(const void* src, int64_t src_ld, const int32_t* pad_offsets, int nu
 /* hexa_esmm on fp32 data with scratch: where it pays (by sizes) and the arguments allow, the products run on the tensor
  * cores as six bf16 term products per k-block with fp32 additions between k-blocks, closer to the exact result than the
  * FMA chain of the CUDA-core kernel, which computes the call otherwise, whenever an operand holds a value that is not
- * finite or beyond bf16's range, and for HEXA_EPI_ACT with HEXA_ACT_RELU (the sign of a pre-activation near zero must not
+ * finite, beyond bf16's range or below 2^-109 (zero aside), whenever the operands' magnitudes let a sum overflow or leave
+ * every product below 2^-100, and for HEXA_EPI_ACT with HEXA_ACT_RELU (the sign of a pre-activation near zero must not
  * depend on the path).  workspace: hexa_esmm_f32_workspace_bytes() bytes (0: none is used), contents irrelevant.
  * hexa_estmm does the same for fp32 inputs given hexa_estmm_workspace_bytes(..., HEXA_F32). */
 size_t hexa_esmm_f32_workspace_bytes(int num_experts, int64_t row_capacity, int64_t n_out, int64_t k);

@@ -114,8 +114,56 @@ def test_values_without_planes_take_the_fma_chain(bad, where):
         assert torch.equal(dw.nan_to_num(7.0, 8.0, 9.0), dw2.nan_to_num(7.0, 8.0, 9.0))
 
 
+def _scaled(x, e):
+    """x * 2^e with the exponent in two steps (2^e alone may be out of range)."""
+    return x * 2.0 ** (e // 2) * 2.0 ** (e - e // 2)
+
+
+# Exponents of two operands of normal data: inside the range where planes hold, at both of its ends, and beyond.  Where
+# they do not hold the answer is the FMA chain's own: bits are lost, products overflow in terms of either sign, or all fall
+# below the normal range.
+@pytest.mark.parametrize("ea,eb,planes", [(0, 0, True), (-80, 0, True), (-80, 60, True), (90, 20, True), (-60, -36, True), (55, 55, True),
+                                          (-100, 0, False), (0, -112, False), (-116, 20, False), (-124, 100, False), (-140, 0, False),
+                                          (-60, -50, False), (-64, -64, False), (-66, -66, False), (60, 60, False), (62, 62, False),
+                                          (100, 20, False), (100, 100, False), (0, 126, False)])
+def test_magnitudes_decide_between_planes_and_chain(ea, eb, planes):
+    L, ops = _mods()
+    T, K, N, E = 12000, 256, 512, 4
+    r, g = _routing(ops, T, E, 2, 5)
+    xs = ops.gather_rows(_scaled(torch.randn(T, K, generator=g, device="cuda"), ea), r)
+    w = _scaled(torch.randn(E, N, K, generator=g, device="cuda"), eb)
+    n_pad = int(r.pad_offsets[-1])
+    po = r.pad_offsets.tolist()
+    got, chain = (ops.esmm(xs, w, L.B_NK, r, engine=e)[:n_pad] for e in (L.ENGINE_AUTO, L.ENGINE_SIMT))
+    if not planes:
+        assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), chain.nan_to_num(7.0, 8.0, 9.0))
+        return
+    exact = torch.cat([xs[po[e]:po[e + 1]].double() @ w[e].double().t() for e in range(E)])
+    assert not torch.equal(got, chain) and _rel(got, exact) <= _rel(chain, exact)
+
+
+@pytest.mark.parametrize("value,planes", [(2.0 ** -109, True), (-2.0 ** -109 * (1 - 2.0 ** -24), False), (2.0 ** -149, False), (0.0, True),
+                                          (3.3895e38, False), (2.0 ** 105, True), (2.0 ** 127, False)])
+@pytest.mark.parametrize("op", ["a", "b", "tn"])
+def test_one_value_decides(value, planes, op):
+    """A single value at the ends of the range among normal data, in either operand of ESMM or one of ESTMM."""
+    L, ops = _mods()
+    T, K, N, E = 12000, 256, 2048, 4
+    r, g = _routing(ops, T, E, 2, 3)
+    x, w = torch.randn(T, K, generator=g, device="cuda"), torch.randn(E, N, K, generator=g, device="cuda")
+    (w[2] if op == "b" else x)[17, 5] = value
+    xs = ops.gather_rows(x, r)
+    n_pad = int(r.pad_offsets[-1])
+    if op == "tn":
+        q = ops.gather_rows(torch.randn(T, N, generator=g, device="cuda"), r)
+        got, chain = (ops.estmm(xs, q, r, engine=e) for e in (L.ENGINE_AUTO, L.ENGINE_SIMT))
+    else:
+        got, chain = (ops.esmm(xs, w, L.B_NK, r, engine=e)[:n_pad] for e in (L.ENGINE_AUTO, L.ENGINE_SIMT))
+    assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), chain.nan_to_num(7.0, 8.0, 9.0)) != planes
+
+
 def test_tiny_values_keep_their_products():
-    """Terms that fall below bf16's normal range: the result stays as close as the FMA chain's."""
+    """Operands around 1e-30, some of which lie below the range of planes: the result stays as close as the FMA chain's."""
     L, ops = _mods()
     r, g = _routing(ops, 12000, 4, 2, 5)
     x = torch.randn(12000, 256, generator=g, device="cuda") * 1e-30
