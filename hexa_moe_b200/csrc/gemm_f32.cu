@@ -6,8 +6,8 @@
 // instruction, so it is never given a long sum.  Per 64-deep k-block the six products of both operands' planes are
 // accumulated in TMEM, smallest first, and the epilogue warps add every k-block's result to fp32 registers with ordinary
 // rounded additions.  Relative error (2-norm, against 64 bits) of a 256 x 256 result of normal data, FMA chain / this:
-//   k = 128: 2.0e-7 / 0.8e-7    512: 4.1e-7 / 1.0e-7    2048: 8.1e-7 / 1.3e-7    8192: 1.6e-6 / 2.2e-7
-// (positive data, the worst for truncation: 1.7 / 0.9, 3.5 / 1.0, 7.0 / 1.2, 14 / 2.0 e-7; with 128-deep blocks the bias
+//   k = 96: 1.8e-7 / 0.8e-7    128: 2.0e-7 / 0.8e-7    512: 4.1e-7 / 1.0e-7    2048: 8.1e-7 / 1.3e-7    8192: 1.6e-6 / 2.2e-7
+// (positive data, the worst for truncation: 1.4 / 0.8, 1.7 / 0.9, 3.5 / 1.0, 7.0 / 1.2, 14 / 2.0 e-7; with 128-deep blocks the bias
 // doubles and reaches the FMA chain's error at k = 128, over the whole k it exceeds it).
 // Not every operand has such planes.  A value that is not finite, or that a bf16 cannot hold, has none; one below 2^-109 has a
 // third term under bf16's smallest step, 2^-133 (operands of 2^-116: 2.2e-6 where the FMA chain has 2.9e-7, of 2^-124: 5.6e-4);
@@ -531,6 +531,10 @@ size_t esmm_f32_workspace_bytes(int E, int64_t row_cap, int64_t n_out, int64_t k
 
 size_t estmm_f32_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n) {
   if (E <= 0 || row_cap <= 0 || m <= 0 || n <= 0) return 0;
+  // A chain of few FMAs is as exact as its last rounding, planes are not: relative error of an expert's gradient from 1 row
+  // 2.5e-8 as a chain, 4.5e-8 from planes, from 8 rows 5.4 / 4.7 (positive data 4.7 / 4.8), from 16 rows 7.4 / 4.8 (6.3 / 4.9).
+  // Of the capacity up to 127 rows per expert are padding, the rest is the real rows.
+  if (row_cap - 127 * (int64_t)E < 16 * (int64_t)E) return 0;
   const int64_t tiles = (int64_t)E * ceil_div(m, 2 * BLOCK_M) * ceil_div(n, BLOCK_N);
   const double rows = (double)row_cap;
   if (!pays(tiles, ceil_div(row_cap / BLOCK_K, E), rows * (double)(m + n), 0.0, m * E, n, rows / E)) return 0;

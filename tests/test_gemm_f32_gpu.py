@@ -36,7 +36,7 @@ def _rel(got, want):
 
 @pytest.mark.parametrize("kind", ["normal", "positive", "wide"])
 @pytest.mark.parametrize("T,K,N,nk", [(12000, 256, 512, True), (12000, 250, 1028, False), (9000, 321, 1000, True), (9000, 324, 1012, False),
-                                      (7000, 1088, 272, False), (6000, 200, 2048, True)])
+                                      (7000, 1088, 272, False), (6000, 200, 2048, True), (32768, 92, 4096, True)])
 def test_esmm_is_closer_than_the_fma_chain(T, K, N, nk, kind):
     L, ops = _mods()
     r, g = _routing(ops, T, 5, 2, K)
@@ -91,6 +91,23 @@ def test_estmm_is_closer_than_the_fma_chain(T, m, n, E, kind):
         assert not torch.equal(got, chain)
     assert _rel(got, exact) <= _rel(chain, exact) and _rel(got, exact) < 6e-7
     assert (got[1] == 0).all() or E <= 2
+
+
+@pytest.mark.parametrize("kind", ["normal", "positive"])
+@pytest.mark.parametrize("T,E", [(1016, 64), (400, 24)])
+def test_estmm_of_few_rows_per_expert(T, E, kind):
+    """From 16 rows per expert on planes are closer than a chain of so few FMAs; below, the chain computes the call."""
+    L, ops = _mods()
+    g = torch.Generator(device="cuda").manual_seed(E)
+    ids = (torch.arange(T, device="cuda") % E).to(torch.int32).view(-1, 1)
+    r = ops.route(ids, E)
+    assert L.lib().hexa_estmm_workspace_bytes(E, r.row_capacity, 2048, 1024, L.F32) > 0
+    assert L.lib().hexa_estmm_workspace_bytes(E, L.lib().hexa_route_row_capacity(8 * E, 1, E, 128), 2048, 1024, L.F32) == 0
+    p, q = ops.gather_rows(_data((T, 2048), g, kind), r), ops.gather_rows(_data((T, 1024), g, kind), r)
+    po = r.pad_offsets.tolist()
+    exact = torch.stack([p[po[e]:po[e + 1]].double().t() @ q[po[e]:po[e + 1]].double() for e in range(E)])
+    got, chain = ops.estmm(p, q, r), ops.estmm(p, q, r, engine=L.ENGINE_SIMT)
+    assert not torch.equal(got, chain) and _rel(got, exact) <= _rel(chain, exact)
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan"), 3.4e38])
