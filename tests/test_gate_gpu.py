@@ -282,3 +282,39 @@ def test_direct_gate_projection(T, d, E, dtype):
     assert ((dw2 - dw).double().abs() <= DY.abs().t() @ X.abs() * (max(T, 8) * 2.0 ** -23) + 1e-30).all()
     only = torch.autograd.grad(_DirectLinear.apply(x.detach(), w), w, dy)[0]
     assert torch.equal(only, dw)
+
+
+def test_direct_gate_projection_leaves_the_linear_to_who_watches_it():
+    """Backward hooks on the gate's linear fire whatever the batch size, torch.func and forward-mode AD pass through it, and
+    rows without a pitch of their own (expanded tokens) are taken."""
+    from hexa_moe_b200.impls import gating
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(64, 128, generator=g, device="cuda")
+    for dtype in (torch.float32, torch.float16):
+        gate = gating.LinearTopKGate(128, 8, fp32_gate=True).cuda()
+        fired = []
+        gate.wg.register_full_backward_hook(lambda *a: fired.append("post"))
+        gate.wg.register_full_backward_pre_hook(lambda *a: fired.append("pre"))
+        gate(x.to(dtype).clone().requires_grad_(True)).sum().backward()
+        assert sorted(fired) == ["post", "pre"]
+    gate = gating.LinearTopKGate(128, 8, fp32_gate=True).cuda()
+    w = gate.wg.weight.detach()
+    want = x @ w.t()
+    # sums of 128 fp32 products of O(1) and O(0.1): within 1e-5 of each other in any order
+    near = lambda a, b: torch.allclose(a, b, rtol=1e-5, atol=1e-5)
+    assert near(torch.func.vmap(gate)(x.view(4, 16, 128)).view(64, 8), want)
+    y, dy = torch.func.jvp(gate, (x,), (x,))
+    assert near(y, want) and near(dy, want)
+    row = x[:1].expand(64, 128)
+    assert not gating._direct_linear_applies(gate.wg, row)
+    assert near(gate(row), want[:1].expand(64, 8))
+    # batched gradients and saved tensors that come back with another layout
+    xi = x.clone().requires_grad_(True)
+    assert gating._direct_linear_applies(gate.wg, xi)
+    eye = torch.eye(8, device="cuda")[:, None].expand(8, 64, 8)
+    (dx,) = torch.autograd.grad(gate(xi), xi, eye, is_grads_batched=True)
+    assert near(dx, w[:, None].expand(8, 64, 128))
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.t().contiguous().t()):
+        y = gate(xi)
+    (dx,) = torch.autograd.grad(y.sum(), xi)
+    assert near(dx, w.sum(0).expand(64, 128))

@@ -308,3 +308,59 @@ def test_weight_gradient_chunks_keep_accumulator_chains_short(E, rows, m, n, chu
         pytest.skip("chunk counts are stated for 148 SMs")
     got = L.lib().hexa_estmm_workspace_bytes(E, rows, m, n, L.BF16)
     assert got == (chunks * E * m * n * 4 if chunks > 1 else 0)
+
+
+def test_direct_gate_projection_steps_aside_for_whoever_watches_the_linear():
+    """Hooks of every kind, a replaced forward, a subclass, and whatever follows operations one by one."""
+    from hexa_moe_b200.impls import gating
+    M = torch.nn.modules.module
+    fresh = lambda: torch.nn.Linear(8, 2, bias=False)
+    assert gating._plain_linear(fresh())
+    for register in ("register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook",
+                     "register_full_backward_pre_hook"):
+        lin = fresh()
+        handle = getattr(lin, register)(lambda *a: None)
+        assert not gating._plain_linear(lin), register
+        handle.remove()
+        assert gating._plain_linear(lin)
+    for register in ("register_module_forward_hook", "register_module_forward_pre_hook", "register_module_full_backward_hook",
+                     "register_module_full_backward_pre_hook"):
+        handle = getattr(M, register)(lambda *a: None)
+        try:
+            assert not gating._plain_linear(fresh()), register
+        finally:
+            handle.remove()
+    lin = fresh()
+    lin.forward = lambda x: x
+    assert not gating._plain_linear(lin)
+    assert not gating._plain_linear(torch.nn.utils.parametrizations.weight_norm(fresh()))
+    assert not gating._plain_linear(torch.nn.Linear(8, 2))
+
+    seen = []
+    look = lambda t: (seen.append(gating.transforming()), t.sum())[1]
+    assert not gating.transforming()
+    torch.func.grad(look)(torch.ones(3))
+    torch.func.vmap(look)(torch.ones(2, 3))
+    torch.func.jvp(look, (torch.ones(3),), (torch.ones(3),))
+    with torch.autograd.forward_ad.dual_level():
+        look(torch.ones(3))
+    torch.jit.trace(look, torch.ones(3), check_trace=False)
+    from torch.utils.flop_counter import FlopCounterMode
+    with FlopCounterMode(display=False):
+        look(torch.ones(3))
+    assert seen and all(seen) and not gating.transforming()
+
+    class Twice(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, t):
+            return t * 2
+
+        @staticmethod
+        def backward(ctx, grad):
+            seen.append(gating.transforming(grad))
+            return grad * 2
+    t = torch.ones(3, requires_grad=True)
+    torch.autograd.grad(Twice.apply(t), t, torch.eye(3), is_grads_batched=True)
+    assert seen[-1]
+    torch.autograd.grad(Twice.apply(t), t, torch.ones(3))
+    assert not seen[-1]
