@@ -498,14 +498,19 @@ _DENSE_ROUTING = {}
 
 def dense_routing(num_tokens: int, device: torch.device) -> Routing:
     """Routing of `num_tokens` rows to a single expert: sorted row i is token i, the tail up to the next multiple
-    of 128 is padding.  Built once per (size, device) by the routing kernel itself and kept."""
-    key = (int(num_tokens), device.index if device.index is not None else torch.cuda.current_device())
+    of 128 is padding.  Built by the routing kernel itself and kept per size, device and stream: the tables are then
+    written, read and, once dropped, reused in the order of that one stream.  Under graph capture they are built in the
+    graph, which must not depend on tables that may be dropped, nor leave its own behind."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    build = lambda: route(torch.zeros(num_tokens, 1, dtype=torch.int32, device=device), 1, L.ROW_TILE)
+    if torch.cuda.is_current_stream_capturing():
+        return build()
+    key = (int(num_tokens), index, torch._C._cuda_getCurrentRawStream(index))
     r = _DENSE_ROUTING.get(key)
     if r is None:
         if len(_DENSE_ROUTING) >= 64:
             _DENSE_ROUTING.clear()
-        r = route(torch.zeros(num_tokens, 1, dtype=torch.int32, device=device), 1, L.ROW_TILE)
-        _DENSE_ROUTING[key] = r
+        r = _DENSE_ROUTING[key] = build()
     return r
 
 

@@ -292,3 +292,32 @@ def test_dense_depth_widths_on_the_kernels(dim, act, on_kernels):
     if act != "relu":
         for a, b in zip(got, want):
             assert float((a.float() - b.float()).norm()) <= 1.2e-2 * float(b.float().norm())
+
+
+def test_dense_routing_belongs_to_its_stream():
+    """Tables built on one stream are not handed to another, and a captured graph has tables of its own."""
+    from hexa_moe_b200 import _lib as L, ops
+    dev = torch.device("cuda", torch.cuda.current_device())
+    here = ops.dense_routing(300, dev)
+    assert ops.dense_routing(300, dev) is here
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        there = ops.dense_routing(300, dev)
+        assert there is not here and ops.dense_routing(300, dev) is there
+    torch.cuda.synchronize()
+    assert torch.equal(there.row_token[:300], here.row_token[:300]) and torch.equal(there.pad_offsets, here.pad_offsets)
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, w1, w2 = (torch.randn(*n, generator=g, device="cuda").bfloat16() for n in ((301, 64), (256, 64), (256, 64)))
+    call = lambda: ops.dense_forward(x, w1, w2, None, None, L.ACT_GELU, need_state=False)[0]
+    want = call().clone()
+    before = len(ops._DENSE_ROUTING)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = call()
+    assert len(ops._DENSE_ROUTING) == before
+    ops._DENSE_ROUTING.clear()
+    junk = [torch.full((4096,), 7, dtype=torch.int32, device="cuda") for _ in range(64)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and len(junk) == 64
