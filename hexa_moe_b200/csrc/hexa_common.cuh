@@ -166,10 +166,11 @@ __device__ __forceinline__ float tanh_fast(float x) {
 template <int ACT> __device__ __forceinline__ float act_fast(float x) {
   if (ACT == HEXA_ACT_RELU) return fmaxf(x, 0.f);
   if (ACT == HEXA_ACT_GELU) {
-    // x Phi(x) with Phi = 1 - u for x >= 0 and u for x < 0: both cases are max(x, 0) - |x u|, no compare or select
+    // x Phi(x) with Phi = 1 - u for x >= 0 and u for x < 0: both cases are max(x, 0) - |x u|, no compare or select.  u is zero
+    // long before the bound on x, which is there for +inf (inf * 0 would be NaN; -inf gives NaN, as in x Phi(x))
     float u, e;
     gelu_parts(x, u, e);
-    return fmaxf(x, 0.f) - fabsf(x * u);
+    return fmaxf(x, 0.f) - fabsf(fminf(x, 1e4f) * u);
   }
   if (ACT == HEXA_ACT_GELU_TANH) return 0.5f * x * (1.f + tanh_fast(0.7978845608028654f * fmaf(0.044715f * x * x, x, x)));
   if (ACT == HEXA_ACT_SILU) return x * rcp_fast(1.f + __expf(-x));

@@ -32,6 +32,7 @@ import torch.distributed as dist
 from torch import Tensor
 
 from . import losses
+from .gating import transforming
 
 
 # ------------------------------------------------------------------------------------------------
@@ -240,14 +241,25 @@ def _dense_on_kernels(cfg, x: Tensor) -> bool:
     Tokens at least 64 wide: forward + backward at widths 64 to 248 and 16 to 65000 tokens 295-440 us against 430-1106 with
     PyTorch operations.  A ReLU takes the kernels from 256 on: the two ways round a pre-activation differently (once from
     the fp32 sum here, before and after the bias there), which moves a derivative that jumps at zero by more than the
-    rounding itself.  HEXA_DENSE_MIN_DIM sets the width for all."""
+    rounding itself.  HEXA_DENSE_MIN_DIM sets the width for all.  Below 256 the layer also keeps what it allowed as PyTorch
+    operations: more tokens than the kernels take, torch.func and tracing, any layout (see MLP_Implement for the backward)."""
     if os.environ.get("HEXA_DENSE_KERNELS", "1") == "0":        # A/B switch: keep the dense FFN on PyTorch ops
         return False
     from .. import _lib
     least = os.environ.get("HEXA_DENSE_MIN_DIM") or (256 if getattr(cfg, "act_id", -1) == _lib.ACT_RELU else 64)
     return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and getattr(cfg, "act_id", -1) >= 0
             and getattr(cfg, "backend", None) is not None and hasattr(cfg.backend, "dense_forward")
-            and x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.shape[1] >= int(least))
+            and x.shape[0] > 0 and x.shape[1] % 8 == 0 and x.shape[1] >= int(least)
+            and (x.shape[1] >= _DENSE_WIDE or (x.shape[0] <= _DENSE_MAX_TOKENS and not transforming())))
+
+
+_DENSE_WIDE = 256
+_DENSE_MAX_TOKENS = 65535 * 128      # the column sums launch a row of blocks per 128 tokens
+
+
+def _unit_rows(w: Tensor) -> Tensor:
+    """A matrix with unit inner stride and rows that do not overlap, as the GEMMs read it."""
+    return w if w.stride(1) == 1 and w.stride(0) >= w.shape[1] else w.contiguous()
 
 
 class MLP_Implement(torch.autograd.Function):
@@ -266,11 +278,17 @@ class MLP_Implement(torch.autograd.Function):
         ctx.fused = _dense_on_kernels(config, tokens_input) and fc1_w.shape[0] % 8 == 0 and fc2_w.shape[1] % 8 == 0
         if ctx.fused:
             x = tokens_input.contiguous()
-            w1, w2 = _cast(fc1_w.detach(), dtype), _cast(fc2_w.detach(), dtype)
+            w1, w2 = _unit_rows(_cast(fc1_w.detach(), dtype)), _unit_rows(_cast(fc2_w.detach(), dtype))
             y, st = config.backend.dense_forward(x, w1, w2, None if fc1_bias is None else fc1_bias.detach(),
                                                  None if fc2_bias is None else fc2_bias.detach(), config.act_id,
                                                  need_state=any(ctx.needs_input_grad))
-            ctx.state, ctx.w = st, (w1, w2)
+            ctx.kept = None
+            if x.shape[1] >= _DENSE_WIDE:
+                ctx.kept = (st, w1, w2)
+            elif st is not None:      # autograd keeps the tensors: several backward passes, checks for changes in place, hooks
+                ctx.rebuild = type(st), st.routing
+                ctx.casts = [None if c.data_ptr() == w.data_ptr() else c for c, w in ((w1, fc1_w), (w2, fc2_w))]
+                ctx.save_for_backward(tokens_input, st.y1, fc1_w, fc2_w, st.xs, st.h)
             ctx.param_dtypes = (fc1_w.dtype, fc2_w.dtype, None if fc1_bias is None else fc1_bias.dtype,
                                 None if fc2_bias is None else fc2_bias.dtype)
             return y
@@ -286,9 +304,20 @@ class MLP_Implement(torch.autograd.Function):
     @staticmethod
     def backward(ctx: Any, dy: Tensor):
         cfg = ctx.config
-        if ctx.fused:
-            (w1, w2), st = ctx.w, ctx.state
-            ctx.state = ctx.w = None
+        st = None
+        if ctx.fused and ctx.kept is not None:
+            st, w1, w2 = ctx.kept
+            ctx.kept = None
+        else:
+            saved = ctx.saved_tensors
+            if not saved:
+                raise RuntimeError("a dense layer of this width keeps what its backward pass needs for one pass")
+            x, hid, fc1_w, fc2_w, *rows = saved
+            if rows and not torch.is_grad_enabled() and not transforming(dy):
+                state, routing = ctx.rebuild
+                st = state(routing, rows[0], hid, rows[1])
+                w1, w2 = (_unit_rows(w.detach()) if c is None else c for c, w in zip(ctx.casts, (fc1_w, fc2_w)))
+        if st is not None:
             dx, dw1, dw2, db1, db2 = cfg.backend.dense_backward(st, dy.contiguous(), w1, w2, cfg.act_id,
                                                                 has_b1=ctx.has_b1, has_b2=ctx.has_b2,
                                                                 bias_grad_dtype=_common_dtype(*ctx.param_dtypes[2:]))
@@ -296,8 +325,8 @@ class MLP_Implement(torch.autograd.Function):
             dw1, dw2 = dw1.to(pd[0]), dw2.to(pd[1])
             db1 = None if db1 is None else db1.to(pd[2])
             db2 = None if db2 is None else db2.to(pd[3])
-        else:
-            x, hid, fc1_w, fc2_w = ctx.saved_tensors
+        else:      # after a forward on the kernels: create_graph or a batch of gradients, which can follow these operations
+            hid = hid[:x.shape[0]]
             with torch.enable_grad():
                 hh = hid.detach().requires_grad_(True)
                 act = cfg.activation_fn(hh)

@@ -515,8 +515,9 @@ def dense_routing(num_tokens: int, device: torch.device) -> Routing:
 
 
 def _dense_rows(t: torch.Tensor, r: Routing) -> torch.Tensor:
-    """t [T, c] as the [row_capacity, c] operand of the grouped GEMMs: t itself when T is a multiple of 128."""
-    if r.row_capacity == t.shape[0] and t.is_contiguous():
+    """t [T, c] as the [row_capacity, c] operand of the grouped GEMMs: t itself when T is a multiple of 128 and t lies on
+    a 16-byte boundary."""
+    if r.row_capacity == t.shape[0] and t.is_contiguous() and t.data_ptr() % 16 == 0:
         return t
     return gather_rows(t.contiguous(), r)
 
@@ -542,7 +543,7 @@ def dense_backward(st: LayerState, dy, w1, w2, act_id: int, has_b1=True, has_b2=
     sums = _sums_dtype(bias_grad_dtype, dy)
     r = st.routing
     T = r.num_tokens
-    if has_b2 and dy.shape[0] != r.row_capacity:
+    if has_b2 and (dy.shape[0] != r.row_capacity or dy.data_ptr() % 16):
         dys, db2 = gather_rows_ess(dy.contiguous(), r, sums)
     else:
         dys = _dense_rows(dy, r)

@@ -321,3 +321,78 @@ def test_dense_routing_belongs_to_its_stream():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want) and len(junk) == 64
+
+
+@pytest.mark.parametrize("T,dim", [(256, 64), (333, 72)])
+def test_narrow_dense_depths_keep_what_plain_operations_allow(T, dim):
+    """Widths below 256 ran as PyTorch operations before they ran on the kernels: two passes over a kept graph, the check for
+    changes in place, saved-tensor hooks, second derivatives, batched gradients, and tensors of any layout."""
+    import os
+    import torch.nn.functional as F
+    from hexa_moe import moe as hmoe
+    from hexa_moe_b200 import ops
+    torch.manual_seed(dim)
+    m = hmoe.MoE_Cascaded(gate_type={'type': 'top', 'k': 1}, model_dim_list=[dim], moe_idx_list=[], mlp_ratio=4,
+                          num_global_experts=1, total_depth=1, data_centric=True, activation_fn=lambda t: F.gelu(t))
+    with torch.no_grad():
+        for p in m.parameters():
+            p.normal_(0, 0.1)
+    m = m.to(torch.bfloat16).cuda()
+    params = list(m.parameters())
+    flat = torch.randn(2 * T * dim + 2, device="cuda").bfloat16()
+    x = flat[1: T * dim + 1].view(T, dim).requires_grad_(True)            # rows that start between 16-byte boundaries
+    dy = flat[T * dim + 1: 2 * T * dim + 1].view(T, dim)
+    grads = lambda y, d=dy, **kw: torch.autograd.grad(y, [x] + params, d, **kw)
+    near = lambda a, b: float((a.float() - b.float()).norm()) <= 1.2e-2 * float(b.float().norm())
+
+    def plain(f):
+        os.environ["HEXA_DENSE_KERNELS"] = "0"
+        try:
+            return f()
+        finally:
+            del os.environ["HEXA_DENSE_KERNELS"]
+
+    before = ops.LAUNCHES
+    y = m(0, x)[0]
+    first = grads(y, retain_graph=True)
+    assert ops.LAUNCHES - before >= 8                                     # both directions on the kernels
+    for a, b in zip(first, grads(y)):
+        assert torch.equal(a, b)
+    want = plain(lambda: grads(m(0, x)[0]))
+    assert all(near(a, b) for a, b in zip(first, want))
+
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(1), t.cpu())[1], lambda t: t.cuda()):
+        y = m(0, x)[0]
+    assert packed and all(torch.equal(a, b) for a, b in zip(first, grads(y)))
+
+    second = lambda: torch.autograd.grad(grads(m(0, x)[0], create_graph=True)[0].float().square().sum(), params[0])[0]
+    assert near(second(), plain(second))
+    both = torch.stack([dy, -dy])
+    batched = grads(m(0, x)[0], both, is_grads_batched=True)
+    assert all(near(a[0], b) and near(a[1], -b) for a, b in zip(batched, want))
+
+    w = params[0].data.clone()
+    params[0].data = w.t().contiguous().t()                               # columns in memory
+    assert all(torch.equal(a, b) for a, b in zip(first, grads(m(0, x)[0])))
+    params[0].data = w
+
+    y = m(0, x)[0]
+    with torch.no_grad():
+        params[0].add_(0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        grads(y)
+
+
+def test_gelu_of_infinity_is_infinity():
+    """As F.gelu has it, in the 16-bit epilogue too; -inf and NaN stay NaN."""
+    from hexa_moe_b200 import _lib as L, ops
+    r = ops.route(torch.zeros(128, 1, dtype=torch.int32, device="cuda"), 1)
+    for dtype in (torch.bfloat16, torch.float16):
+        x, w = torch.zeros(128, 64, device="cuda", dtype=dtype), torch.zeros(1, 128, 64, device="cuda", dtype=dtype)
+        v = torch.tensor([float("inf"), float("-inf"), float("nan"), 3.0, -3.0, 60000.0], device="cuda").to(dtype)
+        x[:6, 0], w[0, :, 0] = v, 1.0
+        want = torch.nn.functional.gelu(v)
+        for n in (128, 8):
+            got = ops.esmm(x, w[:, :n], L.B_NK, r, None, L.EPI_ACT, L.ACT_GELU, engine=L.ENGINE_TCGEN05)[:6]
+            assert torch.allclose(got, want[:, None].expand(6, n), rtol=1e-2, atol=1e-2, equal_nan=True)
