@@ -75,10 +75,13 @@ void* stream_of(const Tensor& t) {
 }
 
 // Kernels take raw pointers: an operand on another device, or on the host, has to be refused here.
-void on_device_of(const Tensor& anchor, std::initializer_list<const Tensor*> others) {
-  for (const Tensor* t : others)
-    if (t->device() != anchor.device()) fail("operands are on different devices: " + anchor.device().str() + " and " + t->device().str());
+void same_device(const Tensor& anchor, const Tensor& t) {
+  if (t.device() != anchor.device()) fail("operands are on different devices: " + anchor.device().str() + " and " + t.device().str());
 }
+void same_device(const Tensor& anchor, const OptTensor& t) {
+  if (t) same_device(anchor, *t);
+}
+template <typename... Ts> void on_device_of(const Tensor& anchor, const Ts&... others) { (same_device(anchor, others), ...); }
 
 int dt(const Tensor& t) {
   switch (t.scalar_type()) {
@@ -138,7 +141,7 @@ py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
 
 Tensor ids_from_lists(int64_t num_toks, const Tensor& tok_ids_, const Tensor& exp_ids_, int chunk) {
   void* s = stream_of(tok_ids_);
-  on_device_of(tok_ids_, {&exp_ids_});
+  on_device_of(tok_ids_, exp_ids_);
   const bool narrow = tok_ids_.scalar_type() == at::kInt;      // anything else is read as 64 bits: an id must not wrap
   const Tensor tok_ids = tok_ids_.to(narrow ? at::kInt : at::kLong).contiguous(), exp_ids = exp_ids_.to(at::kInt).contiguous();
   if (chunk < 1 || tok_ids.numel() > (int64_t)chunk * exp_ids.numel()) fail("ids_from_lists: more token ids than the expert ids cover");
@@ -154,6 +157,7 @@ Tensor ids_from_lists(int64_t num_toks, const Tensor& tok_ids_, const Tensor& ex
 Tensor gather_rows(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
+  on_device_of(src, row_token, pad_offsets, out_);
   Tensor out = out_ ? *out_ : sorted_buffer(cap, cols, src.scalar_type(), src);
   const int type = dt(src);
   const int64_t lds = ld(src), ldo = ld(out);
@@ -164,6 +168,7 @@ Tensor gather_rows(const Tensor& src, const Tensor& row_token, const Tensor& pad
 std::tuple<Tensor, Tensor> gather_rows_ess(const Tensor& src, const Tensor& row_token, const Tensor& pad_offsets, int E, int64_t cap, at::ScalarType sums_type) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
+  on_device_of(src, row_token, pad_offsets);
   Tensor out = sorted_buffer(cap, cols, src.scalar_type(), src), sums = empty({E, cols}, sums_type, src);
   if (sums_type != at::kFloat && !same16(sums, src)) fail("gather_rows_ess: sums are float32 or of the data's 16-bit type");
   Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
@@ -179,6 +184,7 @@ std::tuple<Tensor, Tensor> gather_rows_ess(const Tensor& src, const Tensor& row_
 Tensor combine_rows(const Tensor& src, const Tensor& token_row, int64_t T, int top_k, const OptTensor& out_) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
+  on_device_of(src, token_row, out_);
   Tensor out = out_ ? *out_ : empty({T, cols}, src.scalar_type(), src);
   const int type = dt(src);
   const int64_t lds = ld(src), ldo = ld(out);
@@ -189,6 +195,7 @@ Tensor combine_rows(const Tensor& src, const Tensor& token_row, int64_t T, int t
 Tensor ess(const Tensor& src, const Tensor& pad_offsets, int E, int64_t cap, const OptTensor& out_, at::ScalarType out_type) {
   const int64_t cols = src.size(1);
   void* s = stream_of(src);
+  on_device_of(src, pad_offsets, out_);
   Tensor out = out_ ? *out_ : empty({E, cols}, out_type, src);
   if (out.scalar_type() != at::kFloat && !same16(out, src)) fail("ess: the result is float32 or of the data's 16-bit type");
   Tensor ws = scratch(api.hexa_ess_workspace_bytes(cap, cols), src);
@@ -210,6 +217,7 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
                sums->stride(1) != 1))
     fail("esmm: sums must be [E, n_out], float32 or of the data's 16-bit type, and needs the full expert range");
   void* s = stream_of(a);
+  on_device_of(a, b, tile_expert, pad_offsets, row_token, pair_block, bias, aux, out_, sums);
   const int type = dt(a) | (bias && bias->scalar_type() != at::kFloat ? HEXA_BIAS_16 : 0);
   Tensor out = out_ ? *out_ : sorted_buffer(cap, n_out, a.scalar_type(), a);
   const int64_t lda = ld(a), ldo = ld(out), ldbias = bias ? ld(*bias) : 0, ldaux = aux ? ld(*aux) : 0;
@@ -267,6 +275,7 @@ Tensor estmm(const Tensor& p, const Tensor& q, const Tensor& pad_offsets, int E,
   }
   if (out.stride(-1) != 1) fail("estmm: out must have unit inner stride");
   void* s = stream_of(p);
+  on_device_of(p, q, pad_offsets, out);
   const int in_type = dt(p), o_type = dt(out);
   const int64_t ldp = ld(p), ldq = ld(q);
   const size_t bytes = engine != HEXA_ENGINE_SIMT ? api.hexa_estmm_workspace_bytes(E, cap, m, n, in_type) : 0;
@@ -298,6 +307,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> gate_topk(const Tensor& logits, int t
 Tensor gate_loss_grad(const Tensor& logits, const Tensor& first_count, const Tensor& dloss_) {
   const int64_t T = logits.size(0), E = logits.size(1);
   void* s = stream_of(logits);
+  on_device_of(logits, first_count, dloss_);
   Tensor out = empty({T, E}, at::kFloat, logits);
   const Tensor dloss = dloss_.detach().to(at::kFloat).reshape({1}).contiguous();
   const int64_t ldl = ld(logits);
@@ -332,6 +342,7 @@ Tensor gate_project(const Tensor& x, const Tensor& w) {
   if (w.scalar_type() != at::kFloat || w.dim() != 2 || !w.is_contiguous() || x.dim() != 2 || x.size(1) != w.size(1))
     fail("gate_project: w must be contiguous float32 [E, d] and x [T, d]");
   void* s = stream_of(x);
+  on_device_of(x, w);
   const int type = dt(x);
   const int64_t ldx = ld(x), T = x.size(0), E = w.size(0);
   Tensor out = empty({T, E}, at::kFloat, x);
@@ -345,6 +356,7 @@ std::tuple<OptTensor, OptTensor> gate_project_grad(const Tensor& g, const Tensor
   if (g.scalar_type() != at::kFloat || g.dim() != 2 || !g.is_contiguous() || g.size(0) != x.size(0) || g.size(1) != w.size(0) || !w.is_contiguous())
     fail("gate_project_grad: g must be contiguous float32 [T, E]");
   void* s = stream_of(g);
+  on_device_of(g, x, w);
   const int type = dt(x);
   const int64_t ldx = ld(x);
   OptTensor dx, dw;

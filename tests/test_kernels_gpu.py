@@ -577,3 +577,25 @@ def test_16_bit_bias_and_sums(ops, dtype, K, N, engine):
     f = torch.zeros(r.row_capacity, 8, device="cuda")
     with pytest.raises(Lb.HexaError):
         ops.ess(f, r, out_dtype=torch.bfloat16)                     # only the data's own type
+
+
+# Kernels take raw pointers: an operand left on the host is refused by the wrappers, whichever it is.
+def test_operands_on_another_device_are_refused(ops):
+    Lb = L()
+    r = ops.route(make_ids(200, 1, 2, 3).cuda(), 2)
+    x, w, b = torch.randn(200, 64), torch.randn(2, 32, 64), torch.randn(2, 32)
+    xs = ops.gather_rows(x.cuda(), r)
+    good = (xs, w.cuda(), Lb.B_NK, r, b.cuda())
+    ops.esmm(*good)
+    out, cpu_r = torch.empty(r.row_capacity, 32), type(r)(**{**vars(r), "pad_offsets": r.pad_offsets.cpu()})
+    calls = [lambda: ops.esmm(xs, w, Lb.B_NK, r), lambda: ops.esmm(xs, w.cuda(), Lb.B_NK, r, b), lambda: ops.esmm(*good, out=out),
+             lambda: ops.esmm(*good, epilogue=Lb.EPI_ACT, act=Lb.ACT_GELU, aux=out), lambda: ops.esmm(*good, sums=torch.empty(2, 32)),
+             lambda: ops.esmm(xs, w.cuda(), Lb.B_NK, cpu_r), lambda: ops.estmm(xs, out, r), lambda: ops.ess(xs, cpu_r),
+             lambda: ops.estmm(xs, xs, r, out=torch.empty(2, 64, 64)), lambda: ops.gather_rows(x.cuda(), cpu_r),
+             lambda: ops.gather_rows_ess(x.cuda(), cpu_r), lambda: ops.combine_rows(xs, r, out=torch.empty(200, 64)),
+             lambda: ops.gate_project(x.cuda(), w[0]), lambda: ops.gate_project_grad(b.cuda(), x.cuda()[:2], w[0], True, True),
+             lambda: ops.gate_loss_grad(x.cuda(), torch.zeros(64, dtype=torch.int32), torch.ones((), device="cuda"))]
+    for i, call in enumerate(calls):
+        with pytest.raises(Lb.HexaError, match="different devices"):
+            call()
+            pytest.fail(f"call {i} went through")
