@@ -109,6 +109,14 @@ Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
   return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
 }
 Tensor scratch(size_t bytes, const Tensor& like) { return empty({(int64_t)(bytes < 4 ? 4 : bytes)}, at::kByte, like); }
+// Scratch that an operator can do without: none when the device has not that much left.
+OptTensor scratch_if_free(size_t bytes, const Tensor& like) {
+  try {
+    return scratch(bytes, like);
+  } catch (const c10::OutOfMemoryError&) {
+    return std::nullopt;
+  }
+}
 
 // [rows, cols] whose row pitch is a multiple of 8 elements (16 bytes of 16-bit data), as the TMA-fed GEMMs need
 Tensor sorted_buffer(int64_t rows, int64_t cols, at::ScalarType type, const Tensor& like) {
@@ -225,16 +233,14 @@ Tensor esmm(const Tensor& a, const Tensor& b, int b_layout, const Tensor& tile_e
   const bool relu = epilogue == HEXA_EPI_ACT && act == HEXA_ACT_RELU;      // stays with the FMA chain, see hexa_esmm_f32
   const size_t planes = type == HEXA_F32 && engine == HEXA_ENGINE_AUTO && pair_block && e0 == 0 && e1 == E && !relu
                             ? api.hexa_esmm_f32_workspace_bytes(E, cap, n_out, k) : 0;
-  if (planes) {
-    {
-      Tensor ws = scratch(planes, a);
-      auto f = [](void* v) { return static_cast<float*>(v); };
-      call("hexa_esmm_f32", [&] {
-        return api.hexa_esmm_f32(f(ptr(a)), lda, f(ptr(b)), b_layout, b.stride(1), b.stride(0), bp, ldbias, f(ptr(aux)), ldaux, f(ptr(out)),
-                                 ldo, i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, epilogue,
-                                 act, ptr(ws), (size_t)ws.numel(), s);
-      });
-    }
+  if (OptTensor ws = planes ? scratch_if_free(planes, a) : std::nullopt) {
+    auto f = [](void* v) { return static_cast<float*>(v); };
+    call("hexa_esmm_f32", [&] {
+      return api.hexa_esmm_f32(f(ptr(a)), lda, f(ptr(b)), b_layout, b.stride(1), b.stride(0), bp, ldbias, f(ptr(aux)), ldaux, f(ptr(out)),
+                               ldo, i32(tile_expert), i32(pad_offsets), i32(row_token), i32(pair_block), E, cap, n_out, k, epilogue,
+                               act, ptr(ws), (size_t)ws->numel(), s);
+    });
+    ws.reset();
     if (sums) ess(out, pad_offsets, E, cap, sums, at::kFloat);
     return out;
   }
@@ -278,9 +284,11 @@ Tensor estmm(const Tensor& p, const Tensor& q, const Tensor& pad_offsets, int E,
   on_device_of(p, q, pad_offsets, out);
   const int in_type = dt(p), o_type = dt(out);
   const int64_t ldp = ld(p), ldq = ld(q);
-  const size_t bytes = engine != HEXA_ENGINE_SIMT ? api.hexa_estmm_workspace_bytes(E, cap, m, n, in_type) : 0;
+  size_t bytes = engine != HEXA_ENGINE_SIMT ? api.hexa_estmm_workspace_bytes(E, cap, m, n, in_type) : 0;
   OptTensor ws;
-  if (bytes) ws = scratch(bytes, p);
+  if (bytes && in_type == HEXA_F32) ws = scratch_if_free(bytes, p);
+  else if (bytes) ws = scratch(bytes, p);      // the chunks of a 16-bit weight gradient bound its error
+  if (!ws) bytes = 0;
   call("hexa_estmm", [&] {
     return api.hexa_estmm(ptr(p), ldp, ptr(q), ldq, i32(pad_offsets), E, cap, m, n, ptr(out), ldo, estride, m_split, split_stride, in_type,
                           o_type, beta, engine, ptr(ws), bytes, s);

@@ -203,3 +203,29 @@ def test_relu_masks_do_not_depend_on_the_path():
     a = [torch.empty(r.row_capacity, 512, device="cuda") for _ in range(2)]
     y = [ops.esmm(xs, w, L.B_NK, r, None, L.EPI_ACT, L.ACT_RELU, aux=a[i], engine=e)[:n_pad] for i, e in enumerate((L.ENGINE_AUTO, L.ENGINE_SIMT))]
     assert torch.equal(y[0], y[1]) and torch.equal(a[0][:n_pad], a[1][:n_pad])
+
+
+def test_without_room_for_planes_the_chain_computes_the_call():
+    """The scratch is optional: when the allocator cannot give it, the CUDA cores do what they did without any."""
+    L, ops = _mods()
+    T, K, N, E = 60000, 512, 2048, 4
+    r, g = _routing(ops, T, E, 1, 1)
+    xs = ops.gather_rows(torch.randn(T, K, generator=g, device="cuda"), r)
+    w = torch.randn(E, N, K, generator=g, device="cuda")
+    n_pad = int(r.pad_offsets[-1])
+    h, dw = torch.empty(r.row_capacity, N, device="cuda"), torch.empty(E, N, K, device="cuda")
+    need = min(L.lib().hexa_esmm_f32_workspace_bytes(E, r.row_capacity, N, K), L.lib().hexa_estmm_workspace_bytes(E, r.row_capacity, N, K, L.F32))
+    assert need > 128 << 20
+    want = ops.esmm(xs, w, L.B_NK, r, engine=L.ENGINE_SIMT)[:n_pad].clone()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+    try:
+        ops.esmm(xs, w, L.B_NK, r, out=h)
+        ops.estmm(h, xs, r, out=dw)
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(h[:n_pad], want)
+    assert torch.equal(dw, ops.estmm(h, xs, r, engine=L.ENGINE_SIMT))
+    assert not torch.equal(ops.esmm(xs, w, L.B_NK, r)[:n_pad], want)      # with room the planes are taken
