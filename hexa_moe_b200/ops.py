@@ -342,8 +342,10 @@ def _f32(t):
 
 
 def _bias(t, x):
-    """Bias as the epilogue reads it: as it is when it has the 16-bit type of the data, else in fp32."""
-    if t is not None and t.dtype == x.dtype and x.dtype != torch.float32 and t.stride(-1) == 1:
+    """Bias as the epilogue reads it: as it is when it has the 16-bit type of the data and rows of its own (an expanded
+    one has not), else in fp32."""
+    if (t is not None and t.dtype == x.dtype and x.dtype != torch.float32 and t.stride(-1) == 1
+            and (t.dim() < 2 or t.stride(0) >= t.shape[-1])):
         return t.detach()
     return _f32(t)
 

@@ -310,6 +310,19 @@ def test_weight_gradient_chunks_keep_accumulator_chains_short(E, rows, m, n, chu
     assert got == (chunks * E * m * n * 4 if chunks > 1 else 0)
 
 
+def test_biases_without_rows_of_their_own_are_laid_out():
+    """The kernels read [E, n] rows; a bias expanded over the experts, or with columns in memory, becomes one."""
+    from hexa_moe_b200 import ops
+    x, one = torch.zeros(4, 8, dtype=torch.bfloat16), torch.arange(16, dtype=torch.bfloat16)
+    own = one.repeat(3, 1)
+    assert ops._bias(own, x).data_ptr() == own.data_ptr() and ops._bias(one, x).data_ptr() == one.data_ptr()
+    wide = torch.zeros(3, 24, dtype=torch.bfloat16)
+    assert ops._bias(wide[:, 4:20], x).stride() == (24, 1)
+    for odd in (one.expand(3, 16), own.t().contiguous().t()):
+        got = ops._bias(odd, x)
+        assert got.stride() == (16, 1) and torch.equal(got.float(), own.float())
+
+
 def test_direct_gate_projection_steps_aside_for_whoever_watches_the_linear():
     """Hooks of every kind, a replaced forward, a subclass, and whatever follows operations one by one."""
     from hexa_moe_b200.impls import gating
