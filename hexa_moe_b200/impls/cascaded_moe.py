@@ -365,8 +365,9 @@ class MoE_Cascaded(torch.nn.Module):
         x = input.reshape(-1, original_shape[-reserve_dims:].numel())
         if torch.is_autocast_enabled():
             x = x.to(torch.get_autocast_gpu_dtype() if x.is_cuda else torch.get_autocast_cpu_dtype())
-        elif self.total_depth_moe + self.total_depth_mlp:      # the dtype of the module's first parameter
-            x = x.to((self.batched_fc1_w if self.total_depth_moe else self.mlp_fc1_w)[0].dtype)
+        else:      # the module's first parameter, which may be one that a subclass or a caller has added
+            first = next(self.parameters(), None)
+            x = x if first is None else x.to(first.dtype)
 
         if not is_moe:
             y = MLP_Implement.apply(cfg, x, self.mlp_fc1_w[i_mlp], self.mlp_fc2_w[i_mlp], self.mlp_fc1_b[i_mlp],

@@ -310,6 +310,17 @@ def test_weight_gradient_chunks_keep_accumulator_chains_short(E, rows, m, n, chu
     assert got == (chunks * E * m * n * 4 if chunks > 1 else 0)
 
 
+def test_tokens_take_the_type_of_the_modules_first_parameter():
+    """One that was added to the module itself comes before those of its lists."""
+    m = _toy()
+    dense = m.mlp_idx_list[0]
+    x = torch.randn(2, 8, m.input_dim_list_mlp[0])
+    plain = m(dense, x)[0]
+    m.own = torch.nn.Parameter(torch.zeros(1, dtype=torch.bfloat16))
+    rounded = m(dense, x)[0]
+    assert rounded.dtype == torch.float32 and torch.equal(rounded, rounded.bfloat16().float()) and not torch.equal(rounded, plain)
+
+
 def test_biases_without_rows_of_their_own_are_laid_out():
     """The kernels read [E, n] rows; a bias expanded over the experts, or with columns in memory, becomes one."""
     from hexa_moe_b200 import ops
