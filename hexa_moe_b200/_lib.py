@@ -38,6 +38,7 @@ SIGNATURES = {
     "hexa_route_workspace_bytes": (sz, [i64, ci, ci]),
     "hexa_route_pair_capacity": (i64, [i64, ci, ci]),
     "hexa_route_launches": (ci, [i64, ci, ci]),
+    "hexa_launch_count": (C.c_uint64, []),
     "hexa_route": (ci, [vp, i64, ci, i64, i64, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "hexa_ids_from_lists": (ci, [vp, vp, i64, ci, i64, vp, vp]),
     "hexa_ids_from_lists_i64": (ci, [vp, vp, i64, ci, i64, vp, vp]),

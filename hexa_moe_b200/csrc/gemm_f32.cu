@@ -513,6 +513,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
     set_error("launch of gemm_f32_kernel<%d> failed: %s", MODE, cudaGetErrorString(e));
     return HEXA_ERR_CUDA;
   }
+  count_launch();
   return HEXA_OK;
 }
 

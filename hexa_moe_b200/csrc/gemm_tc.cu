@@ -814,6 +814,7 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
     set_error("launch of gemm_tc_kernel<%d,%d,%d,%d> failed: %s", BN, MODE, CTAS, OUT, cudaGetErrorString(e));
     return HEXA_ERR_CUDA;
   }
+  count_launch();
   return HEXA_OK;
 }
 

@@ -17,6 +17,7 @@ int32_t* status_word();   // status word of the current device (may be null), se
 int status_pending();     // code an earlier kernel left in the current device's status word, when the host can read it (else 0)
 uint64_t wait_limit_ns(); // limit of the bounded waits inside kernels, see hexa_set_wait_limit_ns
 int tc_debug_flags();     // HEXA_TC_DEBUG / hexa_set_tc_debug
+void count_launch();      // one more kernel launched, see hexa_launch_count
 
 constexpr int kStatusBadToken = 6;   // status code of hexa_ids_from_lists; the others come from bounded waits
 // The status word may live in device memory or in pinned host memory (where the host can poll it without a copy), so
@@ -67,6 +68,7 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
       ::hexa::set_error("launch of %s failed: %s", name, cudaGetErrorString(e_));    \
       return HEXA_ERR_CUDA;                                                          \
     }                                                                                \
+    ::hexa::count_launch();                                                          \
   } while (0)
 
 // Splits a dtype argument into the data type and its flags; false when a flag comes with a type that is not 16 bits wide

@@ -28,7 +28,7 @@ namespace {
 struct Api {
 #define HEXA_API(X)                                                                                                            \
   X(hexa_last_error_string) X(hexa_pending_device_status) X(hexa_route_row_capacity) X(hexa_route_workspace_bytes)             \
-  X(hexa_route_pair_capacity) X(hexa_route_launches) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
+  X(hexa_route_pair_capacity) X(hexa_route) X(hexa_gather_rows) X(hexa_gather_rows_ess)                 \
   X(hexa_combine_rows) X(hexa_esmm_experts) X(hexa_esmm_f32_workspace_bytes) X(hexa_esmm_f32) X(hexa_esmm_ess) X(hexa_estmm_workspace_bytes) X(hexa_estmm)                       \
   X(hexa_ess_workspace_bytes) X(hexa_ess) X(hexa_gate_workspace_bytes) X(hexa_gate_topk) X(hexa_gate_loss_grad)                \
   X(hexa_gate_split_terms) X(hexa_gate_sum_terms) X(hexa_ids_from_lists) X(hexa_ids_from_lists_i64)                          \
@@ -125,7 +125,7 @@ Tensor sorted_buffer(int64_t rows, int64_t cols, at::ScalarType type, const Tens
   return pitch == cols ? t : t.narrow(1, 0, cols);
 }
 
-// (counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block | None, T, k, row_capacity, launches)
+// (counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block | None, T, k, row_capacity)
 py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
   if (ids.scalar_type() != at::kInt) fail("route: ids must be int32");
   if (ids.dim() != 2) fail("route: ids must be 2-D");
@@ -144,7 +144,7 @@ py::tuple route(const Tensor& ids, int E, int align, bool route_major) {
     return api.hexa_route(i32(ids), T, (int)k, st, sk, E, align, out(counts), out(seg), out(pad), out(row_token), out(token_row),
                           out(tiles), pairs ? out(*pairs) : nullptr, ptr(ws), (size_t)ws.numel(), s);
   });
-  return py::make_tuple(counts, seg, pad, row_token, token_row, tiles, pairs, T, k, cap, api.hexa_route_launches(T, (int)k, E));
+  return py::make_tuple(counts, seg, pad, row_token, token_row, tiles, pairs, T, k, cap);
 }
 
 Tensor ids_from_lists(int64_t num_toks, const Tensor& tok_ids_, const Tensor& exp_ids_, int chunk) {

@@ -451,6 +451,9 @@ int tc_debug_flags() {
   return g_tc_debug;
 }
 
+static uint64_t g_launches = 0;
+void count_launch() { __atomic_fetch_add(&g_launches, 1, __ATOMIC_RELAXED); }
+
 static int g_sm_limit = 0;
 int sm_limit() { return g_sm_limit; }
 
@@ -471,6 +474,7 @@ int sm_count() {
 using namespace hexa;
 
 extern "C" int hexa_version(void) { return 100; }
+extern "C" uint64_t hexa_launch_count(void) { return __atomic_load_n(&hexa::g_launches, __ATOMIC_RELAXED); }
 extern "C" int hexa_set_sm_limit(int n) {
   hexa::g_sm_limit = n > 0 ? n : 0;
   return HEXA_OK;

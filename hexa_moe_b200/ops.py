@@ -18,18 +18,21 @@ from ._lib import check, dt, host, lib, ptr, stream_of
 
 
 # ---- optional per-call instrumentation (used by bench.py; off by default) --------------------------
-# LAUNCHES counts kernels launched through the C ABI.  When PROFILE is a list, every wrapper appends
-# (name, start_event, end_event, algorithmic_work, algorithmic_bytes) with CUDA events recorded on the launching stream.
-LAUNCHES = 0
+# LAUNCHES (read-only) is the number of kernels the library has launched in this process.  When PROFILE is a list, every
+# wrapper appends (name, start_event, end_event, algorithmic_work, algorithmic_bytes) with CUDA events recorded on the
+# launching stream.
 PROFILE = None
-_KERNELS_PER_CALL = dict(route=1, gather=1, combine=1, esmm=1, estmm=1, ess=2, mask=1, gate=1, lists=1)
+
+
+def __getattr__(name):
+    if name == "LAUNCHES":
+        return int(lib().hexa_launch_count())
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def _run(name, work, nbytes, fn, args):
-    """fn(*args), counted and, when PROFILE is on, timed."""
-    global LAUNCHES
+    """fn(*args), timed when PROFILE is on."""
     if PROFILE is None:
-        LAUNCHES += _KERNELS_PER_CALL[name.split(":")[0]]
         return fn(*args)
     with _Timed(name, work, nbytes):
         return fn(*args)
@@ -42,8 +45,6 @@ class _Timed:
         self.name, self.work, self.bytes, self.ev = name, work, nbytes, None
 
     def __enter__(self):
-        global LAUNCHES
-        LAUNCHES += _KERNELS_PER_CALL[self.name.split(":")[0]]
         if PROFILE is not None:
             self.ev = torch.cuda.Event(enable_timing=True)
             self.ev.record()
@@ -76,10 +77,8 @@ class Routing:
 
 def route(ids: torch.Tensor, num_experts: int, align: int = L.ROW_TILE, route_major: bool = False) -> Routing:
     """Segment routed rows by expert.  ids: int32 [T, k] (or [k, T] when route_major)."""
-    global LAUNCHES
-    out = _run("route", 12.0 * ids.numel(), 0.0, host().route, (ids, num_experts, align, route_major))
-    LAUNCHES += out[-1] - 1
-    counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, cap, _ = out
+    counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, cap = _run(
+        "route", 12.0 * ids.numel(), 0.0, host().route, (ids, num_experts, align, route_major))
     return Routing(counts, seg, pad, row_token, token_row, tile_expert, pairs, T, k, num_experts, align, cap)
 
 
@@ -112,10 +111,8 @@ def gather_rows(src: torch.Tensor, r: Routing, out: Optional[torch.Tensor] = Non
 
 def gather_rows_ess(src: torch.Tensor, r: Routing, sums_dtype: torch.dtype = torch.float32):
     """(gather_rows(src), ess of the result) from one pass over the rows."""
-    global LAUNCHES
     if r.align % L.ROW_TILE:
         raise L.HexaError("gather_rows_ess: routing must be aligned to 128 rows")
-    LAUNCHES += 1          # the second pass of ESS over the tile sums
     return _run("gather", 2.0 * r.num_tokens * r.top_k * src.shape[1] * src.element_size(), 0.0, host().gather_rows_ess,
                 (src, r.row_token, r.pad_offsets, r.num_experts, r.row_capacity, sums_dtype))
 
@@ -135,7 +132,6 @@ def esmm(a: torch.Tensor, b: torch.Tensor, b_layout: int, r: Routing, bias: Opti
     b may be a view with arbitrary expert / row strides (unit inner stride).  experts = (first, end): only the rows of
     those experts are computed (the other rows of `out` are left as they are).  bias: [E, n_out], float32 or of a's 16-bit
     type.  sums: an [E, n_out] tensor, float32 or of a's 16-bit type, that receives the per-expert column sums of the output (ESS of `out`) from the same launch."""
-    global LAUNCHES
     if r.align % L.ROW_TILE:
         raise L.HexaError("esmm: routing must be aligned to 128 rows")
     if b.dim() != 3 or b.stride(2) != 1:
@@ -153,8 +149,6 @@ def esmm(a: torch.Tensor, b: torch.Tensor, b_layout: int, r: Routing, bias: Opti
         share = (e1 - e0) / max(r.num_experts, 1)        # work of a group, taken as its share of the experts
         work = 2.0 * rows * n_out * k * share
         nbytes = float(es * (rows * k + r.num_experts * n_out * k + rows * n_out * (1 if epilogue == L.EPI_LINEAR else 2))) * share
-    if sums is not None:
-        LAUNCHES += 1          # the second pass of ESS over the block sums
     return _run("esmm:" + (tag or "epilogue%d" % epilogue), work, nbytes, host().esmm,
                 (a, b, b_layout, r.tile_expert, r.pad_offsets, r.row_token, r.pair_block, r.num_experts, r.row_capacity, bias,
                  epilogue, act, aux, out, engine, n_out, k, e0, e1, sums))
@@ -247,8 +241,6 @@ def gate_project(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
 
 def gate_project_grad(g: torch.Tensor, x: torch.Tensor, w: torch.Tensor, want_dx: bool, want_dw: bool):
     """(dx = g w in x's type, dw = g^T x in float32) of gate_project, None where not wanted."""
-    global LAUNCHES
-    LAUNCHES += int(want_dx) + int(want_dw) - 1
     return _run("gate", 2.0 * x.shape[0] * w.numel() * (int(want_dx) + int(want_dw)), 0.0, host().gate_project_grad,
                 (g, x, w, want_dx, want_dw))
 
@@ -267,11 +259,7 @@ def gate_sum_terms(part: torch.Tensor, rows: int, cols: int, lo_first: bool) -> 
 def gate_topk(logits: torch.Tensor, top_k: int):
     """softmax + top-k + GShard loss of float32 logits [T,E] in one kernel.  Returns (ids int32 [k,T] route-major,
     loss float32 scalar tensor, first_count int32 [E], mass float32 [E])."""
-    global LAUNCHES
-    out = _run("gate", 8.0 * logits.numel(), 0.0, host().gate_topk, (logits, top_k))
-    T, E = logits.shape
-    LAUNCHES += T > (512 if E <= 64 else 256 if E <= 128 else 32)      # beyond one block: a second kernel adds the blocks' rows
-    return out
+    return _run("gate", 8.0 * logits.numel(), 0.0, host().gate_topk, (logits, top_k))
 
 
 def gate_loss_grad(logits: torch.Tensor, first_count: torch.Tensor, dloss: torch.Tensor) -> torch.Tensor:

@@ -92,6 +92,8 @@ const char* hexa_last_error_string(void);
  * NULL disables reporting (waits stay bounded).  Replaces, as the way a device-side failure reaches the host,
  * HandleError's printf + exit(1) (hexa_moe_cuda/hexa_moe/kernels/esmm_half.cu:27-36). */
 int hexa_set_status_word(int32_t* status);
+/* Kernels this library has launched in this process so far (all devices and threads; a captured launch counts once). */
+uint64_t hexa_launch_count(void);
 /* Code currently in the current device's status word when that word is host-readable, else 0.  Never synchronises. */
 int hexa_pending_device_status(void);
 /* Limit of every wait inside the kernels, in nanoseconds of the GPU's global timer (process-wide; default 2 s). */

@@ -599,3 +599,34 @@ def test_operands_on_another_device_are_refused(ops):
         with pytest.raises(Lb.HexaError, match="different devices"):
             call()
             pytest.fail(f"call {i} went through")
+
+
+def test_launches_are_counted_where_they_happen(ops):
+    Lb = L()
+
+    def count(call):
+        before = ops.LAUNCHES
+        call()
+        return ops.LAUNCHES - before
+
+    T, E = 12000, 4
+    ids = make_ids(T, 1, E, 5).cuda()
+    r = ops.route(ids, E)
+    xs, w = ops.gather_rows(torch.randn(T, 256, device="cuda"), r), torch.randn(E, 2048, 256, device="cuda")
+    h = ops.esmm(xs, w, Lb.B_NK, r)
+    y1 = torch.empty_like(h)
+    assert count(lambda: ops.esmm(xs, w, Lb.B_NK, r)) == 3                     # split, GEMM, the CUDA cores' stand-by
+    assert count(lambda: ops.esmm(xs, w, Lb.B_NK, r, None, Lb.EPI_ACT, Lb.ACT_GELU, aux=y1)) == 4
+    assert count(lambda: ops.esmm(xs, w, Lb.B_NK, r, engine=Lb.ENGINE_SIMT)) == 1
+    assert count(lambda: ops.estmm(h, xs, r)) == 3
+    xb, hb, wb = xs.bfloat16(), h.bfloat16(), w.bfloat16()
+    assert count(lambda: ops.esmm(xb, wb, Lb.B_NK, r)) == 1
+    assert count(lambda: ops.estmm(hb, xb, r)) == (2 if Lb.lib().hexa_estmm_workspace_bytes(E, r.row_capacity, 2048, 256, Lb.BF16) else 1)
+    assert count(lambda: ops.estmm(hb[:, :256], xb, r)) == 2                    # chunks and their sum
+    assert count(lambda: ops.esmm(xb, wb, Lb.B_NK, r, sums=torch.empty(E, 2048, device="cuda"))) == 2
+    assert count(lambda: ops.ess(xb, r)) == 2 and count(lambda: ops.gather_rows_ess(xb[:T], r)) == 2
+    assert count(lambda: ops.gather_rows(xb[:T], r)) == 1 and count(lambda: ops.combine_rows(xb, r)) == 1
+    for rows, kernels in ((512, 1), (513, 2)):
+        assert count(lambda: ops.gate_topk(torch.randn(rows, 64, device="cuda"), 2)) == kernels
+    for rows, kernels in ((8192, 1), (8193, 2)):
+        assert count(lambda: ops.route(torch.zeros(rows, 1, dtype=torch.int32, device="cuda"), E)) == kernels
