@@ -239,9 +239,10 @@ def _dense_on_kernels(cfg, x: Tensor) -> bool:
     kernels (fused bias + activation, fused activation derivative); anything else is plain PyTorch.
 
     Tokens at least 64 wide: forward + backward at widths 64 to 248 and 16 to 65000 tokens 295-440 us against 430-1106 with
-    PyTorch operations.  A ReLU takes the kernels from 256 on: the two ways round a pre-activation differently (once from
-    the fp32 sum here, before and after the bias there), which moves a derivative that jumps at zero by more than the
-    rounding itself.  HEXA_DENSE_MIN_DIM sets the width for all.  Below 256 the layer also keeps what it allowed as PyTorch
+    PyTorch operations.  A ReLU takes the kernels from 256 on, as all activations once did: PyTorch rounds a pre-activation
+    before and after the bias, which flips its derivative near zero (relative error of bf16 gradients 1.1-1.3e-2 against
+    2.3e-3 on the kernels, 4096 tokens 64 to 192 wide, 405-540 us against 316-428), so that a lower line, though closer to
+    the exact values, would move the gradients of existing calls by as much as a 16-bit tolerance.  HEXA_DENSE_MIN_DIM sets the width for all.  Below 256 the layer also keeps what it allowed as PyTorch
     operations: more tokens than the kernels take, torch.func and tracing, any layout (see MLP_Implement for the backward)."""
     if os.environ.get("HEXA_DENSE_KERNELS", "1") == "0":        # A/B switch: keep the dense FFN on PyTorch ops
         return False

@@ -292,6 +292,16 @@ def test_dense_depth_widths_on_the_kernels(dim, act, on_kernels):
     if act != "relu":
         for a, b in zip(got, want):
             assert float((a.float() - b.float()).norm()) <= 1.2e-2 * float(b.float().norm())
+    if not on_kernels:
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        return
+    # against 64 bits, a ReLU's mask included: the kernels round a pre-activation once, after the sum that decides its sign
+    w1, w2, b1, b2 = P = [p.detach().double().requires_grad_(True) for p in m.parameters()]
+    xd = x.double().requires_grad_(True)
+    y = fn(xd @ w1.t() + b1) @ w2 + b2
+    exact = [y.detach()] + list(torch.autograd.grad(y, [xd] + P, dy.double()))
+    for a, b in zip(got, exact):
+        assert float((a.double() - b).norm()) <= 1.2e-2 * float(b.norm())
 
 
 def test_dense_routing_belongs_to_its_stream():
