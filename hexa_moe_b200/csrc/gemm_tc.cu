@@ -93,9 +93,8 @@ struct Params {
   float* partial;   //        partial results [splits, E, m, n] go here and are added in chunk order by estmm_reduce_kernel
   float* colsum;    // ESMM, optional: fp32 [row_capacity / 128, n]; row b receives the column sums of the 128 output rows
                     // of block b, taken from the values as they are stored (after rounding to the 16-bit type)
-  int debug;        // measurement / test aid (HEXA_TC_DEBUG, hexa_set_tc_debug): bit 0 = the producer skips the TMA loads and
-                    // arrives in their place, bit 1 = the MMA thread skips the MMAs, bit 2 = the producer neither loads
-                    // nor arrives, so that every wait of the pipeline runs into its limit
+  int debug;        // test aid (hexa_set_tc_debug): bit 2 = the producer neither loads nor arrives, bit 3 = the derivative's saved
+                    // pre-activation is not requested, so that the waits behind them run into their limit
   int32_t* status;
   uint64_t wait_limit_ns;   // limit of every mbarrier wait (hexa_set_wait_limit_ns; default 2 s)
 };
@@ -331,8 +330,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           const int bcol = tile.col0 + rank * BNH;     // this CTA's share of the B columns
           if (p.debug & 4) {
             // nothing is loaded and nobody arrives: the consumers' waits run into their limit (error-path test)
-          } else if (p.debug & 1) {   // results are garbage; only the timing of the remaining pipeline is of interest
-            if (rank == 0) mbar_arrive(&full[stage]);
           } else if (CTAS == 2) {
             // bytes of both CTAs are credited to the leader's barrier; only the leader arms it
             const uint32_t lead_full = lead_full0 + 8u * (uint32_t)stage;
@@ -414,12 +411,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (!(ok = mbar_wait_fast(&full[stage], phase, abort_flag, p.status, 3, p.wait_limit_ns))) break;
           const uint64_t adesc = adesc0 + (uint64_t)stage * kStageDesc;
           const uint64_t bdesc = bdesc0 + (uint64_t)stage * kStageDesc;
-          if (!(p.debug & 2)) {
 #pragma unroll
-            for (int j = 0; j < BLOCK_K / UMMA_K; ++j) {
-              if (CTAS == 2) umma_f16_pair(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
-              else umma_f16(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
-            }
+          for (int j = 0; j < BLOCK_K / UMMA_K; ++j) {
+            if (CTAS == 2) umma_f16_pair(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
+            else umma_f16(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
           }
           accumulate = 1;
           // slot reusable (in both CTAs) once these MMAs have read it
@@ -561,6 +556,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       uint32_t seq = 0;             // DACT: blocks done so far; block i uses staging tile i & 1
       bool requested = false;       // DACT, leader: the block about to start has its aux load under way
       auto request_aux = [&](uint32_t block, int64_t col, int row0) {
+        if (p.debug & 8) return;
         uint64_t* bar = &aux_full[part * 2 + (block & 1)];
         mbar_expect_tx(bar, C::kStoreBufBytes);
         tma_load_2d(bufs + (block & 1) * C::kStoreBufBytes, &tmX, bar, (int)col, row0);
@@ -624,7 +620,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (!mbar_wait_fast(&aux_full[part * 2 + (seq & 1)], (seq >> 1) & 1u, abort_flag, p.status, 5, p.wait_limit_ns) && lane == 0)
                 group_abort[part] = 1;
             }
-            const bool two = OUT == OUT_ACT && p.aux != nullptr && !(p.debug & 16);
+            const bool two = OUT == OUT_ACT && p.aux != nullptr;
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
               uint32_t v[16];
@@ -642,8 +638,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               }
               uint32_t x[8], y[8], o[8];
               if (OUT == OUT_DACT) load_half(buf, rloc, hf, x);      // columns past the end came in as zeros
-              if (p.debug & 8) epi_dispatch16<OUT_LINEAR>(0, is_bf16, f, x, y, o);
-              else epi_dispatch16<OUT>(p.act, is_bf16, f, x, y, o);
+              epi_dispatch16<OUT>(p.act, is_bf16, f, x, y, o);
               // registers -> swizzled staging tile(s) -> one TMA store per 128x32 block (full 128-byte lines to L2)
               if (OUT != OUT_DACT && hf == 0) {      // (DACT writes over its own row of the saved pre-activation)
                 if (lane == 0) bulk_wait_read<0>();  // this warp's previous stores have finished reading its rows of the buffers
@@ -656,13 +651,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (OUT == OUT_DACT) {
               group_sync(1 + part);
               if (group_abort[part]) { ok = false; break; }
-              if (leader && !(p.debug & 32)) {
+              if (leader) {
                 tma_store_2d(&tmC, buf, (int)gcol, row0);
                 bulk_commit();
               }
             } else {      // every warp stores its own 32 rows: no warp waits for another
               __syncwarp();
-              if (lane == 0 && !(p.debug & 32)) {
+              if (lane == 0) {
                 uint8_t* mine = buf + q * 2048;
                 if (two) tma_store_2d(&tmX, mine + C::kStoreBufBytes, (int)gcol, row0 + q * 32);
                 tma_store_2d(&tmC, mine, (int)gcol, row0 + q * 32);
@@ -671,7 +666,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (p.colsum != nullptr) group_sync(1 + part);      // the other warps' rows are staged
             }
             ++seq;
-            if (p.colsum != nullptr && !(p.debug & 32)) {
+            if (p.colsum != nullptr) {
               // Column sums of the block that now sits in the staging tile (the output as stored).  The warp whose TMEM
               // quadrant is q takes the 16-byte chunk q of every row: lane = (row mod 8) * 4 + 32-bit word within the
               // chunk (two columns), 16 rows per lane, then the eight row classes meet through three shuffles.  The eight

@@ -424,6 +424,7 @@ struct StatusSlot {
 };
 static StatusSlot g_status[64];
 static uint64_t g_wait_limit_ns = 2000000000ull;
+constexpr int kDebugBits = 4 | 8;
 static int g_tc_debug = -1;
 
 static int current_device() {
@@ -446,7 +447,7 @@ uint64_t wait_limit_ns() { return g_wait_limit_ns; }
 int tc_debug_flags() {
   if (g_tc_debug < 0) {
     const char* s = getenv("HEXA_TC_DEBUG");
-    g_tc_debug = s ? atoi(s) : 0;
+    g_tc_debug = s ? atoi(s) & kDebugBits : 0;
   }
   return g_tc_debug;
 }
@@ -500,7 +501,7 @@ extern "C" int hexa_set_wait_limit_ns(uint64_t ns) {
   return HEXA_OK;
 }
 extern "C" int hexa_set_tc_debug(int flags) {
-  HEXA_REQUIRE(flags >= 0 && flags < 64, "hexa_set_tc_debug: flags must be a combination of bits 0..5");
+  HEXA_REQUIRE((flags & ~hexa::kDebugBits) == 0, "hexa_set_tc_debug: flags must be a combination of bits 2 and 3");
   hexa::g_tc_debug = flags;
   return HEXA_OK;
 }

@@ -98,11 +98,11 @@ uint64_t hexa_launch_count(void);
 int hexa_pending_device_status(void);
 /* Limit of every wait inside the kernels, in nanoseconds of the GPU's global timer (process-wide; default 2 s). */
 int hexa_set_wait_limit_ns(uint64_t ns);
-/* Measurement / test switches of the tcgen05 kernels (process-wide; initial value: environment variable
- * HEXA_TC_DEBUG, default 0).  bit 0: the TMA producer skips its loads and signals their arrival itself; bit 1: the
- * MMA thread skips the MMAs (both: timing of the remaining pipeline, results are garbage); bit 2: the producer
- * neither loads nor signals, so every wait of the pipeline runs into its limit and the kernel reports through the
- * status word (used with a short hexa_set_wait_limit_ns to exercise the error path without any fault). */
+/* Test switches of the tcgen05 kernels, 16-bit and fp32 (process-wide; initial value: environment variable HEXA_TC_DEBUG,
+ * default 0).  bit 2: the producer neither loads nor signals, so every wait of the pipeline runs into its limit and the
+ * kernel reports through the status word; bit 3: the activation-derivative epilogue does not request the saved
+ * pre-activation, whose wait then runs out (both with a short hexa_set_wait_limit_ns, to exercise the error path without
+ * any fault). */
 int hexa_set_tc_debug(int flags);
 
 /* Cap on the SMs the persistent GEMM kernels occupy from now on (process-wide; 0 = all SMs).  Their tile

@@ -73,6 +73,55 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_keeps_working(ops, n_ou
     assert torch.equal(again[:n_pad], good[:n_pad]) and L.device_status() == 0
 
 
+# bit 2 stops every load; bit 3 only the saved pre-activation's, so that the derivative epilogue gives up with an accumulator
+# in hand.  sums: the epilogue that also adds columns meets at more barriers.
+@pytest.mark.parametrize("epilogue,flags,codes", [("act", 4, (1, 2, 3, 4)), ("dact", 4, (1, 2, 3, 4)), ("dact", 8, (5,)), ("sums", 8, (5,))])
+@pytest.mark.parametrize("n_out", [128, 512])
+def test_a_wait_that_runs_out_in_the_activation_epilogues(ops, n_out, epilogue, flags, codes):
+    L, r, xs, w = _case(ops, n_out)
+    lib = L.lib()
+    n_pad = int(r.pad_offsets[-1])
+    y1 = torch.randn(r.row_capacity, n_out, generator=torch.Generator(device="cuda").manual_seed(0), device="cuda").bfloat16()
+    epi = L.EPI_ACT if epilogue == "act" else L.EPI_DACT
+
+    def run():
+        aux, sums = y1.clone(), torch.zeros(r.num_experts, n_out, device="cuda") if epilogue == "sums" else None
+        y = ops.esmm(xs, w, L.B_NK, r, None, epi, L.ACT_GELU, aux=aux, engine=L.ENGINE_TCGEN05, sums=sums)
+        return [t for t in (y[:n_pad], aux[:n_pad], sums) if t is not None]
+
+    good = run()
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+    try:
+        assert lib.hexa_set_wait_limit_ns(5_000_000) == 0 and lib.hexa_set_tc_debug(flags) == 0
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        try:
+            run()
+        except L.HexaError:
+            pass                                      # the wrapper may see the code already
+        t1.record()
+        torch.cuda.synchronize()
+        assert t0.elapsed_time(t1) < 1000.0
+    finally:
+        lib.hexa_set_tc_debug(0)
+        lib.hexa_set_wait_limit_ns(2_000_000_000)
+    assert L.device_status() in codes
+    with pytest.raises(L.HexaError, match="bounded wait"):
+        run()
+    L.clear_device_status()
+    assert all(torch.equal(a, b) for a, b in zip(run(), good))
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+
+
+def test_debug_switches_that_skip_work_are_refused(ops):
+    from hexa_moe_b200 import _lib as L
+    for flags in (1, 2, 16, 32, 64, -1):
+        assert L.lib().hexa_set_tc_debug(flags) != 0
+    assert L.lib().hexa_set_tc_debug(0) == 0
+
+
 @pytest.mark.parametrize("form", ["nk", "kn", "tn"])
 def test_a_wait_that_runs_out_in_the_fp32_kernel(ops, form):
     """The same for fp32 data on the tensor cores (ESMM with either weight layout, ESTMM)."""
