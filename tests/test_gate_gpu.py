@@ -318,3 +318,23 @@ def test_direct_gate_projection_leaves_the_linear_to_who_watches_it():
         y = gate(xi)
     (dx,) = torch.autograd.grad(y.sum(), xi)
     assert near(dx, w.sum(0).expand(64, 128))
+
+
+def test_split_precision_gate_under_modes_and_batched_gradients():
+    """Tokens beyond the direct projection: dispatch modes see operations, and a batch of gradients passes through."""
+    from torch.utils.flop_counter import FlopCounterMode
+    from hexa_moe_b200.impls import gating
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(5000, 64, generator=g, device="cuda").bfloat16().requires_grad_(True)
+    gate = gating.LinearTopKGate(64, 8, fp32_gate=True).cuda()
+    w = gate.wg.weight
+    dy = torch.randn(5000, 8, generator=g, device="cuda")
+    y = gate(x)
+    with FlopCounterMode(display=False) as flops:
+        seen = gate(x)
+    assert flops.get_total_flops() > 0 and torch.allclose(y, seen, rtol=1e-5, atol=1e-5)      # sums of 64 terms, in fp32
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+    bx, bw = torch.autograd.grad(gate(x), (x, w), torch.stack([dy, 2 * dy]), is_grads_batched=True)
+    for b, d in ((bx, dx), (bw, dw)):
+        assert float((b[0] - d).float().norm()) <= 1e-2 * float(d.float().norm())             # one bf16 rounding of dx
+        assert float((b[1] - 2 * d).float().norm()) <= 1e-2 * float((2 * d).float().norm())
