@@ -31,8 +31,9 @@
 //                 STAGED  ESTMM's 16-bit [E, m, n] outputs: 145 us with register stores (a row per lane, half-used
 //                         sectors), 75 through the staging tile (32 experts x 4096 x 1024 from 144 rows each; long
 //                         segments measure the same either way)
-//               The tile's bias is put into shared memory by the group a tile ahead (fc1 + GELU of the first shape: 209 ->
-//               196 us on one box, the 16 per-thread global loads of a block sat in front of the math).  Loading all 32
+//               The tile's bias is put into shared memory by the group a tile ahead (fc1 + GELU of [32768 rows, 3072 x 768]:
+//               209 -> 196 us, the 16 per-thread global loads of a block sat in front of the math; 171-177 with the stores per
+//               warp).  Loading all 32
 //               columns of a block from TMEM at once instead of 16 + 16 spilled and was 20 % slower.
 // so the epilogue of tile i overlaps the MMAs of tile i+1.  Every mbarrier wait is bounded: after ~2 s a CTA
 // raises an abort flag, records a code in the status word and drains; both CTAs of a pair always reach the
@@ -867,9 +868,10 @@ bool esmm_tc_supported(const void* a, int64_t lda, const void* b, int64_t ldb, i
   if (dtype != HEXA_F16 && dtype != HEXA_BF16) return false;
   if (!aligned16(a) || !aligned16(b) || !aligned16(c) || (aux && !aligned16(aux)) || (bias && !aligned16(bias))) return false;
   if (lda % 8 || ldb % 8 || b_estride % 8 || ldc % 8 || (aux && ldaux % 8) || (bias && ldbias % 4)) return false;
-  // n_out itself may be any size (a rank's slice of an unevenly split hidden dimension): the TMA stores clip at
-  // n_out, but the epilogue's 16-byte reads of bias and saved pre-activation run to the end of the last chunk, so
-  // those rows must be padded to whole chunks
+  // n_out itself may be any size (a rank's slice of an unevenly split hidden dimension): TMA stores clip at n_out and TMA
+  // loads of the saved pre-activation fill with zeros.  Rows of aux and of an fp32 bias are asked for in whole 16-byte
+  // chunks all the same: callers allocate them so (sorted_buffer, _f32), and what they get does not hang on the reads of
+  // one version of the epilogue (its bias reads are scalar now, and a 16-bit bias needs no padding).
   const int64_t n8 = (n_out + 7) / 8 * 8, n4 = (n_out + 3) / 4 * 4;
   if ((aux && ldaux < n8) || (bias && ldbias < n4)) return false;
   return true;
