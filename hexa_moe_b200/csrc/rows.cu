@@ -5,7 +5,7 @@
 //   combine  reads top_k*cols*size and writes cols*size per token, 4*top_k B of token_row
 //   ESS      reads cols*size per padded row once; partials add 4*cols B per 128 rows (write + read).  The gather that
 //            makes the rows can sum them on the way (hexa_gather_rows_ess): then only the partials are read.  [262144, 2048]
-//            bf16 by token: gather 318 + first pass 193 us apart, 392 us together.
+//            bf16 by token: gather 318 + first pass 193 us apart, 348 us together.
 #include "hexa_common.cuh"
 
 namespace hexa {
@@ -138,9 +138,12 @@ __global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes
 }
 
 // ---- ESS pass 1: column sums of one 128-row tile (one expert) ------------------------------------
-// block = 32 column groups x 8 row groups; a thread sums 16 rows of V adjacent columns, eight loads in flight.
+// block = 32 column groups x 4 row groups; a thread sums 32 rows (r mod 4) of V adjacent columns, all loads in flight, and
+// the four sums are added in order.  The order is part of the result: a bias gradient is rounded to 16 bits from it.  Eight
+// row groups of 16 rows, eight loads in flight, took 400 us with the gather at [262144, 2048] where this takes 348, and 110
+// us where this takes 95 at [131072, 1024]; below a few thousand rows they were 1-4 us faster (a longer chain per thread).
 // GATHER: the rows come from src[row_token[row]] (zeros for pad rows) and are written to dst as well.
-constexpr int kEssCx = 32, kEssRy = 8;
+constexpr int kEssCx = 32, kEssRy = 4;
 template <typename T, bool GATHER>
 __global__ void __launch_bounds__(kEssCx * kEssRy)
 ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ row_token,
@@ -153,7 +156,7 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
   const int64_t row0 = (int64_t)blockIdx.y * kRowTile;
   if (row0 >= n_pad) return;
   if (GATHER) {
-    if (threadIdx.x < kRowTile) tok_s[threadIdx.x] = __ldg(row_token + row0 + threadIdx.x);
+    for (int i = threadIdx.x; i < kRowTile; i += kEssCx * kEssRy) tok_s[i] = __ldg(row_token + row0 + i);
     __syncthreads();
   }
   const int cx = threadIdx.x & (kEssCx - 1), ry = threadIdx.x / kEssCx;
@@ -164,7 +167,7 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
   if (col < cols) {
     const bool vec_ok = GATHER || ((col + V <= cols) && (src_ld % V == 0));      // GATHER: checked by the host
     if (vec_ok) {
-#pragma unroll 8
+#pragma unroll 32
       for (int r = ry; r < kRowTile; r += kEssRy) {
         uint4 raw = make_uint4(0, 0, 0, 0);
         if (GATHER) {
@@ -200,31 +203,54 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
   }
 }
 
-// ---- ESS pass 2: per expert, add its tiles' partial rows -----------------------------------------
-// 32 columns x 8 slices of the tiles per block, each slice in ascending order, then the slices in order: an expert with
-// 144 tiles is 18 dependent additions deep (one thread per column walked all of them: 13 us for [18432, 512] and its
-// hidden gradient, 5 us now).
+// ---- ESS pass 2: per expert, add its tiles' partial rows in ascending order -----------------------
+// 32 columns per block.  The additions of a column are one chain, whose order the results keep, so what is shared out is the
+// reading: eight warps fetch 64 tiles' rows at a time into shared memory, the next 64 already under way while one warp adds.
+// Experts of up to 8 tiles, a tile per warp, skip the pipeline.  (One thread per column that also loaded walked 144 tiles in
+// 13 us; with the slices of the tiles summed apart, in another order, both passes of [18432, 2048] took 11.3 us, now 11.1.)
+constexpr int kFinalTiles = 64;
 template <typename TO>
 __global__ void __launch_bounds__(256)
 ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
                  int64_t cols, TO* __restrict__ out, int64_t ldo) {
-  __shared__ float red[8][32];
+  __shared__ float rows[kFinalTiles][32];
   const int e = blockIdx.y;
   const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * 32 + cx;
   const int64_t t0 = pad_offsets[e] / kRowTile, t1 = pad_offsets[e + 1] / kRowTile;
-  float s = 0.f;
-  if (c < cols) {
-#pragma unroll 8
-    for (int64_t t = t0 + slice; t < t1; t += 8) s += __ldg(partial + t * cols + c);
+  if (t1 - t0 <= 8) {      // a tile per warp
+    rows[slice][cx] = c < cols && t0 + slice < t1 ? __ldg(partial + (t0 + slice) * cols + c) : 0.f;
+    __syncthreads();
+    if (slice == 0 && c < cols) {
+      float s = 0.f;
+      for (int i = 0; i < (int)(t1 - t0); ++i) s += rows[i][cx];
+      out[(int64_t)e * ldo + c] = from_f32<TO>(s);
+    }
+    return;
   }
-  red[slice][cx] = s;
-  __syncthreads();
-  if (slice == 0 && c < cols) {
+  float next[kFinalTiles / 8];
+  auto fetch = [&](int64_t base) {
 #pragma unroll
-    for (int y = 1; y < 8; ++y) s += red[y][cx];
-    out[(int64_t)e * ldo + c] = from_f32<TO>(s);
+    for (int i = 0; i < kFinalTiles / 8; ++i) {
+      const int64_t t = base + slice + 8 * i;
+      next[i] = c < cols && t < t1 ? __ldg(partial + t * cols + c) : 0.f;
+    }
+  };
+  fetch(t0);
+  float s = 0.f;
+  for (int64_t base = t0; base < t1; base += kFinalTiles) {      // uniform across the block
+#pragma unroll
+    for (int i = 0; i < kFinalTiles / 8; ++i) rows[slice + 8 * i][cx] = next[i];
+    __syncthreads();
+    if (base + kFinalTiles < t1) fetch(base + kFinalTiles);
+    if (slice == 0) {
+      const int n = (int)min((int64_t)kFinalTiles, t1 - base);
+#pragma unroll 16
+      for (int i = 0; i < n; ++i) s += rows[i][cx];
+    }
+    __syncthreads();
   }
+  if (slice == 0 && c < cols) out[(int64_t)e * ldo + c] = from_f32<TO>(s);
 }
 
 }  // namespace

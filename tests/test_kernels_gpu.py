@@ -630,3 +630,25 @@ def test_launches_are_counted_where_they_happen(ops):
         assert count(lambda: ops.gate_topk(torch.randn(rows, 64, device="cuda"), 2)) == kernels
     for rows, kernels in ((8192, 1), (8193, 2)):
         assert count(lambda: ops.route(torch.zeros(rows, 1, dtype=torch.int32, device="cuda"), E)) == kernels
+
+
+# Column sums keep one order of additions, which the bias gradients are rounded from: within a 128-row tile rows r mod 4 in
+# ascending order and the four sums in turn, then the tiles of an expert in ascending order.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,cols", [(1, 1, 8), (1000, 3, 264), (18432, 1, 520), (9000, 2, 203), (8200, 1, 32)])
+def test_column_sums_keep_their_order(ops, dtype, T, E, cols):
+    ids = make_ids(T, 1, E, 3, skew=True)
+    r = ops.route(ids.cuda(), E)
+    x = torch.randn(T, cols, generator=torch.Generator().manual_seed(T)).to(dtype).cuda()
+    rows, both = ops.gather_rows_ess(x, r)
+    n_pad, po = int(r.pad_offsets[-1]), r.pad_offsets.tolist()
+    tiles = rows[:n_pad].float().view(-1, 32, 4, cols)
+    acc = torch.zeros(tiles.shape[0], 4, cols, device="cuda")
+    for i in range(32):
+        acc = acc + tiles[:, i]
+    part = ((acc[:, 0] + acc[:, 1]) + acc[:, 2]) + acc[:, 3]
+    want = torch.zeros(E, cols, device="cuda")
+    for e in range(E):
+        for t in range(po[e] // 128, po[e + 1] // 128):
+            want[e] += part[t]
+    assert torch.equal(both, want) and torch.equal(ops.ess(rows, r), want)
