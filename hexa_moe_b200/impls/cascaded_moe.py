@@ -365,9 +365,10 @@ class MoE_Cascaded(torch.nn.Module):
         x = input.reshape(-1, original_shape[-reserve_dims:].numel())
         if torch.is_autocast_enabled():
             x = x.to(torch.get_autocast_gpu_dtype() if x.is_cuda else torch.get_autocast_cpu_dtype())
-        else:      # the module's first parameter, which may be one that a subclass or a caller has added
-            first = next(self.parameters(), None)
-            x = x if first is None else x.to(first.dtype)
+        else:      # the type of the module's first parameter: one that a subclass or a caller has added, else of its lists
+            lists = self.batched_fc1_w if self.total_depth_moe else self.mlp_fc1_w
+            first = next((p for p in self._parameters.values() if p is not None), None)
+            x = x if first is None and not len(lists) else x.to((lists[0] if first is None else first).dtype)
 
         if not is_moe:
             y = MLP_Implement.apply(cfg, x, self.mlp_fc1_w[i_mlp], self.mlp_fc2_w[i_mlp], self.mlp_fc1_b[i_mlp],
