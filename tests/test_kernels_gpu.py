@@ -652,3 +652,17 @@ def test_column_sums_keep_their_order(ops, dtype, T, E, cols):
         for t in range(po[e] // 128, po[e + 1] // 128):
             want[e] += part[t]
     assert torch.equal(both, want) and torch.equal(ops.ess(rows, r), want)
+
+
+# fp32 weight gradients of 16-bit data (fp32 parameters under autocast): the accumulator truncates, half an ulp (2^-24 of a sum
+# of positive terms, at most) per 16-row MMA of a chain on average, so the chunks that a long segment is cut into bound it.
+@pytest.mark.parametrize("T,E,m,n,chunks", [(18432, 1, 2048, 512, 10), (32768, 8, 1024, 256, 5)])
+def test_fp32_weight_gradient_of_16_bit_data(ops, T, E, m, n, chunks):
+    g = torch.Generator(device="cuda").manual_seed(m)
+    r = ops.route((torch.arange(T, device="cuda") % E).to(torch.int32).view(-1, 1), E)
+    p, q = (ops.gather_rows(torch.randn(T, c, generator=g, device="cuda").abs().bfloat16(), r) for c in (m, n))
+    got = ops.estmm(p, q, r, out_dtype=torch.float32)
+    po = r.pad_offsets.tolist()
+    exact = torch.stack([p[po[e]:po[e + 1]].double().t() @ q[po[e]:po[e + 1]].double() for e in range(E)])
+    chain = -(-(T // E // 64) // chunks) * 4
+    assert float((got.double() - exact).norm() / exact.norm()) <= (chain + chunks) * 2.0 ** -24
