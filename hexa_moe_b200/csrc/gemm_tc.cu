@@ -31,6 +31,9 @@
 //                 STAGED  ESTMM's 16-bit [E, m, n] outputs: 145 us with register stores (a row per lane, half-used
 //                         sectors), 75 through the staging tile (32 experts x 4096 x 1024 from 144 rows each; long
 //                         segments measure the same either way)
+//                 PARTIAL a split ESTMM's fp32 partial results: the accumulator is drained every few k-blocks into fp32
+//                         registers, which bounds its truncating chains whatever the length of a chunk, and the sums
+//                         leave through the staging tile (see estmm_tc_plan)
 //               The tile's bias is put into shared memory by the group a tile ahead (fc1 + GELU of [32768 rows, 3072 x 768]:
 //               209 -> 196 us, the 16 per-thread global loads of a block sat in front of the math; 171-177 with the stores per
 //               warp).  Loading all 32
@@ -91,7 +94,8 @@ struct Params {
   int out_f32;      // ESTMM: fp32 output
   int beta;         // ESTMM: accumulate into out
   int splits;       // ESTMM: > 1 = every expert's row segment is cut into this many chunks, each its own tile, whose fp32
-  float* partial;   //        partial results [splits, E, m, n] go here and are added in chunk order by estmm_reduce_kernel
+                    //        partial results [splits, E, m, n] are added in chunk order by estmm_reduce_kernel
+  int chains;       // ESTMM with splits > 1: a chunk's k-blocks are accumulated in this many chains
   float* colsum;    // ESMM, optional: fp32 [row_capacity / 128, n]; row b receives the column sums of the 128 output rows
                     // of block b, taken from the values as they are stored (after rounding to the 16-bit type)
   int debug;        // test aid (hexa_set_tc_debug): bit 2 = the producer neither loads nor arrives, bit 3 = the derivative's saved
@@ -101,8 +105,8 @@ struct Params {
 };
 
 // What the epilogue does with an accumulator.  ESMM: HEXA_EPI_LINEAR / HEXA_EPI_ACT / HEXA_EPI_DACT; ESTMM: stores from
-// registers (any output form) or through staging tiles (16-bit [E, m, n] outputs).
-enum Out { OUT_LINEAR = HEXA_EPI_LINEAR, OUT_ACT = HEXA_EPI_ACT, OUT_DACT = HEXA_EPI_DACT, OUT_REGISTERS = 3, OUT_STAGED = 4 };
+// registers (any output form) or through staging tiles (16-bit [E, m, n] outputs; fp32 partial results of a split).
+enum Out { OUT_LINEAR = HEXA_EPI_LINEAR, OUT_ACT = HEXA_EPI_ACT, OUT_DACT = HEXA_EPI_DACT, OUT_REGISTERS = 3, OUT_STAGED = 4, OUT_PARTIAL = 5 };
 
 template <int BN, int CTAS, int MODE, int OUT> struct Cfg {
   static constexpr int kEpiWarps = 16;
@@ -136,6 +140,7 @@ struct Tile {
   int valid;      // this CTA has rows to store (the second CTA of a pair may not)
   int skip;       // ESMM: the tile's expert is outside the launch's expert range (every role skips it alike)
   int split;      // ESTMM with splits > 1: which chunk of the segment this tile covers
+  int chain;      // ... and how many k-blocks one accumulation takes
 };
 
 // Tile t of the static list, as seen by CTA `rank` of its pair (rank = 0 when CTAS = 1).  Returns false past the end.
@@ -162,6 +167,7 @@ __device__ __forceinline__ bool get_tile(const Params& p, uint32_t t, int rank, 
     tile.row0 = seg0 + kb0 * BLOCK_K;
     tile.num_kb = max(0, min(kb_per, kb_all - kb0));
     tile.split = (int)c;
+    tile.chain = max(1, (kb_per + p.chains - 1) / p.chains);
     tile.skip = 0;
     tile.valid = tile.m0 < p.m;
     return true;
@@ -401,34 +407,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       int it = -1;
       for (uint32_t t = tile_first; ok && get_tile<BN, MODE, CTAS>(p, t, rank, tile); t += tile_step) {
         if (MODE != ESTMM && tile.skip) continue;
-        ++it;
-        const int acc = it & 1;
-        const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
-        if (!(ok = mbar_wait_fast(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, 2, p.wait_limit_ns))) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-        uint32_t accumulate = 0;
-        for (int kb = 0; kb < tile.num_kb; ++kb) {
-          if (!(ok = mbar_wait_fast(&full[stage], phase, abort_flag, p.status, 3, p.wait_limit_ns))) break;
-          const uint64_t adesc = adesc0 + (uint64_t)stage * kStageDesc;
-          const uint64_t bdesc = bdesc0 + (uint64_t)stage * kStageDesc;
+        int kb = 0;
+        do {      // one accumulation: the whole tile, or (PARTIAL) the next chain of its k-blocks
+          ++it;
+          const int acc = it & 1;
+          const uint32_t acc_phase = (uint32_t)(it >> 1) & 1u;
+          if (!(ok = mbar_wait_fast(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, 2, p.wait_limit_ns))) break;
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+          uint32_t accumulate = 0;
+          const int kb_end = OUT == OUT_PARTIAL ? min(kb + tile.chain, tile.num_kb) : tile.num_kb;
+          for (; kb < kb_end; ++kb) {
+            if (!(ok = mbar_wait_fast(&full[stage], phase, abort_flag, p.status, 3, p.wait_limit_ns))) break;
+            const uint64_t adesc = adesc0 + (uint64_t)stage * kStageDesc;
+            const uint64_t bdesc = bdesc0 + (uint64_t)stage * kStageDesc;
 #pragma unroll
-          for (int j = 0; j < BLOCK_K / UMMA_K; ++j) {
-            if (CTAS == 2) umma_f16_pair(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
-            else umma_f16(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
+            for (int j = 0; j < BLOCK_K / UMMA_K; ++j) {
+              if (CTAS == 2) umma_f16_pair(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
+              else umma_f16(d_tmem, adesc + (uint64_t)(j * a_step), bdesc + (uint64_t)(j * b_step), idesc, j == 0 ? accumulate : 1u);
+            }
+            accumulate = 1;
+            // slot reusable (in both CTAs) once these MMAs have read it
+            if (CTAS == 2) umma_commit_pair(&empty[stage]); else umma_commit(&empty[stage]);
+            if (++stage == kStages) { stage = 0; phase ^= 1; }
           }
-          accumulate = 1;
-          // slot reusable (in both CTAs) once these MMAs have read it
-          if (CTAS == 2) umma_commit_pair(&empty[stage]); else umma_commit(&empty[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        if (tile.num_kb > 0) {
-          if (CTAS == 2) umma_commit_pair(&acc_full[acc]); else umma_commit(&acc_full[acc]);
-        } else {  // empty segment: nothing to wait for, the epilogues write zeros
-          mbar_arrive(&acc_full[acc]);
-          if (CTAS == 2) mbar_arrive_cluster(map_to_cta(&acc_full[acc], 1));
-        }
+          if (!ok) break;
+          if (tile.num_kb > 0) {
+            if (CTAS == 2) umma_commit_pair(&acc_full[acc]); else umma_commit(&acc_full[acc]);
+          } else {  // empty segment: nothing to wait for, the epilogues write zeros
+            mbar_arrive(&acc_full[acc]);
+            if (CTAS == 2) mbar_arrive_cluster(map_to_cta(&acc_full[acc], 1));
+          }
+        } while (OUT == OUT_PARTIAL && kb < tile.num_kb);
       }
     }
     __syncwarp();
@@ -458,7 +468,53 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         else mbar_arrive(&acc_empty[acc]);
       }
     };
-    if constexpr (MODE == ESTMM) {
+    if constexpr (OUT == OUT_PARTIAL) {
+      constexpr int kCols = C::kBlocks * 32;
+      Tile tile;
+      for (uint32_t t = tile_first; ok && get_tile<BN, MODE, CTAS>(p, t, rank, tile); t += tile_step) {
+        float sum[kCols];
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
+        int kb = 0;
+        do {
+          ++it;
+          const int acc = it & 1;
+          if (!(ok = accumulator_ready(acc, (uint32_t)(it >> 1) & 1u))) break;
+          tc_fence_after();
+          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + part_col);
+          if (tile.num_kb > 0) {
+#pragma unroll
+            for (int s = 0; s < kCols / 16; ++s) {
+              uint32_t v[16];
+              tmem_ld16(taddr + s * 16, v);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) sum[s * 16 + i] += __uint_as_float(v[i]);
+            }
+          }
+          accumulator_drained(acc);
+          kb += tile.chain;
+        } while (kb < tile.num_kb);
+        if (!ok) break;
+#pragma unroll
+        for (int s = 0; s < kCols / 16; ++s) {
+          const int64_t gcol = (int64_t)tile.col0 + part_col + s * 16;
+          if (gcol < p.n && tile.valid) {      // uniform across the four warps of a group
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) w[i] = __float_as_uint(sum[s * 16 + i]);
+            if (leader) bulk_wait_read<0>();   // the previous store has finished reading the buffer
+            group_sync(1 + part);
+            stage_row(bufs, rloc, w);
+            fence_async_smem();
+            group_sync(1 + part);
+            if (leader) {      // rows and columns beyond the result are clipped
+              tma_store_3d(&tmC, bufs, (int)gcol, tile.m0, tile.split * p.E + tile.e);
+              bulk_commit();
+            }
+          }
+        }
+      }
+    } else if constexpr (MODE == ESTMM) {
       Tile tile;
       for (uint32_t t = tile_first; get_tile<BN, MODE, CTAS>(p, t, rank, tile); t += tile_step) {
         ++it;
@@ -494,16 +550,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             continue;
           }
           const int64_t mrow = (int64_t)tile.m0 + rloc;
-          if (mrow < p.m && p.splits > 1) {
-            // a chunk's partial result: plain fp32 [splits, E, m, n]
-            float* o = p.partial + (((int64_t)tile.split * p.E + tile.e) * p.m + mrow) * p.n + gcol;
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-              if (gcol + g * 4 < p.n)
-                *reinterpret_cast<float4*>(o + g * 4) = make_float4(__uint_as_float(v[4 * g]), __uint_as_float(v[4 * g + 1]),
-                                                                    __uint_as_float(v[4 * g + 2]), __uint_as_float(v[4 * g + 3]));
-            }
-          } else if (mrow < p.m) {
+          if (mrow < p.m) {
             if (p.out_f32) {
               float* o = (p.n_split ? reinterpret_cast<float*>(p.c_split[mrow / p.m_split])
                                     : reinterpret_cast<float*>(p.c) + (mrow / p.m_split) * p.split_stride) +
@@ -735,9 +782,10 @@ estmm_reduce_kernel(const float* __restrict__ partial, int splits, int E, int64_
     const int64_t c4 = i % n4, row = i / n4;          // row = e * m + mrow
     const int64_t e = row / m, mrow = row - e * m;
     const float* src = partial + row * n + c4 * 4;
-    float4 acc = *reinterpret_cast<const float4*>(src);
+    float4 acc = __ldg(reinterpret_cast<const float4*>(src));
+#pragma unroll 4
     for (int s = 1; s < splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)s * plane);
+      const float4 v = __ldg(reinterpret_cast<const float4*>(src + (int64_t)s * plane));
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     const int64_t off = (mrow / m_split) * split_stride + e * c_estride + (mrow % m_split) * ldc + c4 * 4;
@@ -955,17 +1003,22 @@ bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, 
   return true;
 }
 
-// How many chunks a split ESTMM cuts every expert's segment into (1 = no split).  Only static sizes enter: the tile
-// count without a split against the CTA pairs (or CTAs) of the device, and the average segment length, so that a chunk
-// keeps at least 8 k-blocks.  Few, long segments - the dense FFN's weight gradient (one "expert" owning every row), or a
-// handful of experts with a small d x H - would otherwise leave most SMs idle behind a few serial k-loops.  A chunk is also
-// the length of a chain in the accumulator, which truncates: a count that fills whole waves with fewer, longer chunks is
-// faster ([18432 rows, 2048 x 512] in 4 chunks 47 us, in these 10 63 us) but further from the exact sums: relative error of
-// that shape's fp32 result 5.0e-6 against 1.9e-6 (positive data 17e-6 against 4.7e-6), one chunk 21e-6.
-int estmm_tc_splits(int E, int64_t row_cap, int64_t m, int64_t n) {
+// How a split ESTMM is cut (chunks = 1: no split).  Only static sizes enter.  Few, long segments - the dense FFN's weight
+// gradient (one "expert" owning every row), or a handful of experts with a small d x H - would leave most SMs idle behind a
+// few serial k-loops, so where the output has fewer tiles than two per CTA pair (or CTA) every segment is cut into chunks, each a tile of its
+// own.  Two things are chosen apart:
+//   the length of a chain in the accumulator, which truncates: at least as many chains as make two tiles per CTA pair, of
+//     at least 8 k-blocks (relative error of the fp32 result of [18432 rows, 2048 x 512] in 10 chains 1.9e-6, in 4 5.0e-6, in
+//     one 21e-6; positive data 4.7 / 17 / 94e-6).  Between chains the sums are kept in fp32 registers;
+//   the number of chunks, by time: full waves of a chunk's k-blocks at 0.29 us, 2 us to fill, drain and store a tile, and the
+//     partial results, written and read once, at 5 TB/s.
+// One chunk per chain, partial results stored from registers / this, us: [18432 rows, 2048 x 512] 64 / 43, [65000, 256 x 1024]
+// 61 / 45, [16384, 1024 x 256] x 8 35 / 24, [2000, 768 x 3072] 39 / 25; error of the first 1.9e-6 / 1.6e-6.
+struct EstmmPlan { int chunks, chains; };      // chains per chunk
+EstmmPlan estmm_tc_plan(int E, int64_t row_cap, int64_t m, int64_t n) {
   static int forced = -2;
   if (forced == -2) forced = env_int("HEXA_ESTMM_SPLITS", -1);       // A/B switch: 1 = never split
-  if (n % 4) return 1;
+  if (n % 4) return {1, 1};
   const int BN = n > 128 ? 256 : 128;
   const int ctas = (BN == 256 && m > BLOCK_M && pairs_enabled()) ? 2 : 1;
   const int64_t tiles = (int64_t)E * ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN);
@@ -974,13 +1027,21 @@ int estmm_tc_splits(int E, int64_t row_cap, int64_t m, int64_t n) {
   int64_t s = 1;
   if (tiles < 2 * slots) s = ceil_div(2 * slots, tiles);
   if (s > avg_kb / 8) s = avg_kb / 8;
-  if (forced > 0) s = forced;
+  if (forced > 0) return {(int)(forced < 32 ? forced : 32), 1};
   if (s > 32) s = 32;
-  return s < 1 ? 1 : (int)s;
+  if (s <= 1) return {1, 1};
+  const double plane_us = (double)E * (double)m * (double)n * 8.0 / 5e6;
+  int best = 2;
+  double best_us = 0.0;
+  for (int c = 2; c <= 32 && c <= avg_kb / 8; ++c) {
+    const double us = (double)ceil_div(tiles * c, slots) * ((double)ceil_div(avg_kb, c) * 0.29 + 2.0) + c * plane_us;
+    if (c == 2 || us < best_us) { best = c; best_us = us; }
+  }
+  return {best, (int)ceil_div(s, best)};
 }
 
 size_t estmm_tc_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n) {
-  const int s = estmm_tc_splits(E, row_cap, m, n);
+  const int s = estmm_tc_plan(E, row_cap, m, n).chunks;
   return s > 1 ? (size_t)s * (size_t)E * (size_t)m * (size_t)n * sizeof(float) : 0;
 }
 
@@ -991,7 +1052,8 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   const int is_bf16 = dtype == HEXA_BF16;
   const int BN = n > 128 ? 256 : 128;
   const int ctas = (BN == 256 && m > BLOCK_M && pairs_enabled()) ? 2 : 1;
-  int splits = n_split > 0 ? 1 : estmm_tc_splits(E, row_cap, m, n);
+  const EstmmPlan plan = estmm_tc_plan(E, row_cap, m, n);
+  int splits = n_split > 0 ? 1 : plan.chunks;
   if (splits > 1 && (!workspace || workspace_bytes < (size_t)splits * E * m * n * sizeof(float) || !aligned16(workspace)))
     splits = 1;      // without scratch the operator still runs, one tile per expert's whole segment
   CUtensorMap tmA, tmB;
@@ -1017,7 +1079,7 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   p.n_split = n_split;
   for (int i = 0; i < n_split && i < 16; ++i) p.c_split[i] = split_out[i];
   p.is_bf16 = is_bf16; p.out_f32 = out_dtype == HEXA_F32; p.beta = beta;
-  p.splits = splits; p.partial = static_cast<float*>(workspace);
+  p.splits = splits; p.chains = splits > 1 ? plan.chains : 1;
   p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
   const int64_t max_tiles = (int64_t)E * ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN) * splits;
   HEXA_REQUIRE(max_tiles < (int64_t)0x7fffffff, "hexa_estmm: too many output tiles for a 32-bit tile index");
@@ -1025,9 +1087,26 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   p.per_expert = (uint32_t)(ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN) * splits);
   p.total_tiles = (uint32_t)max_tiles;
   int rc;
-  const bool staged = n_split == 0 && m_split >= m && !beta && !p.out_f32 && splits == 1;
   CUtensorMap tmC = tmA;      // a placeholder for register stores
-  if (staged) {
+  if (splits > 1) {
+    const uint64_t dims[3] = {(uint64_t)n, (uint64_t)m, (uint64_t)splits * (uint64_t)E};
+    const uint64_t str[2] = {(uint64_t)n * 4, (uint64_t)m * (uint64_t)n * 4};
+    const uint32_t box[3] = {16, BLOCK_M, 1};
+    rc = encode_tensor_map(&tmC, workspace, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_64B);
+    if (rc) return rc;
+    if (ctas == 2) rc = launch<256, ESTMM, 2, OUT_PARTIAL>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+    else rc = BN == 256 ? launch<256, ESTMM, 1, OUT_PARTIAL>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
+                        : launch<128, ESTMM, 1, OUT_PARTIAL>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+    if (rc) return rc;
+    const int64_t total = (int64_t)E * m * (n / 4);
+    int64_t blocks = ceil_div(total, 256);
+    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+    estmm_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const float*>(workspace), splits, E, m, n, out, ldo, o_estride,
+                                                            p.m_split, p.split_stride, p.out_f32, is_bf16, beta);
+    HEXA_LAUNCH_CHECK("estmm_reduce_kernel");
+    return HEXA_OK;
+  }
+  if (n_split == 0 && m_split >= m && !beta && !p.out_f32) {
     uint64_t dims[3] = {(uint64_t)n, (uint64_t)m, (uint64_t)E};
     uint64_t str[2] = {(uint64_t)ldo * 2, (uint64_t)o_estride * 2};
     uint32_t box[3] = {32, BLOCK_M, 1};
@@ -1037,17 +1116,9 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
     return BN == 256 ? launch<256, ESTMM, 1, OUT_STAGED>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
                      : launch<128, ESTMM, 1, OUT_STAGED>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
   }
-  if (ctas == 2) rc = launch<256, ESTMM, 2, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
-  else rc = BN == 256 ? launch<256, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
-                      : launch<128, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
-  if (rc != HEXA_OK || splits == 1) return rc;
-  const int64_t total = (int64_t)E * m * (n / 4);
-  int64_t blocks = ceil_div(total, 256);
-  if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-  estmm_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(p.partial, splits, E, m, n, out, ldo, o_estride, p.m_split, p.split_stride,
-                                                          p.out_f32, is_bf16, beta);
-  HEXA_LAUNCH_CHECK("estmm_reduce_kernel");
-  return HEXA_OK;
+  if (ctas == 2) return launch<256, ESTMM, 2, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
+  return BN == 256 ? launch<256, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream)
+                   : launch<128, ESTMM, 1, OUT_REGISTERS>(tmA, tmB, tmC, tmA, p, max_tiles, stream);
 }
 
 }  // namespace hexa

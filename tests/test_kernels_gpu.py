@@ -666,3 +666,26 @@ def test_fp32_weight_gradient_of_16_bit_data(ops, T, E, m, n, chunks):
     exact = torch.stack([p[po[e]:po[e + 1]].double().t() @ q[po[e]:po[e + 1]].double() for e in range(E)])
     chain = -(-(T // E // 64) // chunks) * 4
     assert float((got.double() - exact).norm() / exact.norm()) <= (chain + chunks) * 2.0 ** -24
+
+
+# A split weight gradient: tiles past m and n, empty and short segments next to long ones, every form of the output.  Bound: half
+# an ulp per MMA of a chain (as above; chains of at most 32 k-blocks here), one per partial sum, the rounding of the output.
+@pytest.mark.parametrize("T,E,m,n,skew", [(8200, 1, 136, 40, False), (5000, 3, 264, 520, True), (16384, 5, 640, 128, True), (2200, 2, 96, 1000, False)])
+def test_split_weight_gradient_forms(ops, T, E, m, n, skew):
+    ids = make_ids(T, 1, E, 5, skew=skew)
+    if E > 2:
+        ids[ids == 1] = 0
+    r = ops.route(ids.cuda(), E)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    p, q = (ops.gather_rows(torch.randn(T, c, generator=g, device="cuda").half(), r) for c in (m, n))
+    assert r.row_capacity // 64 // E >= 16      # long enough to be split
+    po = r.pad_offsets.tolist()
+    exact = torch.stack([p[po[e]:po[e + 1]].double().t() @ q[po[e]:po[e + 1]].double() for e in range(E)])
+    size = torch.stack([p[po[e]:po[e + 1]].double().abs().t() @ q[po[e]:po[e + 1]].double().abs() for e in range(E)])
+    bound = size * (32 * 4 + 32) * 2.0 ** -24
+    got = ops.estmm(p, q, r, out_dtype=torch.float32)
+    assert bool(((got.double() - exact).abs() <= bound).all())
+    half = ops.estmm(p, q, r)
+    assert bool(((half.double() - exact).abs() <= bound + exact.abs() * 2.0 ** -11 + 2.0 ** -25).all())
+    assert torch.equal(ops.estmm(p, q, r, out=got.clone(), beta=1), got + got)
+    assert torch.equal(ops.estmm(p, q, r, out_dtype=torch.float32, ranks=2), torch.stack(got.split(m // 2, dim=1)))
