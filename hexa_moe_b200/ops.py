@@ -8,7 +8,7 @@ device, most of it through the native wrappers of csrc/host.cpp; no function has
 from __future__ import annotations
 
 import os
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Optional
 
 import torch
@@ -490,9 +490,16 @@ def dense_routing(num_tokens: int, device: torch.device) -> Routing:
     """Routing of `num_tokens` rows to a single expert: sorted row i is token i, the tail up to the next multiple
     of 128 is padding.  Built by the routing kernel itself and kept per size, device and stream: the tables are then
     written, read and, once dropped, reused in the order of that one stream.  Under graph capture they are built in the
-    graph, which must not depend on tables that may be dropped, nor leave its own behind."""
+    graph, which must not depend on tables that may be dropped, nor leave its own behind.  One expert's rows end with the
+    tile that holds its last token, one tile before the capacity that holds for any routing, so that gradients of whole
+    tiles are read where they lie."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    build = lambda: route(torch.zeros(num_tokens, 1, dtype=torch.int32, device=device), 1, L.ROW_TILE)
+
+    def build():
+        r = route(torch.zeros(num_tokens, 1, dtype=torch.int32, device=device), 1, L.ROW_TILE)
+        cap = (num_tokens + L.ROW_TILE - 1) // L.ROW_TILE * L.ROW_TILE
+        return replace(r, row_token=r.row_token[:cap], tile_expert=r.tile_expert[:cap // L.ROW_TILE], row_capacity=cap)
+
     if torch.cuda.is_current_stream_capturing():
         return build()
     key = (int(num_tokens), index, torch._C._cuda_getCurrentRawStream(index))
@@ -518,7 +525,7 @@ def dense_forward(x, w1, w2, b1, b2, act_id: int, need_state=True, engine=L.ENGI
     fused epilogues of the grouped GEMM.  Returns (y [T,d_out], LayerState)."""
     T = x.shape[0]
     r = dense_routing(T, x.device)
-    xs = _dense_rows(x, r)
+    xs = gather_rows(x, r) if need_state else _dense_rows(x, r)      # the backward pass keeps rows of its own: the caller may write to x
     y1 = sorted_buffer(r.row_capacity, w1.shape[0], x.dtype, x.device)
     h = esmm(xs, w1.unsqueeze(0), L.B_NK, r, None if b1 is None else _bias(b1, x).unsqueeze(0), L.EPI_ACT, act_id, aux=y1,
              engine=engine)
