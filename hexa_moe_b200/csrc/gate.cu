@@ -13,8 +13,8 @@
 // rows in a fixed order with all its threads.  A single block finishes by itself.  Nothing has to start at zero and every
 // float sum has a fixed order: mass and loss are bit-identical from run to run.
 // Bound: latency (a token is ~30 dependent shuffles) up to some 10^4 tokens, then the reading of the logits.
-// [131072, 64] top-2: 102 us -> 26 + 10 us (the last block used to add 592 partial rows one after the other, ~50 us of
-// it, after four memsets), the gradient 23 -> 17 us.
+// [131072, 64] top-2: 102 us at first, then 26 + 10 with parallel partial rows, 21 + 5 with products for the quotients, a tree
+// for each lane's maximum and a third of the partial rows; the gradient 23, 17, 15 us.
 // Load-importance kernels: one warp per token; the block that finishes last adds the partial rows (in block order).
 // Ties: the lowest expert id wins, and the k ids of a token come out in descending score order.  The selection is
 // total: a score that is NaN ranks below every number, so a row of NaN / inf logits (an overflowed fp16 step) still
@@ -94,6 +94,28 @@ __device__ __forceinline__ void group_load(const float* __restrict__ row, int E,
   for (int j = 0; j < PER; ++j) v[j] = (valid && g + G * j < E) ? __ldg(row + g + G * j) : -FLT_MAX;
 }
 
+// s / sum for a token's exponentials (0 <= s <= 1 <= sum <= E, both NaN-free), bit for bit the IEEE quotient: one correctly
+// rounded reciprocal per token and Markstein's remainder correction per element (P. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000, 1990) are three instructions where a division is a dozen.  The remainder has to be exact, so a
+// token with a non-zero exponential below 2^-90, or with a sum that is no such number, takes the division.
+template <int PER>
+__device__ __forceinline__ void normalise(float sum, float (&s)[PER]) {
+  uint32_t least = 0xffffffffu;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) least = min(least, __float_as_uint(s[j]) - 1u);      // zero wraps to the top
+  if (sum >= 1.f && sum <= 1024.f && least >= ((127u - 90u) << 23)) {
+    const float r = __frcp_rn(sum);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const float q = s[j] * r;
+      s[j] = fmaf(fmaf(-q, sum, s[j]), r, q);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) s[j] = s[j] / sum;
+  }
+}
+
 // logits -> softmax in place; columns >= E come out as 0
 template <int G, int PER>
 __device__ __forceinline__ void group_softmax(int E, int g, float (&s)[PER]) {
@@ -104,9 +126,7 @@ __device__ __forceinline__ void group_softmax(int E, int g, float (&s)[PER]) {
   for (int o = G / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
 #pragma unroll
   for (int j = 0; j < PER; ++j) s[j] = g + G * j < E ? expf(s[j] - m) : 0.f;
-  const float sum = group_sum<G, PER>(s);
-#pragma unroll
-  for (int j = 0; j < PER; ++j) s[j] = s[j] / sum;
+  normalise<PER>(group_sum<G, PER>(s), s);
 }
 
 __device__ __forceinline__ void fold_loss(float part, float* red, int64_t T, int E, float* __restrict__ loss) {
@@ -153,20 +173,24 @@ gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E,
 #pragma unroll
       for (int j = 0; j < PER; ++j) acc[j] += s[j];
     }
-    unsigned int taken = 0;
-    for (int i = 0; i < k; ++i) {
-      // candidates: this lane's free columns; NaN counts as -inf, and the first free column is taken even at -inf,
-      // so some lane always has a candidate while fewer than E columns are taken (k <= E is checked by the host)
-      float best = -INFINITY;
-      int bi = 0x7fffffff;
+    // candidates: scores are not negative, so a column that is taken or does not exist counts as -1 and some lane always
+    // has one at 0 or more while fewer than E are taken (k <= E is checked by the host); a NaN counts as 0: it makes the
+    // whole row NaN, whose lowest columns are then taken
 #pragma unroll
-      for (int j = 0; j < PER; ++j) {
-        const int c = g + G * j;
-        if (c < E && !((taken >> j) & 1u)) {
-          const float v = s[j] == s[j] ? s[j] : -INFINITY;
-          if (bi == 0x7fffffff || v > best) { best = v; bi = c; }   // ascending c: the first maximum stays
-        }
-      }
+    for (int j = 0; j < PER; ++j) s[j] = g + G * j < E ? fmaxf(s[j], 0.f) : -1.f;      // fmaxf(NaN, 0) is 0
+    for (int i = 0; i < k; ++i) {
+      // this lane's maximum, neighbours first, so that the lower columns are always on the left; of equal scores they stay
+      float v[PER];
+      int at[PER];
+#pragma unroll
+      for (int j = 0; j < PER; ++j) { v[j] = s[j]; at[j] = j; }
+#pragma unroll
+      for (int w = 1; w < PER; w *= 2)
+#pragma unroll
+        for (int j = 0; j + w < PER; j += 2 * w)
+          if (v[j + w] > v[j]) { v[j] = v[j + w]; at[j] = at[j + w]; }
+      float best = v[0];
+      int bi = g + G * at[0];
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -174,7 +198,9 @@ gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E,
         if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
       }
       const bool valid = (unsigned)bi < (unsigned)E;     // always true; kept so that no index derived from data is trusted
-      if (valid && (bi & (G - 1)) == g) taken |= 1u << (bi / G);
+#pragma unroll
+      for (int j = 0; j < PER; ++j)
+        if (bi == g + G * j) s[j] = -1.f;
       if (g == 0 && live) {
         ids[(int64_t)i * T + t] = valid ? bi : -1;         // -1 is a row the routing kernel skips
         if (i == 0 && valid) atomicAdd(&cnt_s[bi], 1);
@@ -220,8 +246,8 @@ gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int
   if (slice < slices) {
     float m = 0.f;
     int c = 0;
-#pragma unroll 4
-    for (int b = slice; b < blocks; b += slices) {
+#pragma unroll 16
+    for (int b = slice; b < blocks; b += slices) {      // in the order of b; 16 rows are on their way at a time
       const float* row = partial + (int64_t)b * 2 * E;
       m += __ldg(row + e);
       c += __ldg(reinterpret_cast<const int32_t*>(row) + E + e);
@@ -662,11 +688,12 @@ gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ 
   }
 }
 
-// Blocks of the group kernels: one sweep of a block covers kGateWarps * 32 / G tokens, three blocks per SM at most.
-int gate_group_grid(int64_t T, int G) {
-  int64_t cap = (int64_t)sm_count() * 3;
+// Blocks of the group kernels: one sweep of a block covers warps * 32 / G tokens, 24 or 32 warps per SM at most.  Blocks of
+// 32 warps where their column sums fit in shared memory: 148 partial rows instead of 444 for gate_finish_kernel to add.
+int gate_group_grid(int64_t T, int G, int warps) {
+  int64_t cap = (int64_t)sm_count() * (warps == 32 ? 1 : 3);
   if (cap > kGateMaxBlocks / 2) cap = kGateMaxBlocks / 2;      // a block leaves two rows of words
-  const int64_t want = ceil_div(T, kGateWarps * (32 / G));
+  const int64_t want = ceil_div(T, warps * (32 / G));
   return (int)(want < cap ? want : cap);
 }
 // Tokens that one block takes by itself, saving the second launch (~3 us): four sweeps at ~1 us each, of 32 warps where
@@ -728,9 +755,10 @@ extern "C" int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_token
                                                                                   top_k, ids, mass, first_count, loss,     \
                                                                                   partial);                                \
   } else {                                                                                                                 \
-    grid = gate_group_grid(num_tokens, G);                                                                                 \
-    gate_topk_kernel<G, PER, kGateWarps><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, top_k,    \
-                                                                            ids, mass, first_count, loss, partial);        \
+    grid = gate_group_grid(num_tokens, G, lone_warps(G));                                                                  \
+    gate_topk_kernel<G, PER, lone_warps(G)><<<grid, lone_warps(G) * 32, 0, stream>>>(logits, ld, num_tokens, num_experts,  \
+                                                                                     top_k, ids, mass, first_count, loss,  \
+                                                                                     partial);                             \
   }
   HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_FWD)
 #undef HEXA_GATE_FWD
@@ -752,7 +780,7 @@ extern "C" int hexa_gate_loss_grad(const float* logits, int64_t ld, int64_t num_
                "hexa_gate_loss_grad: null pointer or leading dimension < experts");
   int grid = 1;
 #define HEXA_GATE_BWD(G, PER)                                                                                             \
-  grid = gate_group_grid(num_tokens, G);                                                                                  \
+  grid = gate_group_grid(num_tokens, G, kGateWarps);                                                                      \
   gate_loss_grad_kernel<G, PER><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, first_count, dloss, \
                                                                    dlogits, ldd)
   HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_BWD)

@@ -9,7 +9,7 @@
 //                                              threads) instead of waiting for one block to scan them serially; the side
 //                                              tables are shared out over the blocks
 //   beyond that (the re-reading would cost more than a scan) three launches: route_hist, route_scan, route_scatter
-// [131072, 2] ids, 64 experts: 10 + 34 + 11 us with the three launches, 5 + 13 us with two; [2048, 2], 8 experts:
+// [131072, 2] ids, 64 experts: 10 + 34 + 11 us with the three launches, 3 + 9 us with two; [2048, 2], 8 experts:
 // 7 + 5 + 9 us with three, 8 us with one.
 // HBM traffic: ids are read twice (8 B per routed row; once by the single block), row_token and token_row written once.
 #include <stdarg.h>
@@ -184,10 +184,12 @@ __global__ void route_scatter(const int32_t* __restrict__ ids, int64_t T, int to
 }
 
 // ---- one or two launches ------------------------------------------------------------------------------------------------
-constexpr int kIters = 8;                          // rows of a lane: a warp's chunk is at most 256 rows
-constexpr int kCountWarps = 8;
-constexpr int kBlockRows = kCountWarps * 32 * kIters;      // rows of a block when there are several
-constexpr int64_t kSmallRows = 32 * 32 * kIters;           // rows of the single block of 32 warps
+// A block has 2048 rows when there are several: 16 warps of 128 rows, because a warp places its rows 32 at a time, one
+// __match_any_sync after the other ([131072, 2] ids, 64 experts: 3.3 + 8.7 us; 8 warps of 256 rows 5.0 + 12.9).
+constexpr int kIters = 4, kLoneIters = 8;          // 32-row groups of a warp
+constexpr int kCountWarps = 16;
+constexpr int kBlockRows = kCountWarps * 32 * kIters;
+constexpr int64_t kSmallRows = 32 * 32 * kLoneIters;       // rows of the single block of 32 warps
 constexpr int kSmallExperts = 256, kCountExperts = 512;    // (WARPS + 4) * E + 2 words of shared memory stay under 48 KB
 constexpr int64_t kMaxTotals = 65536;
 
@@ -241,7 +243,7 @@ __device__ __forceinline__ int owner(const int32_t* offs, int E, int32_t x) {
 }
 
 // totals: one histogram per block, or null when this is the only block
-template <int WARPS>
+template <int WARPS, int ITERS>
 __global__ void __launch_bounds__(WARPS * 32)
 route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const int32_t* __restrict__ totals, Tables out) {
   extern __shared__ int32_t sm[];
@@ -254,10 +256,10 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunk = (blockIdx.x * (uint32_t)WARPS + (uint32_t)warp) * rows_per_warp;
   const uint32_t chunk_end = min(chunk + rows_per_warp, n_rows);
-  int e[kIters];
-  uint32_t t[kIters], slot[kIters];      // slot = t * top_k + j
+  int e[ITERS];
+  uint32_t t[ITERS], slot[ITERS];      // slot = t * top_k + j
 #pragma unroll
-  for (int i = 0; i < kIters; ++i) {
+  for (int i = 0; i < ITERS; ++i) {
     const uint32_t f = chunk + (uint32_t)i * 32 + (uint32_t)lane;
     e[i] = -1;
     t[i] = slot[i] = 0;
@@ -270,7 +272,7 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
   for (int x = threadIdx.x; x < (WARPS + 2) * E; x += WARPS * 32) sm[x] = 0;
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kIters; ++i)
+  for (int i = 0; i < ITERS; ++i)
     if (e[i] >= 0) atomicAdd(&hist[warp * E + e[i]], 1);
   if (totals) {      // integer sums: the order of the additions is immaterial
     const int slices = max(1, WARPS * 32 / E);
@@ -340,7 +342,7 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
   __syncwarp();
   int32_t* cur = hist + warp * E;
 #pragma unroll
-  for (int i = 0; i < kIters; ++i) {
+  for (int i = 0; i < ITERS; ++i) {
     const uint32_t f = chunk + (uint32_t)i * 32;
     if (f >= chunk_end) break;      // uniform across the warp
     const unsigned peers = __match_any_sync(0xffffffffu, e[i]);
@@ -372,9 +374,10 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
     const int32_t row = (int32_t)(i * out.align);
     out.tile_expert[i] = row < pad[E] ? owner(pad, E, row) : -1;
   }
-  for (int64_t i = tid; i < (int64_t)E * out.align; i += threads) {      // pad slots
-    const int x = (int)(i / out.align), o = (int)(i % out.align);
-    const int32_t row = pad[x] + total[x] + o;
+  const uint32_t align = (uint32_t)out.align, slots = (uint32_t)E * align;      // the host has checked that they fit in 31 bits
+  for (uint32_t i = (uint32_t)tid; i < slots; i += (uint32_t)threads) {         // pad slots
+    const uint32_t x = i / align, o = i - x * align;
+    const int32_t row = pad[x] + total[x] + (int32_t)o;
     if (row < pad[x + 1]) out.row_token[row] = -1;
   }
 }
@@ -551,13 +554,13 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
     const Tables out{counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block, row_cap, pair_cap, align};
     if (plan == 1) {
       const uint32_t rows_per_warp = (uint32_t)ceil_div(ceil_div(n_rows, 32), 32) * 32;
-      route_place<32><<<1, 1024, (36 * (size_t)E + 2) * sizeof(int32_t), stream>>>(in, top_k, (uint32_t)n_rows, rows_per_warp, nullptr, out);
+      route_place<32, kLoneIters><<<1, 1024, (36 * (size_t)E + 2) * sizeof(int32_t), stream>>>(in, top_k, (uint32_t)n_rows, rows_per_warp, nullptr, out);
     } else {
       const unsigned blocks = (unsigned)ceil_div(n_rows, kBlockRows);
       int32_t* totals = (int32_t*)workspace;      // blocks * E words, fewer than the chunk histograms of the third plan
       route_count<<<blocks, kCountWarps * 32, (size_t)E * sizeof(int32_t), stream>>>(in, (uint32_t)n_rows, totals);
       HEXA_LAUNCH_CHECK("route_count");
-      route_place<kCountWarps><<<blocks, kCountWarps * 32, ((kCountWarps + 4) * (size_t)E + 2) * sizeof(int32_t), stream>>>(
+      route_place<kCountWarps, kIters><<<blocks, kCountWarps * 32, ((kCountWarps + 4) * (size_t)E + 2) * sizeof(int32_t), stream>>>(
           in, top_k, (uint32_t)n_rows, 32 * kIters, totals, out);
     }
     HEXA_LAUNCH_CHECK("route_place");

@@ -338,3 +338,22 @@ def test_split_precision_gate_under_modes_and_batched_gradients():
     for b, d in ((bx, dx), (bw, dw)):
         assert float((b[0] - d).float().norm()) <= 1e-2 * float(d.float().norm())             # one bf16 rounding of dx
         assert float((b[1] - 2 * d).float().norm()) <= 1e-2 * float((2 * d).float().norm())
+
+
+# The scores are quotients bit for bit, whatever way they are taken: a block's few tokens and several blocks of them, group sizes
+# 8 to 32, ordinary rows and rows with exponentials too small for the remainder correction; equal scores go to the lowest id.
+@pytest.mark.parametrize("E", [1, 7, 9, 33, 64, 100, 200, 500])
+@pytest.mark.parametrize("T", [3, 2000])
+def test_selection_follows_the_ieee_quotients(E, T):
+    from hexa_moe_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(E + T)
+    logits = torch.randint(-6, 7, (T, E), generator=g, device="cuda").float()          # many equal scores
+    logits[::3] *= 20.0                                                                # e^-200: below 2^-90, down to zero
+    k = min(4, E)
+    ids, _, first, mass = ops.gate_topk(logits, k)
+    order = torch.sort(logits, dim=1, descending=True, stable=True).indices[:, :k]     # integers: distinct logits, distinct scores
+    # scores that underflow to zero tie as well, so compare where the k-th score is not zero
+    live = (logits.gather(1, order[:, -1:]) - logits.max(1, keepdim=True).values)[:, 0] > -80
+    assert bool(live.any()) and torch.equal(ids.t()[live].long(), order[live])
+    assert torch.equal(first, torch.bincount(ids[0].long(), minlength=E).int())
+    assert torch.allclose(mass.double(), torch.softmax(logits.double(), 1).sum(0), rtol=1e-5, atol=1e-6)
