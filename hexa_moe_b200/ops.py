@@ -357,7 +357,8 @@ def moe_forward(x, ids, w1, w2, b1, b2, act_id: int, act_fn=None, route_major=Fa
     xs = gather_rows(x, r)
     b1f, b2f = _bias(b1, x), _bias(b2, x)
     H = w1.shape[1]
-    y1 = sorted_buffer(r.row_capacity, H, x.dtype, x.device)
+    # only a backward pass reads the pre-activation of a fused activation
+    y1 = sorted_buffer(r.row_capacity, H, x.dtype, x.device) if need_state or act_id < 0 else None
     g = None
     groups = fc1_groups if fc1_groups else [(0, E, None)]
     if act_id >= 0:
@@ -526,7 +527,7 @@ def dense_forward(x, w1, w2, b1, b2, act_id: int, need_state=True, engine=L.ENGI
     T = x.shape[0]
     r = dense_routing(T, x.device)
     xs = gather_rows(x, r) if need_state else _dense_rows(x, r)      # the backward pass keeps rows of its own: the caller may write to x
-    y1 = sorted_buffer(r.row_capacity, w1.shape[0], x.dtype, x.device)
+    y1 = sorted_buffer(r.row_capacity, w1.shape[0], x.dtype, x.device) if need_state else None
     h = esmm(xs, w1.unsqueeze(0), L.B_NK, r, None if b1 is None else _bias(b1, x).unsqueeze(0), L.EPI_ACT, act_id, aux=y1,
              engine=engine)
     ys = esmm(h, w2.unsqueeze(0), L.B_KN, r, None if b2 is None else _bias(b2, x).unsqueeze(0), L.EPI_LINEAR, engine=engine)

@@ -406,3 +406,89 @@ def test_gelu_of_infinity_is_infinity():
         for n in (128, 8):
             got = ops.esmm(x, w[:, :n], L.B_NK, r, None, L.EPI_ACT, L.ACT_GELU, engine=L.ENGINE_TCGEN05)[:6]
             assert torch.allclose(got, want[:, None].expand(6, n), rtol=1e-2, atol=1e-2, equal_nan=True)
+
+
+def _filled(m, dtype, seed=0):
+    torch.manual_seed(seed)
+    with torch.no_grad():
+        for n, p in m.named_parameters():
+            p.normal_(0, 0.5 if "gates" in n else 0.1)
+    m = m.to(dtype).cuda().eval()
+    m.gates.float()
+    return m
+
+
+def _step(m, x, dy, depth=2, loss=True):
+    x = x.detach().requires_grad_(True)
+    m.zero_grad(set_to_none=True)
+    y, l_aux = m(depth, x)
+    stage = m.dispatch_params.stage
+    torch.autograd.backward([y] + ([l_aux] if loss else []), [dy] + ([torch.ones_like(l_aux)] if loss else []))
+    assert m.dispatch_params.stage == stage - 1
+    return [y.detach(), l_aux.detach(), x.grad] + [p.grad for p in m.parameters()]
+
+
+def _same(a, b):
+    return len(a) == len(b) and all((u is None) == (v is None) and (u is None or (u.dtype == v.dtype and torch.equal(u, v))) for u, v in zip(a, b))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,d,E,k,b1,b2,act", [(1, 32, 4, 1, True, True, F.gelu), (300, 72, 5, 3, False, True, F.relu), (257, 50, 3, 2, True, False, F.silu),
+                                               (4500, 64, 7, 2, True, True, F.gelu), (130, 64, 4, 1, False, False, lambda t: t.tanh())])
+def test_native_layer_equals_the_general_path(dtype, T, d, E, k, b1, b2, act):
+    """One GPU: the native autograd nodes against the Python functions over the same kernels (which a timed run takes), bit for
+    bit, also without the loss, without gradients and for tokens in three dimensions."""
+    from hexa_moe_b200 import ops
+    m = _filled(_toy(k=k, d=d, E=E, mlp_fc1_bias=b1, mlp_fc2_bias=b2, activation_fn=act), dtype)
+    x, dy = torch.randn(T, d, device="cuda").to(dtype), torch.randn(T, d, device="cuda").to(dtype)
+    run = lambda: (_step(m, x, dy), _step(m, x, dy, loss=False), _step(m, x[None], dy[None], depth=3))
+    native = run()
+    with torch.no_grad():
+        y = m(2, x)[0]
+    assert not y.requires_grad and torch.equal(y, native[0][0])
+    try:
+        ops.PROFILE = []
+        general = run()
+    finally:
+        ops.PROFILE = None
+    assert all(_same(a, b) for a, b in zip(native, general))
+
+
+def test_native_layer_under_hooks_checkpoints_and_failures():
+    from hexa_moe_b200 import _lib as L
+    from torch.utils.checkpoint import checkpoint
+    m = _filled(_toy(k=2, d=64), torch.bfloat16)
+    x, dy = torch.randn(500, 64, device="cuda").bfloat16(), torch.randn(500, 64, device="cuda").bfloat16()
+    want = _step(m, x, dy)
+
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(1), t.cpu())[1], lambda t: t.cuda()):
+        assert _same(_step(m, x, dy), want) and len(packed) >= 4          # tokens and gate weight, logits and counts
+    for reentrant in (True, False):
+        xi = x.clone().requires_grad_(True)
+        m.zero_grad(set_to_none=True)
+        y, l_aux = checkpoint(lambda t: m(2, t), xi, use_reentrant=reentrant)
+        torch.autograd.backward([y, l_aux], [dy, torch.ones_like(l_aux)])
+        assert _same([y.detach(), l_aux.detach(), xi.grad] + [p.grad for p in m.parameters()], want)
+
+    xi = x.clone().requires_grad_(True)
+    y, l_aux = m(2, xi)
+    with torch.no_grad():
+        xi.add_(0)                                                        # the gate's tokens have changed
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        l_aux.backward()
+
+    y, _ = m(2, x.clone().requires_grad_(True))
+    y.backward(dy, retain_graph=True)
+    with pytest.raises(RuntimeError, match="second time"):                # the layer keeps its state for one pass
+        y.backward(dy)
+
+    y, _ = m(2, x.clone().requires_grad_(True))
+    word = L.ensure_status_word(0)
+    try:
+        word[0] = 3                                                       # as if an earlier kernel had given up a wait
+        with pytest.raises(L.HexaError, match="gave up a bounded wait"):
+            y.backward(dy)
+    finally:
+        L.clear_device_status(0)
+    assert _same(_step(m, x, dy), want)
