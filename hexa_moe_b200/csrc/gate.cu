@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, int k, int32_t* __restrict__ ids,
                  float* __restrict__ mass, int32_t* __restrict__ first_count, float* __restrict__ loss,
                  float* __restrict__ partial) {
+  wait_for_previous();
   constexpr int kGroups = 32 / G;
   __shared__ float mass_w[WARPS][G * PER];
   __shared__ int cnt_s[G * PER];
@@ -238,6 +239,7 @@ constexpr int kFinishThreads = 1024;
 __global__ void __launch_bounds__(kFinishThreads)
 gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int E, float* __restrict__ mass,
                    int32_t* __restrict__ first_count, float* __restrict__ loss) {
+  wait_for_previous();
   __shared__ float m_s[kFinishThreads];
   __shared__ int c_s[kFinishThreads];
   __shared__ float red_s[kFinishThreads / 32];
@@ -274,6 +276,7 @@ template <int G, int PER>
 __global__ void __launch_bounds__(kGateThreads)
 gate_loss_grad_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, const int32_t* __restrict__ first_count,
                       const float* __restrict__ dloss, float* __restrict__ dlogits, int64_t ldd) {
+  wait_for_previous();
   constexpr int kGroups = 32 / G;
   const int lane = threadIdx.x & 31, g = lane & (G - 1), grp = lane / G;
   const int64_t first = ((int64_t)blockIdx.x * kGateWarps + (threadIdx.x >> 5)) * kGroups;
@@ -325,6 +328,7 @@ template <> struct Vec<1> { using F = float; using H = uint16_t; };
 template <int V>
 __global__ void __launch_bounds__(256)
 split_terms_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, int64_t cols, int lo_first, __nv_bfloat16* __restrict__ out) {
+  wait_for_previous();
   const int64_t per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / per_row, c = (i - r * per_row) * V;
@@ -352,6 +356,7 @@ split_terms_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, int6
 template <int V>
 __global__ void __launch_bounds__(256)
 sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int lo_first, float* __restrict__ out) {
+  wait_for_previous();
   using F = typename Vec<V>::F;
   const int64_t per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
@@ -394,6 +399,7 @@ __device__ __forceinline__ void load8<float>(const float* __restrict__ p, bool l
 template <typename T>
 __global__ void __launch_bounds__(128)
 gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restrict__ w, int64_t tokens, int E, int64_t d, float* __restrict__ logits) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int64_t groups = (E + 3) / 4;
   const int64_t tile = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -442,6 +448,7 @@ gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restric
 template <typename T>
 __global__ void __launch_bounds__(128)
 gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w, int64_t tokens, int E, int64_t d, T* __restrict__ dx) {
+  wait_for_previous();
   const int64_t chunks = d / 8;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t t0 = i / chunks * 4, c = (i % chunks) * 8;
@@ -478,6 +485,7 @@ gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w,
 template <typename T>
 __global__ void __launch_bounds__(256)
 gate_project_dw_kernel(const float* __restrict__ g, const T* __restrict__ x, int64_t ldx, int64_t tokens, int E, int64_t d, float* __restrict__ dw) {
+  wait_for_previous();
   __shared__ float red[64][33];
   const int cl = threadIdx.x & 3, slice = threadIdx.x >> 2;
   const int64_t c = (int64_t)blockIdx.x * 32 + cl * 8;
@@ -581,6 +589,7 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_topk_li_kernel(const float* __restrict__ logits, const float* __restrict__ noisy, int64_t ld, int64_t T, int E, int k,
                     float inv_sigma, int32_t* __restrict__ ids, float* __restrict__ importance, float* __restrict__ load,
                     float* __restrict__ loss, unsigned int* __restrict__ ticket, float* __restrict__ partial) {
+  wait_for_previous();
   __shared__ float sum_w[kGateWarps][2 * 32 * VPT];
   __shared__ bool last_s;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -645,6 +654,7 @@ __global__ void __launch_bounds__(kGateThreads)
 gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ noisy, int64_t ld, int64_t T, int E, int k,
                     float inv_sigma, const float* __restrict__ importance, const float* __restrict__ load,
                     const float* __restrict__ dloss, float* __restrict__ dlogits, int64_t ldd) {
+  wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kGateWarps + (threadIdx.x >> 5);
   const int64_t nwarps = (int64_t)gridDim.x * kGateWarps;
@@ -751,12 +761,12 @@ extern "C" int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_token
   int grid = 1;
 #define HEXA_GATE_FWD(G, PER)                                                                                              \
   if (num_tokens <= lone_tokens(G)) {                                                                                      \
-    gate_topk_kernel<G, PER, lone_warps(G)><<<1, lone_warps(G) * 32, 0, stream>>>(logits, ld, num_tokens, num_experts,     \
+    after_previous(gate_topk_kernel<G, PER, lone_warps(G)>, 1, lone_warps(G) * 32, 0, stream)(logits, ld, num_tokens, num_experts,     \
                                                                                   top_k, ids, mass, first_count, loss,     \
                                                                                   partial);                                \
   } else {                                                                                                                 \
     grid = gate_group_grid(num_tokens, G, lone_warps(G));                                                                  \
-    gate_topk_kernel<G, PER, lone_warps(G)><<<grid, lone_warps(G) * 32, 0, stream>>>(logits, ld, num_tokens, num_experts,  \
+    after_previous(gate_topk_kernel<G, PER, lone_warps(G)>, grid, lone_warps(G) * 32, 0, stream)(logits, ld, num_tokens, num_experts,  \
                                                                                      top_k, ids, mass, first_count, loss,  \
                                                                                      partial);                             \
   }
@@ -764,7 +774,7 @@ extern "C" int hexa_gate_topk(const float* logits, int64_t ld, int64_t num_token
 #undef HEXA_GATE_FWD
   HEXA_LAUNCH_CHECK("gate_topk_kernel");
   if (grid > 1) {
-    gate_finish_kernel<<<1, kFinishThreads, 0, stream>>>(partial, grid, num_tokens, num_experts, mass, first_count, loss);
+    after_previous(gate_finish_kernel, 1, kFinishThreads, 0, stream)(partial, grid, num_tokens, num_experts, mass, first_count, loss);
     HEXA_LAUNCH_CHECK("gate_finish_kernel");
   }
   return HEXA_OK;
@@ -781,7 +791,7 @@ extern "C" int hexa_gate_loss_grad(const float* logits, int64_t ld, int64_t num_
   int grid = 1;
 #define HEXA_GATE_BWD(G, PER)                                                                                             \
   grid = gate_group_grid(num_tokens, G, kGateWarps);                                                                      \
-  gate_loss_grad_kernel<G, PER><<<grid, kGateThreads, 0, stream>>>(logits, ld, num_tokens, num_experts, first_count, dloss, \
+  after_previous(gate_loss_grad_kernel<G, PER>, grid, kGateThreads, 0, stream)(logits, ld, num_tokens, num_experts, first_count, dloss, \
                                                                    dlogits, ldd)
   HEXA_GATE_DISPATCH(num_experts, HEXA_GATE_BWD)
 #undef HEXA_GATE_BWD
@@ -802,8 +812,8 @@ extern "C" int hexa_gate_split_terms(const float* src, int64_t ld, int64_t rows,
   }
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   const bool v4 = cols % 4 == 0 && ld % 4 == 0 && aligned16(src) && aligned16(out);
-  if (v4) split_terms_kernel<4><<<elementwise_grid(rows * cols / 4), 256, 0, stream>>>(src, ld, rows, cols, by_rows, o);
-  else split_terms_kernel<1><<<elementwise_grid(rows * cols), 256, 0, stream>>>(src, ld, rows, cols, by_rows, o);
+  if (v4) after_previous(split_terms_kernel<4>, elementwise_grid(rows * cols / 4), 256, 0, stream)(src, ld, rows, cols, by_rows, o);
+  else after_previous(split_terms_kernel<1>, elementwise_grid(rows * cols), 256, 0, stream)(src, ld, rows, cols, by_rows, o);
   HEXA_LAUNCH_CHECK("split_terms_kernel");
   return HEXA_OK;
 }
@@ -814,8 +824,8 @@ extern "C" int hexa_gate_sum_terms(const float* part, int64_t rows, int64_t cols
   if (rows == 0 || cols == 0) return HEXA_OK;
   HEXA_REQUIRE(part && out, "hexa_gate_sum_terms: null pointer");
   const bool v4 = cols % 4 == 0 && aligned16(part) && aligned16(out);
-  if (v4) sum_terms_kernel<4><<<elementwise_grid(rows * cols / 4), 256, 0, stream>>>(part, rows, cols, lo_first, out);
-  else sum_terms_kernel<1><<<elementwise_grid(rows * cols), 256, 0, stream>>>(part, rows, cols, lo_first, out);
+  if (v4) after_previous(sum_terms_kernel<4>, elementwise_grid(rows * cols / 4), 256, 0, stream)(part, rows, cols, lo_first, out);
+  else after_previous(sum_terms_kernel<1>, elementwise_grid(rows * cols), 256, 0, stream)(part, rows, cols, lo_first, out);
   HEXA_LAUNCH_CHECK("sum_terms_kernel");
   return HEXA_OK;
 }
@@ -843,7 +853,7 @@ extern "C" int hexa_gate_topk_load_importance(const float* logits, const float* 
   if (grid > kGateMaxBlocks / 2) grid = kGateMaxBlocks / 2;      // two partial rows per block
   const float inv_sigma = 1.f / sigma;
 #define HEXA_GATE_LI(V)                                                                                                     \
-  gate_topk_li_kernel<V><<<grid, kGateThreads, 0, stream>>>(logits, logits_w_noise, ld, num_tokens, num_experts, top_k, inv_sigma, \
+  after_previous(gate_topk_li_kernel<V>, grid, kGateThreads, 0, stream)(logits, logits_w_noise, ld, num_tokens, num_experts, top_k, inv_sigma, \
                                                             ids, importance, load, loss, ticket, partial)
   const int vpt = (num_experts + 31) / 32;
   if (vpt <= 1) HEXA_GATE_LI(1);
@@ -869,7 +879,7 @@ extern "C" int hexa_gate_load_importance_grad(const float* logits, const float* 
   const int grid = gate_grid(num_tokens);
   const float inv_sigma = 1.f / sigma;
 #define HEXA_GATE_LIG(V)                                                                                                     \
-  gate_li_grad_kernel<V><<<grid, kGateThreads, 0, stream>>>(logits, logits_w_noise, ld, num_tokens, num_experts, top_k, inv_sigma, \
+  after_previous(gate_li_grad_kernel<V>, grid, kGateThreads, 0, stream)(logits, logits_w_noise, ld, num_tokens, num_experts, top_k, inv_sigma, \
                                                             importance, load, dloss, dlogits, ldd)
   const int vpt = (num_experts + 31) / 32;
   if (vpt <= 1) HEXA_GATE_LIG(1);
@@ -892,9 +902,9 @@ extern "C" int hexa_gate_project(const void* x, int64_t ldx, const float* w, int
   const int64_t tiles = ceil_div(tokens, 4) * ceil_div(num_experts, 4);
   HEXA_REQUIRE(ceil_div(tiles, 4) < INT32_MAX, "hexa_gate_project: too many tokens");
   const unsigned grid = (unsigned)ceil_div(tiles, 4);
-  if (dtype == HEXA_F32) gate_project_kernel<float><<<grid, 128, 0, stream>>>((const float*)x, ldx, w, tokens, num_experts, d, logits);
-  else if (dtype == HEXA_F16) gate_project_kernel<__half><<<grid, 128, 0, stream>>>((const __half*)x, ldx, w, tokens, num_experts, d, logits);
-  else gate_project_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)x, ldx, w, tokens, num_experts, d, logits);
+  if (dtype == HEXA_F32) after_previous(gate_project_kernel<float>, grid, 128, 0, stream)((const float*)x, ldx, w, tokens, num_experts, d, logits);
+  else if (dtype == HEXA_F16) after_previous(gate_project_kernel<__half>, grid, 128, 0, stream)((const __half*)x, ldx, w, tokens, num_experts, d, logits);
+  else after_previous(gate_project_kernel<__nv_bfloat16>, grid, 128, 0, stream)((const __nv_bfloat16*)x, ldx, w, tokens, num_experts, d, logits);
   HEXA_LAUNCH_CHECK("gate_project_kernel");
   return HEXA_OK;
 }
@@ -908,16 +918,16 @@ extern "C" int hexa_gate_project_grad(const float* g, const void* x, int64_t ldx
   const int64_t blocks = ceil_div(ceil_div(tokens, 4) * (d / 8), 128);
   HEXA_REQUIRE(blocks < INT32_MAX && ceil_div(num_experts, 4) <= 65535, "hexa_gate_project_grad: too many tokens or experts");
   if (dx) {
-    if (dtype == HEXA_F32) gate_project_dx_kernel<float><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (float*)dx);
-    else if (dtype == HEXA_F16) gate_project_dx_kernel<__half><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__half*)dx);
-    else gate_project_dx_kernel<__nv_bfloat16><<<(unsigned)blocks, 128, 0, stream>>>(g, w, tokens, num_experts, d, (__nv_bfloat16*)dx);
+    if (dtype == HEXA_F32) after_previous(gate_project_dx_kernel<float>, (unsigned)blocks, 128, 0, stream)(g, w, tokens, num_experts, d, (float*)dx);
+    else if (dtype == HEXA_F16) after_previous(gate_project_dx_kernel<__half>, (unsigned)blocks, 128, 0, stream)(g, w, tokens, num_experts, d, (__half*)dx);
+    else after_previous(gate_project_dx_kernel<__nv_bfloat16>, (unsigned)blocks, 128, 0, stream)(g, w, tokens, num_experts, d, (__nv_bfloat16*)dx);
     HEXA_LAUNCH_CHECK("gate_project_dx_kernel");
   }
   if (dw) {
     const dim3 grid((unsigned)ceil_div(d, 32), (unsigned)ceil_div(num_experts, 4));
-    if (dtype == HEXA_F32) gate_project_dw_kernel<float><<<grid, 256, 0, stream>>>(g, (const float*)x, ldx, tokens, num_experts, d, dw);
-    else if (dtype == HEXA_F16) gate_project_dw_kernel<__half><<<grid, 256, 0, stream>>>(g, (const __half*)x, ldx, tokens, num_experts, d, dw);
-    else gate_project_dw_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(g, (const __nv_bfloat16*)x, ldx, tokens, num_experts, d, dw);
+    if (dtype == HEXA_F32) after_previous(gate_project_dw_kernel<float>, grid, 256, 0, stream)(g, (const float*)x, ldx, tokens, num_experts, d, dw);
+    else if (dtype == HEXA_F16) after_previous(gate_project_dw_kernel<__half>, grid, 256, 0, stream)(g, (const __half*)x, ldx, tokens, num_experts, d, dw);
+    else after_previous(gate_project_dw_kernel<__nv_bfloat16>, grid, 256, 0, stream)(g, (const __nv_bfloat16*)x, ldx, tokens, num_experts, d, dw);
     HEXA_LAUNCH_CHECK("gate_project_dw_kernel");
   }
   return HEXA_OK;

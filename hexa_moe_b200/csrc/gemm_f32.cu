@@ -140,6 +140,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (every CTA)
@@ -336,6 +337,7 @@ __device__ __forceinline__ uint32_t magnitude(float x) {
 // rows of a and of b.
 __global__ void __launch_bounds__(256)
 split_planes_kernel(const Side a, const Side b, uint32_t* __restrict__ maxima) {
+  wait_for_previous();
   __shared__ uint32_t seen[2][8];
   const int lane = threadIdx.x & 31;
   const int64_t rows_a = a.limit ? min((int64_t)*a.limit, a.rows) : a.rows * a.E;
@@ -397,6 +399,7 @@ template <int V>
 __global__ void __launch_bounds__(256)
 epilogue_rows_kernel(const float* x, int64_t ldx, float* c, int64_t ldc, const int32_t* __restrict__ row_token,
                      const int32_t* __restrict__ pad_offsets, int E, int64_t cols, int epilogue, int act) {
+  wait_for_previous();
   const int64_t rows = pad_offsets[E], per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / per_row, col = (i - r * per_row) * V;
@@ -448,7 +451,7 @@ int split_launch(const Side& a, const Side& b, uint8_t* ws, int64_t terms, Param
   if (blocks > kMaxSplitBlocks) blocks = kMaxSplitBlocks;
   if (want < blocks) blocks = want > 0 ? want : 1;
   uint32_t* maxima = reinterpret_cast<uint32_t*>(ws);
-  split_planes_kernel<<<(unsigned)blocks, 256, 0, stream>>>(a, b, maxima);
+  after_previous(split_planes_kernel, (unsigned)blocks, 256, 0, stream)(a, b, maxima);
   HEXA_LAUNCH_CHECK("split_planes_kernel");
   p.maxima = maxima;
   p.n_maxima = (int)blocks;
@@ -494,11 +497,13 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see after_previous
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (max_clusters[dev] == 0) {
     cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
     int n = 0;
@@ -579,8 +584,8 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
     const int64_t ldx = epilogue == HEXA_EPI_DACT || pre ? ldaux : ldc;
     const bool v4 = n_out % 4 == 0 && ldx % 4 == 0 && ldc % 4 == 0 && aligned16(x) && aligned16(c);
     const unsigned grid = (unsigned)sm_count() * 8;
-    if (v4) epilogue_rows_kernel<4><<<grid, 256, 0, stream>>>(x, ldx, static_cast<float*>(c), ldc, row_token, pad_offsets, E, n_out, epilogue, act);
-    else epilogue_rows_kernel<1><<<grid, 256, 0, stream>>>(x, ldx, static_cast<float*>(c), ldc, row_token, pad_offsets, E, n_out, epilogue, act);
+    if (v4) after_previous(epilogue_rows_kernel<4>, grid, 256, 0, stream)(x, ldx, static_cast<float*>(c), ldc, row_token, pad_offsets, E, n_out, epilogue, act);
+    else after_previous(epilogue_rows_kernel<1>, grid, 256, 0, stream)(x, ldx, static_cast<float*>(c), ldc, row_token, pad_offsets, E, n_out, epilogue, act);
     HEXA_LAUNCH_CHECK("epilogue_rows_kernel");
   }
   return esmm_simt_launch(a, lda, b, b_layout, ldb, b_estride, bias, ldbias, aux, ldaux, c, ldc, tile_expert, pad_offsets, row_token, E,

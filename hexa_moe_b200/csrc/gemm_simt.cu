@@ -169,6 +169,7 @@ esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, 
                  const int32_t* __restrict__ pad_offsets, const int32_t* __restrict__ row_token, int E, int64_t n_out,
                  int64_t k, int epilogue, int act, int e_begin, int e_end, int bias16,
                  const int32_t* __restrict__ only_if) {
+  wait_for_previous(false);
   if (!wanted(only_if)) return;
   const int64_t row0 = (int64_t)blockIdx.y * TILE;
   if (row0 >= pad_offsets[E]) return;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
 estmm_simt_kernel(const T* __restrict__ p, int64_t ldp, const T* __restrict__ q, int64_t ldq,
                   const int32_t* __restrict__ pad_offsets, int64_t m, int64_t n, TO* __restrict__ out, int64_t ldo,
                   int64_t o_estride, int64_t m_split, int64_t split_stride, int beta, const int32_t* __restrict__ only_if) {
+  wait_for_previous(false);
   if (!wanted(only_if)) return;
   const int e = blockIdx.z;
   const int64_t m0 = (int64_t)blockIdx.y * TILE, n0 = (int64_t)blockIdx.x * TILE;
@@ -287,7 +289,7 @@ int esmm_simt_launch(const void* a, int64_t lda, const void* b, int b_layout, in
   const int tile = large ? 128 : 64;
   dim3 grid((unsigned)ceil_div(n_out, tile), (unsigned)(row_cap / tile));
 #define HEXA_ESMM_SIMT(T, TILE, NK, VEC)                                                                               \
-  esmm_simt_kernel<T, TILE, NK, VEC><<<grid, kThreads, 0, stream>>>((const T*)a, lda, (const T*)b, ldb, b_estride, bias, \
+  after_previous(esmm_simt_kernel<T, TILE, NK, VEC>, grid, kThreads, 0, stream, only_if != nullptr)((const T*)a, lda, (const T*)b, ldb, b_estride, bias, \
                                                                     ldbias, (T*)aux, ldaux, (T*)c, ldc, tile_expert,   \
                                                                     pad_offsets, row_token, E, n_out, k, epilogue, act, \
                                                                     e_begin, e_end, bias16, only_if)
@@ -323,7 +325,7 @@ int estmm_simt_launch(const void* p, int64_t ldp, const void* q, int64_t ldq, co
   const int tile = large ? 128 : 64;
   dim3 grid((unsigned)ceil_div(n, tile), (unsigned)ceil_div(m, tile), (unsigned)E);
 #define HEXA_ESTMM_SIMT_V(T, TO, TILE, VEC)                                                                             \
-  estmm_simt_kernel<T, TO, TILE, VEC><<<grid, kThreads, 0, stream>>>((const T*)p, ldp, (const T*)q, ldq, pad_offsets, m, n, \
+  after_previous(estmm_simt_kernel<T, TO, TILE, VEC>, grid, kThreads, 0, stream, only_if != nullptr)((const T*)p, ldp, (const T*)q, ldq, pad_offsets, m, n, \
                                                                      (TO*)out, ldo, o_estride, m_split, split_stride, beta, only_if)
 #define HEXA_ESTMM_SIMT(T, TO, VEC)                    \
   do {                                                 \

@@ -320,6 +320,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (CTAS == 2) cluster_sync_all();   // the peer's barriers exist before anything is sent to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_previous();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (every CTA)
@@ -775,6 +776,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 __global__ void __launch_bounds__(256)
 estmm_reduce_kernel(const float* __restrict__ partial, int splits, int E, int64_t m, int64_t n, void* __restrict__ out, int64_t ldc,
                     int64_t c_estride, int64_t m_split, int64_t split_stride, int out_f32, int is_bf16, int beta) {
+  wait_for_previous();
   const int64_t n4 = n / 4;
   const int64_t total = (int64_t)E * m * n4;
   const int64_t plane = (int64_t)E * m * n;
@@ -834,11 +836,14 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   cfg.blockDim = dim3(C::kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see after_previous
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
   if (CTAS == 2) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
     if (max_clusters[dev] == 0) {   // how many CTA pairs the device can hold at once (one CTA per SM)
       cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
       int n = 0;
@@ -1101,7 +1106,7 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
     const int64_t total = (int64_t)E * m * (n / 4);
     int64_t blocks = ceil_div(total, 256);
     if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-    estmm_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const float*>(workspace), splits, E, m, n, out, ldo, o_estride,
+    after_previous(estmm_reduce_kernel, (unsigned)blocks, 256, 0, stream)(static_cast<const float*>(workspace), splits, E, m, n, out, ldo, o_estride,
                                                             p.m_split, p.split_stride, p.out_f32, is_bf16, beta);
     HEXA_LAUNCH_CHECK("estmm_reduce_kernel");
     return HEXA_OK;

@@ -71,6 +71,34 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
     ::hexa::count_launch();                                                          \
   } while (0)
 
+// A launch that may start while the kernel before it in the stream drains: its blocks take up SMs as they become free, set up
+// and then meet wait_for_previous(), which every kernel launched this way calls before it touches device memory.  Between
+// two kernels of a layer this saves the drain, the launch latency and, for a GEMM, the set-up of barriers and TMEM: 16 tokens
+// through a layer 100 -> 85 us, 2048 tokens 99 -> 82, 4608 tokens x 32 experts both ways 605 -> 578, [131072, 64] router 59.6 -> 57.1.
+template <typename... P> struct AfterPrevious {
+  void (*kernel)(P...);
+  dim3 grid, block;
+  size_t smem;
+  cudaStream_t stream;
+  bool early;
+  template <typename... A> void operator()(A&&... args) const {      // errors are left for HEXA_LAUNCH_CHECK
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  }
+};
+template <typename... P> AfterPrevious<P...> after_previous(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool early = true) {
+  return {kernel, grid, block, smem, stream, early};
+}
+
 // Splits a dtype argument into the data type and its flags; false when a flag comes with a type that is not 16 bits wide
 // or is none of `allowed`.
 inline bool take_flags(int& dtype, int allowed, int& flags) {
@@ -85,6 +113,16 @@ int sm_count();  // SMs of the current device (cached per device)
 int sm_limit();  // upper bound on the SMs persistent kernels may occupy (0 = all), see hexa_set_sm_limit
 
 constexpr int kRowTile = 128;  // rows per GEMM tile == required segment alignment of the GEMM operators
+
+// Until the kernels before this one in the stream have finished and their writes can be seen.  Only then may the next one start
+// to set up, so that at most two kernels share the SMs; or (next_may_start false) not before this one ends, for kernels of many
+// blocks that keep an SM busy: the blocks of an early start go to the SMs that are free first, and a few of them get most of the work
+// (fp32 FMA GEMMs of [4096, 512 x 128]: 30 us each on their own, 45 to 80 us so).  Such kernels are not started early either.
+// Without an early launch both instructions do nothing.
+__device__ __forceinline__ void wait_for_previous(bool next_may_start = true) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (next_may_start) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ---- device-side scalar conversion ------------------------------------------------------------
 template <typename T> __device__ __forceinline__ float to_f32(T v);

@@ -31,6 +31,7 @@ __device__ __forceinline__ int load_id(const int32_t* ids, int64_t f, int64_t T,
 
 __global__ void route_hist(const int32_t* __restrict__ ids, int64_t T, int64_t n_rows, int64_t stride_t,
                            int64_t stride_k, int E, int32_t* __restrict__ chunk_hist) {
+  wait_for_previous();
   extern __shared__ int32_t sm[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int32_t* h = sm + warp * E;
@@ -54,6 +55,7 @@ route_scan(int32_t* __restrict__ chunk_hist, int64_t n_chunks, int E, int align,
            int32_t* __restrict__ counts, int32_t* __restrict__ seg_offsets, int32_t* __restrict__ pad_offsets,
            int32_t* __restrict__ row_token, int32_t* __restrict__ tile_expert, int32_t* __restrict__ pair_off,
            int32_t* __restrict__ pair_block, int64_t pair_cap) {
+  wait_for_previous();
   extern __shared__ int32_t sm[];
   int32_t* s_cnt = sm;          // [E]
   int32_t* s_pad = sm + E;      // [E + 1]
@@ -151,6 +153,7 @@ __global__ void route_scatter(const int32_t* __restrict__ ids, int64_t T, int to
                               int64_t stride_k, int E, const int32_t* __restrict__ chunk_base,
                               const int32_t* __restrict__ pad_offsets, int32_t* __restrict__ row_token,
                               int32_t* __restrict__ token_row) {
+  wait_for_previous();
   extern __shared__ int32_t sm[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int32_t* cur = sm + warp * E;
@@ -208,6 +211,7 @@ struct Ids {
 
 __global__ void __launch_bounds__(kCountWarps * 32)
 route_count(Ids ids, uint32_t n_rows, int32_t* __restrict__ totals) {
+  wait_for_previous();
   extern __shared__ int32_t sm[];
   for (int e = threadIdx.x; e < ids.E; e += blockDim.x) sm[e] = 0;
   __syncthreads();
@@ -246,6 +250,7 @@ __device__ __forceinline__ int owner(const int32_t* offs, int E, int32_t x) {
 template <int WARPS, int ITERS>
 __global__ void __launch_bounds__(WARPS * 32)
 route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const int32_t* __restrict__ totals, Tables out) {
+  wait_for_previous();
   extern __shared__ int32_t sm[];
   const int E = ids.E;
   int32_t* hist = sm;                    // [WARPS][E]: counts, then the next free row of each expert for each warp
@@ -389,6 +394,7 @@ template <typename I>
 __global__ void __launch_bounds__(256)
 ids_from_lists_kernel(const I* __restrict__ tok_ids, const int32_t* __restrict__ exp_ids, int64_t n, int chunk, int64_t num_toks,
                       int32_t* __restrict__ ids, int32_t* status) {
+  wait_for_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int64_t slot = (int64_t)__ldg(tok_ids + i);
@@ -554,13 +560,13 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
     const Tables out{counts, seg_offsets, pad_offsets, row_token, token_row, tile_expert, pair_block, row_cap, pair_cap, align};
     if (plan == 1) {
       const uint32_t rows_per_warp = (uint32_t)ceil_div(ceil_div(n_rows, 32), 32) * 32;
-      route_place<32, kLoneIters><<<1, 1024, (36 * (size_t)E + 2) * sizeof(int32_t), stream>>>(in, top_k, (uint32_t)n_rows, rows_per_warp, nullptr, out);
+      after_previous(route_place<32, kLoneIters>, 1, 1024, (36 * (size_t)E + 2) * sizeof(int32_t), stream)(in, top_k, (uint32_t)n_rows, rows_per_warp, nullptr, out);
     } else {
       const unsigned blocks = (unsigned)ceil_div(n_rows, kBlockRows);
       int32_t* totals = (int32_t*)workspace;      // blocks * E words, fewer than the chunk histograms of the third plan
-      route_count<<<blocks, kCountWarps * 32, (size_t)E * sizeof(int32_t), stream>>>(in, (uint32_t)n_rows, totals);
+      after_previous(route_count, blocks, kCountWarps * 32, (size_t)E * sizeof(int32_t), stream)(in, (uint32_t)n_rows, totals);
       HEXA_LAUNCH_CHECK("route_count");
-      route_place<kCountWarps, kIters><<<blocks, kCountWarps * 32, ((kCountWarps + 4) * (size_t)E + 2) * sizeof(int32_t), stream>>>(
+      after_previous(route_place<kCountWarps, kIters>, blocks, kCountWarps * 32, ((kCountWarps + 4) * (size_t)E + 2) * sizeof(int32_t), stream)(
           in, top_k, (uint32_t)n_rows, 32 * kIters, totals, out);
     }
     HEXA_LAUNCH_CHECK("route_place");
@@ -572,17 +578,17 @@ extern "C" int hexa_route(const int32_t* ids, int64_t T, int top_k, int64_t stri
   warps = warps < 1 ? 1 : (warps > 8 ? 8 : warps);
   const size_t smem = (size_t)warps * E * sizeof(int32_t);
   if (n_chunks > 0) {
-    route_hist<<<(unsigned)ceil_div(n_chunks, warps), warps * 32, smem, stream>>>(ids, T, n_rows, stride_t, stride_k, E,
+    after_previous(route_hist, (unsigned)ceil_div(n_chunks, warps), warps * 32, smem, stream)(ids, T, n_rows, stride_t, stride_k, E,
                                                                                 chunk_hist);
     HEXA_LAUNCH_CHECK("route_hist");
   }
   int32_t* pair_off = chunk_hist + (size_t)(n_chunks > 0 ? n_chunks : 1) * E;
-  route_scan<<<1, 1024, (2 * (size_t)E + 1) * sizeof(int32_t), stream>>>(
+  after_previous(route_scan, 1, 1024, (2 * (size_t)E + 1) * sizeof(int32_t), stream)(
       chunk_hist, n_chunks, E, align, row_cap, counts, seg_offsets, pad_offsets, row_token, tile_expert, pair_off, pair_block,
       pair_cap);
   HEXA_LAUNCH_CHECK("route_scan");
   if (n_chunks > 0) {
-    route_scatter<<<(unsigned)ceil_div(n_chunks, warps), warps * 32, smem, stream>>>(
+    after_previous(route_scatter, (unsigned)ceil_div(n_chunks, warps), warps * 32, smem, stream)(
         ids, T, top_k, n_rows, stride_t, stride_k, E, chunk_hist, pad_offsets, row_token, token_row);
     HEXA_LAUNCH_CHECK("route_scatter");
   }
@@ -600,7 +606,7 @@ int ids_from_lists(const I* tok_ids, const int32_t* exp_ids, int64_t n, int chun
   HEXA_REQUIRE((num_toks == 0 || ids) && (n == 0 || (tok_ids && exp_ids)), "hexa_ids_from_lists: null pointer");
   if (num_toks > 0) HEXA_CUDA(cudaMemsetAsync(ids, 0xFF, (size_t)num_toks * sizeof(int32_t), stream));      // -1: token in no segment
   if (n == 0) return HEXA_OK;
-  ids_from_lists_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, stream>>>(tok_ids, exp_ids, n, chunk, num_toks, ids, status_word());
+  after_previous(ids_from_lists_kernel<I>, (unsigned)ceil_div(n, 256), 256, 0, stream)(tok_ids, exp_ids, n, chunk, num_toks, ids, status_word());
   HEXA_LAUNCH_CHECK("ids_from_lists_kernel");
   return HEXA_OK;
 }

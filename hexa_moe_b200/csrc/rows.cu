@@ -16,6 +16,7 @@ template <int VEC_BYTES>
 __global__ void gather_rows_kernel(const uint8_t* __restrict__ src, int64_t src_ld_bytes,
                                    const int32_t* __restrict__ row_token, const int32_t* __restrict__ pad_offsets,
                                    int E, int64_t row_bytes, uint8_t* __restrict__ dst, int64_t dst_ld_bytes) {
+  wait_for_previous();
   const int64_t n_pad = pad_offsets[E];
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -44,6 +45,7 @@ __global__ void gather_rows_kernel(const uint8_t* __restrict__ src, int64_t src_
 template <typename T, int K>
 __global__ void combine_rows_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ token_row,
                                     int64_t num_tokens, int top_k, int64_t cols, T* __restrict__ dst, int64_t dst_ld) {
+  wait_for_previous();
   constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -116,7 +118,7 @@ void combine_launch(const void* src, int64_t src_ld, const int32_t* token_row, i
   const int warps = 8;
   const unsigned grid = (unsigned)ceil_div(T_, warps);
 #define HEXA_COMBINE(K_)                                                                                              \
-  combine_rows_kernel<T, K_><<<grid, warps * 32, 0, stream>>>((const T*)src, src_ld, token_row, T_, top_k, cols, (T*)dst, dst_ld)
+  after_previous(combine_rows_kernel<T, K_>, grid, warps * 32, 0, stream)((const T*)src, src_ld, token_row, T_, top_k, cols, (T*)dst, dst_ld)
   switch (top_k) {
     case 1: HEXA_COMBINE(1); break;
     case 2: HEXA_COMBINE(2); break;
@@ -129,6 +131,7 @@ void combine_launch(const void* src, int64_t src_ld, const int32_t* token_row, i
 // ---- mask: zero the pad rows of a sorted buffer -------------------------------------------------
 __global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes, const int32_t* __restrict__ row_token,
                                      const int32_t* __restrict__ pad_offsets, int E, int64_t row_bytes) {
+  wait_for_previous();
   const int64_t n_pad = pad_offsets[E];
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -149,6 +152,7 @@ __global__ void __launch_bounds__(kEssCx * kEssRy)
 ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ row_token,
                    const int32_t* __restrict__ pad_offsets, int E, int64_t cols, T* __restrict__ dst, int64_t dst_ld,
                    float* __restrict__ partial) {
+  wait_for_previous();
   constexpr int V = 16 / sizeof(T);
   __shared__ float red[kEssRy][kEssCx * V];
   __shared__ int32_t tok_s[kRowTile];
@@ -213,6 +217,7 @@ template <typename TO>
 __global__ void __launch_bounds__(256)
 ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
                  int64_t cols, TO* __restrict__ out, int64_t ldo) {
+  wait_for_previous();
   __shared__ float rows[kFinalTiles][32];
   const int e = blockIdx.y;
   const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
@@ -272,10 +277,10 @@ extern "C" int hexa_gather_rows(const void* src, int64_t src_ld, const int32_t* 
   const int warps = 8;
   const unsigned grid = (unsigned)ceil_div(row_cap, warps);
   if (v16)
-    gather_rows_kernel<16><<<grid, warps * 32, 0, stream>>>((const uint8_t*)src, sld, row_token, pad_offsets, E, row_bytes,
+    after_previous(gather_rows_kernel<16>, grid, warps * 32, 0, stream)((const uint8_t*)src, sld, row_token, pad_offsets, E, row_bytes,
                                                             (uint8_t*)dst, dld);
   else
-    gather_rows_kernel<2><<<grid, warps * 32, 0, stream>>>((const uint8_t*)src, sld, row_token, pad_offsets, E, row_bytes,
+    after_previous(gather_rows_kernel<2>, grid, warps * 32, 0, stream)((const uint8_t*)src, sld, row_token, pad_offsets, E, row_bytes,
                                                            (uint8_t*)dst, dld);
   HEXA_LAUNCH_CHECK("gather_rows");
   return HEXA_OK;
@@ -308,7 +313,7 @@ extern "C" int hexa_mask_pad_rows(void* buf, int64_t ld, const int32_t* row_toke
   if (row_cap == 0) return HEXA_OK;
   const int64_t es = (int64_t)dtype_size(dtype);
   const int warps = 8;
-  mask_pad_rows_kernel<<<(unsigned)ceil_div(row_cap, warps), warps * 32, 0, stream>>>((uint8_t*)buf, ld * es, row_token,
+  after_previous(mask_pad_rows_kernel, (unsigned)ceil_div(row_cap, warps), warps * 32, 0, stream)((uint8_t*)buf, ld * es, row_token,
                                                                                      pad_offsets, E, cols * es);
   HEXA_LAUNCH_CHECK("mask_pad_rows");
   return HEXA_OK;
@@ -330,7 +335,7 @@ int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int 
     dim3 grid((unsigned)ceil_div(cols, kEssCx * V), (unsigned)tiles);
     HEXA_REQUIRE(tiles <= 65535, "hexa_ess: more than 65535 row tiles (row_capacity %lld)", (long long)row_cap);
 #define HEXA_ESS(T)                                                                                                          \
-  ess_partial_kernel<T, false><<<grid, kEssCx * kEssRy, 0, stream>>>((const T*)src, src_ld, nullptr, pad_offsets, E, cols, nullptr, 0, partial)
+  after_previous(ess_partial_kernel<T, false>, grid, kEssCx * kEssRy, 0, stream)((const T*)src, src_ld, nullptr, pad_offsets, E, cols, nullptr, 0, partial)
     switch (dtype) {
       case HEXA_F32: HEXA_ESS(float); break;
       case HEXA_F16: HEXA_ESS(__half); break;
@@ -346,9 +351,9 @@ int ess_launch(const void* src, int64_t src_ld, const int32_t* pad_offsets, int 
 int ess_finish(const float* partial, const int32_t* pad_offsets, int E, int64_t cols, void* out, int64_t ldo, int out_dtype,
                cudaStream_t stream) {
   dim3 grid2((unsigned)ceil_div(cols, 32), (unsigned)E);
-  if (out_dtype == HEXA_F16) ess_final_kernel<__half><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (__half*)out, ldo);
-  else if (out_dtype == HEXA_BF16) ess_final_kernel<__nv_bfloat16><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (__nv_bfloat16*)out, ldo);
-  else ess_final_kernel<float><<<grid2, 256, 0, stream>>>(partial, pad_offsets, cols, (float*)out, ldo);
+  if (out_dtype == HEXA_F16) after_previous(ess_final_kernel<__half>, grid2, 256, 0, stream)(partial, pad_offsets, cols, (__half*)out, ldo);
+  else if (out_dtype == HEXA_BF16) after_previous(ess_final_kernel<__nv_bfloat16>, grid2, 256, 0, stream)(partial, pad_offsets, cols, (__nv_bfloat16*)out, ldo);
+  else after_previous(ess_final_kernel<float>, grid2, 256, 0, stream)(partial, pad_offsets, cols, (float*)out, ldo);
   HEXA_LAUNCH_CHECK("ess_final");
   return HEXA_OK;
 }
@@ -382,7 +387,7 @@ extern "C" int hexa_gather_rows_ess(const void* src, int64_t src_ld, const int32
   }
   dim3 grid((unsigned)ceil_div(cols, kEssCx * V), (unsigned)tiles);
 #define HEXA_GATHER_ESS(T)                                                                                                   \
-  ess_partial_kernel<T, true><<<grid, kEssCx * kEssRy, 0, stream>>>((const T*)src, src_ld, row_token, pad_offsets, E, cols, (T*)dst, \
+  after_previous(ess_partial_kernel<T, true>, grid, kEssCx * kEssRy, 0, stream)((const T*)src, src_ld, row_token, pad_offsets, E, cols, (T*)dst, \
                                                                     dst_ld, (float*)workspace)
   if (dtype == HEXA_F32) HEXA_GATHER_ESS(float);
   else if (dtype == HEXA_F16) HEXA_GATHER_ESS(__half);

@@ -689,3 +689,28 @@ def test_split_weight_gradient_forms(ops, T, E, m, n, skew):
     assert bool(((half.double() - exact).abs() <= bound + exact.abs() * 2.0 ** -11 + 2.0 ** -25).all())
     assert torch.equal(ops.estmm(p, q, r, out=got.clone(), beta=1), got + got)
     assert torch.equal(ops.estmm(p, q, r, out_dtype=torch.float32, ranks=2), torch.stack(got.split(m // 2, dim=1)))
+
+
+# Kernels may be launched while the one before drains: a chain over ever new data and reused memory, enqueued without a stop and
+# next to PyTorch kernels, against the same chain with the host waiting behind every operator.
+@pytest.mark.parametrize("dtype,T,d,H", [(torch.bfloat16, 300, 64, 256), (torch.float32, 900, 72, 200), (torch.float32, 4000, 256, 1024), (torch.float16, 5000, 128, 512)])
+def test_chains_without_a_stop(ops, dtype, T, d, H):
+    Lb, E, k = L(), 5, 2
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").to(dtype)
+    data = [(torch.randn(T, E, generator=g, device="cuda"), rand(T, d), rand(E, H, d), rand(E, H, d)) for _ in range(6)]
+
+    def chain(logits, x, w1, w2, stop):
+        ids = ops.gate_topk(logits * 1.0, k)[0]; stop()
+        r = ops.route(ids, E, route_major=True); stop()
+        xs, sums = ops.gather_rows_ess(x + 0, r); stop()
+        y1 = ops.sorted_buffer(r.row_capacity, H, dtype, "cuda")
+        h = ops.esmm(xs, w1, Lb.B_NK, r, None, Lb.EPI_ACT, Lb.ACT_GELU, aux=y1); stop()
+        dw = ops.estmm(h, xs, r); stop()
+        ys = ops.esmm(h, w2, Lb.B_KN, r); stop()
+        return [ids, r.token_row, sums, dw, ops.combine_rows(ys, r), ops.ess(h, r)]
+
+    want = [chain(*a, torch.cuda.synchronize) for a in data]
+    got = [chain(*a, lambda: None) for _ in range(5) for a in data]
+    for i, out in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(out, want[i % len(data)])), i
