@@ -714,3 +714,34 @@ def test_chains_without_a_stop(ops, dtype, T, d, H):
     got = [chain(*a, lambda: None) for _ in range(5) for a in data]
     for i, out in enumerate(got):
         assert all(torch.equal(a, b) for a, b in zip(out, want[i % len(data)])), i
+
+
+# Few rows take 128-column tiles of one CTA, more take CTA pairs: either side of the rule, against single-CTA tiles of the other
+# width (no pair list), bit for bit.
+@pytest.mark.parametrize("T,E,n,k", [(1, 3, 136, 64), (96 * 4, 4, 520, 72), (97 * 4, 4, 520, 72), (700, 7, 800, 200), (300, 1, 264, 128), (3000, 2, 2048, 64), (20000, 4, 256, 64)])
+def test_few_rows_take_small_tiles(ops, T, E, n, k):
+    from dataclasses import replace
+    Lb = L()
+    r = ops.route(make_ids(T, 1, E, 9, skew=True).cuda(), E)
+    plain = replace(r, pair_block=None)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w, wt, b = ops.gather_rows(rand(T, k), r), rand(E, n, k), rand(E, k, n), rand(E, n)
+    rows = int(r.pad_offsets[-1])
+
+    def both(layout, wgt, epilogue):
+        out = []
+        for table in (r, plain):
+            aux = ops.sorted_buffer(r.row_capacity, n, x.dtype, "cuda")
+            aux.copy_(saved) if epilogue == Lb.EPI_DACT else aux.zero_()
+            sums = torch.empty(E, n, device="cuda")
+            c = ops.esmm(x, wgt, layout, table, None if epilogue == Lb.EPI_DACT else b, epilogue, Lb.ACT_GELU if epilogue else Lb.ACT_NONE,
+                         aux=aux if epilogue else None, sums=sums)
+            out.append((c[:rows], aux[:rows], sums))
+        return out
+
+    saved = ops.esmm(x, w, Lb.B_NK, r, b)
+    for layout, wgt in ((Lb.B_NK, w), (Lb.B_KN, wt)):
+        for epilogue in (Lb.EPI_LINEAR, Lb.EPI_ACT, Lb.EPI_DACT):
+            a, c = both(layout, wgt, epilogue)
+            assert all(torch.equal(u, v) for u, v in zip(a, c)), (layout, epilogue)
