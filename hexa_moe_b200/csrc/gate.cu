@@ -46,12 +46,12 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // softmax of one token's logits, spread over the warp; columns >= E come out as 0
 template <int VPT>
-__device__ __forceinline__ void warp_softmax(const float* __restrict__ row, int E, int lane, float (&s)[VPT]) {
+__device__ __forceinline__ void warp_softmax(const float* row, int E, int lane, float (&s)[VPT]) {
   float m = -FLT_MAX;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = lane + 32 * i;
-    s[i] = c < E ? __ldg(row + c) : -FLT_MAX;
+    s[i] = c < E ? row[c] : -FLT_MAX;
     m = fmaxf(m, s[i]);
   }
   m = warp_max(m);
@@ -89,9 +89,9 @@ __device__ __forceinline__ float group_sum(const float (&v)[PER]) {
 }
 
 template <int G, int PER>
-__device__ __forceinline__ void group_load(const float* __restrict__ row, int E, int g, bool valid, float (&v)[PER]) {
+__device__ __forceinline__ void group_load(const float* row, int E, int g, bool valid, float (&v)[PER]) {
 #pragma unroll
-  for (int j = 0; j < PER; ++j) v[j] = (valid && g + G * j < E) ? __ldg(row + g + G * j) : -FLT_MAX;
+  for (int j = 0; j < PER; ++j) v[j] = (valid && g + G * j < E) ? row[g + G * j] : -FLT_MAX;
 }
 
 // s / sum for a token's exponentials (0 <= s <= 1 <= sum <= E, both NaN-free), bit for bit the IEEE quotient: one correctly
@@ -144,7 +144,7 @@ __device__ __forceinline__ void fold_loss(float part, float* red, int64_t T, int
 // partial: per block E float column sums, then E int top-1 counts
 template <int G, int PER, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, int k, int32_t* __restrict__ ids,
+gate_topk_kernel(const float* logits, int64_t ld, int64_t T, int E, int k, int32_t* __restrict__ ids,
                  float* __restrict__ mass, int32_t* __restrict__ first_count, float* __restrict__ loss,
                  float* __restrict__ partial) {
   wait_for_previous();
@@ -237,7 +237,7 @@ gate_topk_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E,
 // Adds the blocks' rows: 1024 / E threads per expert take every (1024 / E)-th block, their sums meet in index order.
 constexpr int kFinishThreads = 1024;
 __global__ void __launch_bounds__(kFinishThreads)
-gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int E, float* __restrict__ mass,
+gate_finish_kernel(const float* partial, int blocks, int64_t T, int E, float* __restrict__ mass,
                    int32_t* __restrict__ first_count, float* __restrict__ loss) {
   wait_for_previous();
   __shared__ float m_s[kFinishThreads];
@@ -251,8 +251,8 @@ gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int
 #pragma unroll 16
     for (int b = slice; b < blocks; b += slices) {      // in the order of b; 16 rows are on their way at a time
       const float* row = partial + (int64_t)b * 2 * E;
-      m += __ldg(row + e);
-      c += __ldg(reinterpret_cast<const int32_t*>(row) + E + e);
+      m += row[e];
+      c += reinterpret_cast<const int32_t*>(row)[E + e];
     }
     m_s[threadIdx.x] = m;
     c_s[threadIdx.x] = c;
@@ -274,19 +274,19 @@ gate_finish_kernel(const float* __restrict__ partial, int blocks, int64_t T, int
 // mass = column sums of the softmax (ce counts top-1 choices and carries no gradient)
 template <int G, int PER>
 __global__ void __launch_bounds__(kGateThreads)
-gate_loss_grad_kernel(const float* __restrict__ logits, int64_t ld, int64_t T, int E, const int32_t* __restrict__ first_count,
-                      const float* __restrict__ dloss, float* __restrict__ dlogits, int64_t ldd) {
+gate_loss_grad_kernel(const float* logits, int64_t ld, int64_t T, int E, const int32_t* first_count,
+                      const float* dloss, float* __restrict__ dlogits, int64_t ldd) {
   wait_for_previous();
   constexpr int kGroups = 32 / G;
   const int lane = threadIdx.x & 31, g = lane & (G - 1), grp = lane / G;
   const int64_t first = ((int64_t)blockIdx.x * kGateWarps + (threadIdx.x >> 5)) * kGroups;
   const int64_t step = (int64_t)gridDim.x * kGateWarps * kGroups;
-  const float scale = __ldg(dloss) * ((float)E / (float)T) / (float)T;
+  const float scale = *dloss * ((float)E / (float)T) / (float)T;
   float ge[PER], next[PER];
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const int c = g + G * j;
-    ge[j] = c < E ? scale * (float)__ldg(first_count + c) : 0.f;
+    ge[j] = c < E ? scale * (float)first_count[c] : 0.f;
   }
   group_load<G, PER>(logits + (first + grp) * ld, E, g, first + grp < T, next);
   for (int64_t t0 = first; t0 < T; t0 += step) {
@@ -327,12 +327,12 @@ template <> struct Vec<1> { using F = float; using H = uint16_t; };
 // by_rows, four blocks of rows (lo, mid, hi, hi): src is then one row of rows * cols elements.
 template <int V>
 __global__ void __launch_bounds__(256)
-split_terms_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, int64_t cols, int lo_first, __nv_bfloat16* __restrict__ out) {
+split_terms_kernel(const float* src, int64_t ld, int64_t rows, int64_t cols, int lo_first, __nv_bfloat16* __restrict__ out) {
   wait_for_previous();
   const int64_t per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / per_row, c = (i - r * per_row) * V;
-    const typename Vec<V>::F x = __ldg(reinterpret_cast<const typename Vec<V>::F*>(src + r * ld + c));
+    const typename Vec<V>::F x = *reinterpret_cast<const typename Vec<V>::F*>(src + r * ld + c);
     __align__(8) __nv_bfloat16 t[3][V];
 #pragma unroll
     for (int j = 0; j < V; ++j) {
@@ -355,16 +355,16 @@ split_terms_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, int6
 // out[r, c] = (hi + mid) + lo of a row's three blocks of columns, stored in that order or, with lo_first, reversed
 template <int V>
 __global__ void __launch_bounds__(256)
-sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int lo_first, float* __restrict__ out) {
+sum_terms_kernel(const float* part, int64_t rows, int64_t cols, int lo_first, float* __restrict__ out) {
   wait_for_previous();
   using F = typename Vec<V>::F;
   const int64_t per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / per_row, c = (i - r * per_row) * V;
     const float* p = part + r * 3 * cols + c;
-    const F a = __ldg(reinterpret_cast<const F*>(p + (lo_first ? 2 * cols : 0)));
-    const F b = __ldg(reinterpret_cast<const F*>(p + cols));
-    const F d = __ldg(reinterpret_cast<const F*>(p + (lo_first ? 0 : 2 * cols)));
+    const F a = *reinterpret_cast<const F*>(p + (lo_first ? 2 * cols : 0));
+    const F b = *reinterpret_cast<const F*>(p + cols);
+    const F d = *reinterpret_cast<const F*>(p + (lo_first ? 0 : 2 * cols));
     F o;
 #pragma unroll
     for (int j = 0; j < V; ++j)
@@ -381,24 +381,24 @@ sum_terms_kernel(const float* __restrict__ part, int64_t rows, int64_t cols, int
 // sums meet in 16 shuffles.  Bound: the latency of d / 256 rounds of loads.  [2048, 768], 8 experts: 4 us (fp16 with a
 // cast and a GEMM 22, bf16 in split terms 7 in three launches); [16, 1024], 32 experts: 4 us (split terms 7).
 template <typename T>
-__device__ __forceinline__ void load8(const T* __restrict__ p, bool live, float (&v)[8]) {
+__device__ __forceinline__ void load8(const T* p, bool live, float (&v)[8]) {
   uint4 raw = make_uint4(0, 0, 0, 0);
-  if (live) raw = __ldg(reinterpret_cast<const uint4*>(p));
+  if (live) raw = *reinterpret_cast<const uint4*>(p);
   const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(e[i]);
 }
 
 template <>
-__device__ __forceinline__ void load8<float>(const float* __restrict__ p, bool live, float (&v)[8]) {
+__device__ __forceinline__ void load8<float>(const float* p, bool live, float (&v)[8]) {
   float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-  if (live) { lo = __ldg(reinterpret_cast<const float4*>(p)); hi = __ldg(reinterpret_cast<const float4*>(p) + 1); }
+  if (live) { lo = *reinterpret_cast<const float4*>(p); hi = reinterpret_cast<const float4*>(p)[1]; }
   v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restrict__ w, int64_t tokens, int E, int64_t d, float* __restrict__ logits) {
+gate_project_kernel(const T* x, int64_t ldx, const float* w, int64_t tokens, int E, int64_t d, float* __restrict__ logits) {
   wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int64_t groups = (E + 3) / 4;
@@ -417,8 +417,8 @@ gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restric
     for (int b = 0; b < 4; ++b) {
       float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
       if (e0 + b < E) {
-        lo = __ldg(reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c));
-        hi = __ldg(reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c + 4));
+        lo = *reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c);
+        hi = *reinterpret_cast<const float4*>(w + (int64_t)(e0 + b) * d + c + 4);
       }
       const float wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
@@ -447,7 +447,7 @@ gate_project_kernel(const T* __restrict__ x, int64_t ldx, const float* __restric
 // dx = g W, [T, d]: a thread owns 8 columns of 4 tokens
 template <typename T>
 __global__ void __launch_bounds__(128)
-gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w, int64_t tokens, int E, int64_t d, T* __restrict__ dx) {
+gate_project_dx_kernel(const float* g, const float* w, int64_t tokens, int E, int64_t d, T* __restrict__ dx) {
   wait_for_previous();
   const int64_t chunks = d / 8;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -460,11 +460,11 @@ gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w,
     for (int j = 0; j < 8; ++j) acc[a][j] = 0.f;
 #pragma unroll 2
   for (int e = 0; e < E; ++e) {
-    const float4 lo = __ldg(reinterpret_cast<const float4*>(w + (int64_t)e * d + c)), hi = __ldg(reinterpret_cast<const float4*>(w + (int64_t)e * d + c + 4));
+    const float4 lo = *reinterpret_cast<const float4*>(w + (int64_t)e * d + c), hi = *reinterpret_cast<const float4*>(w + (int64_t)e * d + c + 4);
     const float wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      const float gv = t0 + a < tokens ? __ldg(g + (t0 + a) * E + e) : 0.f;
+      const float gv = t0 + a < tokens ? g[(t0 + a) * E + e] : 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[a][j] = fmaf(gv, wv[j], acc[a][j]);
     }
@@ -484,7 +484,7 @@ gate_project_dx_kernel(const float* __restrict__ g, const float* __restrict__ w,
 // dW = g^T x, fp32 [E, d]: a block owns 32 columns of 4 experts; 64 token slices of 4 column lanes, added in slice order
 template <typename T>
 __global__ void __launch_bounds__(256)
-gate_project_dw_kernel(const float* __restrict__ g, const T* __restrict__ x, int64_t ldx, int64_t tokens, int E, int64_t d, float* __restrict__ dw) {
+gate_project_dw_kernel(const float* g, const T* x, int64_t ldx, int64_t tokens, int E, int64_t d, float* __restrict__ dw) {
   wait_for_previous();
   __shared__ float red[64][33];
   const int cl = threadIdx.x & 3, slice = threadIdx.x >> 2;
@@ -501,7 +501,7 @@ gate_project_dw_kernel(const float* __restrict__ g, const T* __restrict__ x, int
     load8<T>(x + t * ldx + c, c < d, xv);
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const float gv = e0 + b < E ? __ldg(g + t * E + e0 + b) : 0.f;
+      const float gv = e0 + b < E ? g[t * E + e0 + b] : 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[b][j] = fmaf(gv, xv[j], acc[b][j]);
     }
@@ -575,18 +575,18 @@ __device__ __forceinline__ float warp_topk(const float (&v)[VPT], int E, int k, 
 
 // cv2 of an [E] vector and its gradient factors, computed by one warp (every warp that needs them recomputes them:
 // E <= 512 values).  Returns mean and var through references.
-__device__ __forceinline__ void warp_mean_var(const float* __restrict__ v, int E, int lane, float& mean, float& var) {
+__device__ __forceinline__ void warp_mean_var(const float* v, int E, int lane, float& mean, float& var) {
   float s = 0.f;
-  for (int e = lane; e < E; e += 32) s += __ldcg(v + e);
+  for (int e = lane; e < E; e += 32) s += v[e];
   mean = warp_sum(s) / (float)E;
   float q = 0.f;
-  for (int e = lane; e < E; e += 32) { const float d = __ldcg(v + e) - mean; q += d * d; }
+  for (int e = lane; e < E; e += 32) { const float d = v[e] - mean; q += d * d; }
   var = warp_sum(q) / (float)(E - 1);
 }
 
 template <int VPT>
 __global__ void __launch_bounds__(kGateThreads)
-gate_topk_li_kernel(const float* __restrict__ logits, const float* __restrict__ noisy, int64_t ld, int64_t T, int E, int k,
+gate_topk_li_kernel(const float* logits, const float* noisy, int64_t ld, int64_t T, int E, int k,
                     float inv_sigma, int32_t* __restrict__ ids, float* __restrict__ importance, float* __restrict__ load,
                     float* __restrict__ loss, unsigned int* __restrict__ ticket, float* __restrict__ partial) {
   wait_for_previous();
@@ -602,7 +602,7 @@ gate_topk_li_kernel(const float* __restrict__ logits, const float* __restrict__ 
     float s[VPT], v[VPT];
     warp_softmax<VPT>(logits + t * ld, E, lane, s);
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) { const int c = lane + 32 * i; v[i] = c < E ? __ldg(noisy + t * ld + c) : -INFINITY; }
+    for (int i = 0; i < VPT; ++i) { const int c = lane + 32 * i; v[i] = c < E ? noisy[t * ld + c] : -INFINITY; }
     int last_id;
     const float thr = warp_topk<VPT>(v, E, k, lane, ids, T, t, &last_id);
 #pragma unroll
@@ -651,9 +651,9 @@ gate_topk_li_kernel(const float* __restrict__ logits, const float* __restrict__ 
 //   d logits_e = s_e (d s_e - sum_e' s_e' d s_e') + [e = k-th choice] d thr
 template <int VPT>
 __global__ void __launch_bounds__(kGateThreads)
-gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ noisy, int64_t ld, int64_t T, int E, int k,
-                    float inv_sigma, const float* __restrict__ importance, const float* __restrict__ load,
-                    const float* __restrict__ dloss, float* __restrict__ dlogits, int64_t ldd) {
+gate_li_grad_kernel(const float* logits, const float* noisy, int64_t ld, int64_t T, int E, int k,
+                    float inv_sigma, const float* importance, const float* load,
+                    const float* dloss, float* __restrict__ dlogits, int64_t ldd) {
   wait_for_previous();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kGateWarps + (threadIdx.x >> 5);
@@ -661,21 +661,21 @@ gate_li_grad_kernel(const float* __restrict__ logits, const float* __restrict__ 
   float mi, vi, ml, vl;
   warp_mean_var(importance, E, lane, mi, vi);
   warp_mean_var(load, E, lane, ml, vl);
-  const float up = 0.5f * __ldg(dloss);
+  const float up = 0.5f * *dloss;
   const float di = mi * mi + 1e-10f, dl = ml * ml + 1e-10f;
   float gi[VPT], gl[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = lane + 32 * i;
     // d cv2 / d v_e = 2 (v_e - mean) / ((E-1) den) - var * 2 mean / (E den^2)
-    gi[i] = c < E ? up * (2.f * (__ldg(importance + c) - mi) / ((float)(E - 1) * di) - vi * 2.f * mi / ((float)E * di * di)) : 0.f;
-    gl[i] = c < E ? up * (2.f * (__ldg(load + c) - ml) / ((float)(E - 1) * dl) - vl * 2.f * ml / ((float)E * dl * dl)) : 0.f;
+    gi[i] = c < E ? up * (2.f * (importance[c] - mi) / ((float)(E - 1) * di) - vi * 2.f * mi / ((float)E * di * di)) : 0.f;
+    gl[i] = c < E ? up * (2.f * (load[c] - ml) / ((float)(E - 1) * dl) - vl * 2.f * ml / ((float)E * dl * dl)) : 0.f;
   }
   for (int64_t t = warp0; t < T; t += nwarps) {
     float s[VPT], v[VPT];
     warp_softmax<VPT>(logits + t * ld, E, lane, s);
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) { const int c = lane + 32 * i; v[i] = c < E ? __ldg(noisy + t * ld + c) : -INFINITY; }
+    for (int i = 0; i < VPT; ++i) { const int c = lane + 32 * i; v[i] = c < E ? noisy[t * ld + c] : -INFINITY; }
     int last_id;
     const float thr = warp_topk<VPT>(v, E, k, lane, nullptr, T, t, &last_id);
     float ds[VPT];

@@ -226,8 +226,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (blockIdx.x == 1) {      // the second CTA of the first pair issues nothing
       uint32_t amax = 0, bmax = 0;
       for (int i = lane; i < p.n_maxima; i += 32) {
-        amax = max(amax, __ldg(p.maxima + i));
-        bmax = max(bmax, __ldg(p.maxima + p.n_maxima + i));
+        amax = max(amax, p.maxima[i]);
+        bmax = max(bmax, p.maxima[p.n_maxima + i]);
       }
       amax = __reduce_max_sync(0xffffffffu, amax);
       bmax = __reduce_max_sync(0xffffffffu, bmax);
@@ -283,7 +283,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             float v = sum[s * kSlab + i];
-            if (live && col + i < p.n) v += __ldg(p.bias + (int64_t)tile.e * p.ldbias + col + i);
+            if (live && col + i < p.n) v += p.bias[(int64_t)tile.e * p.ldbias + col + i];
             w[i] = __float_as_uint(v);
           }
           if (leader) bulk_wait_read<0>();   // the previous store has finished reading the buffer
@@ -353,17 +353,25 @@ split_planes_kernel(const Side a, const Side b, uint32_t* __restrict__ maxima) {
     const int64_t plane = s.plane;
     uint32_t m = 0;
     if (s.vec) {
-      for (int64_t c = lane * 4; c < s.cols; c += 128) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src + c));
-        float x[4] = {v.x, v.y, v.z, v.w};
+      for (int64_t c0 = lane * 4; c0 < s.cols; c0 += 4 * 128) {
+        float4 v[4];      // requested before the first store, which ordinary loads would stay behind
 #pragma unroll
-        for (int i = 0; i < 4; ++i) m = max(m, magnitude(x[i]));
+        for (int u = 0; u < 4; ++u)
+          if (c0 + u * 128 < s.cols) v[u] = *reinterpret_cast<const float4*>(src + c0 + u * 128);
 #pragma unroll
-        for (int q = 0; q < kPlanes; ++q) {
-          __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[0], x[1]), __floats2bfloat162_rn(x[2], x[3])};
-          *reinterpret_cast<uint2*>(dst + q * plane + c) = *reinterpret_cast<const uint2*>(h);
-          x[0] -= __low2float(h[0]); x[1] -= __high2float(h[0]);
-          x[2] -= __low2float(h[1]); x[3] -= __high2float(h[1]);
+        for (int u = 0; u < 4; ++u) {
+          const int64_t c = c0 + u * 128;
+          if (c >= s.cols) break;
+          float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) m = max(m, magnitude(x[i]));
+#pragma unroll
+          for (int q = 0; q < kPlanes; ++q) {
+            __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x[0], x[1]), __floats2bfloat162_rn(x[2], x[3])};
+            *reinterpret_cast<uint2*>(dst + q * plane + c) = *reinterpret_cast<const uint2*>(h);
+            x[0] -= __low2float(h[0]); x[1] -= __high2float(h[0]);
+            x[2] -= __low2float(h[1]); x[3] -= __high2float(h[1]);
+          }
         }
       }
     } else {
@@ -397,13 +405,13 @@ split_planes_kernel(const Side a, const Side b, uint32_t* __restrict__ maxima) {
 // c = act(x) (x may be c itself) or c = c * act'(x), x [rows, cols], over the rows in use
 template <int V>
 __global__ void __launch_bounds__(256)
-epilogue_rows_kernel(const float* x, int64_t ldx, float* c, int64_t ldc, const int32_t* __restrict__ row_token,
-                     const int32_t* __restrict__ pad_offsets, int E, int64_t cols, int epilogue, int act) {
+epilogue_rows_kernel(const float* x, int64_t ldx, float* c, int64_t ldc, const int32_t* row_token,
+                     const int32_t* pad_offsets, int E, int64_t cols, int epilogue, int act) {
   wait_for_previous();
   const int64_t rows = pad_offsets[E], per_row = cols / V;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = i / per_row, col = (i - r * per_row) * V;
-    const bool live = row_token == nullptr || __ldg(row_token + r) >= 0;
+    const bool live = row_token == nullptr || row_token[r] >= 0;
     float xv[V], cv[V];
     if (V == 4) {
       *reinterpret_cast<float4*>(xv) = *reinterpret_cast<const float4*>(x + r * ldx + col);

@@ -41,7 +41,7 @@ template <typename T, int TILE, bool KMAJOR, bool VEC> struct Slab {
   static constexpr int kPitch = TILE + 4;
   float4 reg[kLoads];
 
-  __device__ __forceinline__ void load(const T* __restrict__ src, int64_t ld, int64_t row0, int64_t rows, int64_t k0, int64_t k_end) {
+  __device__ __forceinline__ void load(const T* src, int64_t ld, int64_t row0, int64_t rows, int64_t k0, int64_t k_end) {
 #pragma unroll
     for (int q = 0; q < kLoads; ++q) {
       const int idx = threadIdx.x + kThreads * q;
@@ -51,7 +51,7 @@ template <typename T, int TILE, bool KMAJOR, bool VEC> struct Slab {
       float v[4] = {0.f, 0.f, 0.f, 0.f};
       if (row < rows && k < k_end) {
         if (VEC) {
-          const float4 w = __ldg(reinterpret_cast<const float4*>(p));
+          const float4 w = *reinterpret_cast<const float4*>(p);
           v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
         } else {
 #pragma unroll
@@ -94,7 +94,7 @@ template <int TILE> struct Acc {
 #pragma unroll
       for (int j = 0; j < 2 * kQuads; ++j) v[i][j] = 0ull;
   }
-  __device__ __forceinline__ void step(const float* __restrict__ a, const float* __restrict__ b) {
+  __device__ __forceinline__ void step(const float* a, const float* b) {
     constexpr int P = TILE + 4;
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
@@ -128,8 +128,8 @@ template <int TILE> struct Acc {
 
 // The k loop shared by both operators: acc += A[k_begin .. k_end)^T-slabs of the two operands.
 template <typename T, int TILE, bool A_KMAJOR, bool B_KMAJOR, bool VEC>
-__device__ __forceinline__ void contract(Acc<TILE>& acc, const T* __restrict__ a, int64_t lda, int64_t a_row0, int64_t a_rows,
-                                         const T* __restrict__ b, int64_t ldb, int64_t b_row0, int64_t b_rows, int64_t k_begin,
+__device__ __forceinline__ void contract(Acc<TILE>& acc, const T* a, int64_t lda, int64_t a_row0, int64_t a_rows,
+                                         const T* b, int64_t ldb, int64_t b_row0, int64_t b_rows, int64_t k_begin,
                                          int64_t k_end) {
   __shared__ __align__(16) float As[2][BK * (TILE + 4)];
   __shared__ __align__(16) float Bs[2][BK * (TILE + 4)];
@@ -159,16 +159,16 @@ __device__ __forceinline__ void contract(Acc<TILE>& acc, const T* __restrict__ a
 }
 
 // A launch with a condition does nothing unless that word is set.
-__device__ __forceinline__ bool wanted(const int32_t* __restrict__ only_if) { return only_if == nullptr || __ldg(only_if) != 0; }
+__device__ __forceinline__ bool wanted(const int32_t* only_if) { return only_if == nullptr || *only_if != 0; }
 
 template <typename T, int TILE, bool B_NK, bool VEC>
 __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
-esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, int64_t ldb,
-                 int64_t b_estride, const void* __restrict__ bias, int64_t ldbias, T* __restrict__ aux, int64_t ldaux,
-                 T* __restrict__ c, int64_t ldc, const int32_t* __restrict__ tile_expert,
-                 const int32_t* __restrict__ pad_offsets, const int32_t* __restrict__ row_token, int E, int64_t n_out,
+esmm_simt_kernel(const T* a, int64_t lda, const T* b, int64_t ldb,
+                 int64_t b_estride, const void* bias, int64_t ldbias, T* __restrict__ aux, int64_t ldaux,
+                 T* __restrict__ c, int64_t ldc, const int32_t* tile_expert,
+                 const int32_t* pad_offsets, const int32_t* row_token, int E, int64_t n_out,
                  int64_t k, int epilogue, int act, int e_begin, int e_end, int bias16,
-                 const int32_t* __restrict__ only_if) {
+                 const int32_t* only_if) {
   wait_for_previous(false);
   if (!wanted(only_if)) return;
   const int64_t row0 = (int64_t)blockIdx.y * TILE;
@@ -227,9 +227,9 @@ esmm_simt_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ b, 
 
 template <typename T, typename TO, int TILE, bool VEC>
 __global__ void __launch_bounds__(kThreads, TILE == 128 ? 2 : 4)
-estmm_simt_kernel(const T* __restrict__ p, int64_t ldp, const T* __restrict__ q, int64_t ldq,
-                  const int32_t* __restrict__ pad_offsets, int64_t m, int64_t n, TO* __restrict__ out, int64_t ldo,
-                  int64_t o_estride, int64_t m_split, int64_t split_stride, int beta, const int32_t* __restrict__ only_if) {
+estmm_simt_kernel(const T* p, int64_t ldp, const T* q, int64_t ldq,
+                  const int32_t* pad_offsets, int64_t m, int64_t n, TO* __restrict__ out, int64_t ldo,
+                  int64_t o_estride, int64_t m_split, int64_t split_stride, int beta, const int32_t* only_if) {
   wait_for_previous(false);
   if (!wanted(only_if)) return;
   const int e = blockIdx.z;

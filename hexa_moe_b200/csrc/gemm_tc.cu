@@ -263,7 +263,7 @@ template <int CTAS>
 __device__ __forceinline__ int tile_entry(const Params& p, uint32_t t, uint32_t row_tiles) {
   const uint32_t row_tile = t / p.nt;
   if (row_tile >= row_tiles) return -1;
-  return CTAS == 2 ? __ldg(p.pair_block + row_tile) : (int)(row_tile * 2);
+  return CTAS == 2 ? p.pair_block[row_tile] : (int)(row_tile * 2);
 }
 
 template <int BN, int MODE, int CTAS, int OUT>
@@ -601,7 +601,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const uint32_t row_tiles = CTAS == 2 ? (uint32_t)p.max_pairs : (uint32_t)(p.pad_offsets[p.E] / BLOCK_M);
       uint32_t t = tile_first;
       int entry = tile_entry<CTAS>(p, t, row_tiles);
-      int e = entry >= 0 ? __ldg(p.tile_expert + (entry >> 1)) : -1;
+      int e = entry >= 0 ? p.tile_expert[entry >> 1] : -1;
       uint32_t seq = 0;             // DACT: blocks done so far; block i uses staging tile i & 1
       bool requested = false;       // DACT, leader: the block about to start has its aux load under way
       auto request_aux = [&](uint32_t block, int64_t col, int row0) {
@@ -618,8 +618,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int64_t col = (int64_t)(tile_index % p.nt) * BN + part_col + gi;
         if (p.bias == nullptr || gi >= kPartCols || col >= p.n) return 0.f;
         const int64_t at = (int64_t)expert * p.ldbias + col;
-        if (!p.bias16) return __ldg(static_cast<const float*>(p.bias) + at);
-        return unpack_lo(__ldg(static_cast<const uint16_t*>(p.bias) + at), is_bf16);
+        if (!p.bias16) return static_cast<const float*>(p.bias)[at];
+        return unpack_lo(static_cast<const uint16_t*>(p.bias)[at], is_bf16);
       };
       float bias_next = entry >= 0 && e >= 0 ? bias_of(e, t) : 0.f;
       while (ok && entry >= 0 && e >= 0) {
@@ -627,7 +627,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (OUT != OUT_DACT && p.bias != nullptr) group_sync(1 + part);
         if (gi < kPartCols) bias_s[part_col + gi] = bias_next;
         const int next = tile_entry<CTAS>(p, t_next, row_tiles);
-        const int e_next = next >= 0 ? __ldg(p.tile_expert + (next >> 1)) : -1;
+        const int e_next = next >= 0 ? p.tile_expert[next >> 1] : -1;
         if (e >= p.e_begin && e < p.e_end) {
           ++it;
           const int acc = it & 1;
@@ -774,7 +774,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // Second pass of a split ESTMM: out = beta * out + sum over chunks (in chunk order) of the fp32 partial results, stored
 // in the output's own type and layout.  One thread per four adjacent columns.
 __global__ void __launch_bounds__(256)
-estmm_reduce_kernel(const float* __restrict__ partial, int splits, int E, int64_t m, int64_t n, void* __restrict__ out, int64_t ldc,
+estmm_reduce_kernel(const float* partial, int splits, int E, int64_t m, int64_t n, void* __restrict__ out, int64_t ldc,
                     int64_t c_estride, int64_t m_split, int64_t split_stride, int out_f32, int is_bf16, int beta) {
   wait_for_previous();
   const int64_t n4 = n / 4;
@@ -784,10 +784,10 @@ estmm_reduce_kernel(const float* __restrict__ partial, int splits, int E, int64_
     const int64_t c4 = i % n4, row = i / n4;          // row = e * m + mrow
     const int64_t e = row / m, mrow = row - e * m;
     const float* src = partial + row * n + c4 * 4;
-    float4 acc = __ldg(reinterpret_cast<const float4*>(src));
+    float4 acc = *reinterpret_cast<const float4*>(src);
 #pragma unroll 4
     for (int s = 1; s < splits; ++s) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(src + (int64_t)s * plane));
+      const float4 v = *reinterpret_cast<const float4*>(src + (int64_t)s * plane);
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     const int64_t off = (mrow / m_split) * split_stride + e * c_estride + (mrow % m_split) * ldc + c4 * 4;

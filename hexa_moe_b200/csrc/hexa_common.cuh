@@ -119,6 +119,9 @@ constexpr int kRowTile = 128;  // rows per GEMM tile == required segment alignme
 // blocks that keep an SM busy: the blocks of an early start go to the SMs that are free first, and a few of them get most of the work
 // (fp32 FMA GEMMs of [4096, 512 x 128]: 30 us each on their own, 45 to 80 us so).  Such kernels are not started early either.
 // Without an early launch both instructions do nothing.
+// What such a kernel reads may be written while it is already resident, so it is no read-only data: inputs are read by ordinary
+// loads, which stay behind the wait, through pointers that are not const __restrict__, and never by __ldg, which the compiler
+// may move ahead of it and whose cache need not see the writes.  (Outputs are __restrict__, so that loads can pass stores.)
 __device__ __forceinline__ void wait_for_previous(bool next_may_start = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (next_may_start) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

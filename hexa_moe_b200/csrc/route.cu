@@ -29,7 +29,7 @@ __device__ __forceinline__ int load_id(const int32_t* ids, int64_t f, int64_t T,
   return ids[t * stride_t + j * stride_k];
 }
 
-__global__ void route_hist(const int32_t* __restrict__ ids, int64_t T, int64_t n_rows, int64_t stride_t,
+__global__ void route_hist(const int32_t* ids, int64_t T, int64_t n_rows, int64_t stride_t,
                            int64_t stride_k, int E, int32_t* __restrict__ chunk_hist) {
   wait_for_previous();
   extern __shared__ int32_t sm[];
@@ -149,9 +149,9 @@ route_scan(int32_t* __restrict__ chunk_hist, int64_t n_chunks, int E, int align,
   }
 }
 
-__global__ void route_scatter(const int32_t* __restrict__ ids, int64_t T, int top_k, int64_t n_rows, int64_t stride_t,
-                              int64_t stride_k, int E, const int32_t* __restrict__ chunk_base,
-                              const int32_t* __restrict__ pad_offsets, int32_t* __restrict__ row_token,
+__global__ void route_scatter(const int32_t* ids, int64_t T, int top_k, int64_t n_rows, int64_t stride_t,
+                              int64_t stride_k, int E, const int32_t* chunk_base,
+                              const int32_t* pad_offsets, int32_t* __restrict__ row_token,
                               int32_t* __restrict__ token_row) {
   wait_for_previous();
   extern __shared__ int32_t sm[];
@@ -204,7 +204,7 @@ struct Ids {
   __device__ __forceinline__ int at(uint32_t f, uint32_t& t, uint32_t& j) const {
     j = f / T;
     t = f - j * T;
-    const int e = __ldg(p + (int64_t)t * stride_t + (int64_t)j * stride_k);
+    const int e = p[(int64_t)t * stride_t + (int64_t)j * stride_k];
     return e >= 0 && e < E ? e : -1;
   }
 };
@@ -249,7 +249,7 @@ __device__ __forceinline__ int owner(const int32_t* offs, int E, int32_t x) {
 // totals: one histogram per block, or null when this is the only block
 template <int WARPS, int ITERS>
 __global__ void __launch_bounds__(WARPS * 32)
-route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const int32_t* __restrict__ totals, Tables out) {
+route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const int32_t* totals, Tables out) {
   wait_for_previous();
   extern __shared__ int32_t sm[];
   const int E = ids.E;
@@ -286,7 +286,7 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
       int b_sum = 0, a_sum = 0;
 #pragma unroll 8
       for (int b = x / E; b < (int)gridDim.x; b += slices) {
-        const int v = __ldg(totals + (int64_t)b * E + ex);
+        const int v = totals[(int64_t)b * E + ex];
         a_sum += v;
         b_sum += b < (int)blockIdx.x ? v : 0;
       }
@@ -392,18 +392,18 @@ route_place(Ids ids, int top_k, uint32_t n_rows, uint32_t rows_per_warp, const i
 // does, and an entry outside [-(num_toks + 1), num_toks] is an error: it writes nothing and leaves a code in the status word.
 template <typename I>
 __global__ void __launch_bounds__(256)
-ids_from_lists_kernel(const I* __restrict__ tok_ids, const int32_t* __restrict__ exp_ids, int64_t n, int chunk, int64_t num_toks,
+ids_from_lists_kernel(const I* tok_ids, const int32_t* exp_ids, int64_t n, int chunk, int64_t num_toks,
                       int32_t* __restrict__ ids, int32_t* status) {
   wait_for_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int64_t slot = (int64_t)__ldg(tok_ids + i);
+  int64_t slot = (int64_t)tok_ids[i];
   if (slot > num_toks || slot < -(num_toks + 1)) {
     report_status(status, kStatusBadToken);
     return;
   }
   if (slot < 0) slot += num_toks + 1;
-  if (slot > 0) ids[slot - 1] = __ldg(exp_ids + i / chunk);
+  if (slot > 0) ids[slot - 1] = exp_ids[i / chunk];
 }
 
 // 1, 2 or 3 launches, see the head of this file

@@ -12,9 +12,11 @@ namespace hexa {
 namespace {
 
 // ---- gather: warp per sorted row, 16-byte vectors ---------------------------------------------
+// Here and below, what a thread reads in several steps it requests before its first store: the loads are ordinary ones (see
+// wait_for_previous), which the compiler leaves behind a store.
 template <int VEC_BYTES>
-__global__ void gather_rows_kernel(const uint8_t* __restrict__ src, int64_t src_ld_bytes,
-                                   const int32_t* __restrict__ row_token, const int32_t* __restrict__ pad_offsets,
+__global__ void gather_rows_kernel(const uint8_t* src, int64_t src_ld_bytes,
+                                   const int32_t* row_token, const int32_t* pad_offsets,
                                    int E, int64_t row_bytes, uint8_t* __restrict__ dst, int64_t dst_ld_bytes) {
   wait_for_previous();
   const int64_t n_pad = pad_offsets[E];
@@ -27,7 +29,15 @@ __global__ void gather_rows_kernel(const uint8_t* __restrict__ src, int64_t src_
     const int64_t n = row_bytes >> 4;
     if (tok >= 0) {
       const uint4* s = reinterpret_cast<const uint4*>(src + (int64_t)tok * src_ld_bytes);
-      for (int64_t i = lane; i < n; i += 32) reinterpret_cast<uint4*>(d)[i] = __ldg(s + i);
+      for (int64_t i = lane; i < n; i += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i + 32 * u < n) v[u] = s[i + 32 * u];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i + 32 * u < n) reinterpret_cast<uint4*>(d)[i + 32 * u] = v[u];
+      }
     } else {
       for (int64_t i = lane; i < n; i += 32) reinterpret_cast<uint4*>(d)[i] = make_uint4(0, 0, 0, 0);
     }
@@ -43,7 +53,7 @@ __global__ void gather_rows_kernel(const uint8_t* __restrict__ src, int64_t src_
 // chunk are issued together before anything is added (the adds keep the order j = 0..K-1, so the result does not
 // depend on K being a template parameter).  K = 0: any top_k.
 template <typename T, int K>
-__global__ void combine_rows_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ token_row,
+__global__ void combine_rows_kernel(const T* src, int64_t src_ld, const int32_t* token_row,
                                     int64_t num_tokens, int top_k, int64_t cols, T* __restrict__ dst, int64_t dst_ld) {
   wait_for_previous();
   constexpr int V = 16 / sizeof(T);
@@ -55,15 +65,16 @@ __global__ void combine_rows_kernel(const T* __restrict__ src, int64_t src_ld, c
     const T* rows[K > 0 ? K : 1];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const int32_t r = __ldg(token_row + t * K + j);
+      const int32_t r = token_row[t * K + j];
       rows[j] = r >= 0 ? src + (int64_t)r * src_ld : nullptr;
     }
-#pragma unroll 2
-    for (int64_t c = (int64_t)lane * V; c < cols; c += 32 * V) {
-      uint4 raw[K > 0 ? K : 1];
+    using Raw = uint4[K > 0 ? K : 1];
+    auto load = [&](int64_t c, Raw& raw) {
 #pragma unroll
       for (int j = 0; j < K; ++j)
-        raw[j] = rows[j] ? __ldg(reinterpret_cast<const uint4*>(rows[j] + c)) : make_uint4(0, 0, 0, 0);
+        raw[j] = rows[j] ? *reinterpret_cast<const uint4*>(rows[j] + c) : make_uint4(0, 0, 0, 0);
+    };
+    auto add = [&](int64_t c, const Raw& raw) {
       float acc[V];
 #pragma unroll
       for (int i = 0; i < V; ++i) acc[i] = 0.f;
@@ -80,6 +91,21 @@ __global__ void combine_rows_kernel(const T* __restrict__ src, int64_t src_ld, c
 #pragma unroll
       for (int i = 0; i < V; ++i) o[i] = from_f32<T>(acc[i]);
       *reinterpret_cast<uint4*>(dst + t * dst_ld + c) = outv;
+    };
+    int64_t c = (int64_t)lane * V;
+    if (K <= 2) {      // two column chunks at a time; four rows of one are as many loads
+      for (; c + 32 * V < cols; c += 64 * V) {
+        Raw a, b;
+        load(c, a);
+        load(c + 32 * V, b);
+        add(c, a);
+        add(c + 32 * V, b);
+      }
+    }
+    for (; c < cols; c += 32 * V) {
+      Raw a;
+      load(c, a);
+      add(c, a);
     }
   } else if (vec_ok) {
     for (int64_t c = (int64_t)lane * V; c < cols; c += 32 * V) {
@@ -89,7 +115,7 @@ __global__ void combine_rows_kernel(const T* __restrict__ src, int64_t src_ld, c
       for (int j = 0; j < top_k; ++j) {
         const int32_t r = token_row[t * top_k + j];
         if (r < 0) continue;
-        uint4 raw = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)r * src_ld + c));
+        uint4 raw = *reinterpret_cast<const uint4*>(src + (int64_t)r * src_ld + c);
         const T* v = reinterpret_cast<const T*>(&raw);
 #pragma unroll
         for (int i = 0; i < V; ++i) acc[i] += to_f32<T>(v[i]);
@@ -129,8 +155,8 @@ void combine_launch(const void* src, int64_t src_ld, const int32_t* token_row, i
 }
 
 // ---- mask: zero the pad rows of a sorted buffer -------------------------------------------------
-__global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes, const int32_t* __restrict__ row_token,
-                                     const int32_t* __restrict__ pad_offsets, int E, int64_t row_bytes) {
+__global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes, const int32_t* row_token,
+                                     const int32_t* pad_offsets, int E, int64_t row_bytes) {
   wait_for_previous();
   const int64_t n_pad = pad_offsets[E];
   const int lane = threadIdx.x & 31;
@@ -141,16 +167,16 @@ __global__ void mask_pad_rows_kernel(uint8_t* __restrict__ buf, int64_t ld_bytes
 }
 
 // ---- ESS pass 1: column sums of one 128-row tile (one expert) ------------------------------------
-// block = 32 column groups x 4 row groups; a thread sums 32 rows (r mod 4) of V adjacent columns, all loads in flight, and
+// block = 32 column groups x 4 row groups; a thread sums 32 rows (r mod 4) of V adjacent columns, eight loads ahead of its stores, and
 // the four sums are added in order.  The order is part of the result: a bias gradient is rounded to 16 bits from it.  Eight
-// row groups of 16 rows, eight loads in flight, took 400 us with the gather at [262144, 2048] where this takes 348, and 110
-// us where this takes 95 at [131072, 1024]; below a few thousand rows they were 1-4 us faster (a longer chain per thread).
+// row groups of 16 rows, eight loads in flight, took 400 us with the gather at [262144, 2048] where this takes 342, and 110
+// us where this takes 89 at [131072, 1024]; below a few thousand rows they were 1-4 us faster (a longer chain per thread).
 // GATHER: the rows come from src[row_token[row]] (zeros for pad rows) and are written to dst as well.
 constexpr int kEssCx = 32, kEssRy = 4;
 template <typename T, bool GATHER>
 __global__ void __launch_bounds__(kEssCx * kEssRy)
-ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __restrict__ row_token,
-                   const int32_t* __restrict__ pad_offsets, int E, int64_t cols, T* __restrict__ dst, int64_t dst_ld,
+ess_partial_kernel(const T* src, int64_t src_ld, const int32_t* row_token,
+                   const int32_t* pad_offsets, int E, int64_t cols, T* __restrict__ dst, int64_t dst_ld,
                    float* __restrict__ partial) {
   wait_for_previous();
   constexpr int V = 16 / sizeof(T);
@@ -160,7 +186,7 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
   const int64_t row0 = (int64_t)blockIdx.y * kRowTile;
   if (row0 >= n_pad) return;
   if (GATHER) {
-    for (int i = threadIdx.x; i < kRowTile; i += kEssCx * kEssRy) tok_s[i] = __ldg(row_token + row0 + i);
+    for (int i = threadIdx.x; i < kRowTile; i += kEssCx * kEssRy) tok_s[i] = row_token[row0 + i];
     __syncthreads();
   }
   const int cx = threadIdx.x & (kEssCx - 1), ry = threadIdx.x / kEssCx;
@@ -171,19 +197,28 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
   if (col < cols) {
     const bool vec_ok = GATHER || ((col + V <= cols) && (src_ld % V == 0));      // GATHER: checked by the host
     if (vec_ok) {
-#pragma unroll 32
-      for (int r = ry; r < kRowTile; r += kEssRy) {
-        uint4 raw = make_uint4(0, 0, 0, 0);
-        if (GATHER) {
-          const int32_t tok = tok_s[r];
-          if (tok >= 0) raw = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)tok * src_ld + col));
-          *reinterpret_cast<uint4*>(dst + (row0 + r) * dst_ld + col) = raw;
-        } else {
-          raw = __ldg(reinterpret_cast<const uint4*>(src + (row0 + r) * src_ld + col));
-        }
-        const T* v = reinterpret_cast<const T*>(&raw);
+      constexpr int kRows = 8;      // at a time
+#pragma unroll(GATHER ? 1 : kRowTile / (kRows * kEssRy))
+      for (int r0 = ry; r0 < kRowTile; r0 += kRows * kEssRy) {
+        uint4 raw[kRows];
 #pragma unroll
-        for (int i = 0; i < V; ++i) acc[i] += to_f32<T>(v[i]);
+        for (int u = 0; u < kRows; ++u) {
+          const int r = r0 + u * kEssRy;
+          raw[u] = make_uint4(0, 0, 0, 0);
+          if (GATHER) {
+            const int32_t tok = tok_s[r];
+            if (tok >= 0) raw[u] = *reinterpret_cast<const uint4*>(src + (int64_t)tok * src_ld + col);
+          } else {
+            raw[u] = *reinterpret_cast<const uint4*>(src + (row0 + r) * src_ld + col);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) {
+          if (GATHER) *reinterpret_cast<uint4*>(dst + (row0 + r0 + u * kEssRy) * dst_ld + col) = raw[u];
+          const T* v = reinterpret_cast<const T*>(&raw[u]);
+#pragma unroll
+          for (int i = 0; i < V; ++i) acc[i] += to_f32<T>(v[i]);
+        }
       }
     } else {
       for (int r = ry; r < kRowTile; r += kEssRy) {
@@ -215,7 +250,7 @@ ess_partial_kernel(const T* __restrict__ src, int64_t src_ld, const int32_t* __r
 constexpr int kFinalTiles = 64;
 template <typename TO>
 __global__ void __launch_bounds__(256)
-ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ pad_offsets,
+ess_final_kernel(const float* partial, const int32_t* pad_offsets,
                  int64_t cols, TO* __restrict__ out, int64_t ldo) {
   wait_for_previous();
   __shared__ float rows[kFinalTiles][32];
@@ -224,7 +259,7 @@ ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ 
   const int64_t c = (int64_t)blockIdx.x * 32 + cx;
   const int64_t t0 = pad_offsets[e] / kRowTile, t1 = pad_offsets[e + 1] / kRowTile;
   if (t1 - t0 <= 8) {      // a tile per warp
-    rows[slice][cx] = c < cols && t0 + slice < t1 ? __ldg(partial + (t0 + slice) * cols + c) : 0.f;
+    rows[slice][cx] = c < cols && t0 + slice < t1 ? partial[(t0 + slice) * cols + c] : 0.f;
     __syncthreads();
     if (slice == 0 && c < cols) {
       float s = 0.f;
@@ -238,7 +273,7 @@ ess_final_kernel(const float* __restrict__ partial, const int32_t* __restrict__ 
 #pragma unroll
     for (int i = 0; i < kFinalTiles / 8; ++i) {
       const int64_t t = base + slice + 8 * i;
-      next[i] = c < cols && t < t1 ? __ldg(partial + t * cols + c) : 0.f;
+      next[i] = c < cols && t < t1 ? partial[t * cols + c] : 0.f;
     }
   };
   fetch(t0);

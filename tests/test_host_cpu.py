@@ -388,3 +388,18 @@ def test_direct_gate_projection_steps_aside_for_whoever_watches_the_linear():
     assert seen[-1]
     torch.autograd.grad(Twice.apply(t), t, torch.ones(3))
     assert not seen[-1]
+
+
+def test_kernels_that_start_early_read_by_ordinary_loads():
+    """A kernel that may be resident while the one before it writes has no read-only inputs: a load marked so (__ldg, or through
+    a const __restrict__ pointer) may be moved ahead of the wait for the kernel before."""
+    import glob
+    files = glob.glob(os.path.join(ROOT, "hexa_moe_b200", "csrc", "*.cu*"))
+    early = [f for f in files if "wait_for_previous(" in open(f).read()]
+    assert len(early) >= 7
+    for f in early:
+        code = re.sub(r"//.*", "", open(f).read())
+        marked = re.findall(r"__ldg\(|const\s+[\w ]+\*\s*__restrict__", code)
+        assert not marked, (os.path.basename(f), len(marked))
+    for f in set(files) - set(early):      # and the others are not launched early
+        assert "after_previous" not in open(f).read() and "ProgrammaticStreamSerialization" not in open(f).read(), f
