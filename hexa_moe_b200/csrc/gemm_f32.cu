@@ -60,6 +60,7 @@ struct Params {
   int debug;      // test aid (hexa_set_tc_debug): bit 2 = the producer neither loads nor arrives, every wait runs into its limit
   int32_t* status;
   uint64_t wait_limit_ns;
+  bool next_may_start;                  // no SM limit is set, see wait_for_previous
 };
 
 struct Tile {
@@ -140,7 +141,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  wait_for_previous();
+  wait_for_previous(p.next_may_start);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (every CTA)
@@ -582,7 +583,7 @@ int esmm_f32_launch(const void* a, int64_t lda, const void* b, int b_layout, int
   p.max_pairs = row_cap / (2 * BLOCK_M) + E;
   p.bias = bias; p.ldbias = ldbias; p.n = n_out; p.k = k; p.E = E;
   p.nt = (uint32_t)ceil_div(n_out, BLOCK_N);
-  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns(); p.next_may_start = sm_limit() == 0;
   HEXA_REQUIRE((row_cap / BLOCK_M + E + 1) * (int64_t)p.nt < (int64_t)0x7fffffff, "hexa_esmm: too many output tiles for a 32-bit tile index");
   const int64_t max_tiles = p.max_pairs * (int64_t)p.nt;
   rc = nk ? launch<NK>(tmA, tmB, tmC, p, max_tiles, stream) : launch<KN>(tmA, tmB, tmC, p, max_tiles, stream);
@@ -623,7 +624,7 @@ int estmm_f32_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, co
   HEXA_REQUIRE(per_expert * E < (int64_t)0x7fffffff, "hexa_estmm: too many output tiles for a 32-bit tile index");
   p.per_expert = (uint32_t)per_expert;
   p.total_tiles = (uint32_t)(per_expert * E);
-  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns(); p.next_may_start = sm_limit() == 0;
   rc = launch<TN>(tmA, tmB, tmC, p, per_expert * E, stream);
   if (rc) return rc;
   return estmm_simt_launch(pp, ldp, q, ldq, pad_offsets, E, m, n, out, ldo, o_estride, m, 0, HEXA_F32, HEXA_F32, 0, stream, p.redo);

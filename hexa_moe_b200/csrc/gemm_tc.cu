@@ -102,6 +102,7 @@ struct Params {
                     // pre-activation is not requested, so that the waits behind them run into their limit
   int32_t* status;
   uint64_t wait_limit_ns;   // limit of every mbarrier wait (hexa_set_wait_limit_ns; default 2 s)
+  bool next_may_start;      // no SM limit is set, see wait_for_previous
 };
 
 // What the epilogue does with an accumulator.  ESMM: HEXA_EPI_LINEAR / HEXA_EPI_ACT / HEXA_EPI_DACT; ESTMM: stores from
@@ -320,7 +321,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (CTAS == 2) cluster_sync_all();   // the peer's barriers exist before anything is sent to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  wait_for_previous();
+  wait_for_previous(p.next_may_start);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (every CTA)
@@ -1000,7 +1001,7 @@ int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int6
   p.bias = bias; p.ldbias = ldbias; p.bias16 = bias16; p.aux = aux; p.ldaux = ldaux; p.c = c; p.ldc = ldc;
   p.n = n_out; p.k = k; p.m = 0; p.E = E; p.e_begin = e_begin; p.e_end = e_end;
   p.epilogue = epilogue; p.act = act; p.is_bf16 = is_bf16; p.colsum = colsum;
-  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns(); p.next_may_start = sm_limit() == 0;
   const int64_t NT = ceil_div(n_out, BN);
   HEXA_REQUIRE((row_cap / BLOCK_M + E + 1) * NT < (int64_t)0x7fffffff, "hexa_esmm: too many output tiles for a 32-bit tile index");
   p.nt = (uint32_t)NT;
@@ -1104,7 +1105,7 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   for (int i = 0; i < n_split && i < 16; ++i) p.c_split[i] = split_out[i];
   p.is_bf16 = is_bf16; p.out_f32 = out_dtype == HEXA_F32; p.beta = beta;
   p.splits = splits; p.chains = splits > 1 ? plan.chains : 1;
-  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns();
+  p.status = status_word(); p.debug = tc_debug_flags(); p.wait_limit_ns = wait_limit_ns(); p.next_may_start = sm_limit() == 0;
   const int64_t max_tiles = (int64_t)E * ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN) * splits;
   HEXA_REQUIRE(max_tiles < (int64_t)0x7fffffff, "hexa_estmm: too many output tiles for a 32-bit tile index");
   p.nt = (uint32_t)ceil_div(n, BN);

@@ -118,6 +118,7 @@ constexpr int kRowTile = 128;  // rows per GEMM tile == required segment alignme
 // to set up, so that at most two kernels share the SMs; or (next_may_start false) not before this one ends, for kernels of many
 // blocks that keep an SM busy: the blocks of an early start go to the SMs that are free first, and a few of them get most of the work
 // (fp32 FMA GEMMs of [4096, 512 x 128]: 30 us each on their own, 45 to 80 us so).  Such kernels are not started early either.
+// Nor while a persistent GEMM keeps off some SMs (sm_limit): an early start would take up those that it leaves to other streams.
 // Without an early launch both instructions do nothing.
 // What such a kernel reads may be written while it is already resident, so it is no read-only data: inputs are read by ordinary
 // loads, which stay behind the wait, through pointers that are not const __restrict__, and never by __ldg, which the compiler

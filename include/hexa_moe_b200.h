@@ -107,7 +107,8 @@ int hexa_set_tc_debug(int flags);
 
 /* Cap on the SMs the persistent GEMM kernels occupy from now on (process-wide; 0 = all SMs).  Their tile
  * schedule is static, so they should not share SMs with long-running kernels of other streams (collectives):
- * set a cap while such kernels may be running.  No counterpart in the reference. */
+ * set a cap while such kernels may be running.  What follows a capped GEMM in its stream starts when that one has ended,
+ * so the SMs left free stay free.  No counterpart in the reference. */
 int hexa_set_sm_limit(int num_sms);
 
 /* ---- routing: replaces launch_count + launch_assign (include/hexa_moe.h:3-22,

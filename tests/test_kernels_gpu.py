@@ -745,3 +745,41 @@ def test_few_rows_take_small_tiles(ops, T, E, n, k):
         for epilogue in (Lb.EPI_LINEAR, Lb.EPI_ACT, Lb.EPI_DACT):
             a, c = both(layout, wgt, epilogue)
             assert all(torch.equal(u, v) for u, v in zip(a, c)), (layout, epilogue)
+
+
+@pytest.mark.parametrize("dtype,T", [(torch.bfloat16, 131072), (torch.float32, 32768)])
+def test_sms_left_free_stay_free(ops, dtype, T):
+    """With an SM limit, the kernels that follow a GEMM in its stream do not take up the SMs that it leaves to other streams: a
+    kernel of another stream that becomes ready in the first of two GEMMs runs then, not behind it."""
+    from hexa_moe_b200 import _lib as L
+    d = 4096
+    r = ops.route(torch.zeros(T, 1, dtype=torch.int32, device="cuda"), 1)
+    xs = torch.randn(r.row_capacity, d, dtype=dtype, device="cuda")
+    w = torch.randn(1, d, d, dtype=dtype, device="cuda")
+    out = torch.empty_like(xs)
+    host, dev = torch.empty(4 << 20, dtype=torch.float32).pin_memory(), torch.empty(4 << 20, device="cuda")
+    small = torch.zeros(64, device="cuda")
+    side = torch.cuda.Stream()
+    start, ran, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+
+    def both():
+        torch.cuda._sleep(2_000_000)                  # the host is ahead of the device
+        start.record()
+        for _ in range(2):
+            ops.esmm(xs, w, L.B_NK, r, out=out)
+        end.record()
+        with torch.cuda.stream(side):                 # a copy engine's work, then a kernel
+            side.wait_event(start)
+            dev.copy_(host, non_blocking=True)
+            small.add_(1)
+            ran.record(side)
+        torch.cuda.synchronize()
+        return start.elapsed_time(ran) / start.elapsed_time(end)
+
+    try:
+        L.lib().hexa_set_sm_limit(torch.cuda.get_device_properties(0).multi_processor_count - 16)
+        both()
+        share = min(both() for _ in range(3))
+    finally:
+        L.lib().hexa_set_sm_limit(0)
+    assert share < 0.4, share                         # behind the first GEMM: at least half
