@@ -935,17 +935,23 @@ bool esmm_tc_supported(const void* a, int64_t lda, const void* b, int64_t ldb, i
 // two 128-row blocks of one expert: where experts have one block, or where there are fewer pair tiles than pairs, half of the SMs'
 // work is for nothing, while the small tiles load an operand value twice as often.  Waves of either are estimated from static sizes
 // (experts of up to 96 rows on average have one block, larger ones half a block or pair more than the rows fill), a wave of small
-// tiles at 0.8 of a wave of pairs (measured 0.7 - 0.9; 0.6 with long rows of tiles).  Pairs / small tiles, us (fc1 + GELU, fc2):
+// tiles at 0.8 of a wave of pairs (measured 0.7 - 0.9; 0.6 with long rows of tiles, some of which
+// one factor for all leaves with pairs although small tiles would be a little faster).  A launch of some experts has their share of the rows, and a cap on the SMs makes its
+// waves.  Pairs / small tiles, us (fc1 + GELU, fc2):
 //   300 rows x 1 [4096x1024] 15 24 / 11 23   16 x 32 [4096x1024] 34 29 / 31 26     700 x 7 [800x200] 14 13 / 9 9
 //   1024 x 8 [3072x768] 21 20 / 17 19        2048 x 32 [4096x1024] 69 59 / 65 53   4096 x 64 [1024x256] 37 14 / 21 11
 // and where the rule stays with pairs: 4608 x 32 [4096x1024] 79 65 / 103 86        4096 x 8 [3072x768] 34 22 / 39 34
 //   18432 x 1 [2048x512] 58 32 / 69 46       4000 x 32 [4096x1024] 75 63 / 81 69   500 x 4 [4096x1024] (fc1) 20 / 19
 // (128 x 256 tiles of one CTA were between the two at nearly all of these).
-bool small_tiles(int E, int64_t row_cap, int64_t n_out) {
-  const double rows = (double)(row_cap > 127 * (int64_t)E ? row_cap - 127 * (int64_t)E : 1), met = rows < E ? rows : E, avg = rows / E;
+bool small_tiles(int E, int e_begin, int e_end, int64_t row_cap, int64_t n_out) {
+  const int experts = (e_end < E ? e_end : E) - (e_begin > 0 ? e_begin : 0);
+  if (experts <= 0) return false;
+  const double all = (double)(row_cap > 127 * (int64_t)E ? row_cap - 127 * (int64_t)E : 1), rows = all * experts / E;
+  const double met = rows < experts ? rows : experts, avg = all / E;
   const double blocks = met * (avg <= 96 ? 1.0 : avg / 128 + 0.5), pairs = met * (avg <= 128 ? 1.0 : avg / 256 + 0.5);
-  const int64_t small_waves = ceil_div((int64_t)blocks * ceil_div(n_out, 128), sm_count());
-  const int64_t pair_waves = ceil_div((int64_t)pairs * ceil_div(n_out, 256), sm_count() / 2);
+  const int sms = sm_limit() > 1 && sm_limit() < sm_count() ? sm_limit() : sm_count();
+  const int64_t small_waves = ceil_div((int64_t)blocks * ceil_div(n_out, 128), sms);
+  const int64_t pair_waves = ceil_div((int64_t)pairs * ceil_div(n_out, 256), sms / 2);
   return 0.8 * (double)small_waves < (double)pair_waves;
 }
 
@@ -956,7 +962,7 @@ int esmm_tc_launch(const void* a, int64_t lda, const void* b, int b_layout, int6
                    int act, cudaStream_t stream, int e_begin, int e_end, int bias16, float* colsum) {
   if (row_cap == 0 || e_begin >= e_end) return HEXA_OK;
   const int is_bf16 = dtype == HEXA_BF16;
-  const bool pairs = n_out > 128 && pair_block != nullptr && pairs_enabled() && !small_tiles(E, row_cap, n_out);
+  const bool pairs = n_out > 128 && pair_block != nullptr && pairs_enabled() && !small_tiles(E, e_begin, e_end, row_cap, n_out);
   const int BN = pairs || (n_out > 128 && (pair_block == nullptr || !pairs_enabled())) ? 256 : 128;
   const int ctas = pairs ? 2 : 1;
   CUtensorMap tmA, tmB;

@@ -783,3 +783,34 @@ def test_sms_left_free_stay_free(ops, dtype, T):
     finally:
         L.lib().hexa_set_sm_limit(0)
     assert share < 0.4, share                         # behind the first GEMM: at least half
+
+
+@pytest.mark.parametrize("T,E,n,limit,experts,small", [
+    (2048, 8, 1536, 0, (0, 8), False), (2048, 8, 1536, 132, (0, 8), True),            # a cap on the SMs
+    (4608, 32, 1024, 0, (0, 32), False), (4608, 32, 1024, 0, (8, 16), True),          # some of the experts
+    (2048, 32, 1024, 0, (0, 32), True), (2048, 32, 1024, 1, (0, 32), True),           # a cap that leaves no pair
+])
+def test_small_tiles_follow_the_launch(ops, T, E, n, limit, experts, small):
+    """Waves of small tiles and of pairs are those of the SMs and the experts that a launch has; results are the same bit for bit."""
+    from torch.profiler import ProfilerActivity, profile
+    from hexa_moe_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(T)
+    r = ops.route(torch.randint(0, E, (T, 1), generator=g, device="cuda").to(torch.int32), E)
+    xs = ops.gather_rows(torch.randn(T, 128, generator=g, device="cuda").bfloat16(), r)
+    w = torch.randn(E, n, 128, generator=g, device="cuda").bfloat16()
+    n_pad = int(r.pad_offsets[-1])
+    rows = slice(int(r.pad_offsets[experts[0]]), int(r.pad_offsets[experts[1]]))
+    want = ops.esmm(xs, w, L.B_NK, r)
+    try:
+        L.lib().hexa_set_sm_limit(limit)
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            got = ops.esmm(xs, w, L.B_NK, r, experts=experts)
+            torch.cuda.synchronize()
+    finally:
+        L.lib().hexa_set_sm_limit(0)
+    assert rows.stop <= n_pad and torch.equal(got[rows], want[rows])
+    names = [e.key for e in prof.key_averages() if "gemm_tc_kernel<" in e.key]
+    if not names:
+        pytest.skip("no kernel records on this machine")
+    ctas = int(names[0].split("gemm_tc_kernel<")[1].split(",")[2])
+    assert (ctas == 1) == small, names
