@@ -394,7 +394,7 @@ class MoE_Cascaded(torch.nn.Module):
 
         if not is_moe:
             y = MLP_Implement.apply(cfg, x, _entry(self.mlp_fc1_w, i_mlp), _entry(self.mlp_fc2_w, i_mlp), _entry(self.mlp_fc1_b, i_mlp),
-                                    _entry(self.mlp_fc2_b, i_mlp)).to(x.dtype)
+                                    _entry(self.mlp_fc2_b, i_mlp), torch.is_grad_enabled()).to(x.dtype)
             y = y.view(list(original_shape[:-reserve_dims]) + list(y.shape[-reserve_dims:])).to(original_dtype)
             return (self.result_func(y) if self.result_func is not None else y), 0
 
@@ -413,7 +413,7 @@ class MoE_Cascaded(torch.nn.Module):
         b2 = _entry(self.batched_fc2_bias, i_moe) if self.has_fc2_bias else None
         y = self._one_gpu_layer(cfg, x, w1, w2, b1, b2)
         if y is None:
-            y = FusedMoE_Shared_CudaCore.apply(cfg, x, w1, w2, b1, b2)
+            y = FusedMoE_Shared_CudaCore.apply(cfg, x, w1, w2, b1, b2, torch.is_grad_enabled())
         y = y.to(x.dtype)
         if not flat:
             y = y.view(list(original_shape[:-reserve_dims]) + list(y.shape[-reserve_dims:]))

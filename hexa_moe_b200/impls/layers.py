@@ -7,7 +7,9 @@ Function-level contract of the reference (hexa_moe/impls/layers.py:18-478), kept
     MLP_Implement.apply(config, x[T,d], fc1_w[H,d], fc2_w[H,d_out], fc1_b[H] | None, fc2_b[d_out] | None)
 
 `config.indices_` carries the k routing-id vectors out of band and `config.stage` selects the MoE
-layer; backward returns gradients shaped like the inputs and decrements `config.stage`.
+layer; backward returns gradients shaped like the inputs and decrements `config.stage`.  A last argument, `keep`
+(default True), is False where no backward pass can follow (no_grad, inference): inside a Function the parameters count as
+wanting gradients in any mode, and what only a backward pass reads would be written for nothing.
 
 Differences from the reference, all deliberate:
   * the expert math runs through `config.backend` (hexa_moe_b200.ops: the sm_100a kernels behind
@@ -268,7 +270,7 @@ class MLP_Implement(torch.autograd.Function):
     averaged over the data-parallel ranks inside backward (reference layers.py:18-88)."""
 
     @staticmethod
-    def forward(ctx: Any, config: Any, tokens_input: Tensor, fc1_w, fc2_w, fc1_bias, fc2_bias):
+    def forward(ctx: Any, config: Any, tokens_input: Tensor, fc1_w, fc2_w, fc1_bias, fc2_bias, keep=True):
         ctx.config = config
         assert tokens_input.shape[1] == fc1_w.shape[1] and fc1_w.shape[0] == fc2_w.shape[0]
         if getattr(config, "dense_reducer", None) is not None:
@@ -282,7 +284,7 @@ class MLP_Implement(torch.autograd.Function):
             w1, w2 = _unit_rows(_cast(fc1_w.detach(), dtype)), _unit_rows(_cast(fc2_w.detach(), dtype))
             y, st = config.backend.dense_forward(x, w1, w2, None if fc1_bias is None else fc1_bias.detach(),
                                                  None if fc2_bias is None else fc2_bias.detach(), config.act_id,
-                                                 need_state=any(ctx.needs_input_grad))
+                                                 need_state=keep and any(ctx.needs_input_grad))
             ctx.kept = None
             if x.shape[1] >= _DENSE_WIDE:
                 ctx.kept = (st, w1, w2)
@@ -345,11 +347,11 @@ class MLP_Implement(torch.autograd.Function):
         if _world(cfg.group) > 1 and reducer is not None and os.environ.get("HEXA_DEFER_GRADS", "1") != "0":
             # bucketed, on a side stream, delivered to .grad when the backward pass ends (see DenseGradReducer)
             reducer.add(list(zip(ctx.params, (dw1, dw2, db1, db2))))
-            return None, dx, None, None, None, None
+            return None, dx, None, None, None, None, None
         for g in (dw2, db2, dw1, db1):
             if g is not None:
                 all_reduce_avg(g, cfg.group)
-        return None, dx, dw1, dw2, db1, db2
+        return None, dx, dw1, dw2, db1, db2, None
 
 
 # ------------------------------------------------------------------------------------------------
@@ -358,7 +360,7 @@ class MLP_Implement(torch.autograd.Function):
 class FusedMoE_Shared_CudaCore(torch.autograd.Function):
 
     @staticmethod
-    def forward(ctx: Any, config: Any, tokens_input: Tensor, fc1_w, fc2_w, fc1_bias, fc2_bias):
+    def forward(ctx: Any, config: Any, tokens_input: Tensor, fc1_w, fc2_w, fc1_bias, fc2_bias, keep=True):
         cfg = config
         ctx.config = cfg
         stage = cfg.stage
@@ -372,7 +374,7 @@ class FusedMoE_Shared_CudaCore(torch.autograd.Function):
         ctx.has_b1, ctx.has_b2 = fc1_bias is not None, fc2_bias is not None
         ctx.param_dtypes = (fc1_w.dtype, fc2_w.dtype,
                             None if fc1_bias is None else fc1_bias.dtype, None if fc2_bias is None else fc2_bias.dtype)
-        need_state = any(ctx.needs_input_grad)
+        need_state = keep and any(ctx.needs_input_grad)
 
         if cfg.data_centric:
             if W > 1:
@@ -516,4 +518,4 @@ class FusedMoE_Shared_CudaCore(torch.autograd.Function):
             db1 = db1.to(b1_dt)
         if db2 is not None:
             db2 = db2.to(b2_dt)
-        return None, dx, dw1, dw2, db1, db2
+        return None, dx, dw1, dw2, db1, db2, None

@@ -403,3 +403,39 @@ def test_kernels_that_start_early_read_by_ordinary_loads():
         assert not marked, (os.path.basename(f), len(marked))
     for f in set(files) - set(early):      # and the others are not launched early
         assert "after_previous" not in open(f).read() and "ProgrammaticStreamSerialization" not in open(f).read(), f
+
+
+def test_no_state_is_kept_where_no_backward_pass_follows():
+    """The grad mode decides, not the parameters alone: inside an autograd function they want gradients in any mode."""
+    import sys
+    import types
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import oracle_backend
+    from hexa_moe import moe as hmoe
+    seen = []
+
+    def moe_forward(x, ids, w1, w2, *args, need_state=True, **kw):
+        seen.append(need_state)
+        if not need_state:      # (the oracle differentiates, which inference mode does not allow)
+            return x.new_zeros(x.shape[0], w2.shape[2]), None
+        return oracle_backend.moe_forward(x, ids, w1, w2, *args, **kw)
+
+    spy = types.SimpleNamespace(**{k: v for k, v in vars(oracle_backend).items() if not k.startswith("__")})
+    spy.moe_forward = moe_forward
+    for data_centric in (True, False):
+        m = hmoe.MoE_Cascaded(gate_type={'type': 'top', 'k': 1, 'fp32_gate': True}, model_dim_list=[16], moe_idx_list=[0], mlp_ratio=2,
+                              num_global_experts=2, total_depth=1, data_centric=data_centric, activation_fn=lambda t: F.gelu(t))
+        m.dispatch_params.backend = spy
+        x = torch.randn(6, 16)
+        del seen[:]
+        with torch.no_grad():
+            m(0, x)
+        with torch.inference_mode():
+            m(0, x)
+        y, _ = m(0, x.clone().requires_grad_(True))
+        y.sum().backward()
+        for p in m.parameters():
+            p.requires_grad_(False)
+        m(0, x)
+        assert seen == [False, False, True, False]
+        assert m.batched_fc1_w[0].grad is not None

@@ -492,3 +492,30 @@ def test_native_layer_under_hooks_checkpoints_and_failures():
     finally:
         L.clear_device_status(0)
     assert _same(_step(m, x, dy), want)
+
+
+@pytest.mark.parametrize("T,dim,launches", [(256, 256, 2), (333, 256, 3), (256, 64, 2)])
+def test_dense_depths_without_gradients_write_no_state(T, dim, launches):
+    """Under no_grad a dense depth is its two GEMMs, after a gather where the tokens do not fill whole tiles, and the
+    pre-activation, which only a backward pass reads, is not written; the output is that of a pass with gradients."""
+    import torch.nn.functional as F
+    from hexa_moe import moe as hmoe
+    from hexa_moe_b200 import ops
+    torch.manual_seed(dim)
+    m = hmoe.MoE_Cascaded(gate_type={'type': 'top', 'k': 1}, model_dim_list=[dim], moe_idx_list=[], mlp_ratio=4,
+                          num_global_experts=1, total_depth=1, data_centric=True, activation_fn=lambda t: F.gelu(t))
+    m = m.to(torch.bfloat16).cuda()
+    x = torch.randn(T, dim, device="cuda").bfloat16()
+    want = m(0, x)[0].detach()
+    kept = []
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            m(0, x)                                       # the routing's tables are built once
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            base, before = torch.cuda.memory_allocated(), ops.LAUNCHES
+            y = m(0, x)[0]
+            assert ops.LAUNCHES - before == launches and torch.equal(y, want)
+            kept.append(torch.cuda.max_memory_allocated() - base)
+    rows = (T + 127) // 128 * 128
+    assert max(kept) < rows * (4 * dim + dim + dim + 2 * dim) * 2      # hidden, output, rows of its own; no second [rows, hidden]
