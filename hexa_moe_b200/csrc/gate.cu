@@ -95,9 +95,10 @@ __device__ __forceinline__ void group_load(const float* row, int E, int g, bool 
 }
 
 // s / sum for a token's exponentials (0 <= s <= 1 <= sum <= E, both NaN-free), bit for bit the IEEE quotient: one correctly
-// rounded reciprocal per token and Markstein's remainder correction per element (P. Markstein, Computation of elementary
+// rounded reciprocal per lane and Markstein's remainder correction per element (P. Markstein, Computation of elementary
 // functions on the IBM RISC System/6000, 1990) are three instructions where a division is a dozen.  The remainder has to be exact, so a
-// token with a non-zero exponential below 2^-90, or with a sum that is no such number, takes the division.
+// lane with a non-zero exponential below 2^-90, or with a sum that is no such number, takes the division.  Lanes of one token may
+// go different ways: equal exponentials are equal scores all the same, and the lowest id wins, because both give the quotient.
 template <int PER>
 __device__ __forceinline__ void normalise(float sum, float (&s)[PER]) {
   uint32_t least = 0xffffffffu;

@@ -357,3 +357,61 @@ def test_selection_follows_the_ieee_quotients(E, T):
     assert bool(live.any()) and torch.equal(ids.t()[live].long(), order[live])
     assert torch.equal(first, torch.bincount(ids[0].long(), minlength=E).int())
     assert torch.allclose(mass.double(), torch.softmax(logits.double(), 1).sum(0), rtol=1e-5, atol=1e-6)
+
+
+def _warp_order_sum(e):
+    """fp32 sum of a row's exponentials in the kernel's order: columns c mod 32 in turn, then pairs 16, 8, 4, 2, 1 apart."""
+    import numpy as np
+    cls = np.zeros(32, np.float32)
+    for c in range(0, len(e), 32):
+        part = e[c:c + 32]
+        cls[:len(part)] += part
+    at = np.arange(32)
+    for o in (16, 8, 4, 2, 1):
+        cls = cls + cls[at ^ o]
+    assert (cls == cls[0]).all()
+    return cls[0]
+
+
+# One token's column sums of the softmax are its scores.  Ordinary logits; exponentials on both sides of 2^-90 = e^-62.4 and down
+# to zero; sums a few steps below whole numbers, whose significands are nearly all ones where the number is a power of two.
+@pytest.mark.parametrize("E", [1, 2, 4, 7, 8, 9, 16, 31, 33, 64, 100, 200, 256, 500])
+def test_scores_are_the_ieee_quotients_bit_for_bit(E):
+    import numpy as np
+    from hexa_moe_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(E)
+    rand = lambda: torch.rand(1, E, generator=g, device="cuda")
+    near = lambda: -torch.randint(0, 5, (1, E), generator=g, device="cuda").float() * 2.0 ** -23
+    rows = []
+    for _ in range(6):
+        rows += [3 * torch.randn(1, E, generator=g, device="cuda"), -100 * rand(), -60 - 5 * rand(), near(),
+                 torch.where(rand() < 0.3, -61.5 - 2 * rand(), near())]
+        rows[-3][0, int(torch.randint(0, E, (1,), generator=g, device="cuda"))] = 0.0
+    products_differ = 0
+    for l in rows:
+        mass = ops.gate_topk(l, min(4, E))[3]
+        e = torch.exp(l - l.max())[0].cpu().numpy()
+        total = _warp_order_sum(e)
+        want = e / total
+        assert want.dtype == np.float32 and np.array_equal(mass.cpu().numpy(), want)
+        products_differ += int((e * (np.float32(1) / total) != want).sum())
+    assert products_differ or E <= 2 or E in (4, 8)      # these rows tell quotients from products with the reciprocal
+
+
+@pytest.mark.parametrize("E", [16, 64, 128, 200])
+def test_equal_scores_of_lanes_that_go_different_ways(E):
+    """Pairs of equal logits, one of them in a lane with an exponential below 2^-90: the lower id comes first."""
+    from hexa_moe_b200 import ops
+    T, lanes = 300, 8 if E <= 64 else 16 if E <= 128 else 32
+    g = torch.Generator(device="cuda").manual_seed(E)
+    logits = -20 - 10 * torch.rand(T, E, generator=g, device="cuda")
+    cols = torch.stack([torch.randperm(E, generator=g, device="cuda") for _ in range(T)])
+    at = torch.arange(T, device="cuda")
+    for level in range(2):      # two pairs a token, e apart
+        logits[at, cols[:, 2 * level]] = logits[at, cols[:, 2 * level + 1]] = -float(level)
+    tiny = cols[:, 4:].clone()                            # of the other columns, those in the lane of the first pair's first
+    tiny[(tiny % lanes) != (cols[:, :1] % lanes)] = -1
+    for t in range(T):
+        logits[t, tiny[t][tiny[t] >= 0]] = -70.0
+    ids = ops.gate_topk(logits, 4)[0]
+    assert torch.equal(ids.t().long(), torch.sort(logits, dim=1, descending=True, stable=True).indices[:, :4])
