@@ -175,6 +175,45 @@ def test_a_wait_that_runs_out_in_the_fp32_kernel(ops, form):
     assert L.device_status() == 0
 
 
+# The weight gradient's epilogues: partial results of a split (chains drained into registers), 16-bit results through staging
+# tiles, and stores from registers; CTA pairs, one CTA with 256 columns, one with 128.
+@pytest.mark.parametrize("m,n", [(256, 512), (128, 512), (256, 128)])
+@pytest.mark.parametrize("T,E,out,split", [(8192, 2, torch.bfloat16, True), (8192, 2, torch.float32, True),
+                                           (4608, 32, torch.bfloat16, False), (4608, 32, torch.float32, False)])
+def test_a_wait_that_runs_out_in_the_weight_gradient(ops, T, E, out, split, m, n):
+    from hexa_moe_b200 import _lib as L
+    lib = L.lib()
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    r = ops.route(torch.randint(0, E, (T, 1), generator=g, device="cuda").to(torch.int32), E)
+    p, q = (ops.gather_rows(torch.randn(T, w, generator=g, device="cuda").bfloat16(), r) for w in (m, n))
+    assert (lib.hexa_estmm_workspace_bytes(E, r.row_capacity, m, n, L.BF16) > 0) == split
+    run = lambda: ops.estmm(p, q, r, out_dtype=out, engine=L.ENGINE_TCGEN05)
+    good = run()
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+    try:
+        assert lib.hexa_set_wait_limit_ns(5_000_000) == 0 and lib.hexa_set_tc_debug(4) == 0
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        try:
+            run()
+        except L.HexaError:
+            pass                                      # the wrapper may see the code already
+        t1.record()
+        torch.cuda.synchronize()
+        assert t0.elapsed_time(t1) < 1000.0
+    finally:
+        lib.hexa_set_tc_debug(0)
+        lib.hexa_set_wait_limit_ns(2_000_000_000)
+    assert L.device_status() in (1, 2, 3, 4)
+    with pytest.raises(L.HexaError, match="bounded wait"):
+        run()
+    L.clear_device_status()
+    assert torch.equal(run(), good)
+    torch.cuda.synchronize()
+    assert L.device_status() == 0
+
+
 def test_status_word_is_shared_by_host_threads(ops):
     """Backward runs on the autograd engine's thread: the word installed from the main thread must be the one a
     kernel launched from another thread reports to."""
