@@ -120,7 +120,6 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* acc_empty = acc_full + 2;          // [2] epilogues -> MMA                (used in the leader CTA)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* group_abort = abort_flag + 1;  // [kParts]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();     // 0 = leader of the pair
   const uint32_t tile_first = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
@@ -129,7 +128,6 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], kEpiWarps * 2); }
     *abort_flag = 0;
-    for (int g = 0; g < kParts; ++g) group_abort[g] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -270,9 +268,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
       }
       // the four warps of a group leave together
-      if (!good && lane == 0) group_abort[part] = 1;
-      group_sync(1 + part);
-      if (group_abort[part]) break;
+      if (!group_all(1 + part, good)) break;
       if (!tile.valid) continue;      // uniform across the CTA
       const int64_t row = (int64_t)(MODE == TN ? tile.m0 : tile.row0) + rloc;
       const bool live = MODE != TN && p.bias != nullptr && (p.row_token == nullptr || p.row_token[row] >= 0);

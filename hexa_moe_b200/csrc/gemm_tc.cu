@@ -290,7 +290,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* acc_empty = bars + 2 * kStages + 2;   // [2] epilogues -> MMA    (used in the leader CTA)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* group_abort = abort_flag + 1;   // [4]: one per group of four epilogue warps
   uint64_t* aux_full = bars + 2 * kStages + 8;   // [kParts][2] DACT: the saved pre-activation is in the group's staging tile
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -302,7 +301,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], kEpiWarps * CTAS); }
     *abort_flag = 0;
-    for (int g = 0; g < kEpiWarps / 4; ++g) group_abort[g] = 0;
     if (OUT == OUT_DACT)
       for (int g = 0; g < 2 * C::kParts; ++g) mbar_init(&aux_full[g], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -455,12 +453,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int part_col = part * (BN / C::kParts);
     bool ok = true;
     int it = -1;
-    // The four warps of a group meet at named barriers inside the tile, so they must leave together: each warp
-    // publishes a failed wait, the group synchronises, and all four read the same verdict.
+    // The four warps of a group meet at named barriers inside the tile, so they must leave together: after a wait that may
+    // fail they meet at a barrier that gives all four the same verdict.
     auto accumulator_ready = [&](int acc, uint32_t acc_phase) {
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, 4, p.wait_limit_ns) && lane == 0) group_abort[part] = 1;
-      group_sync(1 + part);
-      return group_abort[part] == 0;
+      return group_all(1 + part, mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, 4, p.wait_limit_ns));
     };
     auto accumulator_drained = [&](int acc) {      // hand it back to the (leader's) MMA warp
       tc_fence_before();
@@ -667,8 +663,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
               }
               __syncwarp();
-              if (!mbar_wait_fast(&aux_full[part * 2 + (seq & 1)], (seq >> 1) & 1u, abort_flag, p.status, 5, p.wait_limit_ns) && lane == 0)
-                group_abort[part] = 1;
+              ok = mbar_wait_fast(&aux_full[part * 2 + (seq & 1)], (seq >> 1) & 1u, abort_flag, p.status, 5, p.wait_limit_ns);
             }
             const bool two = OUT == OUT_ACT && p.aux != nullptr;
 #pragma unroll
@@ -699,8 +694,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             fence_async_smem();
             if (OUT == OUT_DACT) {
-              group_sync(1 + part);
-              if (group_abort[part]) { ok = false; break; }
+              if (!(ok = group_all(1 + part, ok))) break;
               if (leader) {
                 tma_store_2d(&tmC, buf, (int)gcol, row0);
                 bulk_commit();
