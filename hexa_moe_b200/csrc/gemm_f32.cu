@@ -22,8 +22,8 @@
 // 16 epilogue warps keep the tile's sums in registers (64 per thread), drain one of two TMEM accumulators per k-block and
 // store through 64B-swizzled staging tiles.  The activation and its derivative are a pass over the result
 // (epilogue_rows_kernel): in the epilogue they would hold up the next tile's k-blocks.
-// fp32 layer of 8192 tokens, d=512, hidden 2048, 8 experts, top-2 (a launch, CUDA cores / this): fc1 + GELU 811 / 274 us,
-// fc2 790 / 233, GELU' 848 / 300, weight gradient 822 / 235.
+// fp32 layer of 8192 tokens, d=512, hidden 2048, 8 experts, top-2 (a launch, CUDA cores / this): fc1 + GELU 811 / 259 us,
+// fc2 790 / 224, GELU' 848 / 312, weight gradient 822 / 235.
 #include "gemm_launch.h"
 #include "hexa_common.cuh"
 #include "tc_ptx.cuh"

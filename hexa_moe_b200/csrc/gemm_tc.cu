@@ -18,7 +18,7 @@
 //               and publishes finished accumulators (multicast to both CTAs of a pair)
 //   warps 2..17 epilogue: tcgen05.ld of the accumulator (lane quadrant = warp % 4, each group of four warps owns a column
 //               range), fused epilogue math; results go through 64B-swizzled staging tiles and one TMA store per 128x32
-//               block (ESTMM with fp32, accumulating, split or scattered output stores from registers).  A kernel per
+//               block (an unsplit ESTMM with fp32, accumulating or scattered output stores from registers).  A kernel per
 //               epilogue (Out below), because they want different things of shared memory:
 //                 LINEAR, ACT  every warp stages and stores its own 32 rows (ACT: pre-activation and output side by side, two
 //                         staging tiles per group), so that no warp waits for the group between the tile's first barrier
@@ -1032,11 +1032,13 @@ bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, 
 // gradient (one "expert" owning every row), or a handful of experts with a small d x H - would leave most SMs idle behind a
 // few serial k-loops, so where the output has fewer tiles than two per CTA pair (or CTA) every segment is cut into chunks, each a tile of its
 // own.  Two things are chosen apart:
-//   the length of a chain in the accumulator, which truncates: at least as many chains as make two tiles per CTA pair, of
-//     at least 8 k-blocks (relative error of the fp32 result of [18432 rows, 2048 x 512] in 10 chains 1.9e-6, in 4 5.0e-6, in
+//   the length of a chain in the accumulator, which truncates: as many chains as make two tiles per CTA pair, of 8 k-blocks or more
+//     of an average segment; chunks and chains are then both rounded up, so that a chain is never longer than that but may be
+//     shorter ([5120 rows, 2048 x 512]: 4 chunks of 20 k-blocks, chains of 7; an expert far below the average: 1) (relative error of the fp32 result of [18432 rows, 2048 x 512] in 10 chains 1.9e-6, in 4 5.0e-6, in
 //     one 21e-6; positive data 4.7 / 17 / 94e-6).  Between chains the sums are kept in fp32 registers;
 //   the number of chunks, by time: full waves of a chunk's k-blocks at 0.29 us, 2 us to fill, drain and store a tile, and the
-//     partial results, written and read once, at 5 TB/s.  At most as many as chains.
+//     partial results, written and read once, at 5 TB/s (a drain between chains overlaps the next chain's MMAs and is not
+//     counted).  At most as many as chains.
 // One chunk per chain, partial results stored from registers / this, us: [18432 rows, 2048 x 512] 64 / 43, [65000, 256 x 1024]
 // 61 / 45, [16384, 1024 x 256] x 8 35 / 24, [2000, 768 x 3072] 39 / 25; error of the first 1.9e-6 / 1.6e-6.
 struct EstmmPlan { int chunks, chains; };      // chains per chunk

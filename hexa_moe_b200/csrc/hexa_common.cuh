@@ -74,7 +74,7 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
 // A launch that may start while the kernel before it in the stream drains: its blocks take up SMs as they become free, set up
 // and then meet wait_for_previous(), which every kernel launched this way calls before it touches device memory.  Between
 // two kernels of a layer this saves the drain, the launch latency and, for a GEMM, the set-up of barriers and TMEM: 16 tokens
-// through a layer 100 -> 85 us, 2048 tokens 99 -> 82, 4608 tokens x 32 experts both ways 605 -> 578, [131072, 64] router 59.6 -> 57.1.
+// through a layer 100 -> 85 us, 2048 tokens 99 -> 82, 4608 tokens x 32 experts both ways 605 -> 578, [131072, 64] router 59.6 -> 57.3.
 template <typename... P> struct AfterPrevious {
   void (*kernel)(P...);
   dim3 grid, block;

@@ -4,7 +4,7 @@
 // Why: a layer step is ~20 launches of a few microseconds each at small sizes, and a wrapper that collects two dozen
 // pointers, strides and sizes in Python and hands them to ctypes cost ~20 us per operator.  Here it is one call:
 // 16 tokens forward 370 -> 204 us, the README layer's step 941 -> 593 us, 4608 tokens x 32 experts 1037 -> 709 us when it came
-// (158, 559 and 644 us with the fewer launches since).
+// (82, 279 and 574 us with fewer launches, the nodes below and early starts since).
 // The C ABI is bound at run time from the library that _lib.py has loaded (bind()), so this module links against torch only.
 // The interpreter lock is released around every library call: a launch can block on a full queue, and the thread that
 // would resolve the stall may need the lock.
