@@ -1038,14 +1038,14 @@ bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, 
 //     one 21e-6; positive data 4.7 / 17 / 94e-6).  Between chains the sums are kept in fp32 registers;
 //   the number of chunks, by time: full waves of a chunk's k-blocks at 0.29 us, 2 us to fill, drain and store a tile, and the
 //     partial results, written and read once, at 5 TB/s (a drain between chains overlaps the next chain's MMAs and is not
-//     counted).  At most as many as chains.
+//     counted).  At most as many as chains: the scratch is sized for a chunk of each.
 // One chunk per chain, partial results stored from registers / this, us: [18432 rows, 2048 x 512] 64 / 43, [65000, 256 x 1024]
 // 61 / 45, [16384, 1024 x 256] x 8 35 / 24, [2000, 768 x 3072] 39 / 25; error of the first 1.9e-6 / 1.6e-6.
-struct EstmmPlan { int chunks, chains; };      // chains per chunk
+struct EstmmPlan { int chunks, chains, scratch; };      // chains per chunk, chunks the scratch has to hold
 EstmmPlan estmm_tc_plan(int E, int64_t row_cap, int64_t m, int64_t n) {
   static int forced = -2;
   if (forced == -2) forced = env_int("HEXA_ESTMM_SPLITS", -1);       // A/B switch: 1 = never split
-  if (n % 4) return {1, 1};
+  if (n % 4) return {1, 1, 1};
   const int BN = n > 128 ? 256 : 128;
   const int ctas = (BN == 256 && m > BLOCK_M && pairs_enabled()) ? 2 : 1;
   const int64_t tiles = (int64_t)E * ceil_div(m, BLOCK_M * ctas) * ceil_div(n, BN);
@@ -1056,7 +1056,7 @@ EstmmPlan estmm_tc_plan(int E, int64_t row_cap, int64_t m, int64_t n) {
   if (s > avg_kb / 8) s = avg_kb / 8;
   if (forced > 0) s = forced;
   if (s > 32) s = 32;
-  if (s <= 1 || forced > 0) return {s < 1 ? 1 : (int)s, 1};
+  if (s <= 1 || forced > 0) return {s < 1 ? 1 : (int)s, 1, s < 1 ? 1 : (int)s};
   const double plane_us = (double)E * (double)m * (double)n * 8.0 / 5e6;
   int best = 2;
   double best_us = 0.0;
@@ -1064,11 +1064,11 @@ EstmmPlan estmm_tc_plan(int E, int64_t row_cap, int64_t m, int64_t n) {
     const double us = (double)ceil_div(tiles * c, slots) * ((double)ceil_div(avg_kb, c) * 0.29 + 2.0) + c * plane_us;
     if (c == 2 || us < best_us) { best = c; best_us = us; }
   }
-  return {best, (int)ceil_div(s, best)};
+  return {best, (int)ceil_div(s, best), (int)s};
 }
 
 size_t estmm_tc_workspace_bytes(int E, int64_t row_cap, int64_t m, int64_t n) {
-  const int s = estmm_tc_plan(E, row_cap, m, n).chunks;
+  const int s = estmm_tc_plan(E, row_cap, m, n).scratch;
   return s > 1 ? (size_t)s * (size_t)E * (size_t)m * (size_t)n * sizeof(float) : 0;
 }
 
@@ -1081,7 +1081,7 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   const int ctas = (BN == 256 && m > BLOCK_M && pairs_enabled()) ? 2 : 1;
   const EstmmPlan plan = estmm_tc_plan(E, row_cap, m, n);
   int splits = n_split > 0 ? 1 : plan.chunks;
-  if (splits > 1 && (!workspace || workspace_bytes < (size_t)splits * E * m * n * sizeof(float) || !aligned16(workspace)))
+  if (splits > 1 && (!workspace || workspace_bytes < (size_t)plan.scratch * E * m * n * sizeof(float) || !aligned16(workspace)))
     splits = 1;      // without scratch the operator still runs, one tile per expert's whole segment
   CUtensorMap tmA, tmB;
   // the maps need at least one row even when no token was routed

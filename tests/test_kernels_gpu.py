@@ -814,23 +814,3 @@ def test_small_tiles_follow_the_launch(ops, T, E, n, limit, experts, small):
         pytest.skip("no kernel records on this machine")
     ctas = int(names[0].split("gemm_tc_kernel<")[1].split(",")[2])
     assert (ctas == 1) == small, names
-
-
-@pytest.mark.parametrize("T,E,m,n", [(18432, 1, 512, 2048), (8192, 2, 256, 512), (30000, 1, 256, 128), (16384, 8, 1024, 256)])
-def test_scratch_of_a_split_weight_gradient_is_what_it_writes(ops, T, E, m, n):
-    """hexa_estmm_workspace_bytes asks for the partial results that the kernel writes, and that much makes the call a split one."""
-    from hexa_moe_b200 import _lib as L
-    lib = L.lib()
-    g = torch.Generator(device="cuda").manual_seed(T)
-    r = ops.route(torch.randint(0, E, (T, 1), generator=g, device="cuda").to(torch.int32), E)
-    p, q = (ops.gather_rows(torch.randn(T, w, generator=g, device="cuda").bfloat16(), r) for w in (m, n))
-    size = lib.hexa_estmm_workspace_bytes(E, r.row_capacity, m, n, L.BF16)
-    assert size > E * m * n * 4 and size % (E * m * n * 4) == 0
-    mark = 0x7fc12345                                     # a NaN that no sum is
-    ws = torch.full((size // 4 + 256,), mark, dtype=torch.int32, device="cuda")
-    out = torch.empty(E, m, n, device="cuda")
-    assert lib.hexa_estmm(p.data_ptr(), m, q.data_ptr(), n, r.pad_offsets.data_ptr(), E, r.row_capacity, m, n, out.data_ptr(), n, m * n,
-                          0, 0, L.BF16, L.F32, 0, L.ENGINE_AUTO, ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream) == 0
-    torch.cuda.synchronize()
-    assert not bool((ws[:size // 4] == mark).any()) and bool((ws[size // 4:] == mark).all())
-    assert torch.equal(out, ops.estmm(p, q, r, out_dtype=torch.float32))
