@@ -1034,14 +1034,15 @@ bool estmm_tc_supported(const void* p, int64_t ldp, const void* q, int64_t ldq, 
 // own.  Two things are chosen apart:
 //   the length of a chain in the accumulator, which truncates: as many chains as make two tiles per CTA pair, of 8 k-blocks or more
 //     of an average segment; chunks and chains are then both rounded up, so that a chain is never longer than that but may be
-//     shorter ([5120 rows, 2048 x 512]: 4 chunks of 20 k-blocks, chains of 7; an expert far below the average: 1) (relative error of the fp32 result of [18432 rows, 2048 x 512] in 10 chains 1.9e-6, in 4 5.0e-6, in
-//     one 21e-6; positive data 4.7 / 17 / 94e-6).  Between chains the sums are kept in fp32 registers;
+//     shorter ([5120 rows, 2048 x 512]: 4 chunks of 20 k-blocks, chains of 7; an expert far below the average: 1).  Relative error
+//     of the fp32 result of [18432 rows, 2048 x 512] in 10 chains 1.9e-6, in 4 5.0e-6, in one 21e-6 (positive data 4.7 / 17 /
+//     94e-6).  Between chains the sums are kept in fp32 registers;
 //   the number of chunks, by time: full waves of a chunk's k-blocks at 0.29 us, 2 us to fill, drain and store a tile, and the
 //     partial results, written and read once, at 5 TB/s (a drain between chains overlaps the next chain's MMAs and is not
-//     counted).  At most as many as chains: the scratch is sized for a chunk of each.
+//     counted).  At most as many as chains: the query asks for scratch of a chunk for each, and any that holds the chunks will do.
 // One chunk per chain, partial results stored from registers / this, us: [18432 rows, 2048 x 512] 64 / 43, [65000, 256 x 1024]
 // 61 / 45, [16384, 1024 x 256] x 8 35 / 24, [2000, 768 x 3072] 39 / 25; error of the first 1.9e-6 / 1.6e-6.
-struct EstmmPlan { int chunks, chains, scratch; };      // chains per chunk, chunks the scratch has to hold
+struct EstmmPlan { int chunks, chains, scratch; };      // chains per chunk, chunks the query asks scratch for
 EstmmPlan estmm_tc_plan(int E, int64_t row_cap, int64_t m, int64_t n) {
   static int forced = -2;
   if (forced == -2) forced = env_int("HEXA_ESTMM_SPLITS", -1);       // A/B switch: 1 = never split
@@ -1081,7 +1082,7 @@ int estmm_tc_launch(const void* pp, int64_t ldp, const void* q, int64_t ldq, con
   const int ctas = (BN == 256 && m > BLOCK_M && pairs_enabled()) ? 2 : 1;
   const EstmmPlan plan = estmm_tc_plan(E, row_cap, m, n);
   int splits = n_split > 0 ? 1 : plan.chunks;
-  if (splits > 1 && (!workspace || workspace_bytes < (size_t)plan.scratch * E * m * n * sizeof(float) || !aligned16(workspace)))
+  if (splits > 1 && (!workspace || workspace_bytes < (size_t)splits * E * m * n * sizeof(float) || !aligned16(workspace)))
     splits = 1;      // without scratch the operator still runs, one tile per expert's whole segment
   CUtensorMap tmA, tmB;
   // the maps need at least one row even when no token was routed

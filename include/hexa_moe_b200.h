@@ -213,7 +213,7 @@ int hexa_esmm_experts(const void* a, int64_t lda, const void* b, int b_layout, i
  * idle.  With hexa_estmm_workspace_bytes(...) bytes of 16-byte aligned scratch the tcgen05 kernel cuts every segment
  * into chunks (the count depends only on the static sizes), writes fp32 partial results there and adds them in chunk
  * order in a second kernel: deterministic, same rounding of the final result.  The query returns 0 when no split
- * would be used; NULL / too small a workspace runs the unsplit kernel.  (The reference accumulates a whole segment in
+ * would be used, else an upper bound; a workspace that does not hold the chunks (or NULL) runs the unsplit kernel.  (The reference accumulates a whole segment in
  * one program, kernels/fused.py:183-235.) */
 size_t hexa_estmm_workspace_bytes(int num_experts, int64_t row_capacity, int64_t m, int64_t n, int dtype);
 int hexa_estmm(const void* p, int64_t ldp, const void* q, int64_t ldq, const int32_t* pad_offsets,

@@ -814,3 +814,32 @@ def test_small_tiles_follow_the_launch(ops, T, E, n, limit, experts, small):
         pytest.skip("no kernel records on this machine")
     ctas = int(names[0].split("gemm_tc_kernel<")[1].split(",")[2])
     assert (ctas == 1) == small, names
+
+
+@pytest.mark.parametrize("T,E,m,n", [(18432, 1, 512, 2048), (8192, 2, 256, 512), (30000, 1, 256, 128), (16384, 8, 1024, 256)])
+def test_scratch_that_holds_the_chunks_is_enough(ops, T, E, m, n):
+    """A split weight gradient takes any scratch that holds what it writes, which may be less than the query asks for."""
+    from hexa_moe_b200 import _lib as L
+    lib = L.lib()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    r = ops.route(torch.randint(0, E, (T, 1), generator=g, device="cuda").to(torch.int32), E)
+    p, q = (ops.gather_rows(torch.randn(T, w, generator=g, device="cuda").bfloat16(), r) for w in (m, n))
+    plane = E * m * n
+    most = lib.hexa_estmm_workspace_bytes(E, r.row_capacity, m, n, L.BF16) // (4 * plane)
+    assert most > 1
+    mark = 0x7fc12345                                     # a NaN that no sum is
+
+    def run(planes):
+        ws = torch.full((most, plane), mark, dtype=torch.int32, device="cuda")
+        out, before = torch.empty(E, m, n, device="cuda"), ops.LAUNCHES
+        assert lib.hexa_estmm(p.data_ptr(), m, q.data_ptr(), n, r.pad_offsets.data_ptr(), E, r.row_capacity, m, n, out.data_ptr(), n,
+                              m * n, 0, 0, L.BF16, L.F32, 0, L.ENGINE_AUTO, ws.data_ptr(), planes * plane * 4,
+                              torch.cuda.current_stream().cuda_stream) == 0
+        return out, ops.LAUNCHES - before, int((ws != mark).all(1).sum()), int((ws != mark).any(1).sum())
+
+    want, launches, whole, touched = run(most)
+    assert launches == 2 and whole == touched >= 2
+    got, launches, *used = run(whole)
+    assert launches == 2 and used == [whole, whole] and torch.equal(got, want)
+    _, launches, *used = run(whole - 1)                   # the unsplit kernel
+    assert launches == 1 and used == [0, 0]
